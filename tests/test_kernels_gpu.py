@@ -192,6 +192,19 @@ def test_gemm_f32_rows_do_not_depend_on_the_batch():
         assert torch.equal(part, full[rows])
 
 
+@pytest.mark.parametrize("N,K", [(16, 64), (130, 68), (257, 1000), (2048, 512)])
+def test_gemm_f32_gives_the_same_bits_from_every_kernel(N, K):
+    """The kernel for few rows (1 to 32, by groups of four) and the tile shapes for more add up in the same order; a
+    float64 product bounds them: K terms, each rounded once more than exactly, 2^-24 of the sum of magnitudes each."""
+    a, w = rnd(300, K, seed=13), rnd(N, K, seed=14)
+    full = ops().gemm_f32(a.to(DEV), w.to(DEV))
+    want = a.double() @ w.double().T
+    bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert ((full.cpu().double() - want).abs() <= bound).all()
+    for M in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 129):
+        assert torch.equal(ops().gemm_f32(a[:M].to(DEV), w.to(DEV)), full[:M]), M
+
+
 def test_gemm_f32_is_not_reduced_precision():
     # products that a 10-bit (TF32) or 8-bit (bf16) mantissa would lose
     a = torch.tensor([[1.0 + 2.0 ** -20, 1.0]], device=DEV)
