@@ -551,6 +551,272 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// The same product for at most 16 tokens without an exchange between blocks (the route of a decode step).
+//
+// What bounds it: one reading of W, and behind the last byte whatever a block still has to do.  The kernel
+// above cuts k across blocks and spends two dependent round trips to the L2 and a fence on adding the partial
+// tiles up; here a block owns `span` rows of W over the whole of k (N / 148 rows, so every SM streams the same
+// bytes), and its eight warps split k between them and add up in shared memory.  The price is x, which every
+// block reads whole from the L2, 8 rows of x beside 28 of W at N = 4096.  Rows of W are the M side of
+// mma.sync.m16n8k16, 8 tokens its N side: a matrix that passes once at 44 bytes per ns and SM needs one such
+// instruction per 70 cycles and scheduler, far below what even this path can do, and unlike a tensor-memory
+// accumulator its fragments are summed without a round trip.
+//
+//   warp 8     issues the TMA loads: per stage a box of `tile_rows` rows of W x kb * 64 k and the tokens' k range, both
+//              with the 128-byte swizzle.  The ring is filled with weights before the wait for the kernel before and with
+//              x behind it, a lane per stage side by side (one issuing thread alone would be a good part of a small
+//              product's time); from then on lane 0 issues W and lane 1 x
+//   warps 0-7  warp w multiplies the stage's k range [64 w, 64 w + 64) (a stage has up to eight boxes of 64) for all
+//              rows of the tile; at the tile's end warp w adds up and stores token w (and w + 8), a lane per pair of rows
+//
+// A block's rows are cut into tiles of at most 64 rows of equal size (the output head: 14 tiles).  stats_in and
+// stats_out of EpilogueFusion hold one row of 16 sums per block here instead of one per 128 features.
+// ------------------------------------------------------------------------------------------
+#define GR_WARPS 8
+#define GR_THREADS (32 * (GR_WARPS + 1))
+#define GR_TILE 64                  // most rows of W per tile
+#define GR_MAX_STAGES 32
+#define GR_STATS 5                  // rows of sums per lane (32 lanes) held in registers: all that 148 blocks leave
+#define GR_BUDGET (200 * 1024)
+
+__device__ __forceinline__ void gr_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                       uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void gr_ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ uint64_t l2_policy_evict_normal() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;\n" : "=l"(p));
+  return p;
+}
+
+template <typename OutT, int NT, bool kFused, int kAct>
+__global__ void __launch_bounds__(GR_THREADS, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                 OutT* __restrict__ y, int ldy, int M, int N, int K, int tile_rows, int n_row_tiles, int stages, int kb,
+                 int chunked, int swiglu, const EpilogueFusion fus, int w_evict_first) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  constexpr int TOK = 8 * NT;
+  // one box of 64 k.  A box of x has the M rows that there are: boxes filled up with rows beyond M cost more time than
+  // rows of x (one token, 2048 wide, a layer's four products: 25.4 us filled up to 8 rows).  The fragments of tokens
+  // beyond M are then whatever lies behind the box; an instruction's columns do not mix, and nothing stores those.
+  const uint32_t w_box = (uint32_t)tile_rows * TILE_K * 2, x_box = (uint32_t)M * TILE_K * 2;
+  const uint32_t w_bytes = (w_box * kb + 1023) & ~1023u;                              // the tokens' boxes start aligned
+  const uint32_t stage_bytes = w_bytes + ((x_box * kb + 1023) & ~1023u);
+  const int m_tiles = (tile_rows + 15) / 16, pitch = m_tiles * 16 + 4;     // (the pitch spreads the shares over the banks)
+  float* shares = reinterpret_cast<float*>(smem + (size_t)stages * stage_bytes);     // [GR_WARPS][TOK][pitch]
+  __shared__ __align__(8) uint64_t full[GR_MAX_STAGES], empty[GR_MAX_STAGES];
+  __shared__ int give_up;
+
+  mi_pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int kchunks = (K + TILE_K * kb - 1) / (TILE_K * kb);
+  const int row_begin = blockIdx.x * tile_rows * n_row_tiles;
+  const int tiles = min(n_row_tiles, (N - row_begin + tile_rows - 1) / tile_rows);
+  volatile int* gu = &give_up;
+
+  if (warp == GR_WARPS) {
+    if (lane < stages) {
+      mbar_init(&full[lane], 2);         // W and x report to it
+      mbar_init(&empty[lane], GR_WARPS);
+    }
+    if (lane == 0) give_up = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    __syncwarp();
+    asm volatile("bar.arrive 2, 288;\n" ::: "memory");
+    const int units = tiles * kchunks, first_turn = min(stages, units);
+    const uint64_t w_policy = w_evict_first ? l2_policy_evict_first() : l2_policy_evict_normal();
+    const uint64_t x_policy = l2_policy_evict_normal();
+    // the boxes of unit u, of W or of x, to their part of stage st
+    auto load = [&](bool of_w, int st, int u) {
+      const int tile = u / kchunks, kc = u - tile * kchunks;
+      const int row = of_w ? row_begin + tile * tile_rows : 0;
+      const CUtensorMap* map = of_w ? &map_w : &map_x;
+      const uint32_t bytes = of_w ? w_box : x_box;
+      const uint64_t policy = of_w ? w_policy : x_policy;
+      unsigned char* dst = smem + (size_t)st * stage_bytes + (of_w ? 0u : w_bytes);
+      mbar_expect_tx(&full[st], bytes * kb);
+      if (chunked) {
+        tma_load_3d_hint(dst, map, 0, row, kc * kb, &full[st], policy);
+      } else {
+        for (int b = 0; b < kb; ++b) tma_load_2d_hint(dst + b * bytes, map, (kc * kb + b) * TILE_K, row, &full[st], policy);
+      }
+    };
+    if (lane < first_turn) load(true, lane, lane);     // weights depend on no kernel before this one
+    mi_pdl_wait();
+    if (lane < first_turn) load(false, lane, lane);
+    __syncwarp();
+    if (lane < 2) {
+      int st = 0, round = 0;
+      for (int u = first_turn; u < units; ++u) {
+        if (!mbar_wait(&empty[st], round & 1, gu)) break;
+        load(lane == 0, st, u);
+        if (++st == stages) { st = 0; ++round; }
+      }
+    }
+    return;
+  }
+
+  if (kFused) mi_pdl_wait();                         // the statistics and the stream come from the kernels before
+  // the sums of squares of this warp's tokens: asked for here, added up at the first tile's end (the adds would stand
+  // still for a round trip to the L2 in front of the stream)
+  float scale[NT], sums[NT][GR_STATS];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    scale[t] = 1.f;
+#pragma unroll
+    for (int i = 0; i < GR_STATS; ++i)
+      sums[t][i] = (kFused && fus.stats_in && lane + 32 * i < fus.n_stat_tiles)
+                       ? __ldcg(fus.stats_in + (lane + 32 * i) * FUSED_MAX_TOKENS + warp + 8 * t) : 0.f;
+  }
+  asm volatile("bar.sync 2, 288;\n" ::: "memory");   // the barriers are initialised (warp 8 arrived)
+  // fragment addresses within a stage: row l of the boxes (W: box * tile_rows + row, x: box * M + token) lies at
+  // l * 128, its 16-byte chunks permuted by l modulo 8
+  const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_chunk = lane >> 4;
+  const int b_row = lane & 7, b_chunk = lane >> 3;
+  const uint32_t base = smem_u32(smem);
+  float sq[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) sq[t] = 0.f;
+  int st = 0, round = 0;
+  bool ok = true;
+#pragma unroll 1
+  for (int tile = 0; tile < tiles; ++tile) {
+    const int n = row_begin + tile * tile_rows + 2 * lane;          // this lane's pair of rows of W at the end
+    const bool in0 = 2 * lane < tile_rows && n < N, in1 = 2 * lane + 1 < tile_rows && n + 1 < N;
+    float res[NT][2], g0 = 0.f, g1 = 0.f;
+    if (kFused && fus.residual) {       // asked for ahead of the stream
+      g0 = in0 ? __ldg(fus.gain + n) : 0.f;
+      g1 = in1 ? __ldg(fus.gain + n + 1) : 0.f;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int tok = warp + 8 * t;
+        res[t][0] = in0 && tok < M ? __ldcg(fus.residual + (size_t)tok * N + n) : 0.f;
+        res[t][1] = in1 && tok < M ? __ldcg(fus.residual + (size_t)tok * N + n + 1) : 0.f;
+      }
+    }
+    float acc[GR_TILE / 16][NT][4];
+#pragma unroll
+    for (int m = 0; m < GR_TILE / 16; ++m)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][t][e] = 0.f;
+#pragma unroll 1
+    for (int kc = 0; kc < kchunks; ++kc) {
+      if (ok && !mbar_wait(&full[st], round & 1, gu)) ok = false;
+      if (ok && warp < kb) {
+        const uint32_t wa = base + (uint32_t)st * stage_bytes, xa = wa + w_bytes;
+        uint32_t bf[NT][2][4];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int l = warp * M + 8 * t + b_row;
+          gr_ldmatrix_x4(bf[t][0], xa + l * 128 + ((b_chunk ^ (l & 7)) << 4));
+          gr_ldmatrix_x4(bf[t][1], xa + l * 128 + (((b_chunk + 4) ^ (l & 7)) << 4));
+        }
+#pragma unroll
+        for (int m = 0; m < GR_TILE / 16; ++m) {
+          if (m < m_tiles) {
+            const int l = warp * tile_rows + m * 16 + a_row;
+            uint32_t af[4][4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) gr_ldmatrix_x4(af[k], wa + l * 128 + (((a_chunk + 2 * k) ^ (l & 7)) << 4));
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+              for (int t = 0; t < NT; ++t)
+                gr_mma(acc[m][t], af[k][0], af[k][1], af[k][2], af[k][3], bf[t][k >> 1][(k & 1) * 2], bf[t][k >> 1][(k & 1) * 2 + 1]);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+      if (++st == stages) { st = 0; ++round; }
+    }
+    if (kFused && fus.stats_in && tile == 0) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < GR_STATS; ++i) sum += sums[t][i];
+        for (int i = lane + 32 * GR_STATS; i < fus.n_stat_tiles; i += 32)
+          sum += __ldcg(fus.stats_in + i * FUSED_MAX_TOKENS + warp + 8 * t);
+        scale[t] = rsqrtf(mi_warp_sum(sum) * fus.inv_width + fus.eps);
+      }
+    }
+    // every warp's share of the tile, then token by token
+#pragma unroll
+    for (int m = 0; m < GR_TILE / 16; ++m) {
+      if (m < m_tiles) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            shares[(warp * TOK + 8 * t + 2 * (lane & 3) + (e & 1)) * pitch + m * 16 + (lane >> 2) + (e >> 1) * 8] = acc[m][t][e];
+      }
+    }
+    asm volatile("bar.sync 1, 256;\n" ::: "memory");
+    if (ok) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int tok = warp + 8 * t;
+        if (tok >= M || !in0) continue;
+        float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+        for (int w = 0; w < GR_WARPS; ++w) {
+          const float2 p = *reinterpret_cast<const float2*>(shares + (w * TOK + tok) * pitch + 2 * lane);
+          v0 += p.x;
+          v1 += p.y;
+        }
+        if (kFused && fus.stats_in) {
+          v0 *= scale[t];
+          v1 *= scale[t];
+        }
+        OutT* yr = y + (size_t)tok * ldy;
+        if (kFused && fus.residual) {
+          v0 += res[t][0];
+          v1 += res[t][1];
+          float* h = fus.residual + (size_t)tok * N + n;
+          h[0] = v0;
+          yr[n] = mi_from_float<OutT>(v0 * g0);
+          sq[t] = fmaf(v0, v0, sq[t]);
+          if (in1) {
+            h[1] = v1;
+            yr[n + 1] = mi_from_float<OutT>(v1 * g1);
+            sq[t] = fmaf(v1, v1, sq[t]);
+          }
+        } else if (kAct) {
+          yr[n] = mi_from_float<OutT>(kAct == ACT_RELU2 ? mi_relu2(v0) : mi_xielu_bf16(v0, fus.act_a, fus.act_b));
+          if (in1) yr[n + 1] = mi_from_float<OutT>(kAct == ACT_RELU2 ? mi_relu2(v1) : mi_xielu_bf16(v1, fus.act_a, fus.act_b));
+        } else if (swiglu) {      // rows alternate gate, up; a tile begins with a gate
+          yr[n >> 1] = mi_from_float<OutT>(mi_glu_act(v0, swiglu) * v1);
+        } else {
+          yr[n] = mi_from_float<OutT>(v0);
+          if (in1) yr[n + 1] = mi_from_float<OutT>(v1);
+        }
+      }
+    }
+    if (tile + 1 < tiles) asm volatile("bar.sync 1, 256;\n" ::: "memory");   // the shares are read before the next tile's
+  }
+  if (kFused && fus.residual) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const float s = mi_warp_sum(sq[t]);
+      if (lane == 0) fus.stats_out[blockIdx.x * FUSED_MAX_TOKENS + warp + 8 * t] = s;
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------- host
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -729,4 +995,86 @@ extern "C" int mi_gemm_tma(const void* x, long long ldx, const void* w, void* y,
                            int out_dtype, int swiglu, int blocks, float* partials, int* counters, cudaStream_t stream) {
   return mi_gemm_tma_fused(x, ldx, w, y, ldy, M, N, K, out_dtype, swiglu, blocks, partials, counters, nullptr, 0, 0,
                            0.f, nullptr, nullptr, nullptr, 0.f, 0.f, stream);
+}
+
+// How gemm_rows_kernel cuts N rows of W over `blocks` blocks: equal tiles of at most 64 rows (an even number, so
+// that gate/up pairs stay together), as many per block as it takes.
+struct RowPlan { int tile_rows, tiles, grid; };
+static RowPlan row_plan(int N, int blocks) {
+  RowPlan p;
+  p.tiles = (N + GR_TILE * blocks - 1) / (GR_TILE * blocks);
+  const int per = blocks * p.tiles;
+  p.tile_rows = ((N + per - 1) / per + 1) / 2 * 2;
+  const int span = p.tile_rows * p.tiles;
+  p.grid = (N + span - 1) / span;
+  return p;
+}
+
+// rows of the table of sums that a product with N features leaves (one per block)
+extern "C" int mi_gemm_rows_stat_rows(int N, int blocks) { return N > 0 && blocks > 0 ? row_plan(N, blocks).grid : 0; }
+
+// The product for at most 16 rows of x on gemm_rows_kernel; arguments as mi_gemm_tma_fused, without its workspace.
+// stats_in is [stat_rows][16] and stats_out [mi_gemm_rows_stat_rows(N)][16]: one row of sums per block that wrote them.
+extern "C" int mi_gemm_rows(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K,
+                            int out_dtype, int swiglu, int blocks, const float* stats_in, int stat_rows, int width, float eps,
+                            float* residual, const float* gain, float* stats_out, float act_a, float act_b,
+                            cudaStream_t stream) {
+  const EpilogueFusion fus = {stats_in, stat_rows, width > 0 ? 1.f / (float)width : 0.f, eps, residual, gain, stats_out, act_a, act_b};
+  const bool single = swiglu == ACT_XIELU || swiglu == ACT_RELU2, fused = stats_in || residual;
+  if (M <= 0 || N <= 0) return 0;
+  if (M > FUSED_MAX_TOKENS) MI_REFUSE("gemm_rows: %d rows of x; this kernel takes at most %d", M, FUSED_MAX_TOKENS);
+  if (stats_in && (stat_rows <= 0 || width <= 0))
+    MI_REFUSE("gemm_rows: row statistics need their row count and width (%d, %d)", stat_rows, width);
+  if (residual && (!gain || !stats_out || swiglu))
+    MI_REFUSE("gemm_rows: the residual epilogue needs a gain and room for its statistics, and no gate/up pairs");
+  if (swiglu < 0 || swiglu > ACT_RELU2) MI_REFUSE("gemm_rows: unknown activation %d", swiglu);
+  if (single && (fused || out_dtype != MI_DTYPE_BF16))
+    MI_REFUSE("gemm_rows: an activation of single values goes with the plain product and a bfloat16 result");
+  if (swiglu && !single && (N % 2)) MI_REFUSE("gemm_rows: the gate/up epilogue needs an even number of rows of W, got %d", N);
+  if (K <= 0 || K % 8 != 0 || ldx % 8 != 0)
+    MI_REFUSE("gemm_rows: K (%d) and the row stride of x (%lld) must be multiples of 8 (16-byte rows)", K, ldx);
+  if (!mi_aligned(x, 16) || !mi_aligned(w, 16)) MI_REFUSE("gemm_rows: operands must be 16-byte aligned");
+  if (blocks <= 0) MI_REFUSE("gemm_rows: bad block count %d", blocks);
+  if (out_dtype != MI_DTYPE_BF16 && out_dtype != MI_DTYPE_F32) MI_REFUSE("gemm_rows: unknown output dtype %d", out_dtype);
+  const RowPlan p = row_plan(N, blocks);
+  const int nt = M <= 8 ? 1 : 2, tok = 8 * nt;
+  const int kb = K > 7 * TILE_K ? 8 : (K + TILE_K - 1) / TILE_K;     // 64-wide boxes per stage, one per warp
+  const int kchunks = (K + TILE_K * kb - 1) / (TILE_K * kb);
+  const int stage_bytes = ((p.tile_rows * TILE_K * 2 * kb + 1023) & ~1023) + ((M * TILE_K * 2 * kb + 1023) & ~1023);
+  const int share_bytes = GR_WARPS * tok * ((p.tile_rows + 15) / 16 * 16 + 4) * (int)sizeof(float);
+  int stages = (GR_BUDGET - share_bytes) / stage_bytes;
+  if (stages > GR_MAX_STAGES) stages = GR_MAX_STAGES;
+  if (stages > kchunks * p.tiles) stages = kchunks * p.tiles;
+  if (stages < 1) stages = 1;
+  // (the last fragment of a box may reach 15 rows, 1920 bytes, behind it: the next stage or the shares lie there)
+  const size_t smem = (size_t)stages * stage_bytes + (share_bytes < 2048 ? 2048 : share_bytes) + 1024;
+  CUtensorMap map_w, map_x;
+  const int chunked = (K % TILE_K == 0 && kb > 1) ? 1 : 0;
+  const bool maps_ok = chunked ? (make_map_chunked(&map_w, w, N, K, K, p.tile_rows, kb) && make_map_chunked(&map_x, x, M, K, ldx, M, kb))
+                               : (make_map(&map_w, w, N, K, K, p.tile_rows) && make_map(&map_x, x, M, K, ldx, M));
+  if (!maps_ok) MI_REFUSE("gemm_rows: the driver refused a tensor map (N %d, K %d, M %d)", N, K, M);
+  const int w_evict_first = mi_l2_hints_enabled() ? 1 : 0;
+  cudaError_t e;
+#define GR_LAUNCH(T, NT, FUSED, ACT)                                                                                  \
+  {                                                                                                                   \
+    auto kern = gemm_rows_kernel<T, NT, FUSED, ACT>;                                                                  \
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
+    if (e != cudaSuccess) return (int)e;                                                                              \
+    MI_LAUNCH((kern), p.grid, GR_THREADS, smem, stream, map_w, map_x, (T*)y, (int)ldy, M, N, K, p.tile_rows, p.tiles, \
+              stages, kb, chunked, swiglu, fus, w_evict_first);                                                       \
+  }
+#define GR_TOKENS(T, FUSED, ACT) \
+  if (nt == 1) GR_LAUNCH(T, 1, FUSED, ACT) else GR_LAUNCH(T, 2, FUSED, ACT)
+  if (swiglu == ACT_XIELU) {
+    GR_TOKENS(bf16, false, ACT_XIELU)
+  } else if (swiglu == ACT_RELU2) {
+    GR_TOKENS(bf16, false, ACT_RELU2)
+  } else if (out_dtype == MI_DTYPE_BF16) {
+    if (fused) { GR_TOKENS(bf16, true, 0) } else { GR_TOKENS(bf16, false, 0) }
+  } else {
+    if (fused) { GR_TOKENS(float, true, 0) } else { GR_TOKENS(float, false, 0) }
+  }
+#undef GR_TOKENS
+#undef GR_LAUNCH
+  MI_RETURN_LAUNCH_STATUS();
 }

@@ -1,0 +1,416 @@
+// Gated linear attention over long portions in chunks of 64 tokens, as products instead of a walk.
+//
+// Per head S_t = diag(alpha_t) S_(t-1) + k_t v_t^T, o_t = S_t^T (q_t * q_scale) (see mi_gla_scan in recurrent.cu for the
+// forms of alpha, k and v).  With D_t the product of the chunk's alphas up to and with t, and S the state the chunk begins
+// with, per key channel:
+//
+//   o_t     = (q_t D_t)^T S + sum_(s <= t) P_ts v_s,     P_ts = sum_k q_t k_s D_t / D_s
+//   S_end   = D_end S + sum_s (k_s D_end / D_s) v_s^T
+//
+//   gla_fold_kernel    per (request, chunk, head): sum_s (k_s prod_(r > s) alpha_r) v_s^T and D_end
+//   gla_carry_kernel   per state element: the states the chunks begin with, one fused multiply-add per chunk
+//   gla_out_kernel     per (request, chunk, head, 128 value columns): the two products of o
+//
+// Everything is fp32, on fused multiply-adds two columns wide; decays are products of alphas (never differences of
+// logarithms), so their error does not grow with how far a channel decays.  What bounds it: 2 dk dv multiply-adds per
+// token and head with the state and 32 (dk + dv) within the chunk, at 0.5 to 0.6 of the fp32 rate; the token-by-token walk
+// does as many and stands still between them.  The quotient D_t / D_s is taken as (q D_t) (k / D_s) where no
+// channel of the chunk falls below 1e-30 (|log alpha| up to 1.08 per token on average); a chunk where one does multiplies
+// its pairs' decays out one by one.
+#include "common.cuh"
+
+MI_DEFINE_ERROR_API()
+
+#define GC_T 64                // tokens per chunk
+#define GC_W 128               // key channels and value columns per tile
+#define GC_PITCH (GC_W + 4)
+#define GC_PP (GC_T + 4)       // row pitch of the pair weights
+#define GC_SLAB 32             // rows of S or v staged at a time
+#define GC_THREADS 256
+#define GC_SMALLEST 1e-30f
+
+struct GlaArgs {
+  const void *q, *k, *v;
+  int qk_stride, stride;
+  const float* z;
+  int z_stride;
+  const float* z_bias;
+  float inv_tau, q_scale;
+  float* state;
+  long long state_stride;
+  const int *q_start, *q_len, *state_slot;
+  float* o;
+  int o_stride, heads, dk, dv, extra_col, n_chunks;
+  float* scratch;              // per (request, chunk, head): D_end [dk], then [dk][dv]
+  const float *head_decay, *tok_gates;
+};
+
+__device__ __forceinline__ float gc_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+__device__ __forceinline__ float gc_alpha(const GlaArgs& a, int head, size_t m, int ch) {
+  if (a.tok_gates) return a.tok_gates[(m * a.heads + head) * 3];
+  if (a.head_decay) return a.head_decay[head];
+  const float zz = a.z[m * a.z_stride + head * a.dk + ch] + (a.z_bias ? a.z_bias[head * a.dk + ch] : 0.f);
+  return expf(-gc_softplus(-zz) * a.inv_tau);        // sigmoid(zz)^(1/tau)
+}
+template <typename TQ>
+__device__ __forceinline__ float gc_key(const GlaArgs& a, int head, size_t m, int ch) {
+  const float k = mi_to_float(reinterpret_cast<const TQ*>(a.k)[m * a.qk_stride + head * a.dk + ch]);
+  return a.tok_gates ? k * a.tok_gates[(m * a.heads + head) * 3 + 1] : k;
+}
+template <typename T>
+__device__ __forceinline__ float gc_value(const GlaArgs& a, int head, size_t m, int j) {
+  const int dv_in = a.dv - a.extra_col;
+  return j < dv_in ? mi_to_float(reinterpret_cast<const T*>(a.v)[m * a.stride + head * dv_in + j]) : (j < a.dv ? 1.f : 0.f);
+}
+__device__ __forceinline__ float* gc_unit(const GlaArgs& a, int req, int chunk, int head) {
+  return a.scratch + (((size_t)req * a.n_chunks + chunk) * a.heads + head) * ((size_t)a.dk + (size_t)a.dk * a.dv);
+}
+
+__device__ __forceinline__ uint64_t gc_pack(float x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void gc_unpack(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ void gc_fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+// ------------------------------------------------------------------------------------------ the chunks' own part of S
+template <typename TQ, typename T>
+__global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
+  mi_pdl_enter();
+  extern __shared__ __align__(16) float gsm[];
+  float* ks = gsm;                              // [GC_T][GC_PITCH]
+  float* vs = ks + GC_T * GC_PITCH;             // [GC_T][GC_PITCH]
+  __shared__ float tail[GC_W];
+  const int col_tiles = (a.dv + GC_W - 1) / GC_W;
+  const int r0 = (blockIdx.x / col_tiles) * GC_W, j0 = (blockIdx.x % col_tiles) * GC_W;
+  const int head = blockIdx.y, req = blockIdx.z / a.n_chunks, chunk = blockIdx.z - req * a.n_chunks;
+  const int len = a.q_len[req] - chunk * GC_T;  // tokens from here on
+  if (len <= 0) return;
+  const int n = min(GC_T, len);
+  const size_t m0 = (size_t)a.q_start[req] + (size_t)chunk * GC_T;
+  const int tid = threadIdx.x, ch = tid & (GC_W - 1), half = tid >> 7;
+  const bool mine = r0 + ch < a.dk;
+  // k times the decays of the tokens behind it: 32 tokens per thread from the end, then the later half's whole decay
+  float p = 1.f;
+#pragma unroll 8
+  for (int t = half * 32 + 31; t >= half * 32; --t) {
+    float kv = 0.f, al = 1.f;
+    if (mine && t < n) {
+      kv = gc_key<TQ>(a, head, m0 + t, r0 + ch);
+      al = gc_alpha(a, head, m0 + t, r0 + ch);
+    }
+    ks[t * GC_PITCH + ch] = kv * p;
+    p *= al;
+  }
+  if (half == 1) tail[ch] = p;
+  for (int i = tid; i < GC_T * GC_W; i += GC_THREADS) {
+    const int t = i >> 7, j = j0 + (i & (GC_W - 1));
+    vs[t * GC_PITCH + (i & (GC_W - 1))] = t < n && j < a.dv ? gc_value<T>(a, head, m0 + t, j) : 0.f;
+  }
+  __syncthreads();
+  float* unit = gc_unit(a, req, chunk, head);
+  if (half == 0) {
+    const float f = tail[ch];
+    for (int t = 0; t < 32; ++t) ks[t * GC_PITCH + ch] *= f;
+    if (j0 == 0 && mine) unit[r0 + ch] = p * f;
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  uint64_t acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+#pragma unroll 4
+  for (int t = 0; t < GC_T; ++t) {
+    const float4 k0 = *reinterpret_cast<const float4*>(ks + t * GC_PITCH + ty * 4);
+    const float4 k1 = *reinterpret_cast<const float4*>(ks + t * GC_PITCH + 64 + ty * 4);
+    const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(vs + t * GC_PITCH + tx * 4);
+    const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(vs + t * GC_PITCH + 64 + tx * 4);
+    const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint64_t w = gc_pack(kk[i]);
+      gc_fma2(acc[i][0], w, v0.x);
+      gc_fma2(acc[i][1], w, v0.y);
+      gc_fma2(acc[i][2], w, v1.x);
+      gc_fma2(acc[i][3], w, v1.y);
+    }
+  }
+  float* B = unit + a.dk;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = r0 + (i >> 2) * 64 + ty * 4 + (i & 3);
+    if (row >= a.dk) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = j0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
+      float x, y;
+      gc_unpack(acc[i][j], x, y);
+      if (col < a.dv) B[(size_t)row * a.dv + col] = x;
+      if (col + 1 < a.dv) B[(size_t)row * a.dv + col + 1] = y;
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------ the states in between
+// One thread per state element; a chunk's place in the scratch receives the state that the chunk begins with.  The loads
+// do not depend on the chain and run eight chunks ahead.
+__global__ void __launch_bounds__(GC_THREADS) gla_carry_kernel(const GlaArgs a) {
+  mi_pdl_enter();
+  const int head = blockIdx.y, req = blockIdx.z;
+  const long long e = (long long)blockIdx.x * GC_THREADS + threadIdx.x, elems = (long long)a.dk * a.dv;
+  if (e >= elems) return;
+  const int chunks = (a.q_len[req] + GC_T - 1) / GC_T;
+  float* S = a.state + (size_t)a.state_slot[req] * a.state_stride + (size_t)head * elems + e;
+  const size_t step = (size_t)a.heads * (a.dk + elems);
+  float* unit = gc_unit(a, req, 0, head);
+  const float* A = unit + e / a.dv;
+  float* B = unit + a.dk + e;
+  float s = *S;
+  for (int c0 = 0; c0 < chunks; c0 += 8) {
+    float av[8], bv[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const bool in = c0 + i < chunks;
+      av[i] = in ? A[(c0 + i) * step] : 1.f;
+      bv[i] = in ? B[(c0 + i) * step] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (c0 + i < chunks) {
+        B[(c0 + i) * step] = s;
+        s = fmaf(av[i], s, bv[i]);
+      }
+    }
+  }
+  *S = s;
+}
+
+// ------------------------------------------------------------------------------------------ the outputs
+// acc[4][4] (rows 4 ty.., two columns each: 4 tx.. and 64 + 4 tx..) += rows [.][k] times mat [k][columns], `depth` of k
+__device__ __forceinline__ void gc_product(uint64_t (&acc)[4][4], const float* rows, int pitch, const float* mat, int depth,
+                                           int tx) {
+#pragma unroll 2
+  for (int k = 0; k < depth; k += 4) {
+    float4 r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(rows + i * pitch + k);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(mat + (k + kk) * GC_PITCH + tx * 4);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(mat + (k + kk) * GC_PITCH + 64 + tx * 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint64_t w = gc_pack(kk == 0 ? r[i].x : kk == 1 ? r[i].y : kk == 2 ? r[i].z : r[i].w);
+        gc_fma2(acc[i][0], w, b0.x);
+        gc_fma2(acc[i][1], w, b0.y);
+        gc_fma2(acc[i][2], w, b1.x);
+        gc_fma2(acc[i][3], w, b1.y);
+      }
+    }
+  }
+}
+
+template <typename TQ, typename T>
+__global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a) {
+  mi_pdl_enter();
+  extern __shared__ __align__(16) float gsm[];
+  float* qs = gsm;                              // [GC_T][GC_PITCH]  q D
+  float* ks = qs + GC_T * GC_PITCH;             // [GC_T][GC_PITCH]  k / D
+  float* slab = ks + GC_T * GC_PITCH;           // [GC_SLAB][GC_PITCH]
+  float* ps = slab + GC_SLAB * GC_PITCH;        // [GC_T][GC_PP]
+  __shared__ float tail[GC_W];
+  const int j0 = blockIdx.x * GC_W;
+  const int head = blockIdx.y, req = blockIdx.z / a.n_chunks, chunk = blockIdx.z - req * a.n_chunks;
+  const int len = a.q_len[req] - chunk * GC_T;
+  if (len <= 0) return;
+  const int n = min(GC_T, len);
+  const size_t m0 = (size_t)a.q_start[req] + (size_t)chunk * GC_T;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, ch = tid & (GC_W - 1), half = tid >> 7;
+  const float* S = gc_unit(a, req, chunk, head) + a.dk;
+  const TQ* q = reinterpret_cast<const TQ*>(a.q);
+
+  uint64_t acc[4][4];
+  float pair[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[i][j] = 0;
+      pair[i][j] = 0.f;
+    }
+  for (int i = tid; i < GC_T * GC_PP; i += GC_THREADS) ps[i] = 0.f;
+
+  for (int c0 = 0; c0 < a.dk; c0 += GC_W) {      // 128 key channels at a time
+    const bool mine = c0 + ch < a.dk;
+    if (c0) __syncthreads();
+    // D of every token: 32 tokens per thread, then the earlier half's whole decay
+    float p = 1.f;
+#pragma unroll 8
+    for (int t = half * 32; t < half * 32 + 32; ++t) {
+      if (mine && t < n) p *= gc_alpha(a, head, m0 + t, c0 + ch);
+      qs[t * GC_PITCH + ch] = p;
+    }
+    if (half == 0) tail[ch] = p;
+    __syncthreads();
+    const float f = half ? tail[ch] : 1.f;
+    const bool quotient = __syncthreads_and(p * f >= GC_SMALLEST) != 0;
+#pragma unroll 8
+    for (int t = half * 32; t < half * 32 + 32; ++t) {
+      float qv = 0.f, kv = 0.f;
+      const float d = qs[t * GC_PITCH + ch] * f;
+      if (mine && t < n) {
+        qv = mi_to_float(q[(m0 + t) * a.qk_stride + head * a.dk + c0 + ch]) * a.q_scale;
+        kv = gc_key<TQ>(a, head, m0 + t, c0 + ch);
+      }
+      qs[t * GC_PITCH + ch] = qv * d;
+      ks[t * GC_PITCH + ch] = quotient ? kv / d : kv;
+    }
+    __syncthreads();
+    // the pairs' weights
+    if (quotient) {
+#pragma unroll 2
+      for (int k = 0; k < GC_W; k += 4) {
+        float4 r[4], c[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * GC_PITCH + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * GC_PITCH + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            pair[i][j] = fmaf(r[i].x, c[j].x, pair[i][j]);
+            pair[i][j] = fmaf(r[i].y, c[j].y, pair[i][j]);
+            pair[i][j] = fmaf(r[i].z, c[j].z, pair[i][j]);
+            pair[i][j] = fmaf(r[i].w, c[j].w, pair[i][j]);
+          }
+      }
+    } else {
+      // a channel all but dies within the chunk: every key's decay token by token, a warp per key
+      const int lane = tid & 31;
+      for (int s = tid >> 5; s < n; s += GC_THREADS / 32) {
+        float w[GC_W / 32];
+#pragma unroll
+        for (int i = 0; i < GC_W / 32; ++i) w[i] = ks[s * GC_PITCH + lane + 32 * i];
+        for (int t = s; t < n; ++t) {
+          float sum = 0.f;
+#pragma unroll
+          for (int i = 0; i < GC_W / 32; ++i) {
+            const int c = c0 + lane + 32 * i;
+            if (c < a.dk) {
+              if (t > s) w[i] *= gc_alpha(a, head, m0 + t, c);
+              sum = fmaf(mi_to_float(q[(m0 + t) * a.qk_stride + head * a.dk + c]) * a.q_scale, w[i], sum);
+            }
+          }
+          sum = mi_warp_sum(sum);
+          if (lane == 0) ps[t * GC_PP + s] += sum;
+        }
+      }
+    }
+    // what the state the chunk began with gives, 32 channels of it at a time
+    const int depth = min(GC_W, a.dk - c0);
+    for (int k0 = 0; k0 < depth; k0 += GC_SLAB) {
+      __syncthreads();
+      for (int i = tid; i < GC_SLAB * GC_W; i += GC_THREADS) {
+        const int r = i >> 7, j = i & (GC_W - 1);
+        slab[r * GC_PITCH + j] = (k0 + r < depth && j0 + j < a.dv) ? S[(size_t)(c0 + k0 + r) * a.dv + j0 + j] : 0.f;
+      }
+      __syncthreads();
+      gc_product(acc, qs + (ty * 4) * GC_PITCH + k0, GC_PITCH, slab, GC_SLAB, tx);
+    }
+  }
+  // the chunk's own keys (a pair's weight counts from the key's token on)
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int t = ty * 4 + i, s = tx + 16 * j;
+      ps[t * GC_PP + s] = s <= t ? ps[t * GC_PP + s] + pair[i][j] : 0.f;
+    }
+  for (int s0 = 0; s0 < n; s0 += GC_SLAB) {
+    __syncthreads();
+    for (int i = tid; i < GC_SLAB * GC_W; i += GC_THREADS) {
+      const int r = i >> 7, j = i & (GC_W - 1);
+      slab[r * GC_PITCH + j] = (s0 + r < n && j0 + j < a.dv) ? gc_value<T>(a, head, m0 + s0 + r, j0 + j) : 0.f;
+    }
+    __syncthreads();
+    // (rows of four tokens see no key behind their last)
+    gc_product(acc, ps + (ty * 4) * GC_PP + s0, GC_PP, slab, max(0, min(GC_SLAB, ty * 4 + 4 - s0)), tx);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = ty * 4 + i;
+    if (t >= n) continue;
+    float* dst = a.o + (m0 + t) * a.o_stride + head * a.dv;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = j0 + (j >> 1) * 64 + tx * 4 + (j & 1) * 2;
+      float x, y;
+      gc_unpack(acc[i][j], x, y);
+      if (col < a.dv) dst[col] = x;
+      if (col + 1 < a.dv) dst[col + 1] = y;
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------ host
+
+extern "C" int mi_gla_chunk_tokens() { return GC_T; }
+
+// floats of scratch for portions of up to n_chunks chunks
+extern "C" long long mi_gla_chunks_scratch(int n_requests, int n_chunks, int heads, int dk, int dv) {
+  return (long long)n_requests * n_chunks * heads * ((long long)dk + (long long)dk * dv);
+}
+
+template <typename TQ, typename T>
+static cudaError_t gla_chunks_launch(const GlaArgs& a, int n_requests, cudaStream_t stream) {
+  const int col_tiles = (a.dv + GC_W - 1) / GC_W, row_tiles = (a.dk + GC_W - 1) / GC_W;
+  const size_t fold_smem = (size_t)2 * GC_T * GC_PITCH * sizeof(float);
+  const size_t out_smem = ((size_t)(2 * GC_T + GC_SLAB) * GC_PITCH + (size_t)GC_T * GC_PP) * sizeof(float);
+  auto fold = gla_fold_kernel<TQ, T>;
+  auto out = gla_out_kernel<TQ, T>;
+  cudaError_t e = cudaFuncSetAttribute(fold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fold_smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+  if (e != cudaSuccess) return e;
+  const unsigned z = (unsigned)(n_requests * a.n_chunks);
+  e = MI_LAUNCH(fold, dim3(col_tiles * row_tiles, a.heads, z), GC_THREADS, fold_smem, stream, a);
+  if (e != cudaSuccess) return e;
+  const long long elems = (long long)a.dk * a.dv;
+  e = MI_LAUNCH(gla_carry_kernel, dim3((unsigned)((elems + GC_THREADS - 1) / GC_THREADS), a.heads, n_requests), GC_THREADS, 0,
+                stream, a);
+  if (e != cudaSuccess) return e;
+  return MI_LAUNCH(out, dim3(col_tiles, a.heads, z), GC_THREADS, out_smem, stream, a);
+}
+
+// Arguments as mi_gla_scan (recurrent.cu); n_chunks: 64-token chunks of the longest portion, scratch as
+// mi_gla_chunks_scratch says.  Three launches.
+extern "C" int mi_gla_chunks(const void* q, const void* k, int qk_stride, int qk_dtype, const void* v, int stride,
+                             const float* z, int z_stride, const float* z_bias, float inv_tau, float q_scale, float* state,
+                             long long state_stride, const int* q_start, const int* q_len, const int* state_slot, float* o,
+                             int o_stride, int n_requests, int heads, int dk, int dv, float* scratch, int n_chunks,
+                             const float* head_decay, const float* tok_gates, int extra_col, int dtype,
+                             cudaStream_t stream) {
+  if (n_requests <= 0 || n_chunks <= 0) return 0;
+  if (!z && !head_decay && !tok_gates) MI_REFUSE("gla: neither decays per channel nor per head nor per token");
+  if (extra_col != 0 && extra_col != 1) MI_REFUSE("gla: one extra column or none");
+  if (dv - extra_col <= 0) MI_REFUSE("gla: no value columns");
+  if (!scratch) MI_REFUSE("gla: chunks need scratch memory");
+  if ((long long)n_requests * n_chunks > 65535) MI_REFUSE("gla: too many chunks for one launch");
+  if (dk <= 0 || dk > 256 || dv <= 0) MI_REFUSE("gla: key size %d must lie in [1, 256], value size %d above 0", dk, dv);
+  if (heads > 65535) MI_REFUSE("gla: too many heads for one launch");
+  const GlaArgs a = {q, k, v, qk_stride, stride, z, z_stride, z_bias, inv_tau, q_scale, state, state_stride, q_start, q_len,
+                     state_slot, o, o_stride, heads, dk, dv, extra_col, n_chunks, scratch, head_decay, tok_gates};
+  cudaError_t e;
+  if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_BF16) e = gla_chunks_launch<bf16, bf16>(a, n_requests, stream);
+  else if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_F32) e = gla_chunks_launch<float, bf16>(a, n_requests, stream);
+  else MI_REFUSE("gla: dtypes %d (q, k) and %d (v) are not taken together in chunks", qk_dtype, dtype);
+  if (e != cudaSuccess) return (int)e;
+  MI_RETURN_LAUNCH_STATUS();
+}

@@ -205,6 +205,10 @@ def _sig_gemm_tma(lib: ctypes.CDLL) -> None:
                                           ctypes.POINTER(c_int)]
     lib.mi_gemm_tma_status.argtypes = [c_int]
     lib.mi_set_status_word.argtypes = [c_void_p]
+    lib.mi_gemm_rows_stat_rows.argtypes = [c_int, c_int]
+    lib.mi_gemm_rows.argtypes = [c_void_p, ctypes.c_longlong, c_void_p, c_void_p, ctypes.c_longlong, c_int, c_int, c_int,
+                                 c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
+                                 c_float, c_float, c_void_p]
 
 
 def _sig_attention_tc(lib: ctypes.CDLL) -> None:
@@ -1058,9 +1062,10 @@ TMA_GEMM_TILE_ROWS = 128    # rows of W per tile: one row of a statistics table
 
 
 class RowStats:
-    """Sums of squares of the rows of an fp32 stream ``[M, width]``, 128 features at a time
-    (``sums [ceil(width / 128), 16]``, column = row of the stream), as the residual epilogue of
-    ``gemm_tma`` leaves them, with the ``eps`` of the norm they are meant for."""
+    """Sums of squares of the rows of an fp32 stream ``[M, width]``, a range of features at a time
+    (``sums [ranges, 16]``, column = row of the stream), as the residual epilogue of ``gemm_tma`` (128
+    features each) or of ``gemm_rows`` (a block's features each) leaves them, with the ``eps`` of the norm
+    they are meant for."""
 
     __slots__ = ("sums", "width", "eps")
 
@@ -1128,6 +1133,49 @@ def gemm_tma(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bf
     return out
 
 
+def gemm_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, swiglu: int = 0,
+              row_stats: RowStats | None = None, residual: torch.Tensor | None = None, gain: torch.Tensor | None = None,
+              eps: float = 0.0, act: tuple[str, tuple[float, float]] | None = None):
+    """``gemm_tma`` for at most 16 rows of ``x`` on the kernel of decode steps, whose blocks own rows of ``w`` over the
+    whole of k and exchange nothing; the same forms, the statistics a row of 16 sums per block instead of per 128 features."""
+    _cuda(x, w)
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        raise KernelError("gemm_rows: operands must be bfloat16")
+    if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] or x.stride(1) != 1 or not w.is_contiguous():
+        raise KernelError(f"gemm_rows: shapes {tuple(x.shape)} x {tuple(w.shape)}^T do not match")
+    M, K = x.shape
+    N = w.shape[0]
+    lib = _waiting_lib("gemm_tma", x.device)
+    blocks = _sms(x.device)
+    if act is not None and (swiglu or residual is not None or row_stats is not None or out_dtype != torch.bfloat16):
+        raise KernelError("gemm_rows: an activation of single values goes with the plain product")
+    n_out = N // 2 if swiglu else N
+    out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+    sums_in, rows_in, width, eps_in = None, 0, 0, 0.0
+    if row_stats is not None:
+        sums_in, width, eps_in = row_stats.sums, row_stats.width, row_stats.eps
+        rows_in = sums_in.shape[0]
+        if (width != K or sums_in.dtype != torch.float32 or not sums_in.is_contiguous() or sums_in.dim() != 2
+                or sums_in.shape[1] != TMA_GEMM_STAT_TOKENS):
+            raise KernelError(f"gemm_rows: row statistics {tuple(sums_in.shape)} of width {width} do not fit K = {K}")
+    stats_out = None
+    if residual is not None:
+        if (gain is None or gain.dtype != torch.float32 or gain.numel() != N or not gain.is_contiguous()
+                or residual.dtype != torch.float32 or tuple(residual.shape) != (M, N) or not residual.is_contiguous()):
+            raise KernelError("gemm_rows: the residual epilogue needs a contiguous fp32 stream [M, N] and an fp32 gain [N]")
+        _cuda(residual, gain)
+        stats_out = torch.empty((lib.mi_gemm_rows_stat_rows(N, blocks), TMA_GEMM_STAT_TOKENS), dtype=torch.float32,
+                                device=x.device)
+    rc = lib.mi_gemm_rows(_ptr(x), x.stride(0) if M > 1 else K, _ptr(w), _ptr(out), n_out, M, N, K, _code(out_dtype),
+                          UNARY_ACT[act[0]] if act else int(swiglu), blocks, _ptr(sums_in), rows_in, width, eps_in,
+                          _ptr(residual), _ptr(gain), _ptr(stats_out), act[1][0] if act else 0.0, act[1][1] if act else 0.0,
+                          _stream())
+    _finish(lib, rc, "gemm_rows")
+    if residual is not None:
+        return out, RowStats(stats_out, N, eps)
+    return out
+
+
 def gemm_tma_status(reset: bool = True) -> int:
     """Non-zero when a block of the streaming product gave up a bounded wait since the last
     reset (its output is then wrong).  Synchronises the device."""
@@ -1154,7 +1202,7 @@ def linear_into_stream(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor,
     statistics a product with ``row_stats`` needs to finish an RMS norm with ``eps``."""
     if not linear_fusable(x.shape[0], w) or not gemm_tma_ok(x, w):
         raise KernelError("linear_into_stream: these operands have no fused form (ask linear_fusable first)")
-    return gemm_tma(x, w, torch.bfloat16, residual=residual, gain=gain, eps=eps)
+    return gemm_rows(x, w, torch.bfloat16, residual=residual, gain=gain, eps=eps)
 
 
 GLU_ACT = {"silu": 1, "gelu_tanh": 2}
@@ -1171,7 +1219,7 @@ def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, row_stats: "RowStats |
         raise KernelError(f"linear_swiglu: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
             and w_pairs.dtype == torch.bfloat16 and gemm_tma_ok(x, w_pairs)):
-        return gemm_tma(x, w_pairs, torch.bfloat16, swiglu=GLU_ACT[act], row_stats=row_stats)
+        return gemm_rows(x, w_pairs, torch.bfloat16, swiglu=GLU_ACT[act], row_stats=row_stats)
     if row_stats is not None:
         raise KernelError("linear_swiglu: row statistics need the streaming product (ask linear_fusable first)")
     if act == "silu":
@@ -1190,7 +1238,7 @@ def linear_activated(x: torch.Tensor, w: torch.Tensor, act: str, numbers: tuple[
         raise KernelError(f"linear_activated: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
             and w.dtype == torch.bfloat16 and gemm_tma_ok(x, w)):
-        return gemm_tma(x, w, torch.bfloat16, act=(act, numbers))
+        return gemm_rows(x, w, torch.bfloat16, act=(act, numbers))
     y = linear(x, w)
     lib = _lib("stream")
     if act == "relu2":
@@ -1210,7 +1258,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
 
     float32 operands run the true-fp32 CUDA-core kernel (never a library product, which
     could pick a reduced-precision mode).  bfloat16 operands with few rows (decode) run the
-    weight-streaming tcgen05 kernel of gemm_tma.cu, which starts streaming weights while the
+    weight-streaming kernel ``gemm_rows``, which starts streaming weights while the
     kernel before it still runs; other bfloat16 operands use the library product with fp32
     accumulation, as the reference does for every linear layer (``distributed/linear.py:167``).
     ``out_dtype=float32`` keeps the accumulator's precision in the result (used for logits).
@@ -1220,7 +1268,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     if row_stats is not None:
         if not linear_fusable(x.shape[0], w) or not gemm_tma_ok(x, w):
             raise KernelError("linear: row statistics need the streaming product (ask linear_fusable first)")
-        return gemm_tma(x, w, out_dtype or torch.bfloat16, row_stats=row_stats)
+        return gemm_rows(x, w, out_dtype or torch.bfloat16, row_stats=row_stats)
     if x.dtype == torch.float32:
         if w.dtype != torch.float32:
             raise KernelError("linear: fp32 activations need fp32 weights")
@@ -1231,7 +1279,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     if out_dtype not in (None, torch.bfloat16, torch.float32):
         raise KernelError(f"linear: unsupported output dtype {out_dtype}")
     if USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS and gemm_tma_ok(x, w):
-        return gemm_tma(x, w, out_dtype or torch.bfloat16)
+        return gemm_rows(x, w, out_dtype or torch.bfloat16)
     launch_count += 1
     if out_dtype in (None, torch.bfloat16):
         return torch.mm(x, w.t())

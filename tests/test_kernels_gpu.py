@@ -317,6 +317,56 @@ def test_gemm_tma_refuses_what_it_cannot_take():
     assert not ops().gemm_tma_ok(rnd(2, 36, dtype=torch.bfloat16, seed=35).to(DEV), rnd(64, 36, dtype=torch.bfloat16).to(DEV))
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 2, 8), (1, 1000, 64), (3, 51, 448), (7, 296, 512), (8, 9475, 520), (9, 4104, 576),
+                                   (16, 320, 4104), (16, 18945, 72), (8, 4096, 4096)])
+def test_gemm_rows_every_form(M, N, K):
+    """The product of decode steps at the edges of its cuts (rows per block from 2 to 64, several tiles per block, one to
+    eight boxes along k and a ragged last one, one and two groups of eight tokens, odd widths), against float64: the sum
+    of K products in fp32 is off by at most K 2^-24 of the sum of magnitudes, a bfloat16 result by 2^-8 of itself more."""
+    x = rnd(M, K, dtype=torch.bfloat16, seed=60)
+    w = rnd(N, K, dtype=torch.bfloat16, seed=61, scale=0.1)
+    want = x.double() @ w.double().T
+    sums = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    xd, wd = x.to(DEV), w.to(DEV)
+    out = ops().gemm_rows(xd, wd, torch.float32)
+    assert ((out.cpu().double() - want).abs() <= sums + 1e-12).all()
+    assert torch.equal(ops().gemm_rows(xd[M - 1:].contiguous(), wd, torch.float32)[0], out[M - 1])      # whatever shares the call
+    assert ((ops().gemm_rows(xd, wd).cpu().double() - want).abs() <= sums + 2.0 ** -8 * (want.abs() + sums)).all()
+    relu2 = ops().gemm_rows(xd, wd, act=("relu2", (0.0, 0.0))).cpu().double()
+    square = want.clamp(min=0) ** 2
+    assert ((relu2 - square).abs() <= 2 * want.abs() * sums + sums ** 2 + 2.0 ** -8 * (square + 1e-6)).all()
+    if N % 2 == 0:
+        g, u = want[:, 0::2], want[:, 1::2]
+        act = P.silu(g) * u
+        err = sums[:, 0::2] * 1.1 * u.abs() + sums[:, 1::2] * (g.abs() + 1) + 2.0 ** -8 * act.abs() + 1e-5
+        assert ((ops().gemm_rows(xd, wd, swiglu=1).cpu().double() - act).abs() <= err).all()
+    # added to the stream, with the sums of squares that the next product finishes the norm with
+    res, gain = rnd(M, N, seed=62), 1 + 0.1 * rnd(N, seed=63)
+    stream = res.clone().to(DEV)
+    y, stats = ops().gemm_rows(xd, wd, residual=stream, gain=gain.to(DEV), eps=1e-5)
+    h = res.double() + want
+    assert ((stream.cpu().double() - h).abs() <= sums + 2.0 ** -23 * h.abs()).all()
+    assert ((y.cpu().double() - h * gain.double()).abs() <= 1.5 * sums + 2.0 ** -8 * (h * gain.double()).abs() + 1e-6).all()
+    sq = (h ** 2).sum(dim=1)
+    assert ((stats.sums[:, :M].cpu().double().sum(dim=0) - sq).abs() <= 1e-5 * sq).all()
+    if N % 8 == 0:
+        w2 = rnd(33, N, dtype=torch.bfloat16, seed=64, scale=0.1)
+        normed = (y.cpu().double() / torch.sqrt(sq / N + 1e-5)[:, None])
+        err = (N * 2.0 ** -24 + 2e-5) * (normed.abs() @ w2.double().abs().T)
+        assert ((ops().gemm_rows(y, w2.to(DEV), torch.float32, row_stats=stats).cpu().double() - normed @ w2.double().T).abs() <= err).all()
+    assert ops().gemm_tma_status() == 0
+
+
+def test_gemm_rows_refuses_what_it_cannot_take():
+    w = rnd(64, 64, dtype=torch.bfloat16, seed=65).to(DEV)
+    with pytest.raises(ops().KernelError, match="at most 16"):
+        ops().gemm_rows(rnd(17, 64, dtype=torch.bfloat16, seed=66).to(DEV), w)
+    with pytest.raises(ops().KernelError, match="multiples of 8"):
+        ops().gemm_rows(rnd(2, 36, dtype=torch.bfloat16, seed=67).to(DEV), rnd(64, 36, dtype=torch.bfloat16).to(DEV))
+    with pytest.raises(ops().KernelError, match="do not fit"):
+        ops().gemm_rows(rnd(2, 64, dtype=torch.bfloat16, seed=68).to(DEV), w, row_stats=ops().RowStats(torch.zeros(2, 16, device=DEV), 200, 1e-5))
+
+
 def test_linear_library_and_streaming_kernels_agree():
     w = rnd(300, 264, dtype=torch.bfloat16, seed=22, scale=0.1).to(DEV)
     x = rnd(40, 264, dtype=torch.bfloat16, seed=23).to(DEV)
