@@ -23,7 +23,7 @@
 // Three products live here, all with fp32 accumulation, and none lets a row's result depend on which
 // other rows share its tile: float32 on CUDA cores, k ascending (moe_gemm_kernel); bfloat16 tiles of 64
 // rows on the tensor cores (mma.sync m16n8k16, moe_gemm_mma_kernel); bfloat16 tiles of 8 rows that
-// stream an expert's weights, one warp per output column (moe_stream_kernel).  Large bfloat16 steps
+// stream an expert's weights past the tensor cores (moe_rows_kernel).  Large bfloat16 steps
 // whose rows are whole 16-byte pieces go to the library's grouped product instead (the caller gathers
 // the rows with mi_moe_gather and passes the experts' row ranges from the plan).
 #include "common.cuh"
@@ -218,24 +218,41 @@ __global__ void moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* 
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&counts[ids[i]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // rows and tiles in front of every expert: a warp scan per 32 experts, carried on from one to the next by one warp
+  if (threadIdx.x < 32) {
     int* offsets = plan + 1;
     int* tiles = plan + 2 + E;
+    const int lane = threadIdx.x;
     int run = 0, nt = 0;
-    for (int e = 0; e < E; ++e) {
-      offsets[e] = run;
-      cursor[e] = run;
-      const int end = run + counts[e];
-      for (int r0 = run; r0 < end; r0 += tile_rows) {
-        tiles[3 * nt] = e;
-        tiles[3 * nt + 1] = r0;
-        tiles[3 * nt + 2] = min(tile_rows, end - r0);
-        ++nt;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane;
+      const int rows = e < E ? counts[e] : 0, own = (rows + tile_rows - 1) / tile_rows;
+      int rs = rows, ts = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int r = __shfl_up_sync(0xffffffffu, rs, o), t = __shfl_up_sync(0xffffffffu, ts, o);
+        if (lane >= o) {
+          rs += r;
+          ts += t;
+        }
       }
-      run = end;
+      if (e < E) {
+        const int first = run + rs - rows, at = nt + ts - own;
+        offsets[e] = first;
+        cursor[e] = first;
+        for (int i = 0; i < own; ++i) {
+          tiles[3 * (at + i)] = e;
+          tiles[3 * (at + i) + 1] = first + i * tile_rows;
+          tiles[3 * (at + i) + 2] = min(tile_rows, rows - i * tile_rows);
+        }
+      }
+      run += __shfl_sync(0xffffffffu, rs, 31);
+      nt += __shfl_sync(0xffffffffu, ts, 31);
     }
-    offsets[E] = run;
-    plan[0] = nt;
+    if (lane == 0) {
+      offsets[E] = run;
+      plan[0] = nt;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -476,78 +493,96 @@ static int mma_vec_ok(const void* a, long long a_stride, const void* w0, const v
 }
 
 // ------------------------------------------------------------------------------------------ few rows per expert
-// A decode step brings an expert a handful of rows: the product is a stream of that expert's weights.
-// Tiles have at most FEW_ROWS rows; a warp owns one output column, its lanes walk k in 16-byte pieces
-// (several loads in flight per lane), the tile's rows of x come through the L1, and the lanes' sums
-// are added at the end.  bfloat16, k a multiple of 8, 16-byte aligned rows.
-__device__ __forceinline__ void fma8(float& acc, const uint4& w, const uint4& x) {
-  const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&w);
-  const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&x);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 wf = __bfloat1622float2(wp[i]), xf = __bfloat1622float2(xp[i]);
-    acc = fmaf(wf.x, xf.x, acc);
-    acc = fmaf(wf.y, xf.y, acc);
-  }
+// A decode step brings an expert a handful of rows: the product is a stream of that expert's weights.  Tiles have at
+// most FEW_ROWS rows, which are the N side of mma.sync.m16n8k16; a block owns 16 rows of both gated matrices (or 32 of
+// the plain one), the M side, and its eight warps take the 64-wide pieces of k in turn and add up in shared memory.  A
+// lane's fragments come straight from global memory, 16 bytes (8 consecutive k, taken as the k of two instructions in
+// an order that is the same for both operands) at a time, two pieces of k, 16 loads, in flight: with one warp per output
+// column and fused multiply-adds the same 630 MB (25 experts of 3 x 1024 x 4096) took 179 us, 0.54 of the copy
+// bandwidth, most of it conversions and the columns' short lives.  bfloat16, k a multiple of 8, 16-byte aligned rows.
+#define MR_WARPS 8
+#define MR_PIECE 64
+__device__ __forceinline__ uint4 mr_load(const bf16* p, bool in) {       // weights: read once
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (in) asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];\n"
+                       : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 
 template <bool GATED>
-__global__ void __launch_bounds__(256)
-moe_stream_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict__ w0, const bf16* __restrict__ w1,
-                  long long w_expert_stride, const int* __restrict__ perm, int top, const int* __restrict__ plan,
-                  int E, void* __restrict__ out_, int N, int K, float limit, float alpha, float offset) {
+__global__ void __launch_bounds__(32 * MR_WARPS, 2)
+moe_rows_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict__ w0, const bf16* __restrict__ w1,
+                long long w_expert_stride, const int* __restrict__ perm, int top, const int* __restrict__ plan,
+                int E, void* __restrict__ out_, int N, int K, float limit, float alpha, float offset) {
   mi_pdl_enter();
   const int tile = blockIdx.y;
   if (tile >= plan[0]) return;
   const int* td = plan + 2 + E + 3 * tile;
   const int e = td[0], row0 = td[1], rows = td[2];
-  __shared__ const bf16* aptr[FEW_ROWS];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < FEW_ROWS)
-    aptr[tid] = tid < rows ? a + (size_t)(GATED ? perm[row0 + tid] / top : row0 + tid) * a_stride : nullptr;
-  __syncthreads();
-  const int n = blockIdx.x * 8 + warp;
-  if (n >= N) return;
-  const bf16* wr0 = w0 + (size_t)e * w_expert_stride + (size_t)n * K;
-  const bf16* wr1 = GATED ? w1 + (size_t)e * w_expert_stride + (size_t)n * K : nullptr;
-  float acc0[FEW_ROWS], acc1[FEW_ROWS];
+  __shared__ float shares[MR_WARPS][FEW_ROWS][32 + 4];      // [warp][row of x][row of either matrix]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  constexpr int COLS = GATED ? 16 : 32;                     // output columns of the block
+  const int n0 = blockIdx.x * COLS;
+  // rows g and g + 8 of the two halves: gate and up, or columns n0.. and n0 + 16..  (rows beyond N repeat the last one)
+  const bf16* base[2] = {w0 + (size_t)e * w_expert_stride, (GATED ? w1 : w0) + (size_t)e * w_expert_stride};
+  const bf16* wp[2][2];
 #pragma unroll
-  for (int r = 0; r < FEW_ROWS; ++r) acc0[r] = acc1[r] = 0.f;
-  // two pieces of every weight row per turn, all four loads in flight before the first is used
-  for (int k = lane * 8; k < K; k += 512) {
-    const bool two = k + 256 < K;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    const uint4 wa0 = *reinterpret_cast<const uint4*>(wr0 + k);
-    const uint4 wb0 = two ? *reinterpret_cast<const uint4*>(wr0 + k + 256) : zero;
-    const uint4 wa1 = GATED ? *reinterpret_cast<const uint4*>(wr1 + k) : zero;
-    const uint4 wb1 = (GATED && two) ? *reinterpret_cast<const uint4*>(wr1 + k + 256) : zero;
+  for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int r = 0; r < FEW_ROWS; ++r) {
-      if (r < rows) {
-        const uint4 xa = __ldg(reinterpret_cast<const uint4*>(aptr[r] + k));
-        fma8(acc0[r], wa0, xa);
-        if (GATED) fma8(acc1[r], wa1, xa);
-        if (two) {
-          const uint4 xb = __ldg(reinterpret_cast<const uint4*>(aptr[r] + k + 256));
-          fma8(acc0[r], wb0, xb);
-          if (GATED) fma8(acc1[r], wb1, xb);
-        }
+    for (int r = 0; r < 2; ++r)
+      wp[h][r] = base[h] + (size_t)min(N - 1, n0 + (GATED ? 0 : 16 * h) + g + 8 * r) * K + q * 8;
+  const bool has_x = g < rows;
+  const bf16* xp = a + (size_t)(has_x ? (GATED ? perm[row0 + g] / top : row0 + g) : 0) * a_stride + q * 8;
+  const int pieces = (K + MR_PIECE - 1) / MR_PIECE;
+  float acc[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[h][i] = 0.f;
+  for (int c = warp; c < pieces; c += 2 * MR_WARPS) {
+    uint4 w[2][2][2][2], x[2][2];     // [piece][half of it][matrix][row]
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int k = (c + p * MR_WARPS) * MR_PIECE + s * 32;
+        const bool in = k + q * 8 < K;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) w[p][s][h][r] = mr_load(wp[h][r] + k, in);
+        x[p][s] = in && has_x ? __ldg(reinterpret_cast<const uint4*>(xp + k)) : make_uint4(0u, 0u, 0u, 0u);
       }
-    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 u = w[p][s][h][0], v = w[p][s][h][1], xx = x[p][s];
+          const uint32_t a0[4] = {u.x, v.x, u.y, v.y}, b0[2] = {xx.x, xx.y};
+          const uint32_t a1[4] = {u.z, v.z, u.w, v.w}, b1[2] = {xx.z, xx.w};
+          mma_bf16(acc[h], a0, b0);
+          mma_bf16(acc[h], a1, b1);
+        }
   }
 #pragma unroll
-  for (int r = 0; r < FEW_ROWS; ++r) {
-    if (r < rows) {
-      const float s0 = mi_warp_sum(acc0[r]);
-      const float s1 = GATED ? mi_warp_sum(acc1[r]) : 0.f;
-      if (lane == 0) {
-        if (GATED)
-          reinterpret_cast<bf16*>(out_)[(size_t)(row0 + r) * N + n] =
-              __float2bfloat16_rn(mi_clamped_glu_value(s0, s1, limit, alpha, offset));
-        else
-          reinterpret_cast<float*>(out_)[(size_t)(row0 + r) * N + n] = s0;
-      }
-    }
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) shares[warp][2 * q + (i & 1)][16 * h + g + (i >> 1) * 8] = acc[h][i];
+  __syncthreads();
+  const int r = tid >> 5, j = tid & 31;       // a warp per row of x
+  if (r >= rows) return;
+  float v = 0.f;
+#pragma unroll
+  for (int s = 0; s < MR_WARPS; ++s) v += shares[s][r][j];
+  if (GATED) {
+    const float up = __shfl_down_sync(0xffffffffu, v, 16);
+    if (j < 16 && n0 + j < N)
+      reinterpret_cast<bf16*>(out_)[(size_t)(row0 + r) * N + n0 + j] =
+          __float2bfloat16_rn(mi_clamped_glu_value(v, up, limit, alpha, offset));
+  } else if (n0 + j < N) {
+    reinterpret_cast<float*>(out_)[(size_t)(row0 + r) * N + n0 + j] = v;
   }
 }
 
@@ -561,9 +596,9 @@ extern "C" int mi_moe_gate_up(const void* x, int x_stride, const void* w_gate, c
   if (tile_rows == FEW_ROWS) {
     if (dtype != MI_DTYPE_BF16 || !mma_vec_ok(x, x_stride, w_gate, w_up, H))
       MI_REFUSE("moe: the streaming product takes bfloat16 rows of whole 16-byte pieces");
-    dim3 g((ff + 7) / 8, max_tiles(n_entries, E, FEW_ROWS));
+    dim3 g((ff + 15) / 16, max_tiles(n_entries, E, FEW_ROWS));
     if (g.y > 65535) MI_REFUSE("moe: too many row tiles for one launch");
-    MI_LAUNCH((moe_stream_kernel<true>), g, 256, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
+    MI_LAUNCH((moe_rows_kernel<true>), g, 32 * MR_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
               (const bf16*)w_up, w_expert_stride, perm, top, plan, E, act, ff, H, limit, alpha, offset);
     MI_RETURN_LAUNCH_STATUS();
   }
@@ -587,9 +622,9 @@ extern "C" int mi_moe_down(const void* act, const void* w_down, long long w_expe
   if (tile_rows == FEW_ROWS) {
     if (dtype != MI_DTYPE_BF16 || !mma_vec_ok(act, ff, w_down, nullptr, ff))
       MI_REFUSE("moe: the streaming product takes bfloat16 rows of whole 16-byte pieces");
-    dim3 g((H + 7) / 8, max_tiles(n_entries, E, FEW_ROWS));
+    dim3 g((H + 31) / 32, max_tiles(n_entries, E, FEW_ROWS));
     if (g.y > 65535) MI_REFUSE("moe: too many row tiles for one launch");
-    MI_LAUNCH((moe_stream_kernel<false>), g, 256, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
+    MI_LAUNCH((moe_rows_kernel<false>), g, 32 * MR_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
               (const bf16*)nullptr, w_expert_stride, (const int*)nullptr, 1, plan, E, (void*)y, H, ff, 0.f, 0.f, 0.f);
     MI_RETURN_LAUNCH_STATUS();
   }
