@@ -41,6 +41,7 @@ LIBRARIES: dict[str, tuple[list[str], list[str], list[str]]] = {
     "layernorm": (["layernorm.cu"], ["common.cuh"], []),
     "rope_norm": (["rope_norm.cu"], ["common.cuh"], []),
     "recurrent": (["recurrent.cu"], ["common.cuh"], []),
+    "gla_chunks": (["gla_chunks.cu"], ["common.cuh"], []),
     "moe": (["moe.cu"], ["common.cuh"], []),
     "stream": (["stream.cu"], ["common.cuh"], []),
     "qk_prepare": (["qk_prepare.cu"], ["common.cuh"], []),

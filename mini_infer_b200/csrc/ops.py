@@ -262,25 +262,27 @@ def _sig_recurrent(lib: ctypes.CDLL) -> None:
     lib.mi_rglru_scan.argtypes = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int,
                                   c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, ll, c_int,
                                   c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
-    lib.mi_rglru_scan_chunked.argtypes = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int,
-                                          c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, ll, c_int,
-                                          c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int,
-                                          c_int, c_int, c_void_p]
-    lib.mi_rglru_chunked_scratch.argtypes = [c_int, c_int, c_int]
-    lib.mi_rglru_chunked_scratch.restype = ll
+    lib.mi_rglru_scan_long.argtypes = lib.mi_rglru_scan.argtypes
     lib.mi_gla_scan.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                 c_void_p, ll, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]
+                                c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]
     lib.mi_mlstm_gates.argtypes = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, ll, ll, c_void_p,
                                    c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
     lib.mi_delta_scan.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                   c_int, c_float, c_float, c_void_p, ll, ll, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                   c_void_p]
-    lib.mi_gla_chunked_scratch.argtypes = [c_int, c_int, c_int, c_int, c_int]
-    lib.mi_gla_chunked_scratch.restype = ll
     lib.mi_headnorm_gate.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                      c_int, c_float, c_int, c_float, c_int, c_void_p, c_float, c_int, c_void_p]
+
+
+def _sig_gla_chunks(lib: ctypes.CDLL) -> None:
+    ll = ctypes.c_longlong
+    lib.mi_gla_chunks_scratch.argtypes = [c_int, c_int, c_int, c_int, c_int]
+    lib.mi_gla_chunks_scratch.restype = ll
+    lib.mi_gla_chunks.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
+                                  c_void_p, ll, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                  c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]
 
 
 def _sig_moe(lib: ctypes.CDLL) -> None:
@@ -387,6 +389,7 @@ _SIGNATURES = {
     "layernorm": _sig_layernorm,
     "rope_norm": _sig_rope_norm,
     "recurrent": _sig_recurrent,
+    "gla_chunks": _sig_gla_chunks,
     "moe": _sig_moe,
     "attention_tc": _sig_attention_tc,
     "gemm_tma": _sig_gemm_tma,
@@ -1498,7 +1501,7 @@ def _max_q_len(ctx) -> int:
     return 1 if ctx.decode_only else max(ctx.host_q_len)
 
 
-RGLRU_CHUNK = 64     # tokens per chunk of the chunked walk; portions up to this long are walked plainly
+RGLRU_LONG = 32      # portions up to this long are walked by one thread per channel
 
 
 def rglru_scan(gates: torch.Tensor, gate_bias_r: torch.Tensor, gate_bias_i: torch.Tensor, lam: torch.Tensor,
@@ -1528,21 +1531,15 @@ def rglru_scan(gates: torch.Tensor, gate_bias_r: torch.Tensor, gate_bias_i: torc
         raise KernelError("rglru: state row too short")
     lib = _lib("recurrent")
     longest = _max_q_len(ctx)
-    if u.dtype == torch.bfloat16 and longest > RGLRU_CHUNK:
-        # long portions: chunks side by side (the float32 path keeps the plain walk, whose sums do not
-        # depend on where a portion starts)
-        global launch_count
-        n_chunks = -(-longest // RGLRU_CHUNK)
-        scratch = torch.empty(lib.mi_rglru_chunked_scratch(ctx.n_requests, n_chunks, C), dtype=torch.float32,
-                              device=u.device)
-        rc = lib.mi_rglru_scan_chunked(_ptr(gates), M, bw, _ptr(gate_bias_r), _ptr(gate_bias_i), _ptr(lam),
-                                       float(decay_scale), _ptr(u), u.stride(0), _ptr(y), y.stride(0), _ptr(y_bias),
-                                       _ptr(x_in), x_in.stride(0), _ptr(x_in_bias), _ptr(state), stride, int(taps),
-                                       _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(out),
-                                       out.stride(0), ctx.n_requests, C, _ptr(scratch), n_chunks, RGLRU_CHUNK,
-                                       _code(u.dtype), _stream())
+    if u.dtype == torch.bfloat16 and longest > RGLRU_LONG:
+        # long portions: a channel's tokens side by side (the float32 path keeps the plain walk, whose sums do
+        # not depend on where a portion starts)
+        rc = lib.mi_rglru_scan_long(_ptr(gates), M, bw, _ptr(gate_bias_r), _ptr(gate_bias_i), _ptr(lam),
+                                    float(decay_scale), _ptr(u), u.stride(0), _ptr(y), y.stride(0), _ptr(y_bias),
+                                    _ptr(x_in), x_in.stride(0), _ptr(x_in_bias), _ptr(state), stride, int(taps),
+                                    _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(out),
+                                    out.stride(0), ctx.n_requests, C, _code(u.dtype), _stream())
         _finish(lib, rc, "rglru")
-        launch_count += 1
         return
     rc = lib.mi_rglru_scan(_ptr(gates), M, bw, _ptr(gate_bias_r), _ptr(gate_bias_i), _ptr(lam), float(decay_scale),
                            _ptr(u), u.stride(0), _ptr(y), y.stride(0), _ptr(y_bias), _ptr(x_in), x_in.stride(0),
@@ -1551,7 +1548,7 @@ def rglru_scan(gates: torch.Tensor, gate_bias_r: torch.Tensor, gate_bias_i: torc
     _finish(lib, rc, "rglru")
 
 
-GLA_CHUNK = 128      # tokens per chunk of the chunked walk of gated linear attention
+GLA_LONG = 32        # portions up to this long are walked token by token
 
 
 def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor | None, z_bias: torch.Tensor | None,
@@ -1592,24 +1589,29 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor 
     if stride < heads * dk * dvx:
         raise KernelError("gla: state row too short")
     o = torch.empty((M, heads * dvx), dtype=torch.float32, device=q.device)
-    lib = _lib("recurrent")
     longest = _max_q_len(ctx)
-    n_chunks, scratch = 1, None
-    if v.dtype == torch.bfloat16 and longest > GLA_CHUNK:
-        # long portions: chunks side by side, two launches (the float32 path keeps the plain walk, whose
-        # sums do not depend on where a portion starts)
+    if v.dtype == torch.bfloat16 and longest > GLA_LONG:
+        # long portions: chunks side by side as products (the float32 path keeps the plain walk, whose sums do not
+        # depend on where a portion starts)
         global launch_count
-        n_chunks = -(-longest // GLA_CHUNK)
-        scratch = torch.empty(lib.mi_gla_chunked_scratch(ctx.n_requests, n_chunks, heads, dk, dvx), dtype=torch.float32,
+        lib = _lib("gla_chunks")
+        n_chunks = -(-longest // lib.mi_gla_chunk_tokens())
+        scratch = torch.empty(lib.mi_gla_chunks_scratch(ctx.n_requests, n_chunks, heads, dk, dvx), dtype=torch.float32,
                               device=q.device)
-        launch_count += 1
+        rc = lib.mi_gla_chunks(_ptr(q), _ptr(k), q.stride(0), _code(q.dtype), _ptr(v), v.stride(0), _ptr(z),
+                               z.stride(0) if z is not None else 0, _ptr(z_bias), 1.0 / float(tau), float(q_scale),
+                               _ptr(state), stride, _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(o),
+                               o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(scratch), n_chunks, _ptr(head_decay),
+                               _ptr(tok_gates), 1 if extra_col else 0, _code(v.dtype), _stream())
+        _finish(lib, rc, "gla")
+        launch_count += 2
+        return o
+    lib = _lib("recurrent")
     rc = lib.mi_gla_scan(_ptr(q), _ptr(k), q.stride(0), _code(q.dtype), _ptr(v), v.stride(0), _ptr(z),
-                         z.stride(0) if z is not None else 0,
-                         _ptr(z_bias), 1.0 / float(tau),
-                         float(q_scale), _ptr(state), stride, _ptr(ctx.q_start), _ptr(ctx.q_len),
-                         _ptr(ctx.state_slot), _ptr(o), o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(scratch),
-                         n_chunks, GLA_CHUNK, _ptr(head_decay), _ptr(tok_gates), 1 if extra_col else 0,
-                         _code(v.dtype), _stream())
+                         z.stride(0) if z is not None else 0, _ptr(z_bias), 1.0 / float(tau), float(q_scale),
+                         _ptr(state), stride, _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(o),
+                         o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(head_decay), _ptr(tok_gates),
+                         1 if extra_col else 0, _code(v.dtype), _stream())
     _finish(lib, rc, "gla")
     return o
 

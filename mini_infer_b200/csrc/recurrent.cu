@@ -3,8 +3,8 @@
 // Every request of a step brings q_len[b] consecutive tokens (rows q_start[b] .. of the packed
 // activations) and owns row state_slot[b] of a state arena (fp32, zeroed when the request is
 // admitted).  All recurrences run in fp32, token by token in the order of the positions, so a
-// result never depends on how a prompt was cut into steps or on what else is in the batch (the
-// chunked walk of long bfloat16 portions folds whole chunks first, which moves the fp32 rounding).
+// result never depends on how a prompt was cut into steps or on what else is in the batch (long bfloat16
+// portions are taken in chunks, here and in gla_chunks.cu, which moves the fp32 rounding).
 //
 //   mi_causal_conv     per channel: out[t] = b + sum_j w[j] * in[t - (taps-1-j)], in = x + x_bias,
 //                      with the taps-1 inputs before the portion taken from the state (zeros before
@@ -73,6 +73,119 @@ __global__ void causal_conv_kernel(const T* __restrict__ x, int x_stride, const 
   }
 }
 
+// The same with two to four taps on whole 16-byte pieces: a thread keeps the last taps-1 inputs of its 4 or 8
+// channels in registers and walks `tile` tokens, so every input is read once per tile instead of once per tap
+// (2048 tokens of 12288 bfloat16 channels: 93 us element by element; DRAM floor 16 us).
+template <typename T>
+struct ConvPiece;
+template <>
+struct ConvPiece<float> {
+  static constexpr int N = 4;
+  static __device__ __forceinline__ void load(const float* p, float (&f)[4]) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+  }
+  static __device__ __forceinline__ void store(float* p, const float (&f)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+  }
+};
+template <>
+struct ConvPiece<bf16> {
+  static constexpr int N = 8;
+  static __device__ __forceinline__ void load(const bf16* p, float (&f)[8]) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+      f[2 * i] = x.x;
+      f[2 * i + 1] = x.y;
+    }
+  }
+  static __device__ __forceinline__ void store(bf16* p, const float (&f)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 x = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&x);
+    }
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+};
+
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128) causal_conv_pieces_kernel(
+    const T* __restrict__ x, int x_stride, const float* __restrict__ x_bias, const float* __restrict__ w,
+    const float* __restrict__ b, const float* __restrict__ state, long long state_stride,
+    const int* __restrict__ q_start, const int* __restrict__ q_len, const int* __restrict__ state_slot,
+    T* __restrict__ out, int out_stride, int C, int tile, int act) {
+  mi_pdl_enter();
+  constexpr int N = ConvPiece<T>::N;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * N;
+  const int req = blockIdx.z, t0 = blockIdx.y * tile;
+  const int len = q_len[req];
+  if (c >= C || t0 >= len) return;
+  const int row0 = q_start[req];
+  const float* tail = state + (size_t)state_slot[req] * state_stride;
+  float wv[TAPS][N], xb[N], bias[N], in[TAPS][N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    xb[i] = x_bias ? x_bias[c + i] : 0.f;
+    bias[i] = b ? b[c + i] : 0.f;
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) wv[j][i] = w[(size_t)(c + i) * TAPS + j];
+  }
+#pragma unroll
+  for (int j = 0; j < TAPS - 1; ++j) {
+    const int src = t0 - (TAPS - 1) + j;
+    if (src >= 0) {
+      ConvPiece<T>::load(x + (size_t)(row0 + src) * x_stride + c, in[j]);
+#pragma unroll
+      for (int i = 0; i < N; ++i) in[j][i] += xb[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) in[j][i] = tail[(size_t)(TAPS - 1 + src) * C + c + i];
+    }
+  }
+  const int t1 = min(len, t0 + tile);
+#pragma unroll 4
+  for (int t = t0; t < t1; ++t) {
+    ConvPiece<T>::load(x + (size_t)(row0 + t) * x_stride + c, in[TAPS - 1]);
+    float acc[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      in[TAPS - 1][i] += xb[i];
+      acc[i] = bias[i];
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) acc[i] = fmaf(wv[j][i], in[j][i], acc[i]);
+      if (act == 1) acc[i] = acc[i] / (1.f + expf(-acc[i]));   // SiLU
+#pragma unroll
+      for (int j = 0; j < TAPS - 1; ++j) in[j][i] = in[j + 1][i];
+    }
+    ConvPiece<T>::store(out + (size_t)(row0 + t) * out_stride + c, acc);
+  }
+}
+
+template <typename T>
+static bool conv_in_pieces(const T* x, int x_stride, const float* x_bias, const float* w, const float* b,
+                           const float* state, long long state_stride, const int* q_start, const int* q_len,
+                           const int* state_slot, T* out, int out_stride, int n_requests, int max_q_len, int C, int taps,
+                           int act, cudaStream_t stream) {
+  constexpr int N = ConvPiece<T>::N;
+  if (taps < 2 || taps > 4 || C % N || x_stride % N || out_stride % N || !mi_aligned(x, 16) || !mi_aligned(out, 16)) return false;
+  const int tile = max_q_len >= 16 ? 16 : max_q_len;
+  dim3 grid((C / N + 127) / 128, (max_q_len + tile - 1) / tile, n_requests);
+  if (grid.y > 65535 || grid.z > 65535) return false;
+#define MI_GO(TAPS)                                                                                                    \
+  MI_LAUNCH((causal_conv_pieces_kernel<T, TAPS>), grid, 128, 0, stream, x, x_stride, x_bias, w, b, state, state_stride, \
+            q_start, q_len, state_slot, out, out_stride, C, tile, act)
+  if (taps == 2) MI_GO(2);
+  else if (taps == 3) MI_GO(3);
+  else MI_GO(4);
+#undef MI_GO
+  return true;
+}
+
 extern "C" int mi_causal_conv(const void* x, int x_stride, const float* x_bias, const float* w, const float* b,
                               const float* state, long long state_stride, const int* q_start, const int* q_len,
                               const int* state_slot, void* out, int out_stride, int n_requests, int max_q_len,
@@ -80,6 +193,13 @@ extern "C" int mi_causal_conv(const void* x, int x_stride, const float* x_bias, 
   if (n_requests <= 0 || max_q_len <= 0) return 0;
   if (act != 0 && act != 1) MI_REFUSE("causal_conv: unknown activation %d", act);
   if (taps < 1 || taps > MAX_TAPS) MI_REFUSE("causal_conv: %d taps (1 to %d are taken)", taps, MAX_TAPS);
+  if (dtype == MI_DTYPE_F32
+          ? conv_in_pieces((const float*)x, x_stride, x_bias, w, b, state, state_stride, q_start, q_len, state_slot,
+                           (float*)out, out_stride, n_requests, max_q_len, C, taps, act, stream)
+          : dtype == MI_DTYPE_BF16 &&
+                conv_in_pieces((const bf16*)x, x_stride, x_bias, w, b, state, state_stride, q_start, q_len, state_slot,
+                               (bf16*)out, out_stride, n_requests, max_q_len, C, taps, act, stream))
+    MI_RETURN_LAUNCH_STATUS();
   const int tile = 16;
   dim3 grid((C + 127) / 128, (max_q_len + tile - 1) / tile, n_requests);
   if (grid.y > 65535 || grid.z > 65535) MI_REFUSE("causal_conv: too many tiles for one launch");
@@ -183,11 +303,13 @@ extern "C" int mi_rglru_scan(const float* gates, int M, int bw, const float* br,
 }
 
 // ------------------------------------------------------------------------------------------
-// The same recurrence for long portions, cut into chunks of `chunk` tokens that run side by side.
-// Pass 1: every (request, chunk, channel) folds its chunk into S_end = A * S_begin + B.  Pass 2: it
-// walks the chunks before its own to get S_begin (from the state as pass 1 saved it), then its own
-// tokens exactly as the walk above does.  The last chunk stores the state and the convolution's tail.
-// scratch: [requests][max_chunks][2][C] chunk summaries, then [requests][C] the states at the start.
+// The same recurrence for long portions.  A block owns 16 channels of a request and takes its tokens 256 at a time: 32
+// threads per channel hold eight tokens' (a, b) each in registers and fold them into S_end = A S_begin + B, a warp per
+// channel scans the 32 folds, and every thread walks its eight tokens from the state it then knows.  (Blocks of twice the
+// threads leave room for one per SM: 160 blocks of 2560 channels then run in two turns.)  What bounds it is
+// the arithmetic of the gates (five exponentials, two divisions, a root per token and channel), which is done
+// once; two passes of one thread per 64 tokens did it twice and stood still for their loads (2048 tokens of 2560
+// channels: 60 + 90 us).
 // ------------------------------------------------------------------------------------------
 struct RglruTerms { float a, b; };
 
@@ -202,57 +324,87 @@ __device__ __forceinline__ RglruTerms rglru_terms(const float* g, int bw, float 
   return t;
 }
 
-template <typename T, int PASS>
-__global__ void rglru_chunk_kernel(const float* __restrict__ gates, int M, int bw,
-                                   const float* __restrict__ br, const float* __restrict__ bi,
-                                   const float* __restrict__ lam, float decay_scale,
-                                   const T* __restrict__ u, int u_stride,
-                                   const T* __restrict__ y, int y_stride, const float* __restrict__ y_bias,
-                                   const T* __restrict__ xin, int xin_stride, const float* __restrict__ xin_bias,
-                                   float* __restrict__ state, long long state_stride, int taps,
-                                   const int* __restrict__ q_start, const int* __restrict__ q_len,
-                                   const int* __restrict__ state_slot, T* __restrict__ out, int out_stride, int C,
-                                   float* __restrict__ scratch, int max_chunks, int chunk, int n_requests) {
+#define RU_CH 16       // channels per block: 64 bytes of a row of gates
+#define RU_SEG 32      // threads per channel: the lanes of the warp that scans their folds
+#define RU_TOK 8       // tokens per thread and round
+#define RU_THREADS (RU_CH * RU_SEG)
+
+template <typename T>
+__global__ void __launch_bounds__(RU_THREADS, 2)
+rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* __restrict__ br, const float* __restrict__ bi,
+                  const float* __restrict__ lam, float decay_scale, const T* __restrict__ u, int u_stride,
+                  const T* __restrict__ y, int y_stride, const float* __restrict__ y_bias,
+                  const T* __restrict__ xin, int xin_stride, const float* __restrict__ xin_bias,
+                  float* __restrict__ state, long long state_stride, int taps, const int* __restrict__ q_start,
+                  const int* __restrict__ q_len, const int* __restrict__ state_slot, T* __restrict__ out, int out_stride,
+                  int C) {
   mi_pdl_enter();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ci = blockIdx.y, req = blockIdx.z;
-  if (c >= C) return;
+  __shared__ float fold_a[RU_SEG][RU_CH + 1], fold_b[RU_SEG][RU_CH + 1];   // then: the state a thread begins with (b)
+  __shared__ float carry[RU_CH];
+  const int tid = threadIdx.x, cl = tid % RU_CH, seg = tid / RU_CH, c = blockIdx.x * RU_CH + cl, req = blockIdx.y;
   const int len = q_len[req], row0 = q_start[req];
-  const int t0 = ci * chunk;
-  if (t0 >= len) return;
-  const int t1 = min(len, t0 + chunk);
+  const bool in = c < C;
   float* st = state + (size_t)state_slot[req] * state_stride;
-  float* summ = scratch + ((size_t)req * max_chunks) * 2 * C;
-  float* start = scratch + (size_t)n_requests * max_chunks * 2 * C + (size_t)req * C;
-  const int blk = c / bw, cj = c - blk * bw;
-  const float* g = gates + ((size_t)blk * M + row0 + t0) * (2 * bw) + cj;
-  const float vbr = br[c], vbi = bi[c];
-  const float sp = decay_scale * mi_softplus(lam[c]);
-  if (PASS == 1) {
-    float A = 1.f, B = 0.f;
-#pragma unroll 4
-    for (int t = t0; t < t1; ++t, g += 2 * bw) {
-      const RglruTerms k = rglru_terms(g, bw, vbr, vbi, sp, u, (size_t)(row0 + t), u_stride, c);
-      B = fmaf(k.a, B, k.b);
-      A *= k.a;
+  const int blk = in ? c / bw : 0, cj = c - blk * bw;
+  const float* g = gates + ((size_t)blk * M + row0) * (2 * bw) + cj;
+  const float vbr = in ? br[c] : 0.f, vbi = in ? bi[c] : 0.f, yb = in && y_bias ? y_bias[c] : 0.f;
+  const float sp = in ? decay_scale * mi_softplus(lam[c]) : 0.f;
+  if (seg == 0) carry[cl] = in ? st[(size_t)(taps - 1) * C + c] : 0.f;
+  for (int t0 = 0; t0 < len; t0 += RU_SEG * RU_TOK) {
+    const int first = t0 + seg * RU_TOK;
+    RglruTerms k[RU_TOK];
+    float yv[RU_TOK];
+#pragma unroll
+    for (int i = 0; i < RU_TOK; ++i) {
+      const int t = first + i;
+      k[i].a = 1.f;
+      k[i].b = 0.f;
+      yv[i] = 0.f;
+      if (in && t < len) {
+        k[i] = rglru_terms(g + (size_t)t * (2 * bw), bw, vbr, vbi, sp, u, (size_t)(row0 + t), u_stride, c);
+        yv[i] = mi_to_float(y[(size_t)(row0 + t) * y_stride + c]);
+      }
     }
-    summ[((size_t)ci * 2) * C + c] = A;
-    summ[((size_t)ci * 2 + 1) * C + c] = B;
-    if (ci == 0) start[c] = st[(size_t)(taps - 1) * C + c];
-    return;
+    float A = 1.f, B = 0.f;
+#pragma unroll
+    for (int i = 0; i < RU_TOK; ++i) {
+      B = fmaf(k[i].a, B, k[i].b);
+      A *= k[i].a;
+    }
+    fold_a[seg][cl] = A;
+    fold_b[seg][cl] = B;
+    __syncthreads();
+    // warp w, lane l: fold l of channel w
+    const int warp = tid >> 5, lane = tid & 31;
+    if (warp < RU_CH) {
+      float sa = fold_a[lane][warp], sb = fold_b[lane][warp];      // then: all folds up to here as one
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const float pa = __shfl_up_sync(0xffffffffu, sa, off), pb = __shfl_up_sync(0xffffffffu, sb, off);
+        if (lane >= off) {
+          sb = fmaf(sa, pb, sb);
+          sa *= pa;
+        }
+      }
+      const float S0 = carry[warp];
+      const float end = fmaf(sa, S0, sb);                 // the state behind this lane's fold
+      const float before = __shfl_up_sync(0xffffffffu, end, 1);
+      fold_b[lane][warp] = lane ? before : S0;
+      __syncwarp();
+      if (lane == 31) carry[warp] = end;
+    }
+    __syncthreads();
+    float S = fold_b[seg][cl];
+#pragma unroll
+    for (int i = 0; i < RU_TOK; ++i) {
+      const int t = first + i;
+      S = fmaf(k[i].a, S, k[i].b);
+      if (in && t < len) out[(size_t)(row0 + t) * out_stride + c] = mi_from_float<T>(S * mi_gelu_tanh(yv[i] + yb));
+    }
+    __syncthreads();                                      // the folds are read before the next round's
   }
-  float S = start[c];
-  for (int p = 0; p < ci; ++p) S = fmaf(summ[((size_t)p * 2) * C + c], S, summ[((size_t)p * 2 + 1) * C + c]);
-  const float yb = y_bias ? y_bias[c] : 0.f;
-#pragma unroll 4
-  for (int t = t0; t < t1; ++t, g += 2 * bw) {
-    const RglruTerms k = rglru_terms(g, bw, vbr, vbi, sp, u, (size_t)(row0 + t), u_stride, c);
-    S = fmaf(k.a, S, k.b);
-    const float yv = mi_gelu_tanh(mi_to_float(y[(size_t)(row0 + t) * y_stride + c]) + yb);
-    out[(size_t)(row0 + t) * out_stride + c] = mi_from_float<T>(S * yv);
-  }
-  if (t1 < len) return;
-  st[(size_t)(taps - 1) * C + c] = S;
+  if (seg != 0 || !in) return;
+  st[(size_t)(taps - 1) * C + c] = carry[cl];
   if (taps > 1) {
     const float xb = xin_bias ? xin_bias[c] : 0.f;
     float keep[MAX_TAPS];
@@ -270,36 +422,21 @@ __global__ void rglru_chunk_kernel(const float* __restrict__ gates, int M, int b
   }
 }
 
-extern "C" long long mi_rglru_chunked_scratch(int n_requests, int max_chunks, int C) {
-  return ((long long)n_requests * max_chunks * 2 + n_requests) * C;
-}
-
-extern "C" int mi_rglru_scan_chunked(const float* gates, int M, int bw, const float* br, const float* bi,
-                                     const float* lam, float decay_scale, const void* u, int u_stride, const void* y,
-                                     int y_stride, const float* y_bias, const void* xin, int xin_stride,
-                                     const float* xin_bias, float* state, long long state_stride, int taps,
-                                     const int* q_start, const int* q_len, const int* state_slot, void* out,
-                                     int out_stride, int n_requests, int C, float* scratch, int max_chunks, int chunk,
-                                     int dtype, cudaStream_t stream) {
-  if (n_requests <= 0 || max_chunks <= 0) return 0;
+extern "C" int mi_rglru_scan_long(const float* gates, int M, int bw, const float* br, const float* bi,
+                                  const float* lam, float decay_scale, const void* u, int u_stride, const void* y,
+                                  int y_stride, const float* y_bias, const void* xin, int xin_stride,
+                                  const float* xin_bias, float* state, long long state_stride, int taps,
+                                  const int* q_start, const int* q_len, const int* state_slot, void* out,
+                                  int out_stride, int n_requests, int C, int dtype, cudaStream_t stream) {
+  if (n_requests <= 0) return 0;
   if (taps < 1 || taps > MAX_TAPS) MI_REFUSE("rglru: %d taps (1 to %d are taken)", taps, MAX_TAPS);
   if (bw <= 0 || C % bw) MI_REFUSE("rglru: %d channels are no whole number of blocks of %d", C, bw);
-  if (chunk <= 0 || max_chunks > 65535 || n_requests > 65535) MI_REFUSE("rglru: too many chunks or requests for one launch");
-  dim3 grid((C + 127) / 128, max_chunks, n_requests);
-#define MI_GO(T, PASS)                                                                                               \
-  MI_LAUNCH((rglru_chunk_kernel<T, PASS>), grid, 128, 0, stream, gates, M, bw, br, bi, lam, decay_scale, (const T*)u, \
-            u_stride, (const T*)y, y_stride, y_bias, (const T*)xin, xin_stride, xin_bias, state, state_stride, taps,   \
-            q_start, q_len, state_slot, (T*)out, out_stride, C, scratch, max_chunks, chunk, n_requests)
-  if (dtype == MI_DTYPE_F32) {
-    MI_GO(float, 1);
-    MI_GO(float, 2);
-  } else if (dtype == MI_DTYPE_BF16) {
-    MI_GO(bf16, 1);
-    MI_GO(bf16, 2);
-  } else {
-    MI_REFUSE("rglru: unknown dtype %d", dtype);
-  }
-#undef MI_GO
+  if (n_requests > 65535) MI_REFUSE("rglru: too many requests for one launch");
+  if (dtype != MI_DTYPE_BF16) MI_REFUSE("rglru: long portions are taken in bfloat16 only, got dtype %d", dtype);
+  dim3 grid((C + RU_CH - 1) / RU_CH, n_requests);
+  MI_LAUNCH((rglru_long_kernel<bf16>), grid, RU_THREADS, 0, stream, gates, M, bw, br, bi, lam, decay_scale, (const bf16*)u,
+            u_stride, (const bf16*)y, y_stride, y_bias, (const bf16*)xin, xin_stride, xin_bias, state, state_stride, taps,
+            q_start, q_len, state_slot, (bf16*)out, out_stride, C);
   MI_RETURN_LAUNCH_STATUS();
 }
 
@@ -320,19 +457,13 @@ __global__ void __launch_bounds__(MAXT) gla_scan_kernel(const TQ* __restrict__ q
                                 float inv_tau, float q_scale, float* __restrict__ state, long long state_stride,
                                 const int* __restrict__ q_start, const int* __restrict__ q_len,
                                 const int* __restrict__ state_slot, float* __restrict__ o, int o_stride,
-                                int heads, int dk, int dv, int pass, int chunk_len, int n_chunks,
-                                float* __restrict__ scratch, const float* __restrict__ head_decay,
+                                int heads, int dk, int dv, const float* __restrict__ head_decay,
                                 const float* __restrict__ tok_gates, int extra_col) {
   // head_decay [heads]: one fixed decay per head in the place of alpha (z is then not read).
   // tok_gates [M, heads, 3]: per token and head the decay (all key channels alike) and a factor on k
   // (z and head_decay are then not read).  extra_col: the head has dv + 1 value columns, the last one
   // all ones, in the state and in o alike (dv below counts it; v has one column less).
   // q and k may be fp32 rows of their own (what a rotation left in fp32) beside bfloat16 values.
-  // pass 0: the whole portion, from and into the state.  Long portions run as chunks side by side:
-  // pass 1 folds every chunk into (A, B) with S_end = diag(A) S_begin + B (and saves the state the
-  // portion starts from), pass 2 walks the chunks before its own to get S_begin and then its own
-  // tokens as pass 0 does; the last chunk stores the state.
-  // scratch: per (request, chunk, head) A [dk] and B [dk, dv]; then per (request, head) the state at the start.
   mi_pdl_enter();
   extern __shared__ float sm[];
   const int KP = blockDim.y;
@@ -342,38 +473,16 @@ __global__ void __launch_bounds__(MAXT) gla_scan_kernel(const TQ* __restrict__ q
   float* vs = as + GLA_L * dk;          // [GLA_L][32]
   float* part = vs + GLA_L * 32;        // [GLA_L][KP][32]
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx, nthreads = KP * 32;
-  const int head = blockIdx.y, req = blockIdx.z / n_chunks, chunk = blockIdx.z - req * n_chunks;
+  const int head = blockIdx.y, req = blockIdx.z;
   const int j = blockIdx.x * 32 + tx;   // value column
   const int dv_in = dv - extra_col;     // columns that v brings
-  const int len_all = q_len[req];
-  const int c0 = pass ? chunk * chunk_len : 0;
-  if (c0 >= len_all) return;
-  const int len = (pass ? min(len_all, c0 + chunk_len) : len_all) - c0, row0 = q_start[req] + c0;
-  const bool last = c0 + len == len_all;
+  const int len = q_len[req], row0 = q_start[req];
   float* S = state + (size_t)state_slot[req] * state_stride + (size_t)head * dk * dv;
-  const size_t unit = (size_t)dk + (size_t)dk * dv;
-  const int n_req = gridDim.z / n_chunks;
-  float* summ = scratch ? scratch + (((size_t)req * n_chunks + chunk) * heads + head) * unit : nullptr;
-  float* begin = scratch ? scratch + (size_t)n_req * n_chunks * heads * unit + ((size_t)req * heads + head) * dk * dv
-                         : nullptr;
-  float s[GLA_R], pa[GLA_R];
+  float s[GLA_R];
 #pragma unroll
   for (int i = 0; i < GLA_R; ++i) {
     const int kk = ty * GLA_R + i;
-    const bool mine = kk < dk && j < dv;
-    pa[i] = 1.f;
-    if (pass == 0) {
-      s[i] = mine ? S[(size_t)kk * dv + j] : 0.f;
-    } else if (pass == 1) {
-      s[i] = 0.f;
-      if (chunk == 0 && mine) begin[(size_t)kk * dv + j] = S[(size_t)kk * dv + j];
-    } else {
-      s[i] = mine ? begin[(size_t)kk * dv + j] : 0.f;
-      for (int p = 0; p < chunk; ++p) {
-        const float* ps = scratch + (((size_t)req * n_chunks + p) * heads + head) * unit;
-        if (mine) s[i] = fmaf(ps[kk], s[i], ps[dk + (size_t)kk * dv + j]);
-      }
-    }
+    s[i] = (kk < dk && j < dv) ? S[(size_t)kk * dv + j] : 0.f;
   }
   // A group's q, k, z and v are fetched into registers while the group before is worked on, so that
   // the walk does not stand still for a round trip to memory at every group.
@@ -441,14 +550,13 @@ __global__ void __launch_bounds__(MAXT) gla_scan_kernel(const TQ* __restrict__ q
         if (kk < dk) {
           const float al = as[l * dk + kk];
           s[i] = fmaf(al, s[i], ks[l * dk + kk] * vv);
-          if (pass == 1) pa[i] *= al;
-          else po = fmaf(s[i], qs[l * dk + kk], po);
+          po = fmaf(s[i], qs[l * dk + kk], po);
         }
       }
-      if (pass != 1) part[(l * KP + ty) * 32 + tx] = po;
+      part[(l * KP + ty) * 32 + tx] = po;
     }
     __syncthreads();
-    if (pass != 1) for (int l = ty; l < n; l += KP) {
+    for (int l = ty; l < n; l += KP) {
       float sum = 0.f;
       for (int p = 0; p < KP; ++p) sum += part[(l * KP + p) * 32 + tx];
       if (j < dv) o[(size_t)(row0 + t0 + l) * o_stride + head * dv + j] = sum;
@@ -457,39 +565,25 @@ __global__ void __launch_bounds__(MAXT) gla_scan_kernel(const TQ* __restrict__ q
 #pragma unroll
   for (int i = 0; i < GLA_R; ++i) {
     const int kk = ty * GLA_R + i;
-    if (pass == 1) {
-      if (kk < dk && j < dv) summ[dk + (size_t)kk * dv + j] = s[i];
-      if (kk < dk && j == 0) summ[kk] = pa[i];
-      continue;
-    }
-    if (!last) continue;
     if (kk < dk && j < dv) S[(size_t)kk * dv + j] = s[i];
   }
-}
-
-extern "C" long long mi_gla_chunked_scratch(int n_requests, int n_chunks, int heads, int dk, int dv) {
-  const long long unit = (long long)dk + (long long)dk * dv;
-  return (long long)n_requests * n_chunks * heads * unit + (long long)n_requests * heads * dk * dv;
 }
 
 extern "C" int mi_gla_scan(const void* q, const void* k, int qk_stride, int qk_dtype, const void* v, int stride,
                            const float* z, int z_stride,
                            const float* z_bias, float inv_tau, float q_scale, float* state, long long state_stride,
                            const int* q_start, const int* q_len, const int* state_slot, float* o, int o_stride,
-                           int n_requests, int heads, int dk, int dv, float* scratch, int n_chunks, int chunk_len,
-                           const float* head_decay, const float* tok_gates, int extra_col, int dtype,
-                           cudaStream_t stream) {
+                           int n_requests, int heads, int dk, int dv, const float* head_decay, const float* tok_gates,
+                           int extra_col, int dtype, cudaStream_t stream) {
   // dv counts the value columns of the state and of o; with extra_col v brings one less
   if (n_requests <= 0) return 0;
   if (!z && !head_decay && !tok_gates) MI_REFUSE("gla: neither decays per channel nor per head nor per token");
   if (extra_col != 0 && extra_col != 1) MI_REFUSE("gla: one extra column or none");
   if (dv - extra_col <= 0) MI_REFUSE("gla: no value columns");
-  if (n_chunks < 1 || (n_chunks > 1 && (!scratch || chunk_len <= 0))) MI_REFUSE("gla: chunks need scratch memory");
-  if ((long long)n_requests * n_chunks > 65535) MI_REFUSE("gla: too many chunks for one launch");
   if (dk <= 0 || dk > 256 || dv <= 0) MI_REFUSE("gla: key size %d must lie in [1, 256], value size %d above 0", dk, dv);
   if (heads > 65535 || n_requests > 65535) MI_REFUSE("gla: too many heads or requests for one launch");
   const int KP = max(4, (dk + GLA_R - 1) / GLA_R);     // at least 128 threads: they also stage the inputs
-  dim3 grid((dv + 31) / 32, heads, n_requests * n_chunks), block(32, KP);
+  dim3 grid((dv + 31) / 32, heads, n_requests), block(32, KP);
   const size_t smem = ((size_t)3 * GLA_L * dk + GLA_L * 32 + (size_t)GLA_L * KP * 32) * sizeof(float);
 #define MI_GO(TQ, T)                                                                                      \
   do {                                                                                                    \
@@ -498,10 +592,9 @@ extern "C" int mi_gla_scan(const void* q, const void* k, int qk_stride, int qk_d
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) return (int)e;                                                                \
     }                                                                                                     \
-    for (int pass = n_chunks > 1 ? 1 : 0; pass <= (n_chunks > 1 ? 2 : 0); ++pass)                         \
-      MI_LAUNCH(kern, grid, block, smem, stream, (const TQ*)q, (const TQ*)k, qk_stride, (const T*)v, stride, z, z_stride, \
-                z_bias, inv_tau, q_scale, state, state_stride, q_start, q_len, state_slot, o, o_stride, heads, \
-                dk, dv, pass, chunk_len, n_chunks, scratch, head_decay, tok_gates, extra_col);              \
+    MI_LAUNCH(kern, grid, block, smem, stream, (const TQ*)q, (const TQ*)k, qk_stride, (const T*)v, stride, z, z_stride, \
+              z_bias, inv_tau, q_scale, state, state_stride, q_start, q_len, state_slot, o, o_stride, heads,  \
+              dk, dv, head_decay, tok_gates, extra_col);                                                      \
   } while (0)
   if (dtype == MI_DTYPE_F32 && qk_dtype == MI_DTYPE_F32) MI_GO(float, float);
   else if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_BF16) MI_GO(bf16, bf16);

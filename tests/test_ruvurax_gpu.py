@@ -344,6 +344,83 @@ def test_gated_linear_attention_state(heads, dk, dv, dtype, portions):
     assert (out.cpu().double() - ref).abs().max() <= 1e-5 * max(1.0, ref.abs().max())
 
 
+@pytest.mark.parametrize("heads,dk,dv,portions", [(2, 128, 128, (64, 33, 65)), (1, 130, 129, (200,)), (2, 16, 8, (127, 1, 128)),
+                                                  (1, 256, 40, (70, 64))])
+@pytest.mark.parametrize("decays", ["slow", "steep", "dead", "head"])
+def test_linear_attention_in_chunks(heads, dk, dv, portions, decays):
+    """Portions taken as products per 64 tokens at the edges of the chunks and of the 128-wide tiles, with decays that stay
+    near 1, that fall by e^-100 within a chunk, that are exactly 0 now and then, and one per head, against the token loop
+    in float64.  The error of a sum of products in fp32 is bounded by the number of roundings on the way (64 within a
+    chunk, dk + 64 for the sums, a few per chunk) times 2^-24 of the sum of the terms' magnitudes."""
+    Tn = sum(portions)
+    q, k, v = rnd(Tn, heads * dk, seed=70).bfloat16(), rnd(Tn, heads * dk, seed=71).bfloat16(), rnd(Tn, heads * dv, seed=72).bfloat16()
+    z = rnd(Tn, heads * dk, seed=73, scale={"slow": 1.0, "steep": 12.0, "dead": 1.0, "head": 1.0}[decays])
+    if decays == "dead":
+        z[::7] = -1e4
+    per_head = torch.tensor([0.97, 0.2][:heads]) if decays == "head" else None
+    alpha = torch.sigmoid(z.double()).reshape(Tn, heads, dk) if per_head is None else per_head.double()[None, :, None].expand(Tn, heads, dk)
+    S = torch.zeros(heads, dk, dv, dtype=torch.float64)
+    size, want, terms = S.clone(), torch.empty(Tn, heads, dv, dtype=torch.float64), torch.empty(Tn, heads, dv, dtype=torch.float64)
+    for t in range(Tn):
+        qt, kt, vt = (x[t].double().reshape(heads, -1) for x in (q, k, v))
+        S = alpha[t][:, :, None] * S + kt[:, :, None] * vt[:, None, :]
+        size = alpha[t][:, :, None] * size + (kt[:, :, None] * vt[:, None, :]).abs()
+        want[t], terms[t] = torch.einsum("hkv,hk->hv", S, qt), torch.einsum("hkv,hk->hv", size, qt.abs())
+    state = torch.zeros(2, heads, dk, dv, device=DEV)
+    got, t0 = [], 0
+    for n in portions:
+        part = [x[t0:t0 + n].to(DEV) for x in (q, k, v)]
+        got.append(ops().gla_scan(*part, None if per_head is not None else z[t0:t0 + n].to(DEV).contiguous(), None, 1.0, 1.0,
+                                  heads, dk, dv, state, ctx_for([n], [1]),
+                                  head_decay=per_head.to(DEV) if per_head is not None else None).cpu().double())
+        t0 += n
+    rounds = 64 + (dk + 64) + 4 * (Tn // 64 + 1)
+    assert ((torch.cat(got).reshape(Tn, heads, dv) - want).abs() <= rounds * 2.0 ** -24 * terms + 1e-30).all()
+    assert ((state[1].cpu().double() - S).abs() <= rounds * 2.0 ** -24 * size + 1e-30).all()
+
+
+@pytest.mark.parametrize("C,bw,taps,act,portions", [(48, 16, 4, "silu", (1, 2, 40, 33)), (40, 20, 3, None, (259,)), (24, 24, 2, None, (33, 256, 1)),
+                                                    (36, 12, 4, None, (600,)), (40, 8, 5, "silu", (40, 1))])
+def test_convolution_and_recurrent_unit_in_long_portions(C, bw, taps, act, portions):
+    """The convolution on whole 16-byte pieces (C a multiple of 8, two to four taps) and element by element, and the
+    unit's walk with 32 threads per channel at the edges of its rounds of 256 tokens, in bfloat16 against the plain
+    formulas in float64 on the same rounded inputs: results are off by their rounding to bfloat16, 2^-8 of themselves, and the
+    fp32 sums (the unit's state by 2^-20 of the largest)."""
+    Tn = sum(portions)
+    x, y = rnd(Tn, C, seed=80).bfloat16(), rnd(Tn, C, seed=81).bfloat16()
+    w, b, xb, lam, yb = rnd(C, taps, seed=82), rnd(C, seed=83), rnd(C, seed=84), rnd(C, seed=85), rnd(C, seed=86)
+    br, bi = rnd(C, seed=87), rnd(C, seed=88)
+    gates = rnd(C // bw, Tn, 2 * bw, seed=89)
+    state = torch.zeros(2, taps, C, device=DEV)
+    us, outs, t0 = [], [], 0
+    for n in portions:
+        ctx, xs = ctx_for([n], [1]), x[t0:t0 + n].to(DEV)
+        u = torch.empty(n, C, dtype=torch.bfloat16, device=DEV)
+        ops().causal_conv(xs, xb.to(DEV), w.to(DEV), b.to(DEV), state, ctx, u, act=act)
+        out = torch.empty(n, C, dtype=torch.bfloat16, device=DEV)
+        ops().rglru_scan(gates[:, t0:t0 + n].contiguous().to(DEV), br.to(DEV), bi.to(DEV), lam.to(DEV), 8.0, u,
+                         y[t0:t0 + n].to(DEV), yb.to(DEV), xs, xb.to(DEV), taps, state, ctx, out)
+        us.append(u.cpu().double())
+        outs.append(out.cpu().double())
+        t0 += n
+    u, out = torch.cat(us), torch.cat(outs)
+    want = P.causal_conv(x.double() + xb.double(), w.double(), b.double())
+    want = torch.nn.functional.silu(want) if act else want
+    assert ((u - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+    r = torch.sigmoid(torch.cat(list(gates[:, :, :bw].double()), dim=1) + br.double())
+    i = torch.sigmoid(torch.cat(list(gates[:, :, bw:].double()), dim=1) + bi.double())
+    log_a = -8.0 * r * torch.nn.functional.softplus(lam.double())
+    a, inp = log_a.exp(), torch.sqrt(-torch.expm1(2 * log_a)) * i * u
+    S, states = torch.zeros(C, dtype=torch.float64), []
+    for t in range(Tn):
+        S = a[t] * S + inp[t]
+        states.append(S)
+    ref = torch.stack(states) * P.gelu_tanh(y.double() + yb.double())
+    assert ((out - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
+    assert ((state[1, taps - 1].cpu().double() - S).abs() <= 2.0 ** -20 * torch.stack(states).abs().max()).all()
+    assert torch.equal(state[1, :taps - 1].cpu(), (x.float() + xb)[Tn - (taps - 1):])
+
+
 @pytest.mark.parametrize("E,top,ff,H,M", [(5, 2, 24, 40, 33), (3, 1, 20, 48, 5), (4, 4, 16, 36, 70), (12, 3, 72, 64, 200),
                                           (6, 2, 24, 40, 7), (3, 3, 16, 64, 8), (16, 1, 8, 264, 100)])
 @pytest.mark.parametrize("dtype,bound", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
