@@ -654,6 +654,12 @@ attention_decode_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restri
 // (units + G) * 8 * d floats, part_ml (units + G) * 8 * 2, counters one int per unit (zero
 // between calls).  No host-side plan: the blocks work the stretches out from kv_len themselves.
 
+// a / b for a >= 0, b > 0: a 64-bit division is a few hundred instructions, and hardly ever needed
+__device__ __forceinline__ long long balanced_div(long long a, long long b) {
+  if (((a | b) >> 31) == 0) return (long long)((uint32_t)a / (uint32_t)b);
+  return a / b;
+}
+
 // The row: request after request, each with U units of (ov + its chunks) positions; request b
 // starts at position (cum[b] + ov * b) * U.  The part of the row's stretch [i, i1) that lies in
 // the unit holding position i: request b, unit u within it, `seg` chunks from chunk c_rel of the
@@ -671,7 +677,7 @@ __device__ __forceinline__ int balanced_part(long long i, long long i1, const in
   n_b = cum[b + 1] - cum[b];
   const int nv = n_b + ov;
   const long long r = i - (long long)(cum[b] + ov * b) * U;
-  u = (int)(r / nv);
+  u = (int)balanced_div(r, nv);
   const int p = (int)(r - (long long)u * nv);
   const int len = (int)min((long long)(nv - p), i1 - i);
   const int first = max(p, ov);
@@ -680,76 +686,50 @@ __device__ __forceinline__ int balanced_part(long long i, long long i1, const in
   return len;
 }
 
-// The stretches g_first .. g_last of one unit into its output row (head r of the unit's group,
-// this thread's columns cgrp, cgrp + 16, ...), in block order.  Out of line: its many loads in
-// flight need registers that the main loop's accumulators would otherwise have to share.
-template <int DMAX>
+// Four columns (c4 ..) of one head's stretches g_first .. g_last into its output row, in block order.  Every stretch's
+// (max, sum) and columns are asked for eight stretches at a time before any of them is used: one round trip to the
+// L2 in the usual case.  Out of line and short: the code runs once per unit and comes from memory itself (72 scalar loads per
+// thread, all unrolled, took 2.7 to 5 us; `out` of a four-token group at 1024 tokens).
 __device__ __noinline__ void balanced_merge_unit(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                 int unit, int g_first, int g_last, int r, int cgrp, int d,
+                                                 int unit, int g_first, int g_last, int r, int c4, int d,
                                                  bf16* __restrict__ orow, float sink_l2) {
   // sink_l2: a score (times log2 e) that joins the denominator without a key or a value; minus infinity: none
-  const float2* ml = reinterpret_cast<const float2*>(part_ml);
-  float mm = -INFINITY, LL = 0.f, acc[DMAX / 16];
-#pragma unroll
-  for (int k = 0; k < DMAX / 16; ++k) acc[k] = 0.f;
-  if (g_last - g_first < 8 && DMAX <= 128) {
-    // Few stretches (the usual case): everything this thread needs is asked for before any of it
-    // is used, so the merge costs one round trip to the L2.
+  float mm = -INFINITY, L = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int gb = g_first; gb <= g_last; gb += 8) {
     float2 v[8];
-    float po[8][DMAX <= 128 ? DMAX / 16 : 1];
+    float4 o[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const bool live = g_first + k <= g_last;
-      const size_t slot = ((size_t)unit + g_first + k) * DEC_HEADS + r;
-      v[k] = live ? __ldcg(ml + slot) : make_float2(-INFINITY, 0.f);
-#pragma unroll
-      for (int c = 0; c < (DMAX <= 128 ? DMAX / 16 : 1); ++c)
-        po[k][c] = (live && cgrp + 16 * c < d) ? __ldcg(part_o + slot * d + cgrp + 16 * c) : 0.f;
+      const size_t slot = ((size_t)unit + min(gb + k, g_last)) * DEC_HEADS + r;
+      v[k] = __ldcg(reinterpret_cast<const float2*>(part_ml) + slot);
+      o[k] = __ldcg(reinterpret_cast<const float4*>(part_o + slot * d + c4));
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) mm = fmaxf(mm, v[k].x);
+    float m = mm;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const float fk = (v[k].x == -INFINITY) ? 0.f : exp2f(v[k].x - mm);
-      LL += v[k].y * fk;
-#pragma unroll
-      for (int c = 0; c < (DMAX <= 128 ? DMAX / 16 : 1); ++c) acc[c] += fk != 0.f ? fk * po[k][c] : 0.f;
+      if (gb + k > g_last) v[k] = make_float2(-INFINITY, 0.f);
+      m = fmaxf(m, v[k].x);
     }
-  } else {
-    for (int gb = g_first; gb <= g_last; gb += 8) {   // eight stretches' (max, sum) in flight at a time
-      float2 v[8];
+    const float keep = mm == -INFINITY ? 0.f : exp2f(mm - m);
+    L *= keep;
+    acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+    mm = m;
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        v[k] = gb + k <= g_last ? __ldcg(ml + ((size_t)unit + gb + k) * DEC_HEADS + r) : make_float2(-INFINITY, 0.f);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) mm = fmaxf(mm, v[k].x);
-    }
-    for (int gb = g_first; gb <= g_last; gb += 4) {   // four stretches' columns in flight at a time
-      float2 v[4];
-      float po[4][DMAX / 16];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const bool live = gb + k <= g_last;
-        const size_t slot = ((size_t)unit + gb + k) * DEC_HEADS + r;
-        v[k] = live ? __ldcg(ml + slot) : make_float2(-INFINITY, 0.f);
-#pragma unroll
-        for (int c = 0; c < DMAX / 16; ++c)
-          po[k][c] = (live && cgrp + 16 * c < d) ? __ldcg(part_o + slot * d + cgrp + 16 * c) : 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float fk = (v[k].x == -INFINITY) ? 0.f : exp2f(v[k].x - mm);
-        LL += v[k].y * fk;
-#pragma unroll
-        for (int c = 0; c < DMAX / 16; ++c) acc[c] += fk != 0.f ? fk * po[k][c] : 0.f;
-      }
+    for (int k = 0; k < 8; ++k) {
+      if (v[k].x == -INFINITY) continue;       // (a stretch without a visible key holds nothing)
+      const float f = exp2f(v[k].x - mm);
+      L = fmaf(v[k].y, f, L);
+      acc.x = fmaf(f, o[k].x, acc.x); acc.y = fmaf(f, o[k].y, acc.y);
+      acc.z = fmaf(f, o[k].z, acc.z); acc.w = fmaf(f, o[k].w, acc.w);
     }
   }
-  if (sink_l2 != -INFINITY && mm != -INFINITY) LL += exp2f(sink_l2 - mm);
-  const float inv = LL > 0.f ? 1.f / LL : 0.f;
-#pragma unroll
-  for (int c = 0; c < DMAX / 16; ++c)
-    if (cgrp + 16 * c < d) orow[cgrp + 16 * c] = __float2bfloat16_rn(acc[c] * inv);
+  if (sink_l2 != -INFINITY && mm != -INFINITY) L += exp2f(sink_l2 - mm);
+  const float inv = L > 0.f ? 1.f / L : 0.f;
+  uint32_t* dst = reinterpret_cast<uint32_t*>(orow + c4);
+  dst[0] = pack_bf16(acc.x * inv, acc.y * inv);
+  dst[1] = pack_bf16(acc.z * inv, acc.w * inv);
 }
 
 #define BAL_THREADS (NTHREADS + 64)   // four consumer warps, the copy warp, the store warp (ROPE only)
@@ -769,9 +749,9 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
   // sinks [nq] (optional): per head a score that joins the softmax's denominator with neither key nor value.
   // ROPE (the head size is then DMAX exactly): rope_cs holds per query token [d / 2] sines then
   // [d / 2] cosines of its rotary angles; q arrives un-rotated and is rotated here, in registers; and with store_kv
-  // the block that comes to a request's newest chunk first rotates the new key, writes it and
-  // the new value into their page (they follow q in the token's row: q heads, k heads, v heads)
-  // and only then copies the chunk.  One kernel and one kernel boundary less per layer.
+  // the block that reads a request's newest chunk rotates the new key, writes it and the new value into their page (they
+  // follow q in the token's row: q heads, k heads, v heads) and puts both into the chunk's copy in shared memory, which
+  // was fetched with whatever that row held before.  One kernel and one kernel boundary less per layer.
   mi_pdl_launch_dependents();   // (what this kernel may touch before it waits: see attention_decode_kernel)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* Ks = reinterpret_cast<bf16*>(smem_raw);                      // [DEC_STAGES][64][d]
@@ -780,7 +760,7 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
   int* cum = reinterpret_cast<int*>(merge_o + 4 * DEC_HEADS * d);    // [B + 1] chunks of the requests before b
   const int swz_mask = mi_swizzle_mask(d, 2);
   __shared__ float merge_m[4][DEC_HEADS], merge_l[4][DEC_HEADS];
-  __shared__ __align__(8) uint64_t bars[DEC_STAGES], empty[DEC_STAGES], stored;
+  __shared__ __align__(8) uint64_t bars[DEC_STAGES], empty[DEC_STAGES], reached, patched;
   __shared__ int is_last;
   __shared__ volatile int dead;   // a warp gave up waiting for a copy: everybody leaves at the next common point
 
@@ -823,19 +803,19 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
     const long long units = (long long)B * U, chunks = (long long)cum[B] * U;
     const int n0 = cum[1];
     // a stretch shorter than min_chunks costs more in set-up and merging than it spreads
-    const int g_plain = (int)min((long long)gridDim.x, max((long long)1, chunks / max(1, min_chunks)));
+    const int g_plain = (int)min((long long)gridDim.x, max((long long)1, balanced_div(chunks, max(1, min_chunks))));
     if (units < g_plain && chunks == units * n0) {
       ov = 0;
-      G = (int)(units * (g_plain / units));
+      G = (int)units * (g_plain / (int)units);
     } else {
-      G = (int)min((long long)gridDim.x, max((long long)1, (chunks + units * ov) / max(1, min_chunks)));
+      G = (int)min((long long)gridDim.x, max((long long)1, balanced_div(chunks + units * ov, max(1, min_chunks))));
     }
   }
   const long long W = (long long)(cum[B] + ov * B) * U;
   if (W == 0) G = 1;
   if ((int)blockIdx.x >= G) return;
   if (status && *reinterpret_cast<volatile int*>(status)) return;   // an earlier block gave up waiting
-  const long long i0 = W * blockIdx.x / G, i1 = W * (blockIdx.x + 1) / G;
+  const long long i0 = balanced_div(W * blockIdx.x, G), i1 = balanced_div(W * (blockIdx.x + 1), G);
 
   if (tid == 0) {
 #pragma unroll
@@ -843,16 +823,21 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
       mbar_init(&bars[i], 1);
       mbar_init(&empty[i], 4);
     }
-    mbar_init(&stored, 1);
+    mbar_init(&reached, 1);
+    mbar_init(&patched, 1);
     fence_mbar_init();
   }
   __syncthreads();
 
   if (warp == 4) {
-    // the copy warp: walks the stretch chunk by chunk and keeps the ring full
-    PageLoader loader;
+    // the copy warp: walks the stretch chunk by chunk and keeps the ring full.  A chunk's page ids are asked for while
+    // the chunk before it is under way (where a lane per piece is enough), so that refilling a stage does not begin
+    // with a round trip to the block table.
+    PageLoader loader, ahead;
     const int pieces = 2 * (KCHUNK / PageLoader::piece_rows(page_size, page_shift));
-    bool ok = true, waited = false, stored_seen = false;
+    const bool lane_each = pieces <= 32;
+    loader.t = ahead.t = lane;
+    bool ok = true, waited = false;
     int it = 0;
     for (long long i = i0; i < i1 && ok;) {
       int b, u, c_rel, seg, n_b;
@@ -862,30 +847,36 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
       const int lo_w = first_visible(kl - 1, window);
       const MiKeyWalk<EXT> walk(lo_w, keep, KCHUNK);
       const int* table = block_table + (size_t)(table_rows ? table_rows[b] : b) * bt_stride;
+      // a chunk with kept keys is copied from its beginning
+      auto low = [&](int c) { return EXT && c * KCHUNK < keep ? 0 : lo_w; };
+      if (lane_each && seg > 0) {
+        const int c = walk.chunk(c_rel);
+        ahead.fetch(table, page_size, page_shift, c, low(c), kl);
+      }
       for (int s = 0; s < seg && ok; ++s, ++it) {
         const int c = walk.chunk(c_rel + s), st = it % DEC_STAGES;
-        const int lo = EXT && c * KCHUNK < keep ? 0 : lo_w;     // a chunk with kept keys is copied from its beginning
+        const int lo = low(c);
+        loader.pg = ahead.pg;
+        if (lane_each && s + 1 < seg) {
+          const int next = walk.chunk(c_rel + s + 1);
+          ahead.fetch(table, page_size, page_shift, next, low(next), kl);
+        }
         if (it >= DEC_STAGES)
           ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[st], ((it / DEC_STAGES) - 1) & 1, status));
         if (!ok) break;
-        if ((c + 1) * KCHUNK >= kl) {   // the chunk with the newest position: written by this step
-          if (!waited) {
-            mi_pdl_wait();
-            waited = true;
-          }
-          if (ROPE && store_kv && !stored_seen) {
-            // the other warps have rotated and stored the newest keys and values of this block's requests
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&stored, 0, status));
-            if (!ok) break;
-            fence_proxy_async_all();
-            stored_seen = true;
-          }
+        // The chunk with the newest position, which this step writes: a kernel before this one does, or the store
+        // warp below, which then also puts it into shared memory behind this copy.
+        if (!(ROPE && store_kv) && !waited && (c + 1) * KCHUNK >= kl) {
+          mi_pdl_wait();
+          waited = true;
         }
         if (lane == 0) mbar_expect_tx(&bars[st], PageLoader::chunk_bytes(c, lo, kl, d, page_size, page_shift));
         __syncwarp();
         for (int t0 = 0; t0 < pieces; t0 += 32) {
-          loader.t = t0 + lane;
-          loader.fetch(table, page_size, page_shift, c, lo, kl);
+          if (!lane_each) {
+            loader.t = t0 + lane;
+            loader.fetch(table, page_size, page_shift, c, lo, kl);
+          }
           loader.issue<true>(Ks + st * KCHUNK * d, Vs + st * KCHUNK * d, kcache, vcache, page_size, page_shift, c, nkv, kvh,
                        d, &bars[st]);
         }
@@ -898,48 +889,65 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
   if (ROPE && warp == 5) {
     // The store warp (only when this kernel rotates and stores by itself): the newest key
     // (rotated) and value of every request whose last chunk this block reads go into their
-    // pages, beside the other warps' work and long before the copy warp gets there.  Blocks
+    // pages and, once the other warps have come to the chunk's copy, over the copy's row of that position.  Blocks
     // that read the same chunk (other head groups of the key/value head) write the same bytes.
     if (!store_kv) return;
     mi_pdl_wait();
     const int half = d >> 1, n_rot = half >> 3, cpr = d >> 3, per_unit = n_rot + cpr;
+    int it = 0, n_new = 0;
     for (long long i = i0; i < i1;) {
       int b, u, c_rel, seg, n_b;
       const int len = balanced_part(i, i1, cum, B, U, ov, b, u, c_rel, seg, n_b);
+      it += seg;
       if (seg > 0 && c_rel + seg == n_b) {
-        const int kvh = u / hblocks, kl = kv_len[b], tok = q_start[b], pos = kl - 1;
+        const int kvh = u / hblocks, kl = kv_len[b], tok = q_start[b], pos = kl - 1, st = (it - 1) % DEC_STAGES;
         const int* table = block_table + (size_t)(table_rows ? table_rows[b] : b) * bt_stride;
         const int page = table[page_shift >= 0 ? (pos >> page_shift) : (pos / page_size)];
         const int off = inpage_of(pos, page_size, page_shift), swz = off & swz_mask;
         const bf16* krow = q + (size_t)tok * q_stride + (size_t)(nq + kvh) * d;
         const bf16* vrow = krow + (size_t)nkv * d;
         const size_t row = (((size_t)page * nkv + kvh) * page_size + off) * d;
-        bf16* kdst = const_cast<bf16*>(kcache) + row;
-        bf16* vdst = const_cast<bf16*>(vcache) + row;
+        const size_t copy = ((size_t)st * KCHUNK + (pos & (KCHUNK - 1))) * d;
         const float* cs = rope_cs + (size_t)tok * d;
-        for (int item = lane; item < per_unit; item += 32) {
+        uint4 a, bb;
+        auto load = [&](int item) {        // 8 of a half's numbers and their partners, or 8 of the value's
           if (item < n_rot) {
-            uint4 a = *reinterpret_cast<const uint4*>(krow + item * 8);
-            uint4 bb = *reinterpret_cast<const uint4*>(krow + half + item * 8);
+            a = *reinterpret_cast<const uint4*>(krow + item * 8);
+            bb = *reinterpret_cast<const uint4*>(krow + half + item * 8);
             const float* sn = cs + item * 8;
             const float* cn = cs + half + item * 8;
             rotate_words(a.x, bb.x, sn + 0, cn + 0);
             rotate_words(a.y, bb.y, sn + 2, cn + 2);
             rotate_words(a.z, bb.z, sn + 4, cn + 4);
             rotate_words(a.w, bb.w, sn + 6, cn + 6);
+          } else if (item < per_unit) {
+            a = *reinterpret_cast<const uint4*>(vrow + (item - n_rot) * 8);
+          }
+        };
+        auto store = [&](int item, bf16* kdst, bf16* vdst) {
+          if (item < n_rot) {
             *reinterpret_cast<uint4*>(kdst + ((item ^ swz) << 3)) = a;
             *reinterpret_cast<uint4*>(kdst + (((n_rot + item) ^ swz) << 3)) = bb;
-          } else {
-            const int j = item - n_rot;
-            *reinterpret_cast<uint4*>(vdst + ((j ^ swz) << 3)) = *reinterpret_cast<const uint4*>(vrow + j * 8);
+          } else if (item < per_unit) {
+            *reinterpret_cast<uint4*>(vdst + (((item - n_rot) ^ swz) << 3)) = a;
           }
+        };
+        for (int item = lane; item < per_unit; item += 32) {
+          load(item);
+          store(item, const_cast<bf16*>(kcache) + row, const_cast<bf16*>(vcache) + row);
         }
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&reached, n_new & 1, status))) return;
+        ++n_new;
+        for (int item = lane; item < per_unit; item += 32) {
+          if (per_unit > 32) load(item);     // (else the one turn's numbers are still there)
+          store(item, Ks + copy, Vs + copy);
+        }
+        fence_proxy_async();   // these writes come before the copy engine's next writes to the stage
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&patched);
       }
       i += len;
     }
-    fence_proxy_async_all();   // a bulk copy reads these plain stores next
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&stored);
     return;
   }
 
@@ -948,8 +956,8 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
   const float sc = scale * LOG2E;
   const int src0 = (2 * t4) * 4 + (qd >> 1), src1 = (2 * t4 + 1) * 4 + (qd >> 1);
   const bool odd_head = qd & 1;
-  const int r = tid >> 4, cgrp = tid & 15;   // the merges' layout: 8 heads x 16 threads
   int it = 0;
+  int n_new = 0;     // newest chunks so far: the phase of `reached` and `patched`
   bool warp_dead = false;   // this warp's wait ran out: it keeps in step with the others but computes nothing more
   for (long long i = i0; i < i1;) {
     int b, u, c_rel, seg, n_b;
@@ -998,8 +1006,13 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
 
     for (int s = 0; s < seg; ++s, ++it) {
       const int c = walk.chunk(c_rel + s), buf = it % DEC_STAGES;
-      const bool arrived =
+      bool arrived =
           !warp_dead && __all_sync(0xffffffffu, mbar_wait_bounded(&bars[buf], (it / DEC_STAGES) & 1, status));
+      if (ROPE && store_kv && (c + 1) * KCHUNK >= kl) {      // the newest key and value come from the store warp
+        if (arrived && tid == 0) mbar_arrive(&reached);
+        arrived = arrived && __all_sync(0xffffffffu, mbar_wait_bounded(&patched, n_new & 1, status));
+        ++n_new;
+      }
       if (!arrived && !warp_dead) {
         warp_dead = true;
         if (lane == 0) dead = 1;
@@ -1110,60 +1123,57 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
       }
     consumer_barrier(NTHREADS);
     if (dead) break;   // (status is set; the output is invalid) all four warps see the same value here
-    float m = -INFINITY, L = 0.f, f[4];
-    if (r < heads_here) {
-      m = merge_m[0][r];
+    const bool whole = seg == n_b;   // this block held the whole unit: no scratch, no counter
+    const int quads = d >> 2;
+    // four columns of a head per thread and turn (one turn for four heads of 128)
+#pragma unroll 1
+    for (int item = tid; item < heads_here * quads; item += NTHREADS) {
+      const int r = item / quads, c4 = (item - r * quads) * 4;
+      float m = merge_m[0][r], L = 0.f;
 #pragma unroll
       for (int w = 1; w < 4; ++w) m = fmaxf(m, merge_m[w][r]);
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
-        f[w] = (merge_m[w][r] == -INFINITY) ? 0.f : exp2f(merge_m[w][r] - m);
-        L += merge_l[w][r] * f[w];
+        const float f = (merge_m[w][r] == -INFINITY) ? 0.f : exp2f(merge_m[w][r] - m);
+        const float4 v = *reinterpret_cast<const float4*>(merge_o + ((size_t)w * DEC_HEADS + r) * d + c4);
+        L = fmaf(merge_l[w][r], f, L);
+        acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y);
+        acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
       }
-    }
-    const bool whole = seg == n_b;   // this block held the whole unit: no scratch, no counter
-    const int head = head0 + r;
-    if (r < heads_here) {
       if (whole) {
-        if (sinks && m != -INFINITY) L += exp2f(sinks[head] * LOG2E - m);
+        if (sinks && m != -INFINITY) L += exp2f(sinks[head0 + r] * LOG2E - m);
         const float inv = L > 0.f ? 1.f / L : 0.f;
-        bf16* orow = out + (size_t)tok * out_stride + (size_t)head * d;
-        for (int k = cgrp; k < d; k += 16) {
-          float acc = 0.f;
-#pragma unroll
-          for (int w = 0; w < 4; ++w) acc += f[w] * merge_o[((size_t)w * DEC_HEADS + r) * d + k];
-          orow[k] = __float2bfloat16_rn(acc * inv);
-        }
+        uint32_t* dst = reinterpret_cast<uint32_t*>(out + (size_t)tok * out_stride + (size_t)(head0 + r) * d + c4);
+        dst[0] = pack_bf16(acc.x * inv, acc.y * inv);
+        dst[1] = pack_bf16(acc.z * inv, acc.w * inv);
       } else {
         const size_t slot = ((size_t)unit + blockIdx.x) * DEC_HEADS + r;
-        float* po = part_o + slot * d;
-        for (int k = cgrp; k < d; k += 16) {
-          float acc = 0.f;
-#pragma unroll
-          for (int w = 0; w < 4; ++w) acc += f[w] * merge_o[((size_t)w * DEC_HEADS + r) * d + k];
-          po[k] = acc;
-        }
-        if (cgrp == 0) {
-          part_ml[slot * 2] = m;
-          part_ml[slot * 2 + 1] = L;
-        }
+        *reinterpret_cast<float4*>(part_o + slot * d + c4) = acc;
+        if (c4 == 0) *reinterpret_cast<float2*>(part_ml + slot * 2) = make_float2(m, L);
       }
     }
     if (!whole) {
-      // count this stretch's chunks in; whoever completes the unit merges its stretches in block order
-      __threadfence();
+      // Count this stretch's chunks in; whoever completes the unit merges its stretches in block order.  One thread's
+      // fence behind the barrier orders all threads' stores before the count.
       consumer_barrier(NTHREADS);
-      if (tid == 0) is_last = (atomicAdd(&counters[unit], seg) + seg == n_b) ? 1 : 0;
+      if (tid == 0) {
+        __threadfence();
+        is_last = (atomicAdd(&counters[unit], seg) + seg == n_b) ? 1 : 0;
+        if (is_last) __threadfence();
+      }
       consumer_barrier(NTHREADS);
       if (is_last) {
-        __threadfence();
         // the blocks whose stretches hold the unit's chunks: its positions from `ov` on
         const long long start = (long long)(cum[b] + ov * b) * U + (long long)u * (n_b + ov) + ov;
-        const int g_first = (int)(((start + 1) * G - 1) / W), g_last = (int)(((start + n_b) * G - 1) / W);
-        if (r < heads_here)
-          balanced_merge_unit<DMAX>(part_o, part_ml, unit, g_first, g_last, r, cgrp, d,
-                                    out + (size_t)tok * out_stride + (size_t)head * d,
-                                    sinks ? sinks[head] * LOG2E : -INFINITY);
+        const int g_first = (int)balanced_div((start + 1) * G - 1, W), g_last = (int)balanced_div((start + n_b) * G - 1, W);
+#pragma unroll 1
+        for (int item = tid; item < heads_here * quads; item += NTHREADS) {
+          const int r = item / quads, c4 = (item - r * quads) * 4;
+          balanced_merge_unit(part_o, part_ml, unit, g_first, g_last, r, c4, d,
+                              out + (size_t)tok * out_stride + (size_t)(head0 + r) * d,
+                              sinks ? sinks[head0 + r] * LOG2E : -INFINITY);
+        }
         if (tid == 0) counters[unit] = 0;   // ready for the next call
       }
     }
@@ -1627,6 +1637,9 @@ extern "C" int mi_attention_decode_balanced_unit_cost(int chunks) {
   return before;
 }
 
+// Stretches are not made shorter than this many chunks: their set-up and merge then cost more than they spread.  (One request
+// of 1024 tokens, a pass of Llama 3.1 8B sizes: 4 chunks 199.4 ms, 2 196.5, 1 198.5; 8 x 2048 within noise.)
+#define BAL_MIN_CHUNKS 2
 static size_t balanced_smem_bytes(int B, int d) {   // the ring, the warps' merge buffer, the running sum of chunks
   return (size_t)(2 * DEC_STAGES * KCHUNK) * d * sizeof(bf16) + (size_t)4 * DEC_HEADS * d * sizeof(float) +
          (size_t)(B + 1) * sizeof(int);
@@ -1664,8 +1677,8 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
     MI_REFUSE("attention: rotating inside the decode kernel needs a head size of 64, 128 or 256, got %d", d);
   if (int rc = check_common(q, q_stride, out, out_stride, kcache, vcache, nq, nkv, d, page_size, window)) return rc;
   if (grid <= 0 || !part_o || !part_ml || !counters) MI_REFUSE("attention: the balanced kernel needs its grid and scratch");
-  if (!mi_aligned(part_o, 4) || !mi_aligned(part_ml, 8) || !mi_aligned(counters, 4))
-    MI_REFUSE("attention: scratch must be aligned (part_o and counters to 4 bytes, part_ml to 8)");
+  if (!mi_aligned(part_o, 16) || !mi_aligned(part_ml, 8) || !mi_aligned(counters, 4))
+    MI_REFUSE("attention: scratch must be aligned (part_o to 16 bytes, part_ml to 8, counters to 4)");
   if (B > 16384) MI_REFUSE("attention: %d requests in one decode step", B);
   const int page_shift = shift_of(page_size);
   const size_t smem = balanced_smem_bytes(B, d);
@@ -1678,7 +1691,7 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
     }                                                                                                     \
     MI_LAUNCH((kern), grid, ROPE ? BAL_THREADS : DEC_THREADS, smem, stream, (const bf16*)q, q_stride,     \
               (bf16*)out, out_stride, (const bf16*)kcache, (const bf16*)vcache, block_table, bt_stride,   \
-              table_rows, page_size, page_shift, q_start, kv_len, B, nq, nkv, d, scale, window, 4,        \
+              table_rows, page_size, page_shift, q_start, kv_len, B, nq, nkv, d, scale, window, BAL_MIN_CHUNKS, \
               g_unit_cost, part_o, part_ml, counters, wait_status_ptr(), rope_cs, store_kv, sinks, keep,  \
               cap_k, cap_h);                                                                              \
   } while (0)
