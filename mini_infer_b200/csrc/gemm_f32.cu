@@ -1,64 +1,79 @@
 // True 32-bit matrix product on CUDA cores:  C[M,N] = A[M,K] * W[N,K]^T
 // (both operands K-contiguous, as linear layers store them).  No tensor cores, no
-// reduced-precision mode.  Every output element is accumulated over k = 0..K-1 in that
-// order with fused multiply-adds, whatever tile it falls in and whatever kernel and tile shape are
-// chosen, so a row's result does not depend on which other rows share the call.
+// reduced-precision mode.  Every output element is the sum, in this order, of four parts of k of equal length (a
+// multiple of 32, the last one shorter), each accumulated from its first k on with fused multiply-adds, whatever kernel and
+// tile it falls in, so a row's result does not depend on which other rows share the call.
 //
 //   gemm_f32_rows_kernel   up to 32 rows (decode): bound by one reading of W
-//   gemm_f32_tile_kernel   more rows, or operands without 16-byte rows: bound by the fused multiply-adds
+//   gemm_f32_tile_kernel   more rows: bound by the fused multiply-adds
+//   gemm_f32_any_kernel    operands without 16-byte rows
 #include "common.cuh"
 
 MI_DEFINE_ERROR_API()
 
-// ------------------------------------------------------------------------------------------
-// Few rows.  A block owns 16 columns of the result (rows of W) and streams them, with the rows of A beside
-// them, through a ring of shared-memory stages filled by cp.async; 16 x 4 threads, RM rows of A each.  One element's
-// sum is a chain of K multiply-adds (4 cycles each: 4.3 us at K = 2048), so the columns have to be spread wide, 128
-// blocks for N = 2048, and the ring deep.  The first stages of W are asked for before the wait for the kernel before.
-// ------------------------------------------------------------------------------------------
-#define RB_COLS 16
-#define RB_K 64
-#define RB_PITCH (RB_K + 4)      // floats per staged row: eight rows' 16-byte pieces touch every bank once
-#define RB_STAGES 8
-#define RB_MAX_ROWS 32
+#define PARTS 4
+// where part p of k begins (a multiple of 32, so that a staged piece lies in one part)
+__host__ __device__ __forceinline__ int part_begin(int K, int p) {
+  const int len = ((K + PARTS - 1) / PARTS + 31) / 32 * 32;
+  const int at = p * len;
+  return at < K ? at : K;
+}
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   const int n = in ? 16 : 0;       // nothing read, zeros written
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
+// the 64 threads of a part among themselves
+__device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync %0, 64;\n" ::"r"(part + 1) : "memory"); }
 
-template <int RM>
-__global__ void __launch_bounds__(64) gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                           float* __restrict__ C, int M, int N, int K, int lda, int ldw,
-                                                           int ldc) {
+// ------------------------------------------------------------------------------------------
+// Few rows.  A block owns 16 columns of the result (rows of W); 64 threads per part of k stream their part of
+// them, with the rows of A beside it, through a ring of stages filled by cp.async, 16 x 4 threads, RM rows of A each.  One
+// element's sum is a chain of K / 4 multiply-adds (4 cycles each: 1.1 us at K = 2048).  The first stages of W are asked for
+// before the wait for the kernel before.  2 x 3072 x 2048 behind one another: 19 us with one part (a chain four times
+// as long behind a ring four times as narrow), 322 us with 128 columns per block and no ring; 3.9 us of bytes.
+// ------------------------------------------------------------------------------------------
+#define RB_COLS 16
+#define RB_K 32
+#define RB_PITCH (RB_K + 4)      // floats per staged row: eight rows' 16-byte pieces touch every bank once
+#define RB_MAX_ROWS 32
+
+template <int RM, int STAGES>
+__global__ void __launch_bounds__(64 * PARTS) gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
+                                                                   float* __restrict__ C, int M, int N, int K, int lda,
+                                                                   int ldw, int ldc) {
   extern __shared__ __align__(16) float rsm[];
   constexpr int ROWS = 4 * RM;
   constexpr int STAGE = (RB_COLS + ROWS) * RB_PITCH;
+  __shared__ float sums[PARTS - 1][ROWS][RB_COLS];
   mi_pdl_launch_dependents();
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int part = threadIdx.x >> 6, tid = threadIdx.x & 63, tx = tid & 15, ty = tid >> 4;
   const int n0 = blockIdx.x * RB_COLS;
-  const int chunks = (K + RB_K - 1) / RB_K;
+  const int k_begin = part_begin(K, part), k_end = part_begin(K, part + 1);
+  const int chunks = (k_end - k_begin + RB_K - 1) / RB_K;
+  float* ring = rsm + part * STAGES * STAGE;
   auto load_w = [&](int kc) {
-    float* dst = rsm + (kc % RB_STAGES) * STAGE;
+    float* dst = ring + (kc % STAGES) * STAGE;
+#pragma unroll
     for (int i = tid; i < RB_COLS * (RB_K / 4); i += 64) {
-      const int r = i / (RB_K / 4), c = (i % (RB_K / 4)) * 4, k = kc * RB_K + c;
-      const bool in = n0 + r < N && k < K;
+      const int r = i / (RB_K / 4), c = (i % (RB_K / 4)) * 4, k = k_begin + kc * RB_K + c;
+      const bool in = n0 + r < N && k < k_end;
       cp_async16(dst + r * RB_PITCH + c, in ? W + (size_t)(n0 + r) * ldw + k : W, in);
     }
   };
   auto load_a = [&](int kc) {
-    float* dst = rsm + (kc % RB_STAGES) * STAGE + RB_COLS * RB_PITCH;
+    float* dst = ring + (kc % STAGES) * STAGE + RB_COLS * RB_PITCH;
     for (int i = tid; i < M * (RB_K / 4); i += 64) {
-      const int r = i / (RB_K / 4), c = (i % (RB_K / 4)) * 4, k = kc * RB_K + c;
-      const bool in = k < K;
+      const int r = i / (RB_K / 4), c = (i % (RB_K / 4)) * 4, k = k_begin + kc * RB_K + c;
+      const bool in = k < k_end;
       cp_async16(dst + r * RB_PITCH + c, in ? A + (size_t)r * lda + k : A, in);
     }
   };
-  const int ahead = min(RB_STAGES - 1, chunks);
+  const int ahead = min(STAGES - 1, chunks);
   for (int s = 0; s < ahead; ++s) load_w(s);      // weights depend on no kernel before this one
   mi_pdl_wait();
-  for (int s = 0; s < RB_STAGES - 1; ++s) {
+  for (int s = 0; s < STAGES - 1; ++s) {
     if (s < chunks) load_a(s);
     asm volatile("cp.async.commit_group;\n" ::: "memory");   // (W's first stages ride in the first group)
   }
@@ -66,190 +81,218 @@ __global__ void __launch_bounds__(64) gemm_f32_rows_kernel(const float* __restri
 #pragma unroll
   for (int i = 0; i < RM; ++i) acc[i] = 0.f;
   for (int kc = 0; kc < chunks; ++kc) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(RB_STAGES - 2) : "memory");
-    __syncthreads();               // stage kc is there, and stage kc - 1 is consumed
-    const int next = kc + RB_STAGES - 1;
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    part_barrier(part);            // stage kc is there, and stage kc - 1 is consumed
+    const int next = kc + STAGES - 1;
     if (next < chunks) {
       load_w(next);
       load_a(next);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const float* ws = rsm + (kc % RB_STAGES) * STAGE + tx * RB_PITCH;
-    const float* as = rsm + (kc % RB_STAGES) * STAGE + (RB_COLS + ty * RM) * RB_PITCH;
-#pragma unroll 8
-    for (int k = 0; k < RB_K; k += 4) {
-      const float4 w = *reinterpret_cast<const float4*>(ws + k);
+    const float* ws = ring + (kc % STAGES) * STAGE + tx * RB_PITCH;
+    const float* as = ring + (kc % STAGES) * STAGE + (RB_COLS + ty * RM) * RB_PITCH;
+    // a batch's pieces are read before its multiply-adds (each piece's chain alone would wait for it)
+    constexpr int BATCH = RM <= 2 ? 8 : RM <= 4 ? 4 : 2;
 #pragma unroll
-      for (int i = 0; i < RM; ++i) {
-        const float4 a = *reinterpret_cast<const float4*>(as + i * RB_PITCH + k);
-        acc[i] = fmaf(a.w, w.w, fmaf(a.z, w.z, fmaf(a.y, w.y, fmaf(a.x, w.x, acc[i]))));
+    for (int k0 = 0; k0 < RB_K; k0 += 4 * BATCH) {
+      float4 w[BATCH], a[BATCH][RM];
+#pragma unroll
+      for (int j = 0; j < BATCH; ++j) {
+        w[j] = *reinterpret_cast<const float4*>(ws + k0 + 4 * j);
+#pragma unroll
+        for (int i = 0; i < RM; ++i) a[j][i] = *reinterpret_cast<const float4*>(as + i * RB_PITCH + k0 + 4 * j);
       }
+#pragma unroll
+      for (int j = 0; j < BATCH; ++j)
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+          acc[i] = fmaf(a[j][i].w, w[j].w, fmaf(a[j][i].z, w[j].z, fmaf(a[j][i].y, w[j].y, fmaf(a[j][i].x, w[j].x, acc[i]))));
     }
   }
+  if (part) {
+#pragma unroll
+    for (int i = 0; i < RM; ++i) sums[part - 1][ty * RM + i][tx] = acc[i];
+  }
+  __syncthreads();
+  if (part) return;
   const int n = n0 + tx;
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
     const int m = ty * RM + i;
-    if (m < M && n < N) C[(size_t)m * ldc + n] = acc[i];
+    float v = acc[i];
+#pragma unroll
+    for (int p = 0; p < PARTS - 1; ++p) v += sums[p][m][tx];
+    if (m < M && n < N) C[(size_t)m * ldc + n] = v;
   }
 }
 
 // ------------------------------------------------------------------------------------------
-// Many rows.  A BM x BN tile per block, TM x TN results per thread (two groups of four rows and of four columns,
-// half a tile apart), k in steps of 16 through two shared-memory buffers: the next step's pieces come from global memory into
-// registers while this one is multiplied.  The multiply-adds are the two-wide form, two columns at a time.
+// More rows.  An 8 TM x 64 tile per block and part of k: 64 threads per part, 8 x 8, TM x 8 results each (rows and
+// columns 8 apart, so that a warp's reads of one operand are at most 128 different bytes), k in steps of 32 through two
+// stages filled by cp.async, both operands as they lie in memory: a thread reads four k of its rows and columns.  The parts
+// bring four times the warps of a tile to an SM, which a product of a few hundred rows needs: with one part a step of 16 k took
+// 1400 cycles, most of it waiting (262 x 2048 x 2048: 148 us, now 63; 31 us of multiply-adds; 1024 x 6144 x 2048: 623 us, 358 of
+// multiply-adds).  TM = 4: two blocks per SM; 2, 6 and 8 take 91, 94 and 114 us for the first and 913, 690 and 648 for the second.
 // ------------------------------------------------------------------------------------------
-#define TB_K 16
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
+#define TB_K 32
+#define TB_PITCH (TB_K + 4)
+#define TB_STAGES 2
+#define TB_N 64
 
-template <int BM, int BN, int TM, int TN, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
-                     int M, int N, int K, int lda, int ldw, int ldc) {
-  mi_pdl_enter();   // inputs come from the kernels before this one
-  constexpr int THREADS = (BM / TM) * (BN / TN);
-  constexpr int GM = TM / 4, GN = TN / 4;                 // groups of four
-  constexpr int PA = BM * (TB_K / 4) / THREADS, PW = BN * (TB_K / 4) / THREADS;   // 16-byte pieces per thread and step
-  static_assert(PA * THREADS == BM * (TB_K / 4) && PW * THREADS == BN * (TB_K / 4), "whole pieces per thread");
-  __shared__ __align__(16) float As[2][TB_K][BM + 4];
-  __shared__ __align__(16) float Ws[2][TB_K][BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-
-  auto piece = [&](const float* p, int row, int rows, int ld, int k) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row >= rows) return v;
-    const float* src = p + (size_t)row * ld + k;
-    if (VEC) {           // K % 4 == 0 and 16-byte rows
-      if (k < K) v = *reinterpret_cast<const float4*>(src);
-    } else {
-      if (k < K) v.x = src[0];
-      if (k + 1 < K) v.y = src[1];
-      if (k + 2 < K) v.z = src[2];
-      if (k + 3 < K) v.w = src[3];
-    }
-    return v;
-  };
-  float4 pa[PA], pw[PW];
-  auto fetch = [&](int k0) {
+template <int TM>
+__global__ void __launch_bounds__(64 * PARTS) gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
+                                                                   float* __restrict__ C, int M, int N, int K, int lda,
+                                                                   int ldw, int ldc) {
+  extern __shared__ __align__(16) float tsm[];
+  constexpr int BM = 8 * TM, STAGE = (BM + TB_N) * TB_PITCH;
+  mi_pdl_enter();
+  const int part = threadIdx.x >> 6, tid = threadIdx.x & 63, tx = tid & 7, ty = tid >> 3;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * TB_N;
+  const int k_begin = part_begin(K, part), k_end = part_begin(K, part + 1);
+  const int chunks = (k_end - k_begin + TB_K - 1) / TB_K;
+  float* ring = tsm + part * TB_STAGES * STAGE;
+  // this thread copies rows r0, r0 + 8, ... of A and of W, the four k from c on
+  const int r0 = tid >> 3, c = (tid & 7) * 4;
+  auto load = [&](int kc) {
+    float* dst = ring + (kc & 1) * STAGE + r0 * TB_PITCH + c;
+    const int k = k_begin + kc * TB_K + c;
+    const bool k_in = k < k_end;
 #pragma unroll
-    for (int i = 0; i < PA; ++i) {
-      const int idx = tid + i * THREADS;
-      pa[i] = piece(A, m0 + idx / (TB_K / 4), M, lda, k0 + (idx % (TB_K / 4)) * 4);
+    for (int i = 0; i < TM; ++i) {
+      const bool in = k_in && m0 + r0 + 8 * i < M;
+      cp_async16(dst + 8 * i * TB_PITCH, in ? A + (size_t)(m0 + r0 + 8 * i) * lda + k : A, in);
     }
 #pragma unroll
-    for (int i = 0; i < PW; ++i) {
-      const int idx = tid + i * THREADS;
-      pw[i] = piece(W, n0 + idx / (TB_K / 4), N, ldw, k0 + (idx % (TB_K / 4)) * 4);
+    for (int j = 0; j < TB_N / 8; ++j) {
+      const bool in = k_in && n0 + r0 + 8 * j < N;
+      cp_async16(dst + (BM + 8 * j) * TB_PITCH, in ? W + (size_t)(n0 + r0 + 8 * j) * ldw + k : W, in);
     }
   };
-  auto stage = [&](int buf) {
-#pragma unroll
-    for (int i = 0; i < PA; ++i) {
-      const int idx = tid + i * THREADS, r = idx / (TB_K / 4), c = (idx % (TB_K / 4)) * 4;
-      As[buf][c][r] = pa[i].x; As[buf][c + 1][r] = pa[i].y; As[buf][c + 2][r] = pa[i].z; As[buf][c + 3][r] = pa[i].w;
-    }
-#pragma unroll
-    for (int i = 0; i < PW; ++i) {
-      const int idx = tid + i * THREADS, r = idx / (TB_K / 4), c = (idx % (TB_K / 4)) * 4;
-      Ws[buf][c][r] = pw[i].x; Ws[buf][c + 1][r] = pw[i].y; Ws[buf][c + 2][r] = pw[i].z; Ws[buf][c + 3][r] = pw[i].w;
-    }
-  };
-
-  uint64_t acc[TM][TN / 2];
+  if (chunks > 0) load(0);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  float acc[TM][8];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
-
-  fetch(0);
-  stage(0);
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  for (int kc = 0; kc < chunks; ++kc) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    part_barrier(part);            // stage kc is there, and stage kc - 1 is consumed
+    if (kc + 1 < chunks) load(kc + 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const float* as = ring + (kc & 1) * STAGE + ty * TB_PITCH;
+    const float* ws = ring + (kc & 1) * STAGE + (BM + tx) * TB_PITCH;
+#pragma unroll
+    for (int k = 0; k < TB_K; k += 4) {
+      float4 a[TM], w[8];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + 8 * i * TB_PITCH + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(ws + 8 * j * TB_PITCH + k);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          acc[i][j] = fmaf(a[i].w, w[j].w, fmaf(a[i].z, w[j].z, fmaf(a[i].y, w[j].y, fmaf(a[i].x, w[j].x, acc[i][j]))));
+    }
+  }
+  // the parts' sums, in the order of the parts, through the rings' memory
   __syncthreads();
-  int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += TB_K) {
-    const bool more = k0 + TB_K < K;
-    if (more) fetch(k0 + TB_K);
+  float* sums = tsm;               // [PARTS][BM][TB_N]
 #pragma unroll
-    for (int k = 0; k < TB_K; ++k) {
-      uint64_t w[TN / 2];
-      float a[TM];
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < GN; ++j) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Ws[buf][k][j * (BN / GN) + tx * 4]);
-        w[2 * j] = v.x;
-        w[2 * j + 1] = v.y;
-      }
+    for (int j = 0; j < 8; ++j) sums[(part * BM + ty + 8 * i) * TB_N + tx + 8 * j] = acc[i][j];
+  __syncthreads();
+  for (int i = threadIdx.x; i < BM * TB_N; i += 64 * PARTS) {
+    const int m = m0 + i / TB_N, n = n0 + i % TB_N;
+    float v = sums[i];
 #pragma unroll
-      for (int i = 0; i < GM; ++i) {
-        const float4 v = *reinterpret_cast<const float4*>(&As[buf][k][i * (BM / GM) + ty * 4]);
-        a[4 * i] = v.x; a[4 * i + 1] = v.y; a[4 * i + 2] = v.z; a[4 * i + 3] = v.w;
-      }
-#pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        const uint64_t aa = pack2(a[i], a[i]);
-#pragma unroll
-        for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], aa, w[j]);
-      }
-    }
-    if (more) stage(buf ^ 1);      // (that buffer was last read before the barrier of the step before)
-    __syncthreads();
-    buf ^= 1;
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + (i / 4) * (BM / GM) + ty * 4 + (i & 3);
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN / 2; ++j) {
-      const int n = n0 + (j / 2) * (BN / GN) + tx * 4 + (j & 1) * 2;
-      float v0, v1;
-      unpack2(acc[i][j], v0, v1);
-      if (n < N) C[(size_t)m * ldc + n] = v0;
-      if (n + 1 < N) C[(size_t)m * ldc + n + 1] = v1;
-    }
+    for (int p = 1; p < PARTS; ++p) v += sums[p * BM * TB_N + i];
+    if (m < M && n < N) C[(size_t)m * ldc + n] = v;
   }
 }
 
-template <int BM, int BN, int TM, int TN>
-static void launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
-                        int ldc, bool vec, cudaStream_t stream) {
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  constexpr int THREADS = (BM / TM) * (BN / TN);
-  if (vec)
-    MI_LAUNCH((gemm_f32_tile_kernel<BM, BN, TM, TN, true>), grid, THREADS, 0, stream, A, W, C, M, N, K, lda, ldw, ldc);
-  else
-    MI_LAUNCH((gemm_f32_tile_kernel<BM, BN, TM, TN, false>), grid, THREADS, 0, stream, A, W, C, M, N, K, lda, ldw, ldc);
+// ------------------------------------------------------------------------------------------
+// Operands of any size and alignment: element by element through one stage, the parts one after the other.
+// ------------------------------------------------------------------------------------------
+#define AB_T 64
+#define AB_K 16
+__global__ void __launch_bounds__(256) gemm_f32_any_kernel(const float* __restrict__ A, const float* __restrict__ W,
+                                                           float* __restrict__ C, int M, int N, int K, int lda, int ldw,
+                                                           int ldc) {
+  mi_pdl_enter();
+  __shared__ float As[AB_K][AB_T + 4], Ws[AB_K][AB_T + 4];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * AB_T, n0 = blockIdx.x * AB_T;
+  float total[4][4], acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) total[i][j] = 0.f;
+  for (int p = 0; p < PARTS; ++p) {
+    const int k_end = part_begin(K, p + 1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int k0 = part_begin(K, p); k0 < k_end; k0 += AB_K) {
+      __syncthreads();
+      for (int idx = tid; idx < AB_T * AB_K; idx += 256) {
+        const int r = idx / AB_K, c = idx % AB_K, k = k0 + c;
+        As[c][r] = (m0 + r < M && k < k_end) ? A[(size_t)(m0 + r) * lda + k] : 0.f;
+        Ws[c][r] = (n0 + r < N && k < k_end) ? W[(size_t)(n0 + r) * ldw + k] : 0.f;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < AB_K; ++k) {
+        float a[4], w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) total[i][j] = p ? total[i][j] + acc[i][j] : acc[i][j];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
+      if (m < M && n < N) C[(size_t)m * ldc + n] = total[i][j];
+    }
 }
 
-template <int RM>
+template <int RM, int STAGES>
 static cudaError_t launch_rows(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
                                cudaStream_t stream) {
-  const size_t smem = (size_t)RB_STAGES * (RB_COLS + 4 * RM) * RB_PITCH * sizeof(float);
-  auto kern = gemm_f32_rows_kernel<RM>;
+  const size_t smem = (size_t)PARTS * STAGES * (RB_COLS + 4 * RM) * RB_PITCH * sizeof(float);
+  auto kern = gemm_f32_rows_kernel<RM, STAGES>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return MI_LAUNCH(kern, (N + RB_COLS - 1) / RB_COLS, 64, smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
+  return MI_LAUNCH(kern, (N + RB_COLS - 1) / RB_COLS, 64 * PARTS, smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
 }
 
-// The time of a tile shape in units of multiply-adds: waves over the SMs times the tile, the smaller shapes marked
-// down for what they read from shared memory per multiply-add.
-static double tile_time(int M, int N, int bm, int bn, double weight) {
-  const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-  return (double)((tiles + 147) / 148) * bm * bn * weight;
+template <int TM>
+static cudaError_t launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                               cudaStream_t stream) {
+  const size_t smem = (size_t)PARTS * TB_STAGES * (8 * TM + TB_N) * TB_PITCH * sizeof(float);
+  auto kern = gemm_f32_tile_kernel<TM>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  return MI_LAUNCH(kern, dim3((N + TB_N - 1) / TB_N, (M + 8 * TM - 1) / (8 * TM)), 64 * PARTS, smem, stream, A, W, C, M, N,
+                   K, lda, ldw, ldc);
 }
 
-// Zero-padded K tails add exact zeros at the end of the sum, so they do not change it.
+// Zero-padded tails of a part add exact zeros at the end of its sum, so they do not change it.
 extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
                            int ldw, int ldc, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
@@ -257,23 +300,18 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
   if (lda < K || ldw < K || ldc < N) MI_REFUSE("gemm_f32: leading dimensions too small");
   if ((M + 15) / 16 > 65535) MI_REFUSE("gemm_f32: too many rows (%d)", M);
   const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && mi_aligned(A, 16) && mi_aligned(W, 16);
-  if (vec && M <= RB_MAX_ROWS) {
-    const cudaError_t e = M <= 4    ? launch_rows<1>(A, W, C, M, N, K, lda, ldw, ldc, stream)
-                          : M <= 8  ? launch_rows<2>(A, W, C, M, N, K, lda, ldw, ldc, stream)
-                          : M <= 16 ? launch_rows<4>(A, W, C, M, N, K, lda, ldw, ldc, stream)
-                                    : launch_rows<8>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    if (e != cudaSuccess) return (int)e;
-    MI_RETURN_LAUNCH_STATUS();
+  cudaError_t e = cudaSuccess;
+  if (!vec) {
+    MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
+              lda, ldw, ldc);
+  } else if (M <= RB_MAX_ROWS) {
+    e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, stream)
+        : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, stream)
+        : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, stream)
+                  : launch_rows<8, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  } else {
+    e = launch_tile<4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
   }
-  const double big = tile_time(M, N, 128, 128, 1.0), wide = tile_time(M, N, 64, 128, 1.05),
-               mid = tile_time(M, N, 64, 64, 1.25), small = tile_time(M, N, 32, 64, 1.6);
-  if (big <= wide && big <= mid && big <= small)
-    launch_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
-  else if (wide <= mid && wide <= small)
-    launch_tile<64, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
-  else if (mid <= small)
-    launch_tile<64, 64, 4, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
-  else
-    launch_tile<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
+  if (e != cudaSuccess) return (int)e;
   MI_RETURN_LAUNCH_STATUS();
 }

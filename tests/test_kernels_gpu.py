@@ -194,8 +194,9 @@ def test_gemm_f32_rows_do_not_depend_on_the_batch():
 
 @pytest.mark.parametrize("N,K", [(16, 64), (130, 68), (257, 1000), (2048, 512)])
 def test_gemm_f32_gives_the_same_bits_from_every_kernel(N, K):
-    """The kernel for few rows (1 to 32, by groups of four) and the tile shapes for more add up in the same order; a
-    float64 product bounds them: K terms, each rounded once more than exactly, 2^-24 of the sum of magnitudes each."""
+    """The kernel for few rows (1 to 32, by groups of four), the tiles for more and the kernel for rows that are no whole
+    16-byte pieces add up in the same order; a float64 product bounds them: K terms, each rounded once more than exactly,
+    2^-24 of the sum of magnitudes each."""
     a, w = rnd(300, K, seed=13), rnd(N, K, seed=14)
     full = ops().gemm_f32(a.to(DEV), w.to(DEV))
     want = a.double() @ w.double().T
@@ -203,6 +204,9 @@ def test_gemm_f32_gives_the_same_bits_from_every_kernel(N, K):
     assert ((full.cpu().double() - want).abs() <= bound).all()
     for M in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 129):
         assert torch.equal(ops().gemm_f32(a[:M].to(DEV), w.to(DEV)), full[:M]), M
+    odd = torch.zeros(N, K + 1, device=DEV)
+    odd[:, 1:] = w.to(DEV)
+    assert torch.equal(ops().gemm_f32(a.to(DEV), odd[:, 1:]), full)
 
 
 def test_gemm_f32_is_not_reduced_precision():
