@@ -37,6 +37,12 @@ MI_DEFINE_ERROR_API()
 #define BK 32
 #define NTHREADS 128
 
+// whether the instance for values of up to DMAX fetches these rows a chunk ahead
+template <int DMAX>
+__host__ __device__ __forceinline__ bool rows_ahead(int d, int dv, int v_prefix) {
+  return DMAX <= 128 && d <= DMAX && (d & 3) == 0 && (dv & 3) == 0 && !v_prefix;
+}
+
 template <typename T, int DMAX>
 __global__ void __launch_bounds__(NTHREADS)
 attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride,
@@ -55,8 +61,13 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
   float* Qs = Vs + (v_prefix ? 0 : BK * dvp);   // [BQ][d]
   float* Ks = Qs + BQ * d;                // [BK][d + 1]
   float* Ss = Ks + BK * (d + 1);          // [BQ][BK]
-  int* rowbase = reinterpret_cast<int*>(Ss + BQ * BK);  // [BK] element offset / d of each key row, -1: none
-  int* rowswz = rowbase + BK;                            // [BK] chunk permutation of each key row
+  // With 16-byte pieces and heads of up to 128 the next chunk's rows come into registers while this one is worked on
+  // (a chunk of 32 keys took 18 us when every one began with a round trip to the block table and one to its rows).
+  constexpr int PRE = DMAX <= 128 ? DMAX / 16 : 0;
+  const bool ahead = PRE > 0 && rows_ahead<DMAX>(d, dv, v_prefix);
+  // per key row of the chunk at hand (and of the next): element offset / d (-1: none) and chunk permutation
+  int* rowbase2 = reinterpret_cast<int*>(Ss + BQ * BK);  // [1 or 2][BK]
+  int* rowswz2 = rowbase2 + (ahead ? 2 : 1) * BK;        // [1 or 2][BK]
   constexpr int EPC = 16 / (int)sizeof(T);
   const int swz_mask = mi_swizzle_mask_rows(d, (int)sizeof(T));
   const int swz_mask_v = mi_swizzle_mask_rows(dv, (int)sizeof(T));
@@ -94,20 +105,63 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
 
   const MiKeyWalk<true> walk(j_lo, keep, BK);
   const int n_chunks = walk.count(j_end, BK);
+  auto locate = [&](int ci) {      // the rows of chunk ci, by the first 32 threads
+    const int j = walk.chunk(ci) * BK + tid;
+    int base = -1;
+    if ((j >= j_lo || j < keep) && j < j_end) {
+      const int page = block_table[(size_t)trow * bt_stride + j / page_size];
+      base = (page * nkv + kvh) * page_size + j % page_size;
+    }
+    rowbase2[(ahead ? ci & 1 : 0) * BK + tid] = base;
+    rowswz2[(ahead ? ci & 1 : 0) * BK + tid] = (j % page_size);
+  };
+  Vec4<T> kp[PRE > 0 ? PRE : 1], vp[PRE > 0 ? PRE : 1];
+  auto piece = [&](Vec4<T>& to, const T* cache, int idx, int width, int mask, const int* base_of, const int* swz_of) {
+    const int w4 = width >> 2, jj = idx / w4, k4 = (idx - jj * w4) << 2;
+    const float none[4] = {0.f, 0.f, 0.f, 0.f};
+    to.set(none);
+    if (jj < BK && base_of[jj] >= 0)
+      to.load(cache + (size_t)base_of[jj] * width + ((((k4 / EPC) ^ (swz_of[jj] & mask)) * EPC) + (k4 % EPC)));
+  };
+  auto fetch = [&](int ci) {
+    const int *base_of = rowbase2 + (ci & 1) * BK, *swz_of = rowswz2 + (ci & 1) * BK;
+#pragma unroll
+    for (int i = 0; i < PRE; ++i) piece(kp[i], kcache, tid + i * NTHREADS, d, swz_mask, base_of, swz_of);
+#pragma unroll
+    for (int i = 0; i < PRE; ++i) piece(vp[i], vcache, tid + i * NTHREADS, dv, swz_mask_v, base_of, swz_of);
+  };
+  if (ahead && n_chunks > 0) {
+    if (tid < BK) locate(0);
+    __syncthreads();
+    fetch(0);
+  }
   for (int ci = 0; ci < n_chunks; ++ci) {
     const int j0 = walk.chunk(ci) * BK;
+    const int *rowbase = rowbase2, *rowswz = rowswz2;      // (read by the loads below, not by those ahead)
     __syncthreads();  // previous chunk fully consumed (and Qs written, first time)
-    if (tid < BK) {
-      const int j = j0 + tid;
-      int base = -1;
-      if ((j >= j_lo || j < keep) && j < j_end) {
-        const int page = block_table[(size_t)trow * bt_stride + j / page_size];
-        base = (page * nkv + kvh) * page_size + j % page_size;
+    if (tid < BK && !ahead) locate(ci);
+    if (tid < BK && ahead && ci + 1 < n_chunks) locate(ci + 1);
+    if (ahead) {
+#pragma unroll
+      for (int i = 0; i < PRE; ++i) {
+        const int idx = tid + i * NTHREADS;
+        float f[4];
+        const int kj = idx / (d >> 2), vj = idx / (dv >> 2);
+        if (kj < BK) {
+          kp[i].get(f);
+          float* kd = Ks + kj * dp + ((idx - kj * (d >> 2)) << 2);
+          kd[0] = f[0]; kd[1] = f[1]; kd[2] = f[2]; kd[3] = f[3];
+        }
+        if (vj < BK) {
+          vp[i].get(f);
+          *reinterpret_cast<float4*>(Vs + vj * dvp + ((idx - vj * (dv >> 2)) << 2)) = make_float4(f[0], f[1], f[2], f[3]);
+        }
       }
-      rowbase[tid] = base;
-      rowswz[tid] = (j % page_size);
     }
     __syncthreads();
+    if (ahead) {
+      if (ci + 1 < n_chunks) fetch(ci + 1);
+    } else {
     if ((d & 3) == 0) {
       const int d4 = d >> 2;
       for (int idx = tid; idx < BK * d4; idx += NTHREADS) {
@@ -154,9 +208,11 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
       }
     }
     __syncthreads();
+    }
 
     float s[4] = {0.f, 0.f, 0.f, 0.f};
     const float* qrow = Qs + r * d;
+#pragma unroll 8
     for (int k = 0; k < d; ++k) {
       const float qv = qrow[k];
 #pragma unroll
@@ -195,6 +251,7 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
 #pragma unroll
     for (int e = 0; e < DMAX / 8; ++e) acc[e] *= alpha;
     __syncthreads();
+#pragma unroll 2
     for (int j = 0; j < BK; ++j) {
       const float pj = Ss[r * BK + j];
       const float* vrow = Vrows + j * vpitch + c;
@@ -229,7 +286,7 @@ static int launch(const void* q, int q_stride, void* out, int out_stride, const 
                   int chunk, const float* sinks, const float* slopes, int v_prefix, int keep, float softcap,
                   cudaStream_t stream) {
   const size_t smem = ((v_prefix ? 0 : (size_t)BK * ((dv + 3) & ~3)) + (size_t)BQ * d + (size_t)BK * (d + 1) + BQ * BK) *
-                          sizeof(float) + 2 * BK * sizeof(int);
+                          sizeof(float) + (rows_ahead<DMAX>(d, dv, v_prefix) ? 4 : 2) * BK * sizeof(int);
   auto kern = attention_generic_kernel<T, DMAX>;
   if (smem > 227 * 1024) return MI_REFUSED - 1;
   if (smem > 48 * 1024) {
