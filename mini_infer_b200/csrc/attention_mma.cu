@@ -733,19 +733,21 @@ __device__ __noinline__ void balanced_merge_unit(const float* __restrict__ part_
 }
 
 #define BAL_THREADS (NTHREADS + 64)   // four consumer warps, the copy warp, the store warp (ROPE only)
-// EXT: an instance of its own for kept keys and capped scores, so that the others keep their code.
-template <int DMAX, bool ROPE, bool EXT>
+// EXT: an instance of its own for kept keys and capped scores, so that the others keep their code.  EXACT: the head size is
+// DMAX, known to the compiler: the loops over it lose their conditions, of which a chunk's instructions were a good part.
+template <int DMAX, bool ROPE, bool EXT, bool EXACT>
 __global__ void __launch_bounds__(ROPE ? BAL_THREADS : DEC_THREADS, DMAX <= 128 ? 2 : 1)
 attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out, int out_stride,
                                  const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
                                  const int* __restrict__ block_table, int bt_stride,
                                  const int* __restrict__ table_rows, int page_size, int page_shift,
                                  const int* __restrict__ q_start, const int* __restrict__ kv_len, int B, int nq,
-                                 int nkv, int d, float scale, int window, int min_chunks, int unit_cost,
+                                 int nkv, int d_any, float scale, int window, int min_chunks, int unit_cost,
                                  float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters,
                                  int* __restrict__ status, const float* __restrict__ rope_cs, int store_kv,
                                  const float* __restrict__ sinks, int keep_any, float cap_k, float cap_h) {
   const int keep = EXT ? keep_any : 0;
+  const int d = EXACT ? DMAX : d_any;
   // sinks [nq] (optional): per head a score that joins the softmax's denominator with neither key nor value.
   // ROPE (the head size is then DMAX exactly): rope_cs holds per query token [d / 2] sines then
   // [d / 2] cosines of its rotary angles; q arrives un-rotated and is rotated here, in registers; and with store_kv
@@ -1067,9 +1069,9 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
           const float m_new = fmaxf(m_run[hh], mx);
-          alpha[hh] = exp2f(m_run[hh] - m_new);
-          p[hh] = exp2f(sa[hh] - m_new);
-          p[2 + hh] = exp2f(sa[2 + hh] - m_new);
+          alpha[hh] = mi_fast_exp2(m_run[hh] - m_new);
+          p[hh] = mi_fast_exp2(sa[hh] - m_new);
+          p[2 + hh] = mi_fast_exp2(sa[2 + hh] - m_new);
           m_run[hh] = m_new;
           l_run[hh] = l_run[hh] * alpha[hh] + (p[hh] + p[2 + hh]);
         }
@@ -1682,9 +1684,9 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
   if (B > 16384) MI_REFUSE("attention: %d requests in one decode step", B);
   const int page_shift = shift_of(page_size);
   const size_t smem = balanced_smem_bytes(B, d);
-#define MI_DECODE_BAL(DMAX, ROPE, EXT)                                                                         \
+#define MI_DECODE_BAL(DMAX, ROPE, EXT, EXACT)                                                                  \
   do {                                                                                                    \
-    auto kern = attention_decode_balanced_kernel<DMAX, ROPE, EXT>;                                             \
+    auto kern = attention_decode_balanced_kernel<DMAX, ROPE, EXT, EXACT>;                                      \
     if (smem > 40 * 1024) {                                                                               \
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) return (int)e;                                                                \
@@ -1697,16 +1699,18 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
   } while (0)
   if (rope_cs) {
     if (keep || softcap > 0.f) MI_REFUSE("attention: the decode kernel that rotates takes neither kept keys nor a cap");
-    if (d == 64) MI_DECODE_BAL(64, true, false);
-    else if (d == 128) MI_DECODE_BAL(128, true, false);
-    else MI_DECODE_BAL(256, true, false);
+    if (d == 64) MI_DECODE_BAL(64, true, false, true);
+    else if (d == 128) MI_DECODE_BAL(128, true, false, true);
+    else MI_DECODE_BAL(256, true, false, true);
   } else if (keep || softcap > 0.f) {
-    if (d <= 64) MI_DECODE_BAL(64, false, true);
-    else if (d <= 128) MI_DECODE_BAL(128, false, true);
-    else MI_DECODE_BAL(256, false, true);
-  } else if (d <= 64) MI_DECODE_BAL(64, false, false);
-  else if (d <= 128) MI_DECODE_BAL(128, false, false);
-  else MI_DECODE_BAL(256, false, false);
+    if (d == 128) MI_DECODE_BAL(128, false, true, true);
+    else if (d <= 64) MI_DECODE_BAL(64, false, true, false);
+    else if (d <= 128) MI_DECODE_BAL(128, false, true, false);
+    else MI_DECODE_BAL(256, false, true, false);
+  } else if (d == 128) MI_DECODE_BAL(128, false, false, true);
+  else if (d <= 64) MI_DECODE_BAL(64, false, false, false);
+  else if (d <= 128) MI_DECODE_BAL(128, false, false, false);
+  else MI_DECODE_BAL(256, false, false, false);
 #undef MI_DECODE_BAL
   MI_RETURN_LAUNCH_STATUS();
 }
