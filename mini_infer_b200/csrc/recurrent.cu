@@ -313,14 +313,12 @@ extern "C" int mi_rglru_scan(const float* gates, int M, int bw, const float* br,
 // ------------------------------------------------------------------------------------------
 struct RglruTerms { float a, b; };
 
-template <typename T>
-__device__ __forceinline__ RglruTerms rglru_terms(const float* g, int bw, float vbr, float vbi, float sp, const T* u,
-                                                  size_t row, int u_stride, int c) {
-  const float r = mi_sigmoid(g[0] + vbr), ig = mi_sigmoid(g[bw] + vbi);
+__device__ __forceinline__ RglruTerms rglru_terms(float gr, float gi, float sp, float u) {
+  const float r = mi_sigmoid(gr), ig = mi_sigmoid(gi);
   const float log_a = -sp * r;
   RglruTerms t;
   t.a = expf(log_a);
-  t.b = sqrtf(-expm1f(2.f * log_a)) * (ig * mi_to_float(u[row * u_stride + c]));
+  t.b = sqrtf(-expm1f(2.f * log_a)) * (ig * u);
   return t;
 }
 
@@ -352,18 +350,30 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
   if (seg == 0) carry[cl] = in ? st[(size_t)(taps - 1) * C + c] : 0.f;
   for (int t0 = 0; t0 < len; t0 += RU_SEG * RU_TOK) {
     const int first = t0 + seg * RU_TOK;
+    // what the eight tokens' (a, b) need is asked for before any of it is used, y behind that and ahead of the scan
     RglruTerms k[RU_TOK];
-    float yv[RU_TOK];
+    T uv[RU_TOK];
 #pragma unroll
     for (int i = 0; i < RU_TOK; ++i) {
       const int t = first + i;
-      k[i].a = 1.f;
-      k[i].b = 0.f;
-      yv[i] = 0.f;
+      k[i] = {0.f, 0.f};
+      uv[i] = T(0.f);
       if (in && t < len) {
-        k[i] = rglru_terms(g + (size_t)t * (2 * bw), bw, vbr, vbi, sp, u, (size_t)(row0 + t), u_stride, c);
-        yv[i] = mi_to_float(y[(size_t)(row0 + t) * y_stride + c]);
+        const float* gt = g + (size_t)t * (2 * bw);
+        k[i] = {gt[0], gt[bw]};
+        uv[i] = u[(size_t)(row0 + t) * u_stride + c];
       }
+    }
+    asm volatile("" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < RU_TOK; ++i) {
+      k[i] = rglru_terms(k[i].a + vbr, k[i].b + vbi, sp, mi_to_float(uv[i]));
+      if (first + i >= len) k[i] = {1.f, 0.f};
+    }
+#pragma unroll
+    for (int i = 0; i < RU_TOK; ++i) {
+      const int t = first + i;
+      uv[i] = (in && t < len) ? y[(size_t)(row0 + t) * y_stride + c] : T(0.f);
     }
     float A = 1.f, B = 0.f;
 #pragma unroll
@@ -399,7 +409,7 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
     for (int i = 0; i < RU_TOK; ++i) {
       const int t = first + i;
       S = fmaf(k[i].a, S, k[i].b);
-      if (in && t < len) out[(size_t)(row0 + t) * out_stride + c] = mi_from_float<T>(S * mi_gelu_tanh(yv[i] + yb));
+      if (in && t < len) out[(size_t)(row0 + t) * out_stride + c] = mi_from_float<T>(S * mi_gelu_tanh(mi_to_float(uv[i]) + yb));
     }
     __syncthreads();                                      // the folds are read before the next round's
   }
