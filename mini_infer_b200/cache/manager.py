@@ -41,6 +41,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import Hashable, Iterable, Sequence
 
+import numpy as np
 import torch
 
 
@@ -113,7 +114,19 @@ class AppendPlan:
     state_slots: list[int]
     start: list[int]                     # tokens held before the step, per request
     counts: list[int]                    # new tokens per request
-    token_slots: list[list[int]]         # per group: flat slot of every new token (all requests)
+    slot_parts: list[list]               # per group: flat slots of the new tokens, lists and (long portions) arrays in turn
+
+    @property
+    def token_slots(self) -> list[list[int]]:
+        """Per group: flat slot of every new token (all requests)."""
+        return [[int(x) for part in parts for x in part] for parts in self.slot_parts]
+
+    def slot_array(self, group: int) -> np.ndarray | list[int]:
+        """The same for one group, as one array (or a list, in a step of single tokens)."""
+        parts = self.slot_parts[group]
+        if len(parts) == 1:
+            return parts[0]
+        return np.concatenate([np.asarray(p, dtype=np.int64) for p in parts]) if parts else []
 
 
 def group_needs(needs: Sequence) -> list[GroupSpec]:
@@ -364,13 +377,15 @@ class CacheManager:
                     page = pool.allocate()
                     updates.extend((req.slot, len(table), page))
                     table.append(page)
-                slots = plan.token_slots[gi]
+                parts = plan.slot_parts[gi]
                 if n_new == 1:
-                    slots.append(table[start // ps] * ps + start % ps)
-                else:
-                    for idx in range(start // ps, -(-total // ps)):      # page by page
-                        base = table[idx] * ps
-                        slots.extend(range(base + max(0, start - idx * ps), base + min(ps, total - idx * ps)))
+                    if not parts or not isinstance(parts[-1], list):
+                        parts.append([])
+                    parts[-1].append(table[start // ps] * ps + start % ps)
+                else:                                                    # all pages at once
+                    first = start // ps
+                    pages = np.array(table[first:-(-total // ps)], dtype=np.int64)
+                    parts.append((pages[:, None] * ps + np.arange(ps)).reshape(-1)[start - first * ps:total - first * ps])
             req.length = total
         return plan
 

@@ -27,12 +27,13 @@ class KernelError(RuntimeError):
     pass
 
 
-def _ptr(t: torch.Tensor | None) -> c_void_p:
-    return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
+# (plain integers: every entry point that takes a pointer declares its argument types)
+def _ptr(t: torch.Tensor | None) -> int:
+    return t.data_ptr() if t is not None else 0
 
 
-def _stream() -> c_void_p:
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+def _stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _cuda(*tensors: torch.Tensor | None) -> None:

@@ -105,14 +105,16 @@ class StepRunner:
 
     # ------------------------------------------------------------------ planning
 
-    def _validate(self, entries: Sequence[StepEntry]) -> None:
+    def _validate(self, entries: Sequence[StepEntry]) -> list[np.ndarray | None]:
+        """Raise ``StepError`` for what a step cannot take; the token ids of the long portions as arrays."""
+        arrays: list[np.ndarray | None] = []
         if not entries:
             raise StepError("a step needs at least one entry")
         V = self.vocab_size
         for e in entries:
             if len(e.tokens) == 0:
                 raise StepError(f"request {e.rid!r}: no tokens in this step")
-            check = True
+            check, ids = True, None
             if len(e.tokens) > 8:                # a long portion: one pass, and the loop only to name the token
                 ids = np.asarray(e.tokens)
                 check = ids.dtype.kind not in "iu" or ids.min() < 0 or ids.max() >= V
@@ -120,6 +122,7 @@ class StepRunner:
                 for t in e.tokens:
                     if not 0 <= int(t) < V:
                         raise StepError(f"request {e.rid!r}: token id {t} is outside [0, {V})")
+            arrays.append(None if check else ids)
             for w in e.want:
                 if not 0 <= int(w) < len(e.tokens):
                     raise StepError(f"request {e.rid!r}: wanted place {w} is outside its {len(e.tokens)} tokens")
@@ -128,13 +131,14 @@ class StepRunner:
                     raise StepError(
                         f"request {e.rid!r} would pass the model's {self.max_positions} positions"
                     )
+        return arrays
 
     def host_plan(self, entries: Sequence[StepEntry], graphed: bool = False) -> HostPlan:
         """Reserve pages and lay the step's descriptors out in one host buffer (no device work).
 
         With ``graphed`` the layout depends only on the batch size: every list has a fixed
         length (one token per request, room for one new page per request and group)."""
-        self._validate(entries)
+        arrays = self._validate(entries)
         plan: AppendPlan = self.cache.plan_append([(e.rid, len(e.tokens)) for e in entries])
         updates = self.cache.take_table_updates()
         B = len(entries)
@@ -155,7 +159,8 @@ class StepRunner:
                     want_rows.append(i)
                     rows.append((e.rid, int(w)))
         else:
-            tokens = np.concatenate([np.asarray(e.tokens, dtype=np.int64) for e in entries])
+            tokens = np.concatenate([np.asarray(e.tokens if a is None else a, dtype=np.int64)
+                                     for e, a in zip(entries, arrays)])
             positions = np.concatenate([np.arange(plan.start[i], kv_len[i]) for i in range(B)])
             for i, e in enumerate(entries):
                 for w in e.want:
@@ -170,7 +175,7 @@ class StepRunner:
         n_groups = len(self.cache.groups)
         capacity, overflow = [0] * n_groups, [[] for _ in range(n_groups)]
         for gi, g in enumerate(self.cache.groups):
-            parts.append((f"slots{gi}", plan.token_slots[gi]))
+            parts.append((f"slots{gi}", plan.slot_array(gi)))
             flat = updates[gi]
             if graphed:
                 capacity[gi] = B
