@@ -733,7 +733,7 @@ __device__ __noinline__ void balanced_merge_unit(const float* __restrict__ part_
 }
 
 #define BAL_THREADS (NTHREADS + 64)   // four consumer warps, the copy warp, the store warp (ROPE only)
-// EXT: an instance of its own for kept keys and capped scores, so that the others keep their code.  EXACT: the head size is
+// EXT: an instance of its own for kept keys, capped scores and distance biases, so that the others keep their code.  EXACT: the head size is
 // DMAX, known to the compiler: the loops over it lose their conditions, of which a chunk's instructions were a good part.
 template <int DMAX, bool ROPE, bool EXT, bool EXACT>
 __global__ void __launch_bounds__(ROPE ? BAL_THREADS : DEC_THREADS, DMAX <= 128 ? 2 : 1)
@@ -745,10 +745,14 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
                                  int nkv, int d_any, float scale, int window, int min_chunks, int unit_cost,
                                  float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters,
                                  int* __restrict__ status, const float* __restrict__ rope_cs, int store_kv,
-                                 const float* __restrict__ sinks, int keep_any, float cap_k, float cap_h) {
+                                 const float* __restrict__ sinks, int keep_any, float cap_k, float cap_h,
+                                 const float* __restrict__ slopes) {
   const int keep = EXT ? keep_any : 0;
   const int d = EXACT ? DMAX : d_any;
   // sinks [nq] (optional): per head a score that joins the softmax's denominator with neither key nor value.
+  // slopes [nq] (optional, EXT, no cap): the scaled score of a key `dist` positions back is lowered by slopes[h] * dist
+  // (8 x 700 keys, 16 heads over 4 of 128: 14.9 + 6.5 us in attention_rows.cu and its merge, 8.1 here; a pass of 64
+  // steps with three such layer runs 26.2 -> 24.8 ms).
   // ROPE (the head size is then DMAX exactly): rope_cs holds per query token [d / 2] sines then
   // [d / 2] cosines of its rotary angles; q arrives un-rotated and is rotated here, in registers; and with store_kv
   // the block that reads a request's newest chunk rotates the new key, writes it and the new value into their page (they
@@ -1001,6 +1005,13 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
           }
       }
     }
+    // this lane's scores belong to heads 2 * t4 and 2 * t4 + 1
+    float slope[2] = {0.f, 0.f};
+    if (EXT && slopes) {
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh)
+        if (2 * t4 + hh < heads_here) slope[hh] = slopes[head0 + 2 * t4 + hh] * LOG2E;
+    }
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     float o[DMAX / 16][4];
 #pragma unroll
@@ -1055,6 +1066,12 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
           sa[1] = ok0 ? mi_softcap(sa[1], cap_k, cap_h) : -INFINITY;
           sa[2] = ok1 ? mi_softcap(sa[2], cap_k, cap_h) : -INFINITY;
           sa[3] = ok1 ? mi_softcap(sa[3], cap_k, cap_h) : -INFINITY;
+        } else if (EXT) {           // (without slopes the same numbers as below)
+          const float back0 = (float)(kl - 1 - j0), back1 = (float)(kl - 1 - j1);
+          sa[0] = ok0 ? fmaf(-slope[0], back0, sa[0] * sc) : -INFINITY;
+          sa[1] = ok0 ? fmaf(-slope[1], back0, sa[1] * sc) : -INFINITY;
+          sa[2] = ok1 ? fmaf(-slope[0], back1, sa[2] * sc) : -INFINITY;
+          sa[3] = ok1 ? fmaf(-slope[1], back1, sa[3] * sc) : -INFINITY;
         } else {
           sa[0] = ok0 ? sa[0] * sc : -INFINITY;
           sa[1] = ok0 ? sa[1] * sc : -INFINITY;
@@ -1073,7 +1090,10 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
           p[hh] = mi_fast_exp2(sa[hh] - m_new);
           p[2 + hh] = mi_fast_exp2(sa[2 + hh] - m_new);
           m_run[hh] = m_new;
-          l_run[hh] = l_run[hh] * alpha[hh] + (p[hh] + p[2 + hh]);
+          if (EXT && slopes)   // the denominator counts the weights as the second product reads them
+            l_run[hh] = l_run[hh] * alpha[hh] + (mi_to_float(__float2bfloat16_rn(p[hh])) + mi_to_float(__float2bfloat16_rn(p[2 + hh])));
+          else
+            l_run[hh] = l_run[hh] * alpha[hh] + (p[hh] + p[2 + hh]);
         }
         if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
@@ -1671,10 +1691,11 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
                                             const int* kv_len, int B, int nq, int nkv, int d, float scale, int window,
                                             int grid, float* part_o, float* part_ml, int* counters,
                                             const float* rope_cs, int store_kv, const float* sinks, int keep,
-                                            float softcap, cudaStream_t stream) {
+                                            float softcap, const float* slopes, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (keep < 0 || (keep && window < 0) || !(softcap >= 0.f)) MI_REFUSE("attention: bad kept keys %d or cap %f", keep, softcap);
   const float cap_k = softcap > 0.f ? scale / softcap : 0.f, cap_h = softcap * LOG2E;
+  if (slopes && softcap > 0.f) MI_REFUSE("attention: a distance bias or capped scores, not both");
   if (rope_cs && ((d != 64 && d != 128 && d != 256) || !mi_aligned(rope_cs, 4)))
     MI_REFUSE("attention: rotating inside the decode kernel needs a head size of 64, 128 or 256, got %d", d);
   if (int rc = check_common(q, q_stride, out, out_stride, kcache, vcache, nq, nkv, d, page_size, window)) return rc;
@@ -1695,14 +1716,15 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
               (bf16*)out, out_stride, (const bf16*)kcache, (const bf16*)vcache, block_table, bt_stride,   \
               table_rows, page_size, page_shift, q_start, kv_len, B, nq, nkv, d, scale, window, BAL_MIN_CHUNKS, \
               g_unit_cost, part_o, part_ml, counters, wait_status_ptr(), rope_cs, store_kv, sinks, keep,  \
-              cap_k, cap_h);                                                                              \
+              cap_k, cap_h, slopes);                                                                      \
   } while (0)
   if (rope_cs) {
-    if (keep || softcap > 0.f) MI_REFUSE("attention: the decode kernel that rotates takes neither kept keys nor a cap");
+    if (keep || softcap > 0.f || slopes)
+      MI_REFUSE("attention: the decode kernel that rotates takes neither kept keys nor a cap nor a distance bias");
     if (d == 64) MI_DECODE_BAL(64, true, false, true);
     else if (d == 128) MI_DECODE_BAL(128, true, false, true);
     else MI_DECODE_BAL(256, true, false, true);
-  } else if (keep || softcap > 0.f) {
+  } else if (keep || softcap > 0.f || slopes) {
     if (d == 128) MI_DECODE_BAL(128, false, true, true);
     else if (d <= 64) MI_DECODE_BAL(64, false, true, false);
     else if (d <= 128) MI_DECODE_BAL(128, false, true, false);

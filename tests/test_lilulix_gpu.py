@@ -572,3 +572,56 @@ def test_prompt_portions_on_the_tcgen05_kernel_with_sinks_and_slopes(nq, nkv, d,
     assert torch.isfinite(got).all()
     assert (got - want).abs().max() <= 2e-2 * max(1.0, want.abs().max())
     assert (got[n - 20:, 0] - k.double()[marked, 0]).abs().max() <= 2e-2 * 6.0
+
+
+@pytest.mark.parametrize("nq,nkv,d,page", [(32, 8, 128, 16), (9, 1, 128, 32), (3, 3, 64, 8), (12, 4, 48, 16), (2, 1, 16, 4)])
+def test_single_tokens_with_distance_bias_on_the_balanced_kernel(nq, nkv, d, page):
+    """Every request brings one token: contexts at the edges of a chunk of 64 keys and over many blocks, groups of one
+    head, of a head more than a block of heads takes, and odd ones, with and without sinks, against the plain softmax in
+    float64.  Weights are rounded to bfloat16 (2^-9 of every addend) and so is the result (2^-9); fp32 scores add far less."""
+    o = ops()
+    lens = [1, 63, 64, 65, 500, 2000, 17, 129]
+    per = nq // nkv
+    q = rnd(len(lens), nq, d, seed=3, scale=d ** -0.25).bfloat16()
+    ks = [rnd(n, nkv, d, seed=10 + i, scale=d ** -0.25).bfloat16() for i, n in enumerate(lens)]
+    vs = [rnd(n, nkv, d, seed=40 + i).bfloat16() for i, n in enumerate(lens)]
+    slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / nq) for h in range(nq)], dtype=torch.float64).float()
+    slopes[0] = 0.0
+    sinks = torch.linspace(-3.0, 3.0, nq)
+    width = -(-max(lens) // page)
+    pages = sum(-(-n // page) for n in lens)
+    kc = torch.full((pages, nkv, page, d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    vc = kc.clone()
+    table = torch.full((len(lens), width), -1, dtype=torch.int32)
+    slots, nxt = [], 0
+    for i, n in enumerate(lens):
+        for p in range(-(-n // page)):
+            table[i, p] = nxt
+            nxt += 1
+        slots += [int(table[i, t // page]) * page + t % page for t in range(n)]
+    # written by the kernel that the engine writes them with
+    rows = torch.cat([torch.cat(ks), torch.cat(vs)], dim=1).reshape(len(slots), -1)
+    packed = torch.cat([torch.zeros(len(slots), nq * d, dtype=torch.bfloat16), rows], dim=1).to(DEV)
+    o.qk_bias_norm_store(packed, 0, nq * d, (nq + nkv) * d, nq, nkv, d, d, q_bias=None, k_bias=None, q_gain=None,
+                         k_gain=None, eps=0.0, values_are_keys=False, slots=i32(slots), kcache=kc, vcache=vc)
+    qd = q.reshape(len(lens), nq * d).to(DEV)
+    for sink in (None, sinks):
+        out = torch.full((len(lens), nq * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        o.attention_decode_balanced(qd, qd.stride(0), out, kc, vc, table.to(DEV), page, i32(list(range(len(lens)))),
+                                    i32(lens), len(lens), nq, nkv, d, 0.9, slopes=slopes.to(DEV),
+                                    sinks=None if sink is None else sink.to(DEV))
+        assert o.attention_wait_status() == 0
+        got = out.cpu().double().reshape(len(lens), nq, d)
+        for i, n in enumerate(lens):
+            back = torch.arange(n - 1, -1, -1, dtype=torch.float64)
+            for h in range(nq):
+                s = ks[i][:, h // per].double() @ q[i, h].double() * 0.9 - slopes[h].double() * back
+                v = vs[i][:, h // per].double()
+                if sink is None:
+                    want = torch.softmax(s, 0) @ v
+                else:
+                    want = torch.softmax(torch.cat([s, sink[h:h + 1].double()]), 0)[:n] @ v
+                assert (got[i, h] - want).abs().max() <= 1.25 * 2.0 ** -8 * v.abs().max(), (i, h)
+    with pytest.raises(o.KernelError):        # one or the other
+        o.attention_decode_balanced(qd, qd.stride(0), out, kc, vc, table.to(DEV), page, i32(list(range(len(lens)))),
+                                    i32(lens), len(lens), nq, nkv, d, 0.9, slopes=slopes.to(DEV), softcap=20.0)
