@@ -1034,11 +1034,12 @@ def sample(
 
 
 TMA_GEMM_MAX_ROWS = 128            # what gemm_tma.cu takes
-# ``linear`` routes inputs of up to this many rows to gemm_tma.  Measured on a B200 inside a
-# captured decode step (Llama 3.1 8B sizes, milliseconds per step, own product against the
-# library's): up to 16 rows the own product is ahead, because it marks the weights to leave the
-# L2 first and does the block's additions and norms in its epilogues (batch 8: 3.74 vs 4.05;
-# batch 16: 4.17 vs 4.42); from 32 rows on the library is (5.23 vs 5.15; 64 rows: 7.34 vs 6.63).
+# ``linear`` routes inputs of up to this many rows, all that gemm_rows takes, to it; the library takes larger ones.
+# Measured on a B200 inside a captured decode step (Llama 3.1 8B sizes, milliseconds per step, own
+# product (gemm_tma) against the library's): up to 16 rows the own product is ahead, because it marks the weights
+# to leave the L2 first and does the block's additions and norms in its epilogues (batch 8: 3.74 vs 4.05;
+# batch 16: 4.17 vs 4.42; gemm_rows is another 16 us per layer ahead); from 32 rows on the library is (5.23 vs
+# 5.15; 64 rows: 7.34 vs 6.63).
 TMA_GEMM_DISPATCH_ROWS = 16
 USE_TMA_GEMM = os.environ.get("MINI_INFER_TMA_GEMM", "1") != "0"
 _tma_ws: dict[int, list[tuple[torch.Tensor, torch.Tensor]]] = {}
@@ -1058,7 +1059,7 @@ def _tma_workspace(device: torch.device, floats: int, counters: int) -> tuple[to
 
 
 def gemm_tma_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether ``gemm_tma`` takes these operands (few rows, 16-byte aligned rows)."""
+    """Whether ``gemm_tma``, and up to 16 rows ``gemm_rows``, takes these operands (few rows, 16-byte aligned rows)."""
     return (x.dim() == 2 and w.dim() == 2 and 0 < x.shape[0] <= TMA_GEMM_MAX_ROWS and x.shape[1] % 8 == 0
             and x.stride(1) == 1 and w.is_contiguous() and (x.shape[0] == 1 or x.stride(0) % 8 == 0)
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -1197,7 +1198,7 @@ def fused_norms_enabled() -> bool:
 
 
 def linear_fusable(n_rows: int, w: torch.Tensor) -> bool:
-    """Whether a product of ``n_rows`` rows with ``w`` has the fused forms of ``gemm_tma``
+    """Whether a product of ``n_rows`` rows with ``w`` has the fused forms of ``gemm_rows``
     (``row_stats`` on its input side, ``linear_into_stream`` on its output side)."""
     return (fused_norms_enabled() and 0 < n_rows <= min(TMA_GEMM_DISPATCH_ROWS, TMA_GEMM_FUSED_ROWS)
             and w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous()
@@ -1220,9 +1221,9 @@ def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, row_stats: "RowStats |
                   act: str = "silu") -> torch.Tensor:
     """``act(x Wg^T) * (x Wu^T)`` for a merged projection whose rows alternate gate, up
     (``w_pairs [2 I, K]``); ``act`` is ``"silu"`` or ``"gelu_tanh"``.  Decode-sized bfloat16 inputs
-    run the product and the activation as one kernel (gemm_tma with its gate/up epilogue);
+    run the product and the activation as one kernel (gemm_rows with its gate/up epilogue);
     everything else runs ``linear`` and an activation-and-multiply kernel on the interleaved
-    result.  ``row_stats``: see ``gemm_tma``."""
+    result.  ``row_stats``: see ``RowStats``."""
     if act not in GLU_ACT:
         raise KernelError(f"linear_swiglu: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
@@ -1270,7 +1271,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     kernel before it still runs; other bfloat16 operands use the library product with fp32
     accumulation, as the reference does for every linear layer (``distributed/linear.py:167``).
     ``out_dtype=float32`` keeps the accumulator's precision in the result (used for logits).
-    ``row_stats`` (streaming product only): see ``gemm_tma``.
+    ``row_stats`` (streaming product only): see ``RowStats``.
     """
     global _MM_OUT_DTYPE, launch_count
     if row_stats is not None:

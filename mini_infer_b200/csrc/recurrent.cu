@@ -75,7 +75,7 @@ __global__ void causal_conv_kernel(const T* __restrict__ x, int x_stride, const 
 
 // The same with two to four taps on whole 16-byte pieces: a thread keeps the last taps-1 inputs of its 4 or 8
 // channels in registers and walks `tile` tokens, so every input is read once per tile instead of once per tap
-// (2048 tokens of 12288 bfloat16 channels: 93 us element by element; DRAM floor 16 us).
+// (2048 tokens of 12288 bfloat16 channels: 93 us element by element, 42 now; DRAM floor 16 us).
 template <typename T>
 struct ConvPiece;
 template <>
@@ -308,8 +308,8 @@ extern "C" int mi_rglru_scan(const float* gates, int M, int bw, const float* br,
 // channel scans the 32 folds, and every thread walks its eight tokens from the state it then knows.  (Blocks of twice the
 // threads leave room for one per SM: 160 blocks of 2560 channels then run in two turns.)  What bounds it is
 // the arithmetic of the gates (five exponentials, two divisions, a root per token and channel), which is done
-// once; two passes of one thread per 64 tokens did it twice and stood still for their loads (2048 tokens of 2560
-// channels: 60 + 90 us).
+// once; two passes of one thread per 64 tokens did it twice and stood still for their loads (2000 tokens of 2560
+// channels: 60 + 90 us; 118 with a round's loads where they are used, 68 with all of them first).
 // ------------------------------------------------------------------------------------------
 struct RglruTerms { float a, b; };
 
