@@ -499,7 +499,11 @@ static int mma_vec_ok(const void* a, long long a_stride, const void* w0, const v
 // lane's fragments come straight from global memory, 16 bytes (8 consecutive k, taken as the k of two instructions in
 // an order that is the same for both operands) at a time, two pieces of k, 16 loads, in flight: with one warp per output
 // column and fused multiply-adds the same 630 MB (25 experts of 3 x 1024 x 4096) took 179 us, 0.54 of the copy
-// bandwidth, most of it conversions and the columns' short lives.  bfloat16, k a multiple of 8, 16-byte aligned rows.
+// bandwidth, most of it conversions and the columns' short lives, and takes 114 here (102 of bytes).
+// An instruction adds its 16 products to nothing; what it gives is added up pairwise in fp32, the warps' shares in fp64: the
+// accumulator of a chain of instructions loses more than an fp32 addition does (distance from 64 bits at K = 512, 1024 and
+// 2816: 8.6, 12.9 and 32.8e-8 as one chain, 5.0, 5.6 and 6.7e-8 so, 6.2, 7.0 and 8.5e-8 by fused multiply-adds; 113 us as
+// one chain).  bfloat16, k a multiple of 8, 16-byte aligned rows.
 #define MR_WARPS 8
 #define MR_PIECE 64
 __device__ __forceinline__ uint4 mr_load(const bf16* p, bool in) {       // weights: read once
@@ -554,17 +558,28 @@ moe_rows_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict
         x[p][s] = in && has_x ? __ldg(reinterpret_cast<const uint4*>(xp + k)) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+    for (int h = 0; h < 2; ++h) {
+      float sum[2][4];
 #pragma unroll
-      for (int s = 0; s < 2; ++s)
+      for (int p = 0; p < 2; ++p) {
+        float t[2][4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int s = 0; s < 2; ++s) {
           const uint4 u = w[p][s][h][0], v = w[p][s][h][1], xx = x[p][s];
           const uint32_t a0[4] = {u.x, v.x, u.y, v.y}, b0[2] = {xx.x, xx.y};
           const uint32_t a1[4] = {u.z, v.z, u.w, v.w}, b1[2] = {xx.z, xx.w};
-          mma_bf16(acc[h], a0, b0);
-          mma_bf16(acc[h], a1, b1);
+          float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16(d0, a0, b0);
+          mma_bf16(d1, a1, b1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) t[s][i] = d0[i] + d1[i];
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[p][i] = t[0][i] + t[1][i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[h][i] += sum[0][i] + sum[1][i];
+    }
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h)
@@ -573,9 +588,10 @@ moe_rows_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict
   __syncthreads();
   const int r = tid >> 5, j = tid & 31;       // a warp per row of x
   if (r >= rows) return;
-  float v = 0.f;
+  double all = 0.0;
 #pragma unroll
-  for (int s = 0; s < MR_WARPS; ++s) v += shares[s][r][j];
+  for (int s = 0; s < MR_WARPS; ++s) all += shares[s][r][j];
+  const float v = (float)all;
   if (GATED) {
     const float up = __shfl_down_sync(0xffffffffu, v, 16);
     if (j < 16 && n0 + j < N)

@@ -421,6 +421,36 @@ def test_convolution_and_recurrent_unit_in_long_portions(C, bw, taps, act, porti
     assert torch.equal(state[1, :taps - 1].cpu(), (x.float() + xb)[Tn - (taps - 1):])
 
 
+@pytest.mark.parametrize("K", [256, 520, 1024, 2816, 8192])
+def test_experts_of_few_rows_sum_as_fp32_would(K):
+    """The fp32 result of the streaming product of few rows against float64.  Summing K products one by one in fp32 is off
+    by about 2^-25 of the running sums, sqrt(K / 2) of a typical result: 32 chains of K / 32 fused multiply-adds and a tree over
+    them, the order that an fp32 product of this kind has, are imitated here, and the kernel may be off by no more (an
+    accumulator of tensor-core instructions carried through all of k is off by 1.4 times that at K = 512 and 4 at 2816)."""
+    E, rows, H = 3, 8, 128
+    a = rnd(E * rows, K, seed=90).bfloat16()
+    w = rnd(E, H, K, seed=91, scale=K ** -0.5).bfloat16()
+    plan = torch.tensor([E] + [rows * e for e in range(E + 1)] + [x for e in range(E) for x in (e, rows * e, rows)]
+                        + [0] * (3 * E), dtype=torch.int32, device=DEV)
+    y = torch.empty(E * rows, H, device=DEV)
+    ad, wd = a.to(DEV), w.to(DEV)
+    lib = ops()._lib("moe")
+    rc = lib.mi_moe_down(ad.data_ptr(), wd.data_ptr(), H * K, plan.data_ptr(), E, y.data_ptr(), E * rows, H, K, 8, 1,
+                         torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    prod = (a.double().reshape(E, rows, 1, K) * w.double().reshape(E, 1, H, K)).reshape(E * rows, H, K)
+    want = prod.sum(dim=-1)
+    pad = -K % 256
+    lanes = torch.nn.functional.pad(prod, (0, pad)).reshape(E * rows, H, -1, 32, 8).permute(0, 1, 3, 2, 4).flatten(3)
+    acc = torch.zeros(E * rows, H, 32)
+    for i in range(lanes.shape[-1]):            # a product of two bfloat16 is exact, so this rounds as a fused multiply-add
+        acc = (acc.double() + lanes[..., i]).float()
+    while acc.shape[-1] > 1:
+        acc = acc[..., ::2] + acc[..., 1::2]
+    fp32 = (acc[..., 0].double() - want).norm()
+    assert (y.cpu().double() - want).norm() <= fp32
+
+
 @pytest.mark.parametrize("E,top,ff,H,M", [(5, 2, 24, 40, 33), (3, 1, 20, 48, 5), (4, 4, 16, 36, 70), (12, 3, 72, 64, 200),
                                           (6, 2, 24, 40, 7), (3, 3, 16, 64, 8), (16, 1, 8, 264, 100)])
 @pytest.mark.parametrize("dtype,bound", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2)])
