@@ -574,11 +574,14 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 //
 // A block's rows are cut into tiles of at most 64 rows of equal size (the output head: 14 tiles).  What bounds it: the
 // stream of W, and about 2 us from the launch before to the first sum and from the last byte to the last store.  The four
-// products of a layer behind one another, gemm_tma_kernel against this one: one token at Llama 3.1 8B sizes 87.6 and
+// products of a layer behind one another, gemm_tma_kernel against this one: eight tokens at Llama 3.1 8B sizes 87.6 and
 // 71.4 us (67 of bytes), at 2048 wide (8192 and 3072 features in between) 36.7 and 20.2 us.  Other forms at those 2048: x by
-// plain loads into registers 28, one issuing lane 26.0, boxes of x always 8 rows high 25.4 (one token); a ring of 56 to 216 KB: 200 best.
-// stats_in and
-// stats_out of EpilogueFusion hold one row of 16 sums per block here instead of one per 128 features.
+// plain loads into registers 28, one issuing lane 26.0; with one token 18.7, boxes of x always 8 rows high 25.4; a ring of 56
+// to 216 KB: 200 best.
+// A chain of instructions ends after 64 k and is added to the sum in fp32.  Distance from 64 bits, one chain through all of
+// k, chains of 64, and gemm_tma_kernel: 2048 x 2048 2.4, 0.9 and 2.4e-7, 2048 x 8192 10.0, 1.2 and 9.1e-7, 4096 x 14336 18.1,
+// 1.3 and 38.1e-7; the time is the same (a layer of eight tokens at 8B sizes 70.8 and 70.8 us).
+// stats_in and stats_out of EpilogueFusion hold one row of 16 sums per block here instead of one per 128 features.
 // ------------------------------------------------------------------------------------------
 #define GR_WARPS 8
 #define GR_THREADS (32 * (GR_WARPS + 1))
@@ -738,11 +741,20 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             uint32_t af[4][4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) gr_ldmatrix_x4(af[k], wa + l * 128 + (((a_chunk + 2 * k) ^ (l & 7)) << 4));
+            float part[NT][4];                 // added up in fp32: the accumulator of a longer chain loses more
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) part[t][e] = 0.f;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
               for (int t = 0; t < NT; ++t)
-                gr_mma(acc[m][t], af[k][0], af[k][1], af[k][2], af[k][3], bf[t][k >> 1][(k & 1) * 2], bf[t][k >> 1][(k & 1) * 2 + 1]);
+                gr_mma(part[t], af[k][0], af[k][1], af[k][2], af[k][3], bf[t][k >> 1][(k & 1) * 2], bf[t][k >> 1][(k & 1) * 2 + 1]);
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) acc[m][t][e] += part[t][e];
           }
         }
       }

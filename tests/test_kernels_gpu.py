@@ -361,6 +361,16 @@ def test_gemm_rows_every_form(M, N, K):
     assert ops().gemm_tma_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 512, 4096), (8, 2048, 2048), (8, 2048, 5632), (8, 2048, 8192), (1, 4096, 14336), (8, 24, 16384)])
+def test_gemm_rows_is_no_further_from_64_bits_than_gemm_tma(M, N, K):
+    """Whichever of the two kernels takes a product of few rows, its fp32 sums may be no worse than the other's, whose
+    chains of instructions are short where N is small (k is then cut over many blocks)."""
+    x, w = rnd(M, K, dtype=torch.bfloat16, seed=70).to(DEV), rnd(N, K, dtype=torch.bfloat16, seed=71, scale=K ** -0.5).to(DEV)
+    want = x.double() @ w.double().T
+    rows, tma = ((f(x, w, torch.float32).double() - want).norm() for f in (ops().gemm_rows, ops().gemm_tma))
+    assert rows <= tma
+
+
 def test_gemm_rows_refuses_what_it_cannot_take():
     w = rnd(64, 64, dtype=torch.bfloat16, seed=65).to(DEV)
     with pytest.raises(ops().KernelError, match="at most 16"):
