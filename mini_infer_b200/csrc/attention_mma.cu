@@ -694,36 +694,42 @@ __device__ __noinline__ void balanced_merge_unit(const float* __restrict__ part_
                                                  int unit, int g_first, int g_last, int r, int c4, int d,
                                                  bf16* __restrict__ orow, float sink_l2) {
   // sink_l2: a score (times log2 e) that joins the denominator without a key or a value; minus infinity: none
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + (size_t)unit * DEC_HEADS + r;
   float mm = -INFINITY, L = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 v[8];
+  float4 o[8];
+  auto load = [&](int gb) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int g = min(gb + k, g_last);
+      v[k] = __ldcg(ml + (size_t)g * DEC_HEADS);
+      o[k] = __ldcg(reinterpret_cast<const float4*>(part_o + (((size_t)unit + g) * DEC_HEADS + r) * d + c4));
+    }
+  };
+  load(g_first);
 #pragma unroll 1
-  for (int gb = g_first; gb <= g_last; gb += 8) {
-    float2 v[8];
-    float4 o[8];
+  for (int gb = g_first + 8; gb <= g_last; gb += 16) {      // the other stretches' maxima, beside the first ones' columns
+    float m[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) m[k] = __ldcg(ml + (size_t)min(gb + k, g_last) * DEC_HEADS).x;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) mm = fmaxf(mm, m[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) mm = fmaxf(mm, v[k].x);
+  for (int gb = g_first;;) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const size_t slot = ((size_t)unit + min(gb + k, g_last)) * DEC_HEADS + r;
-      v[k] = __ldcg(reinterpret_cast<const float2*>(part_ml) + slot);
-      o[k] = __ldcg(reinterpret_cast<const float4*>(part_o + slot * d + c4));
-    }
-    float m = mm;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (gb + k > g_last) v[k] = make_float2(-INFINITY, 0.f);
-      m = fmaxf(m, v[k].x);
-    }
-    const float keep = mm == -INFINITY ? 0.f : exp2f(mm - m);
-    L *= keep;
-    acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
-    mm = m;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (v[k].x == -INFINITY) continue;       // (a stretch without a visible key holds nothing)
-      const float f = exp2f(v[k].x - mm);
+      const float f = gb + k > g_last || v[k].x == -INFINITY ? 0.f : exp2f(v[k].x - mm);
+      if (f == 0.f) continue;                    // (a stretch without a visible key holds nothing)
       L = fmaf(v[k].y, f, L);
-      acc.x = fmaf(f, o[k].x, acc.x); acc.y = fmaf(f, o[k].y, acc.y);
-      acc.z = fmaf(f, o[k].z, acc.z); acc.w = fmaf(f, o[k].w, acc.w);
+      acc.x = __fadd_rn(acc.x, __fmul_rn(f, o[k].x)); acc.y = __fadd_rn(acc.y, __fmul_rn(f, o[k].y));
+      acc.z = __fadd_rn(acc.z, __fmul_rn(f, o[k].z)); acc.w = __fadd_rn(acc.w, __fmul_rn(f, o[k].w));
     }
+    gb += 8;
+    if (gb > g_last) break;
+    load(gb);
   }
   if (sink_l2 != -INFINITY && mm != -INFINITY) L += exp2f(sink_l2 - mm);
   const float inv = L > 0.f ? 1.f / L : 0.f;
@@ -1691,8 +1697,11 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
                                             const int* kv_len, int B, int nq, int nkv, int d, float scale, int window,
                                             int grid, float* part_o, float* part_ml, int* counters,
                                             const float* rope_cs, int store_kv, const float* sinks, int keep,
-                                            float softcap, const float* slopes, cudaStream_t stream) {
+                                            float softcap, const float* slopes, int min_chunks, cudaStream_t stream) {
+  // min_chunks: the least chunks of a stretch; 0: BAL_MIN_CHUNKS.  The cuts decide the order of the sums.
   if (B <= 0) return 0;
+  if (min_chunks < 0) MI_REFUSE("attention: stretches of at least %d chunks", min_chunks);
+  if (min_chunks == 0) min_chunks = BAL_MIN_CHUNKS;
   if (keep < 0 || (keep && window < 0) || !(softcap >= 0.f)) MI_REFUSE("attention: bad kept keys %d or cap %f", keep, softcap);
   const float cap_k = softcap > 0.f ? scale / softcap : 0.f, cap_h = softcap * LOG2E;
   if (slopes && softcap > 0.f) MI_REFUSE("attention: a distance bias or capped scores, not both");
@@ -1714,7 +1723,7 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
     }                                                                                                     \
     MI_LAUNCH((kern), grid, ROPE ? BAL_THREADS : DEC_THREADS, smem, stream, (const bf16*)q, q_stride,     \
               (bf16*)out, out_stride, (const bf16*)kcache, (const bf16*)vcache, block_table, bt_stride,   \
-              table_rows, page_size, page_shift, q_start, kv_len, B, nq, nkv, d, scale, window, BAL_MIN_CHUNKS, \
+              table_rows, page_size, page_shift, q_start, kv_len, B, nq, nkv, d, scale, window, min_chunks, \
               g_unit_cost, part_o, part_ml, counters, wait_status_ptr(), rope_cs, store_kv, sinks, keep,  \
               cap_k, cap_h, slopes);                                                                      \
   } while (0)

@@ -23,7 +23,7 @@
 // Three products live here, all with fp32 accumulation, and none lets a row's result depend on which
 // other rows share its tile: float32 on CUDA cores, k ascending (moe_gemm_kernel); bfloat16 tiles of 64
 // rows on the tensor cores (mma.sync m16n8k16, moe_gemm_mma_kernel); bfloat16 tiles of 8 rows that
-// stream an expert's weights past the tensor cores (moe_rows_kernel).  Large bfloat16 steps
+// stream an expert's weights (moe_rows_kernel on the tensor cores, moe_stream_kernel on CUDA cores in a kept order).  Large bfloat16 steps
 // whose rows are whole 16-byte pieces go to the library's grouped product instead (the caller gathers
 // the rows with mi_moe_gather and passes the experts' row ranges from the plan).
 #include "common.cuh"
@@ -494,25 +494,169 @@ static int mma_vec_ok(const void* a, long long a_stride, const void* w0, const v
 
 // ------------------------------------------------------------------------------------------ few rows per expert
 // A decode step brings an expert a handful of rows: the product is a stream of that expert's weights.  Tiles have at
-// most FEW_ROWS rows, which are the N side of mma.sync.m16n8k16; a block owns 16 rows of both gated matrices (or 32 of
-// the plain one), the M side, and its eight warps take the 64-wide pieces of k in turn and add up in shared memory.  A
-// lane's fragments come straight from global memory, 16 bytes (8 consecutive k, taken as the k of two instructions in
-// an order that is the same for both operands) at a time, two pieces of k, 16 loads, in flight: with one warp per output
-// column and fused multiply-adds the same 630 MB (25 experts of 3 x 1024 x 4096) took 179 us, 0.54 of the copy
-// bandwidth, most of it conversions and the columns' short lives, and takes 114 here (102 of bytes).
-// An instruction adds its 16 products to nothing; what it gives is added up pairwise in fp32, the warps' shares in fp64: the
-// accumulator of a chain of instructions loses more than an fp32 addition does (distance from 64 bits at K = 512, 1024 and
-// 2816: 8.6, 12.9 and 32.8e-8 as one chain, 5.0, 5.6 and 6.7e-8 so, 6.2, 7.0 and 8.5e-8 by fused multiply-adds; 113 us as
-// one chain).  bfloat16, k a multiple of 8, 16-byte aligned rows.
-#define MR_WARPS 8
-#define MR_PIECE 64
-__device__ __forceinline__ uint4 mr_load(const bf16* p, bool in) {       // weights: read once
+// most FEW_ROWS rows.  A warp owns pairs of weight rows (gate and up of a column, or two columns of the plain product);
+// lane l takes the 16-byte pieces of k at 8 l, 8 l + 256, ... of both, one fused multiply-add after the other, and the
+// lanes' sums are added by butterfly.  That order is the result's, whatever rows share the tile.
+//
+// What bounds it is the stream of weights.  A warp's pairs are one list of pieces, fetched a batch ahead of the batch that
+// is worked on, so that it does not stand still at the end of a column: a warp per pair without the batch ahead took 179 us
+// for 630 MB (25 experts of 3 x 1024 x 4096), 0.54 of the copy bandwidth, and this takes 129 (2048 wide, 19 experts of
+// 3 x 512 x 2048: 48 and 43).  It is run where a result's order of sums is kept from one version of these kernels to the next
+// (`in_order` of the entry points); moe_rows_kernel below takes the other calls.
+// bfloat16, k a multiple of 8, 16-byte aligned rows.
+#define MS_WARPS 8
+#define MS_UNITS 16       // a warp gets as many pairs as make up this many pieces of 256 k (8, 32: 139 and 124 us, 41 and 52)
+__device__ __forceinline__ uint4 ms_load(const bf16* p, bool in) {       // weights: read once
   uint4 v = make_uint4(0u, 0u, 0u, 0u);
   if (in) asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];\n"
                        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+__device__ __forceinline__ void ms_unpack(const uint4& v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
 
+// the pairs [pair0, pair0 + n_pairs) of a warp for R rows of x, of which `rows` exist
+template <bool GATED, int R>
+__device__ __forceinline__ void moe_stream_pairs(const bf16* __restrict__ a, int a_stride, const bf16* __restrict__ w0,
+                                                 const bf16* __restrict__ w1, const int* __restrict__ perm, int top, int row0,
+                                                 int rows, void* __restrict__ out_, int N, int K, int pair0, int n_pairs,
+                                                 float limit, float alpha, float offset) {
+  constexpr int BATCH = R <= 4 ? 4 : 2;
+  const int lane = threadIdx.x & 31;
+  const int pieces = (K + 255) >> 8, units = n_pairs * pieces;
+  const bf16* xr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int row = row0 + min(r, rows - 1);
+    xr[r] = a + (size_t)(GATED ? perm[row] / top : row) * a_stride + lane * 8;
+  }
+  float acc0[R], acc1[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc0[r] = acc1[r] = 0.f;
+
+  int l_pair = pair0, l_piece = 0;             // the next unit to be fetched
+  auto fetch = [&](uint4 (&w)[BATCH][2]) {
+#pragma unroll
+    for (int b = 0; b < BATCH; ++b) {
+      const int k = l_piece * 256 + lane * 8;
+      const bool in = l_pair < pair0 + n_pairs && k < K;
+      const int n_a = GATED ? l_pair : 2 * l_pair, n_b = GATED ? l_pair : min(2 * l_pair + 1, N - 1);
+      w[b][0] = ms_load(w0 + (size_t)n_a * K + k, in);
+      w[b][1] = ms_load((GATED ? w1 : w0) + (size_t)n_b * K + k, in);
+      if (++l_piece == pieces) {
+        l_piece = 0;
+        ++l_pair;
+      }
+    }
+  };
+  uint4 w[BATCH][2], next[BATCH][2];
+  fetch(w);
+  int pair = pair0, piece = 0;
+#pragma unroll 1
+  for (int u0 = 0; u0 < units; u0 += BATCH) {
+    fetch(next);
+#pragma unroll
+    for (int b = 0; b < BATCH; ++b) {
+      if (u0 + b < units) {
+        const int k = piece * 256 + lane * 8;
+        float wa[8], wb[8];
+        ms_unpack(w[b][0], wa);
+        ms_unpack(w[b][1], wb);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float x[8];
+          ms_unpack(k < K ? __ldg(reinterpret_cast<const uint4*>(xr[r] + piece * 256)) : make_uint4(0u, 0u, 0u, 0u), x);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            acc0[r] = fmaf(wa[i], x[i], acc0[r]);
+            acc1[r] = fmaf(wb[i], x[i], acc1[r]);
+          }
+        }
+        if (++piece == pieces) {               // the pair is done: a lane per row stores it
+          float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const float t0 = mi_warp_sum(acc0[r]), t1 = mi_warp_sum(acc1[r]);
+            if (lane == r) {
+              s0 = t0;
+              s1 = t1;
+            }
+            acc0[r] = acc1[r] = 0.f;
+          }
+          if (lane < rows) {
+            if (GATED) {
+              reinterpret_cast<bf16*>(out_)[(size_t)(row0 + lane) * N + pair] =
+                  __float2bfloat16_rn(mi_clamped_glu_value(s0, s1, limit, alpha, offset));
+            } else {
+              float* o = reinterpret_cast<float*>(out_) + (size_t)(row0 + lane) * N + 2 * pair;
+              o[0] = s0;
+              if (2 * pair + 1 < N) o[1] = s1;
+            }
+          }
+          piece = 0;
+          ++pair;
+        }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < BATCH; ++b) {
+      w[b][0] = next[b][0];
+      w[b][1] = next[b][1];
+    }
+  }
+}
+
+template <bool GATED>
+__global__ void __launch_bounds__(32 * MS_WARPS, 2)
+moe_stream_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict__ w0, const bf16* __restrict__ w1,
+                  long long w_expert_stride, const int* __restrict__ perm, int top, const int* __restrict__ plan,
+                  int E, void* __restrict__ out_, int N, int K, int pairs_per_warp, float limit, float alpha, float offset) {
+  mi_pdl_enter();
+  const int tile = blockIdx.y;
+  if (tile >= plan[0]) return;
+  const int* td = plan + 2 + E + 3 * tile;
+  const int e = td[0], row0 = td[1], rows = td[2];
+  const int n_all = GATED ? N : (N + 1) / 2, pair0 = (blockIdx.x * MS_WARPS + (threadIdx.x >> 5)) * pairs_per_warp;
+  const int n_pairs = min(pairs_per_warp, n_all - pair0);
+  if (n_pairs <= 0) return;
+  const bf16* e0 = w0 + (size_t)e * w_expert_stride;
+  const bf16* e1 = GATED ? w1 + (size_t)e * w_expert_stride : nullptr;
+#define MI_GO(R) \
+  moe_stream_pairs<GATED, R>(a, a_stride, e0, e1, perm, top, row0, rows, out_, N, K, pair0, n_pairs, limit, alpha, offset)
+  if (rows <= 1) MI_GO(1);
+  else if (rows <= 2) MI_GO(2);
+  else if (rows <= 4) MI_GO(4);
+  else MI_GO(8);
+#undef MI_GO
+}
+// Pairs of weight rows per warp: MS_UNITS pieces, or fewer so that small products still fill the chip.
+static int stream_pairs(int K, int n_pairs, int n_entries) {
+  const int pieces = (K + 255) / 256;
+  const long long fill = (long long)n_pairs * n_entries / (2 * 148 * MS_WARPS);
+  const int most = pieces >= MS_UNITS ? 1 : MS_UNITS / pieces;
+  return fill < 1 ? 1 : fill < most ? (int)fill : most;
+}
+static int stream_blocks(int n_pairs, int per_warp) { return (n_pairs + MS_WARPS * per_warp - 1) / (MS_WARPS * per_warp); }
+
+// The same on the tensor cores.  The tile's rows are the N side of mma.sync.m16n8k16; a block owns 16 rows of both gated
+// matrices (or 32 of the plain one), the M side, and its eight warps take the 64-wide pieces of k in turn and add up in
+// shared memory.  A lane's fragments come straight from global memory, 16 bytes (8 consecutive k, taken as the k of two
+// instructions in an order that is the same for both operands) at a time, two pieces of k, 16 loads, in flight.  What bounds
+// it is the stream of weights; gate/up and down of 64 experts of 3 x 1024 x 4096, four each, here and by moe_stream_kernel:
+// 8 tokens 114 and 129 us (102 of bytes), 32 tokens 224 and 320, 128 tokens 311 and 810.
+// An instruction adds its 16 products to nothing; what it gives is added up pairwise in fp32, the warps' shares in fp64: the
+// accumulator of a chain of instructions loses more than an fp32 addition does (distance from 64 bits at K = 512, 1024 and
+// 2816: 8.6, 12.9 and 32.8e-8 as one chain, 5.0, 5.6 and 6.7e-8 so, 6.2, 7.0 and 8.5e-8 by fused multiply-adds), and the time
+// is the same to one part in a hundred.  bfloat16, k a multiple of 8, 16-byte aligned rows.
+#define MR_WARPS 8
+#define MR_PIECE 64
+#define MR_LEAST_K 256     // below, what an instruction cuts off its own sum is not made up: 4.1 against 3.9e-8 at K = 64
 template <bool GATED>
 __global__ void __launch_bounds__(32 * MR_WARPS, 2)
 moe_rows_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict__ w0, const bf16* __restrict__ w1,
@@ -554,7 +698,7 @@ moe_rows_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int r = 0; r < 2; ++r) w[p][s][h][r] = mr_load(wp[h][r] + k, in);
+          for (int r = 0; r < 2; ++r) w[p][s][h][r] = ms_load(wp[h][r] + k, in);
         x[p][s] = in && has_x ? __ldg(reinterpret_cast<const uint4*>(xp + k)) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
@@ -607,15 +751,21 @@ static int max_tiles(int n_entries, int E, int tile_rows) { return (n_entries + 
 extern "C" int mi_moe_gate_up(const void* x, int x_stride, const void* w_gate, const void* w_up,
                               long long w_expert_stride, const int* perm, int top, const int* plan, int E,
                               void* act, int n_entries, int ff, int H, float limit, float alpha, float offset,
-                              int tile_rows, int dtype, cudaStream_t stream) {
+                              int tile_rows, int in_order, int dtype, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (tile_rows == FEW_ROWS) {
     if (dtype != MI_DTYPE_BF16 || !mma_vec_ok(x, x_stride, w_gate, w_up, H))
       MI_REFUSE("moe: the streaming product takes bfloat16 rows of whole 16-byte pieces");
-    dim3 g((ff + 15) / 16, max_tiles(n_entries, E, FEW_ROWS));
+    const int per_warp = stream_pairs(H, ff, n_entries);
+    const bool stream_it = in_order || H < MR_LEAST_K;
+    dim3 g(stream_it ? stream_blocks(ff, per_warp) : (ff + 15) / 16, max_tiles(n_entries, E, FEW_ROWS));
     if (g.y > 65535) MI_REFUSE("moe: too many row tiles for one launch");
-    MI_LAUNCH((moe_rows_kernel<true>), g, 32 * MR_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
-              (const bf16*)w_up, w_expert_stride, perm, top, plan, E, act, ff, H, limit, alpha, offset);
+    if (stream_it)
+      MI_LAUNCH((moe_stream_kernel<true>), g, 32 * MS_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
+                (const bf16*)w_up, w_expert_stride, perm, top, plan, E, act, ff, H, per_warp, limit, alpha, offset);
+    else
+      MI_LAUNCH((moe_rows_kernel<true>), g, 32 * MR_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
+                (const bf16*)w_up, w_expert_stride, perm, top, plan, E, act, ff, H, limit, alpha, offset);
     MI_RETURN_LAUNCH_STATUS();
   }
   dim3 grid((ff + TILE_N - 1) / TILE_N, max_tiles(n_entries, E, TILE_M));
@@ -633,15 +783,22 @@ extern "C" int mi_moe_gate_up(const void* x, int x_stride, const void* w_gate, c
 }
 
 extern "C" int mi_moe_down(const void* act, const void* w_down, long long w_expert_stride, const int* plan, int E,
-                           float* y, int n_entries, int H, int ff, int tile_rows, int dtype, cudaStream_t stream) {
+                           float* y, int n_entries, int H, int ff, int tile_rows, int in_order, int dtype,
+                           cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (tile_rows == FEW_ROWS) {
     if (dtype != MI_DTYPE_BF16 || !mma_vec_ok(act, ff, w_down, nullptr, ff))
       MI_REFUSE("moe: the streaming product takes bfloat16 rows of whole 16-byte pieces");
-    dim3 g((H + 31) / 32, max_tiles(n_entries, E, FEW_ROWS));
+    const int per_warp = stream_pairs(ff, (H + 1) / 2, n_entries);
+    const bool stream_it = in_order || ff < MR_LEAST_K;
+    dim3 g(stream_it ? stream_blocks((H + 1) / 2, per_warp) : (H + 31) / 32, max_tiles(n_entries, E, FEW_ROWS));
     if (g.y > 65535) MI_REFUSE("moe: too many row tiles for one launch");
-    MI_LAUNCH((moe_rows_kernel<false>), g, 32 * MR_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
-              (const bf16*)nullptr, w_expert_stride, (const int*)nullptr, 1, plan, E, (void*)y, H, ff, 0.f, 0.f, 0.f);
+    if (stream_it)
+      MI_LAUNCH((moe_stream_kernel<false>), g, 32 * MS_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
+                (const bf16*)nullptr, w_expert_stride, (const int*)nullptr, 1, plan, E, (void*)y, H, ff, per_warp, 0.f, 0.f, 0.f);
+    else
+      MI_LAUNCH((moe_rows_kernel<false>), g, 32 * MR_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
+                (const bf16*)nullptr, w_expert_stride, (const int*)nullptr, 1, plan, E, (void*)y, H, ff, 0.f, 0.f, 0.f);
     MI_RETURN_LAUNCH_STATUS();
   }
   dim3 grid((H + TILE_N - 1) / TILE_N, max_tiles(n_entries, E, TILE_M));

@@ -12,6 +12,8 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
+from contextlib import contextmanager
 from ctypes import c_float, c_int, c_void_p
 
 import torch
@@ -122,6 +124,32 @@ def recover_from_wait_failure(device: torch.device) -> None:
     torch.cuda.synchronize(device)
 
 
+_sums = threading.local()
+KEPT_MIN_CHUNKS = 4      # chunks of 64 keys that a block of decode attention takes at least, where sums are kept
+
+
+@contextmanager
+def kept_sums():
+    """Inside, and in this thread only, bfloat16 work of decode steps adds up in one order that does not change from one
+    version of the kernels to the next: products of up to 16 rows run ``gemm_tma``, experts with few rows the streaming
+    kernel on CUDA cores, decode attention cuts its keys into stretches of four chunks or more.  Everywhere else the faster kernels run,
+    which are as close to the exact sums or closer.
+
+    It is for models that turn a difference in the last bit into another answer: a router that first picks groups of experts
+    and is undecided between two groups changes several experts with large weights at once (a quarter of such a token's logits'
+    size, against a hundredth for an undecided last expert), and so much of what the model said before."""
+    before = getattr(_sums, "kept", False)
+    _sums.kept = True
+    try:
+        yield
+    finally:
+        _sums.kept = before
+
+
+def _sums_kept() -> bool:
+    return getattr(_sums, "kept", False)
+
+
 def _sig_elementwise(lib: ctypes.CDLL) -> None:
     lib.mi_embedding.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_add_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -184,7 +212,7 @@ def _sig_attention_mma(lib: ctypes.CDLL) -> None:
     lib.mi_attention_decode_balanced.argtypes = [
         c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
         c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-        c_int, c_float, c_void_p, c_void_p]
+        c_int, c_float, c_void_p, c_int, c_void_p]
     lib.mi_attention_decode_balanced_unit_cost.argtypes = [c_int]
     lib.mi_attention_wait_status.argtypes = [c_int]
     lib.mi_set_status_word.argtypes = [c_void_p]
@@ -294,8 +322,9 @@ def _sig_moe(lib: ctypes.CDLL) -> None:
     lib.mi_moe_tile_rows.argtypes = [c_int]
     lib.mi_moe_tile_rows.restype = c_int
     lib.mi_moe_gate_up.argtypes = [c_void_p, c_int, c_void_p, c_void_p, ll, c_void_p, c_int, c_void_p, c_int,
-                                   c_void_p, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p]
-    lib.mi_moe_down.argtypes = [c_void_p, c_void_p, ll, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                   c_void_p, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int,
+                                   c_void_p]
+    lib.mi_moe_down.argtypes = [c_void_p, c_void_p, ll, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                 c_void_p]
     lib.mi_moe_combine.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                    c_void_p, c_int, c_int, c_void_p]
@@ -862,7 +891,7 @@ def attention_decode_balanced(q, q_stride, out, kcache, vcache, block_table, pag
         block_table.stride(0), _ptr(table_rows), int(page_size), _ptr(q_start), _ptr(kv_len), int(n_requests), nq, nkv,
         head_dim, float(scale), int(window), int(grid.value), _ptr(part_o), _ptr(part_ml), _ptr(count),
         _ptr(rope_table), 1 if store_kv else 0, _ptr(sinks), int(keep_first), float(softcap), _ptr(slopes),
-        _stream())
+        KEPT_MIN_CHUNKS if _sums_kept() else 0, _stream())
     _finish(lib, rc, "attention_decode")
 
 
@@ -1185,6 +1214,10 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.b
     return out
 
 
+def _few_rows_product(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, **forms):
+    return (gemm_tma if _sums_kept() else gemm_rows)(x, w, out_dtype, **forms)
+
+
 def gemm_tma_status(reset: bool = True) -> int:
     """Non-zero when a block of the streaming product gave up a bounded wait since the last
     reset (its output is then wrong).  Synchronises the device."""
@@ -1211,7 +1244,7 @@ def linear_into_stream(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor,
     statistics a product with ``row_stats`` needs to finish an RMS norm with ``eps``."""
     if not linear_fusable(x.shape[0], w) or not gemm_tma_ok(x, w):
         raise KernelError("linear_into_stream: these operands have no fused form (ask linear_fusable first)")
-    return gemm_rows(x, w, torch.bfloat16, residual=residual, gain=gain, eps=eps)
+    return _few_rows_product(x, w, torch.bfloat16, residual=residual, gain=gain, eps=eps)
 
 
 GLU_ACT = {"silu": 1, "gelu_tanh": 2}
@@ -1228,7 +1261,7 @@ def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, row_stats: "RowStats |
         raise KernelError(f"linear_swiglu: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
             and w_pairs.dtype == torch.bfloat16 and gemm_tma_ok(x, w_pairs)):
-        return gemm_rows(x, w_pairs, torch.bfloat16, swiglu=GLU_ACT[act], row_stats=row_stats)
+        return _few_rows_product(x, w_pairs, torch.bfloat16, swiglu=GLU_ACT[act], row_stats=row_stats)
     if row_stats is not None:
         raise KernelError("linear_swiglu: row statistics need the streaming product (ask linear_fusable first)")
     if act == "silu":
@@ -1247,7 +1280,7 @@ def linear_activated(x: torch.Tensor, w: torch.Tensor, act: str, numbers: tuple[
         raise KernelError(f"linear_activated: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
             and w.dtype == torch.bfloat16 and gemm_tma_ok(x, w)):
-        return gemm_rows(x, w, torch.bfloat16, act=(act, numbers))
+        return _few_rows_product(x, w, torch.bfloat16, act=(act, numbers))
     y = linear(x, w)
     lib = _lib("stream")
     if act == "relu2":
@@ -1277,7 +1310,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     if row_stats is not None:
         if not linear_fusable(x.shape[0], w) or not gemm_tma_ok(x, w):
             raise KernelError("linear: row statistics need the streaming product (ask linear_fusable first)")
-        return gemm_rows(x, w, out_dtype or torch.bfloat16, row_stats=row_stats)
+        return _few_rows_product(x, w, out_dtype or torch.bfloat16, row_stats=row_stats)
     if x.dtype == torch.float32:
         if w.dtype != torch.float32:
             raise KernelError("linear: fp32 activations need fp32 weights")
@@ -1288,7 +1321,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     if out_dtype not in (None, torch.bfloat16, torch.float32):
         raise KernelError(f"linear: unsupported output dtype {out_dtype}")
     if USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS and gemm_tma_ok(x, w):
-        return gemm_rows(x, w, out_dtype or torch.bfloat16)
+        return _few_rows_product(x, w, out_dtype or torch.bfloat16)
     launch_count += 1
     if out_dtype in (None, torch.bfloat16):
         return torch.mm(x, w.t())
@@ -1828,11 +1861,11 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         act = torch.empty((n, ff), dtype=x.dtype, device=dev)
         rc = lib.mi_moe_gate_up(_ptr(x), x.stride(0), _ptr(w_gate_up), _ptr(w_gate_up[:, ff:]), 2 * ff * H, _ptr(perm),
                                 top, _ptr(plan), E, _ptr(act), n, ff, H, float(limit), float(alpha), float(up_offset),
-                                tile, _code(x.dtype), _stream())
+                                tile, 1 if _sums_kept() else 0, _code(x.dtype), _stream())
         _finish(lib, rc, "moe_gate_up")
         y = torch.empty((n, H), dtype=torch.float32, device=dev)
-        rc = lib.mi_moe_down(_ptr(act), _ptr(w_down), H * ff, _ptr(plan), E, _ptr(y), n, H, ff, tile, _code(x.dtype),
-                             _stream())
+        rc = lib.mi_moe_down(_ptr(act), _ptr(w_down), H * ff, _ptr(plan), E, _ptr(y), n, H, ff, tile,
+                             1 if _sums_kept() else 0, _code(x.dtype), _stream())
         _finish(lib, rc, "moe_down")
     out = torch.empty((M, H), dtype=x.dtype, device=dev)
     if shared_gate is not None and (shared is None or shared_gate.dtype != torch.float32 or shared_gate.shape[0] != M

@@ -173,6 +173,9 @@ class Part:
     # device or changes Python state sets this to False; steps of its model then always run
     # kernel by kernel.
     graph_safe: ClassVar[bool] = True
+    # Whether a difference in the last bit can change this part's output a great deal: a step of its model then
+    # runs under ``ops.kept_sums``.
+    keeps_sums: bool = False
 
     def __init__(self, spec: PartSpec) -> None:
         self.spec = spec

@@ -76,6 +76,11 @@ class RoutedExperts(FeedForward):
             if self.keep_groups * (self.experts // self.groups) < self.top:
                 raise ValueError(f"{self.keep_groups} groups of {self.experts // self.groups} experts cannot give {self.top}")
 
+    @property
+    def keeps_sums(self) -> bool:
+        """Whether the router leaves out whole groups of experts (see ``ops.kept_sums``)."""
+        return self.groups > 1 and self.keep_groups < self.groups
+
     def param_decls(self):
         H, ff = self.hidden, self.ff
         decls = {"router": ParamDecl((self.experts, H))}

@@ -11,6 +11,7 @@ from dataclasses import dataclass
 
 import torch
 
+from ..csrc import ops
 from .base import (
     Arrangement,
     KVNeed,
@@ -79,6 +80,7 @@ class DecoderModel:
                                          for e in spec.schedule]
         self._keeps_embedding = any(getattr(p, "needs_embedding", False) for p in self.before + self.after
                                     if p is not None)
+        self._keeps_sums = any(p.keeps_sums for p in self.all_parts())
         self._bound = False
 
     # ------------------------------------------------------------------ declarations
@@ -197,6 +199,13 @@ class DecoderModel:
         """fp32 logits ``[n_want, vocab]`` at the packed rows ``want_rows`` (int32)."""
         if not self._bound:
             raise RuntimeError("the model has no weights yet")
+        if self._keeps_sums:
+            with ops.kept_sums():
+                return self._forward(ctx, caches, want_rows, n_want)
+        return self._forward(ctx, caches, want_rows, n_want)
+
+    def _forward(self, ctx: StepContext, caches: list[LayerCache], want_rows: torch.Tensor | None,
+                 n_want: int) -> torch.Tensor:
         if len(caches) > len(self.schedule):     # the embedding's own per-request state
             x = self.embedding.forward(ctx, caches[len(self.schedule)])
         else:
