@@ -42,8 +42,8 @@ struct GlaArgs {
   long long state_stride;
   const int *q_start, *q_len, *state_slot;
   float* o;
-  int o_stride, heads, dk, dv, extra_col, n_chunks;
-  float* scratch;              // per (request, chunk, head): D_end [dk], then [dk][dv]
+  int o_stride, n_requests, heads, dk, dv, extra_col, longer_than;
+  float* scratch;              // per (chunk, head): D_end [dk], then [dk][dv]
   const float *head_decay, *tok_gates;
 };
 
@@ -64,8 +64,59 @@ __device__ __forceinline__ float gc_value(const GlaArgs& a, int head, size_t m, 
   const int dv_in = a.dv - a.extra_col;
   return j < dv_in ? mi_to_float(reinterpret_cast<const T*>(a.v)[m * a.stride + head * dv_in + j]) : (j < a.dv ? 1.f : 0.f);
 }
-__device__ __forceinline__ float* gc_unit(const GlaArgs& a, int req, int chunk, int head) {
-  return a.scratch + (((size_t)req * a.n_chunks + chunk) * a.heads + head) * ((size_t)a.dk + (size_t)a.dk * a.dv);
+__device__ __forceinline__ float* gc_unit(const GlaArgs& a, int number, int head) {
+  return a.scratch + ((size_t)number * a.heads + head) * ((size_t)a.dk + (size_t)a.dk * a.dv);
+}
+
+// The step's chunks are numbered through: request after request, those alone whose portion is longer than
+// a.longer_than.  A block works out by itself where chunk `number`, or with `of_request` the number-th such request,
+// lies (a scan over the requests' lengths, 256 at a time, below 1 us against some 80 of a block's work), so that grid
+// and scratch are as large as the step's chunks are many and nothing comes from the host.  All threads of the block.
+struct GcPlace { int req, chunk, first; };      // first: the number of the request's first chunk
+__device__ __forceinline__ bool gc_find(const GlaArgs& a, int number, bool of_request, GcPlace& at) {
+  __shared__ int found[3], totals[GC_THREADS / 32][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int chunks = 0, requests = 0;                 // in front of this turn's
+  if (tid == 0) found[0] = -1;
+  for (int r0 = 0; r0 < a.n_requests; r0 += GC_THREADS) {
+    const int len = r0 + tid < a.n_requests ? a.q_len[r0 + tid] : 0;
+    const int c = len > a.longer_than ? (len + GC_T - 1) / GC_T : 0, one = c > 0 ? 1 : 0;
+    int cs = c, rs = one;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, cs, o), v = __shfl_up_sync(0xffffffffu, rs, o);
+      if (lane >= o) {
+        cs += u;
+        rs += v;
+      }
+    }
+    __syncthreads();
+    if (lane == 31) {
+      totals[warp][0] = cs;
+      totals[warp][1] = rs;
+    }
+    __syncthreads();
+    int cb = chunks + cs - c, rb = requests + rs - one;
+#pragma unroll
+    for (int w = 0; w < GC_THREADS / 32; ++w) {
+      if (w < warp) {
+        cb += totals[w][0];
+        rb += totals[w][1];
+      }
+      chunks += totals[w][0];
+      requests += totals[w][1];
+    }
+    if (one && (of_request ? rb == number : number >= cb && number < cb + c)) {
+      found[0] = r0 + tid;
+      found[1] = of_request ? 0 : number - cb;
+      found[2] = cb;
+    }
+  }
+  __syncthreads();
+  at.req = found[0];
+  at.chunk = found[1];
+  at.first = found[2];
+  return at.req >= 0;
 }
 
 __device__ __forceinline__ uint64_t gc_pack(float x) {
@@ -89,12 +140,11 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
   float* vs = ks + GC_T * GC_PITCH;             // [GC_T][GC_PITCH]
   __shared__ float tail[GC_W];
   const int col_tiles = (a.dv + GC_W - 1) / GC_W;
-  const int r0 = (blockIdx.x / col_tiles) * GC_W, j0 = (blockIdx.x % col_tiles) * GC_W;
-  const int head = blockIdx.y, req = blockIdx.z / a.n_chunks, chunk = blockIdx.z - req * a.n_chunks;
-  const int len = a.q_len[req] - chunk * GC_T;  // tokens from here on
-  if (len <= 0) return;
-  const int n = min(GC_T, len);
-  const size_t m0 = (size_t)a.q_start[req] + (size_t)chunk * GC_T;
+  const int r0 = (blockIdx.z / col_tiles) * GC_W, j0 = (blockIdx.z % col_tiles) * GC_W, head = blockIdx.y;
+  GcPlace at;
+  if (!gc_find(a, blockIdx.x, false, at)) return;
+  const int n = min(GC_T, a.q_len[at.req] - at.chunk * GC_T);
+  const size_t m0 = (size_t)a.q_start[at.req] + (size_t)at.chunk * GC_T;
   const int tid = threadIdx.x, ch = tid & (GC_W - 1), half = tid >> 7;
   const bool mine = r0 + ch < a.dk;
   // k times the decays of the tokens behind it: 32 tokens per thread from the end, then the later half's whole decay
@@ -115,7 +165,7 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
     vs[t * GC_PITCH + (i & (GC_W - 1))] = t < n && j < a.dv ? gc_value<T>(a, head, m0 + t, j) : 0.f;
   }
   __syncthreads();
-  float* unit = gc_unit(a, req, chunk, head);
+  float* unit = gc_unit(a, blockIdx.x, head);
   if (half == 0) {
     const float f = tail[ch];
     for (int t = 0; t < 32; ++t) ks[t * GC_PITCH + ch] *= f;
@@ -165,13 +215,15 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
 // do not depend on the chain and run eight chunks ahead.
 __global__ void __launch_bounds__(GC_THREADS) gla_carry_kernel(const GlaArgs a) {
   mi_pdl_enter();
-  const int head = blockIdx.y, req = blockIdx.z;
+  const int head = blockIdx.y;
+  GcPlace at;
+  if (!gc_find(a, blockIdx.z, true, at)) return;
   const long long e = (long long)blockIdx.x * GC_THREADS + threadIdx.x, elems = (long long)a.dk * a.dv;
   if (e >= elems) return;
-  const int chunks = (a.q_len[req] + GC_T - 1) / GC_T;
-  float* S = a.state + (size_t)a.state_slot[req] * a.state_stride + (size_t)head * elems + e;
+  const int chunks = (a.q_len[at.req] + GC_T - 1) / GC_T;
+  float* S = a.state + (size_t)a.state_slot[at.req] * a.state_stride + (size_t)head * elems + e;
   const size_t step = (size_t)a.heads * (a.dk + elems);
-  float* unit = gc_unit(a, req, 0, head);
+  float* unit = gc_unit(a, at.first, head);
   const float* A = unit + e / a.dv;
   float* B = unit + a.dk + e;
   float s = *S;
@@ -228,14 +280,13 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
   float* slab = ks + GC_T * GC_PITCH;           // [GC_SLAB][GC_PITCH]
   float* ps = slab + GC_SLAB * GC_PITCH;        // [GC_T][GC_PP]
   __shared__ float tail[GC_W];
-  const int j0 = blockIdx.x * GC_W;
-  const int head = blockIdx.y, req = blockIdx.z / a.n_chunks, chunk = blockIdx.z - req * a.n_chunks;
-  const int len = a.q_len[req] - chunk * GC_T;
-  if (len <= 0) return;
-  const int n = min(GC_T, len);
-  const size_t m0 = (size_t)a.q_start[req] + (size_t)chunk * GC_T;
+  const int j0 = blockIdx.z * GC_W, head = blockIdx.y;
+  GcPlace at;
+  if (!gc_find(a, blockIdx.x, false, at)) return;
+  const int n = min(GC_T, a.q_len[at.req] - at.chunk * GC_T);
+  const size_t m0 = (size_t)a.q_start[at.req] + (size_t)at.chunk * GC_T;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, ch = tid & (GC_W - 1), half = tid >> 7;
-  const float* S = gc_unit(a, req, chunk, head) + a.dk;
+  const float* S = gc_unit(a, blockIdx.x, head) + a.dk;
   const TQ* q = reinterpret_cast<const TQ*>(a.q);
 
   uint64_t acc[4][4];
@@ -366,13 +417,13 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
 
 extern "C" int mi_gla_chunk_tokens() { return GC_T; }
 
-// floats of scratch for portions of up to n_chunks chunks
-extern "C" long long mi_gla_chunks_scratch(int n_requests, int n_chunks, int heads, int dk, int dv) {
-  return (long long)n_requests * n_chunks * heads * ((long long)dk + (long long)dk * dv);
+// floats of scratch for this many chunks
+extern "C" long long mi_gla_chunks_scratch(int total_chunks, int heads, int dk, int dv) {
+  return (long long)total_chunks * heads * ((long long)dk + (long long)dk * dv);
 }
 
 template <typename TQ, typename T>
-static cudaError_t gla_chunks_launch(const GlaArgs& a, int n_requests, cudaStream_t stream) {
+static cudaError_t gla_chunks_launch(const GlaArgs& a, int total_chunks, int n_long, cudaStream_t stream) {
   const int col_tiles = (a.dv + GC_W - 1) / GC_W, row_tiles = (a.dk + GC_W - 1) / GC_W;
   const size_t fold_smem = (size_t)2 * GC_T * GC_PITCH * sizeof(float);
   const size_t out_smem = ((size_t)(2 * GC_T + GC_SLAB) * GC_PITCH + (size_t)GC_T * GC_PP) * sizeof(float);
@@ -381,37 +432,35 @@ static cudaError_t gla_chunks_launch(const GlaArgs& a, int n_requests, cudaStrea
   cudaError_t e = cudaFuncSetAttribute(fold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fold_smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
   if (e != cudaSuccess) return e;
-  const unsigned z = (unsigned)(n_requests * a.n_chunks);
-  e = MI_LAUNCH(fold, dim3(col_tiles * row_tiles, a.heads, z), GC_THREADS, fold_smem, stream, a);
+  e = MI_LAUNCH(fold, dim3(total_chunks, a.heads, col_tiles * row_tiles), GC_THREADS, fold_smem, stream, a);
   if (e != cudaSuccess) return e;
   const long long elems = (long long)a.dk * a.dv;
-  e = MI_LAUNCH(gla_carry_kernel, dim3((unsigned)((elems + GC_THREADS - 1) / GC_THREADS), a.heads, n_requests), GC_THREADS, 0,
+  e = MI_LAUNCH(gla_carry_kernel, dim3((unsigned)((elems + GC_THREADS - 1) / GC_THREADS), a.heads, n_long), GC_THREADS, 0,
                 stream, a);
   if (e != cudaSuccess) return e;
-  return MI_LAUNCH(out, dim3(col_tiles, a.heads, z), GC_THREADS, out_smem, stream, a);
+  return MI_LAUNCH(out, dim3(total_chunks, a.heads, col_tiles), GC_THREADS, out_smem, stream, a);
 }
 
-// Arguments as mi_gla_scan (recurrent.cu); n_chunks: 64-token chunks of the longest portion, scratch as
-// mi_gla_chunks_scratch says.  Three launches.
+// The portions longer than `longer_than`; arguments as mi_gla_scan (recurrent.cu).  n_long: how many these are, total_chunks:
+// how many chunks of 64 tokens they make together, scratch as mi_gla_chunks_scratch says.  Three launches.
 extern "C" int mi_gla_chunks(const void* q, const void* k, int qk_stride, int qk_dtype, const void* v, int stride,
                              const float* z, int z_stride, const float* z_bias, float inv_tau, float q_scale, float* state,
                              long long state_stride, const int* q_start, const int* q_len, const int* state_slot, float* o,
-                             int o_stride, int n_requests, int heads, int dk, int dv, float* scratch, int n_chunks,
+                             int o_stride, int n_requests, int heads, int dk, int dv, float* scratch, int total_chunks, int n_long, int longer_than,
                              const float* head_decay, const float* tok_gates, int extra_col, int dtype,
                              cudaStream_t stream) {
-  if (n_requests <= 0 || n_chunks <= 0) return 0;
+  if (n_requests <= 0 || total_chunks <= 0 || n_long <= 0) return 0;
   if (!z && !head_decay && !tok_gates) MI_REFUSE("gla: neither decays per channel nor per head nor per token");
   if (extra_col != 0 && extra_col != 1) MI_REFUSE("gla: one extra column or none");
   if (dv - extra_col <= 0) MI_REFUSE("gla: no value columns");
   if (!scratch) MI_REFUSE("gla: chunks need scratch memory");
-  if ((long long)n_requests * n_chunks > 65535) MI_REFUSE("gla: too many chunks for one launch");
   if (dk <= 0 || dk > 256 || dv <= 0) MI_REFUSE("gla: key size %d must lie in [1, 256], value size %d above 0", dk, dv);
-  if (heads > 65535) MI_REFUSE("gla: too many heads for one launch");
+  if (heads > 65535 || n_long > 65535) MI_REFUSE("gla: too many heads or requests for one launch");
   const GlaArgs a = {q, k, v, qk_stride, stride, z, z_stride, z_bias, inv_tau, q_scale, state, state_stride, q_start, q_len,
-                     state_slot, o, o_stride, heads, dk, dv, extra_col, n_chunks, scratch, head_decay, tok_gates};
+                     state_slot, o, o_stride, n_requests, heads, dk, dv, extra_col, longer_than, scratch, head_decay, tok_gates};
   cudaError_t e;
-  if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_BF16) e = gla_chunks_launch<bf16, bf16>(a, n_requests, stream);
-  else if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_F32) e = gla_chunks_launch<float, bf16>(a, n_requests, stream);
+  if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_BF16) e = gla_chunks_launch<bf16, bf16>(a, total_chunks, n_long, stream);
+  else if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_F32) e = gla_chunks_launch<float, bf16>(a, total_chunks, n_long, stream);
   else MI_REFUSE("gla: dtypes %d (q, k) and %d (v) are not taken together in chunks", qk_dtype, dtype);
   if (e != cudaSuccess) return (int)e;
   MI_RETURN_LAUNCH_STATUS();

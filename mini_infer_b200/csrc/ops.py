@@ -294,7 +294,7 @@ def _sig_recurrent(lib: ctypes.CDLL) -> None:
     lib.mi_rglru_scan_long.argtypes = lib.mi_rglru_scan.argtypes
     lib.mi_gla_scan.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                 c_void_p, ll, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]
+                                c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
     lib.mi_mlstm_gates.argtypes = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, ll, ll, c_void_p,
                                    c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
     lib.mi_delta_scan.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
@@ -307,11 +307,11 @@ def _sig_recurrent(lib: ctypes.CDLL) -> None:
 
 def _sig_gla_chunks(lib: ctypes.CDLL) -> None:
     ll = ctypes.c_longlong
-    lib.mi_gla_chunks_scratch.argtypes = [c_int, c_int, c_int, c_int, c_int]
+    lib.mi_gla_chunks_scratch.argtypes = [c_int, c_int, c_int, c_int]
     lib.mi_gla_chunks_scratch.restype = ll
     lib.mi_gla_chunks.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                   c_void_p, ll, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                  c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]
+                                  c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p]
 
 
 def _sig_moe(lib: ctypes.CDLL) -> None:
@@ -1540,6 +1540,11 @@ def _max_q_len(ctx) -> int:
     return 1 if ctx.decode_only else max(ctx.host_q_len)
 
 
+def _portions_over(ctx, n: int) -> list[int]:
+    """The lengths of the step's portions that are longer than ``n``."""
+    return [] if ctx.decode_only else [k for k in ctx.host_q_len if k > n]
+
+
 RGLRU_LONG = 32      # portions up to this long are walked by one thread per channel
 
 
@@ -1587,7 +1592,11 @@ def rglru_scan(gates: torch.Tensor, gate_bias_r: torch.Tensor, gate_bias_i: torc
     _finish(lib, rc, "rglru")
 
 
-GLA_LONG = 32        # portions up to this long are walked token by token
+# Every portion by itself: up to this long it is walked token by token, longer ones are taken in chunks of 64.  Walk and
+# chunks, us (32 heads of 128 x 128): one request of 64 tokens 28 and 80, 128 52 and 82, 192 76 and 87, 256 101 and 88; 8
+# requests of 33 102 and 134, 64 180 and 140, 128 350 and 260; 32 requests of 64 866 and 798, 96 1268 and 1181, 128 1700 and
+# 1239.  The line lies where both sides lose about as much.  A token alone and beside long portions gives the same bits.
+GLA_LONG = 128
 
 
 def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor | None, z_bias: torch.Tensor | None,
@@ -1628,30 +1637,29 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor 
     if stride < heads * dk * dvx:
         raise KernelError("gla: state row too short")
     o = torch.empty((M, heads * dvx), dtype=torch.float32, device=q.device)
-    longest = _max_q_len(ctx)
-    if v.dtype == torch.bfloat16 and longest > GLA_LONG:
-        # long portions: chunks side by side as products (the float32 path keeps the plain walk, whose sums do not
-        # depend on where a portion starts)
+    # (the float32 path keeps the plain walk for every portion: its sums do not depend on where a portion starts)
+    long = _portions_over(ctx, GLA_LONG) if v.dtype == torch.bfloat16 else []
+    if len(long) < ctx.n_requests:
+        lib = _lib("recurrent")
+        rc = lib.mi_gla_scan(_ptr(q), _ptr(k), q.stride(0), _code(q.dtype), _ptr(v), v.stride(0), _ptr(z),
+                             z.stride(0) if z is not None else 0, _ptr(z_bias), 1.0 / float(tau), float(q_scale),
+                             _ptr(state), stride, _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(o),
+                             o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(head_decay), _ptr(tok_gates),
+                             1 if extra_col else 0, GLA_LONG if long else 2 ** 31 - 1, _code(v.dtype), _stream())
+        _finish(lib, rc, "gla")
+    if long:
         global launch_count
         lib = _lib("gla_chunks")
-        n_chunks = -(-longest // lib.mi_gla_chunk_tokens())
-        scratch = torch.empty(lib.mi_gla_chunks_scratch(ctx.n_requests, n_chunks, heads, dk, dvx), dtype=torch.float32,
-                              device=q.device)
+        tokens = lib.mi_gla_chunk_tokens()
+        chunks = sum(-(-n // tokens) for n in long)
+        scratch = torch.empty(lib.mi_gla_chunks_scratch(chunks, heads, dk, dvx), dtype=torch.float32, device=q.device)
         rc = lib.mi_gla_chunks(_ptr(q), _ptr(k), q.stride(0), _code(q.dtype), _ptr(v), v.stride(0), _ptr(z),
                                z.stride(0) if z is not None else 0, _ptr(z_bias), 1.0 / float(tau), float(q_scale),
                                _ptr(state), stride, _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(o),
-                               o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(scratch), n_chunks, _ptr(head_decay),
-                               _ptr(tok_gates), 1 if extra_col else 0, _code(v.dtype), _stream())
+                               o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(scratch), chunks, len(long), GLA_LONG,
+                               _ptr(head_decay), _ptr(tok_gates), 1 if extra_col else 0, _code(v.dtype), _stream())
         _finish(lib, rc, "gla")
         launch_count += 2
-        return o
-    lib = _lib("recurrent")
-    rc = lib.mi_gla_scan(_ptr(q), _ptr(k), q.stride(0), _code(q.dtype), _ptr(v), v.stride(0), _ptr(z),
-                         z.stride(0) if z is not None else 0, _ptr(z_bias), 1.0 / float(tau), float(q_scale),
-                         _ptr(state), stride, _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(o),
-                         o.stride(0), ctx.n_requests, heads, dk, dvx, _ptr(head_decay), _ptr(tok_gates),
-                         1 if extra_col else 0, _code(v.dtype), _stream())
-    _finish(lib, rc, "gla")
     return o
 
 

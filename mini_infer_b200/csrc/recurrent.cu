@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(MAXT) gla_scan_kernel(const TQ* __restrict__ q
                                 const int* __restrict__ q_start, const int* __restrict__ q_len,
                                 const int* __restrict__ state_slot, float* __restrict__ o, int o_stride,
                                 int heads, int dk, int dv, const float* __restrict__ head_decay,
-                                const float* __restrict__ tok_gates, int extra_col) {
+                                const float* __restrict__ tok_gates, int extra_col, int up_to) {
   // head_decay [heads]: one fixed decay per head in the place of alpha (z is then not read).
   // tok_gates [M, heads, 3]: per token and head the decay (all key channels alike) and a factor on k
   // (z and head_decay are then not read).  extra_col: the head has dv + 1 value columns, the last one
@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(MAXT) gla_scan_kernel(const TQ* __restrict__ q
   const int j = blockIdx.x * 32 + tx;   // value column
   const int dv_in = dv - extra_col;     // columns that v brings
   const int len = q_len[req], row0 = q_start[req];
+  if (len > up_to) return;              // gla_chunks.cu takes it
   float* S = state + (size_t)state_slot[req] * state_stride + (size_t)head * dk * dv;
   float s[GLA_R];
 #pragma unroll
@@ -584,8 +585,9 @@ extern "C" int mi_gla_scan(const void* q, const void* k, int qk_stride, int qk_d
                            const float* z_bias, float inv_tau, float q_scale, float* state, long long state_stride,
                            const int* q_start, const int* q_len, const int* state_slot, float* o, int o_stride,
                            int n_requests, int heads, int dk, int dv, const float* head_decay, const float* tok_gates,
-                           int extra_col, int dtype, cudaStream_t stream) {
-  // dv counts the value columns of the state and of o; with extra_col v brings one less
+                           int extra_col, int up_to, int dtype, cudaStream_t stream) {
+  // dv counts the value columns of the state and of o; with extra_col v brings one less.  Portions longer than up_to are
+  // left alone.
   if (n_requests <= 0) return 0;
   if (!z && !head_decay && !tok_gates) MI_REFUSE("gla: neither decays per channel nor per head nor per token");
   if (extra_col != 0 && extra_col != 1) MI_REFUSE("gla: one extra column or none");
@@ -604,7 +606,7 @@ extern "C" int mi_gla_scan(const void* q, const void* k, int qk_stride, int qk_d
     }                                                                                                     \
     MI_LAUNCH(kern, grid, block, smem, stream, (const TQ*)q, (const TQ*)k, qk_stride, (const T*)v, stride, z, z_stride, \
               z_bias, inv_tau, q_scale, state, state_stride, q_start, q_len, state_slot, o, o_stride, heads,  \
-              dk, dv, head_decay, tok_gates, extra_col);                                                      \
+              dk, dv, head_decay, tok_gates, extra_col, up_to);                                                      \
   } while (0)
   if (dtype == MI_DTYPE_F32 && qk_dtype == MI_DTYPE_F32) MI_GO(float, float);
   else if (dtype == MI_DTYPE_BF16 && qk_dtype == MI_DTYPE_BF16) MI_GO(bf16, bf16);

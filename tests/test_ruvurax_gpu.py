@@ -379,6 +379,57 @@ def test_linear_attention_in_chunks(heads, dk, dv, portions, decays):
     assert ((state[1].cpu().double() - S).abs() <= rounds * 2.0 ** -24 * size + 1e-30).all()
 
 
+@pytest.mark.parametrize("lens", [[1, 200, 33, 1, 64, 129, 5], [65, 64, 63], [1] * 300 + [150] + [2] * 20 + [64, 70]])
+@pytest.mark.parametrize("longer_than", [None, 32])
+@pytest.mark.parametrize("decays", ["channel", "head", "token"])
+def test_linear_attention_of_unequal_portions_in_one_step(lens, longer_than, decays, monkeypatch):
+    """Portions of every length in one call, against the token loop in float64 with the bound of the test above; a portion's
+    numbers are to the bit those it gets alone, whatever shares the step; and scratch is taken for the chunks there are."""
+    o, heads, dk, dv = ops(), 2, 48, 40
+    if longer_than is not None:
+        monkeypatch.setattr(o, "GLA_LONG", longer_than)
+    Tn, starts = sum(lens), np.concatenate([[0], np.cumsum(lens)])
+    q, k, v = rnd(Tn, heads * dk, seed=70).bfloat16(), rnd(Tn, heads * dk, seed=71).bfloat16(), rnd(Tn, heads * dv, seed=72).bfloat16()
+    z = rnd(Tn, heads * dk, seed=73, scale=2.0) if decays == "channel" else None
+    hd = torch.tensor([0.97, 0.6]) if decays == "head" else None
+    tg = torch.sigmoid(rnd(Tn, heads, 3, seed=74) + 1) if decays == "token" else None
+    S0 = rnd(len(lens), heads, dk, dv, seed=75)
+    dev = lambda x, a, b: None if x is None else x[a:b].contiguous().to(DEV)
+
+    def run(which):
+        a, b = starts[which[0]], starts[which[-1] + 1]
+        state = S0[which].to(DEV)
+        out = o.gla_scan(dev(q, a, b), dev(k, a, b), dev(v, a, b), dev(z, a, b), None, 1.0, 1.0, heads, dk, dv, state,
+                         ctx_for([lens[i] for i in which], list(range(len(which)))),
+                         head_decay=None if hd is None else hd.to(DEV), tok_gates=dev(tg, a, b))
+        return out.cpu(), state.cpu()
+
+    run(list(range(len(lens))))
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got, state = run(list(range(len(lens))))
+    held = Tn * heads * (2 * dk + 2 * dv + 3 * dk + dv) * 4 + S0.numel() * 4
+    chunks = sum(-(-n // 64) for n in lens)
+    assert torch.cuda.max_memory_allocated() - before <= held + chunks * heads * (dk + dk * dv) * 4 + (1 << 21)
+    alpha = (torch.sigmoid(z.double()).reshape(Tn, heads, dk) if z is not None else
+             hd.double()[None, :, None].expand(Tn, heads, dk) if hd is not None else tg[..., :1].double().expand(Tn, heads, dk))
+    kk = k.double().reshape(Tn, heads, dk) * (tg[..., 1:2].double() if tg is not None else 1.0)
+    qq, vv = q.double().reshape(Tn, heads, dk), v.double().reshape(Tn, heads, dv)
+    for i, n in enumerate(lens):
+        S, size = S0[i].double(), S0[i].double().abs()
+        rounds = 64 + (dk + 64) + 4 * (n // 64 + 1)
+        for t in range(starts[i], starts[i] + n):
+            add = kk[t][:, :, None] * vv[t][:, None, :]
+            S, size = alpha[t][:, :, None] * S + add, alpha[t][:, :, None] * size + add.abs()
+            want, terms = torch.einsum("hkv,hk->hv", S, qq[t]), torch.einsum("hkv,hk->hv", size, qq[t].abs())
+            assert ((got[t].reshape(heads, dv).double() - want).abs() <= rounds * 2.0 ** -24 * terms + 1e-30).all(), (i, t)
+        assert ((state[i].double() - S).abs() <= rounds * 2.0 ** -24 * size + 1e-30).all(), i
+    for i in sorted({lens.index(n) for n in set(lens)}):
+        alone, alone_state = run([i])
+        assert torch.equal(alone, got[starts[i]:starts[i + 1]]) and torch.equal(alone_state[0], state[i]), i
+
+
 @pytest.mark.parametrize("C,bw,taps,act,portions", [(48, 16, 4, "silu", (1, 2, 40, 33)), (40, 20, 3, None, (259,)), (24, 24, 2, None, (33, 256, 1)),
                                                     (36, 12, 4, None, (600,)), (40, 8, 5, "silu", (40, 1))])
 def test_convolution_and_recurrent_unit_in_long_portions(C, bw, taps, act, portions):
