@@ -12,11 +12,16 @@
 //   gla_out_kernel     per (request, chunk, head, 128 value columns): the two products of o
 //
 // Everything is fp32, on fused multiply-adds two columns wide; decays are products of alphas (never differences of
-// logarithms), so their error does not grow with how far a channel decays.  What bounds it: 2 dk dv multiply-adds per
+// logarithms) kept to twice that precision, so their error does not grow with how far a channel decays, and sums are taken in
+// chains of 16.  Over 1000 tokens o and the state end 1.9 and 1.7e-7 from 64 bits with a decay per channel (2.0 and 1.8 by the
+// walk), 1.8 and 1.8 with one per head (3.4 and 4.0), 1.2 and 0.8 with one per token (1.2 and 0.8); single products and one chain
+// through all terms: 2.9 and 1.9, 8.0 and 10.0, 2.3 and 1.1.  What bounds it: 2 dk dv multiply-adds per
 // token and head with the state and 32 (dk + dv) within the chunk, whose operands come out of shared
 // memory 16 bytes at a time and 4 cycles a piece, so that about 0.2 of the fp32 rate is reached (15 TFLOP/s); the
-// token-by-token walk does as many at 2.  Per 2000 tokens: 4 heads of 128 x 256 512 us by the walk, 160 here; 16 heads of
-// 128 x 128 880 and 390.  Inputs fetched 16 tokens ahead into registers: 194 for 176 us of folds, 329 for 307 of outputs.  The quotient D_t / D_s is taken as (q D_t) (k / D_s) where no
+// token-by-token walk does as many at 2.  Per 2000 tokens, walk and here: 4 heads of 128 x 256 824 and 110 us with a decay per
+// channel, 752 and 92 with one per head; 32 heads of 128 x 128 1026 and 600, 870 and 459.  Inputs fetched 16 tokens ahead into
+// registers: 194 for 176 us of folds, 329 for 307 of outputs; the halves of a chunk's decays one after the other instead of side
+// by side: 814 for 588.  Where decays differ by channel the quotient D_t / D_s is taken as (q D_t) (k / D_s) if no
 // channel of the chunk falls below 1e-30 (|log alpha| up to 1.08 per token on average); a chunk where one does multiplies
 // its pairs' decays out one by one.
 #include "common.cuh"
@@ -28,6 +33,10 @@ MI_DEFINE_ERROR_API()
 #define GC_PITCH (GC_W + 4)
 #define GC_PP (GC_T + 4)       // row pitch of the pair weights
 #define GC_SLAB 32             // rows of S or v staged at a time
+// Terms per chain of additions; the chains' sums are added up.  Distance of o from 64 bits over 1000 tokens (a decay per channel,
+// per head, per token) with one chain through all channels and keys, chains of 32, of 16 and of 8: 2.7, 2.1, 1.9, 1.9e-7; 2.9,
+// 2.0, 1.9, 1.9e-7; 2.2, 1.4, 1.3, 1.3e-7 (by the walk 2.0, 3.4 and 1.2e-7), at 107, 107, 109 and 112 us.
+#define GC_CHAIN 16
 #define GC_THREADS 256
 #define GC_SMALLEST 1e-30f
 
@@ -127,9 +136,27 @@ __device__ __forceinline__ uint64_t gc_pack(float x) {
 __device__ __forceinline__ void gc_unpack(uint64_t v, float& a, float& b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
+__device__ __forceinline__ void gc_mul2(uint64_t& d, uint64_t a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
+__device__ __forceinline__ void gc_add2(uint64_t& d, uint64_t a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
 __device__ __forceinline__ void gc_fma2(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
+
+// A product of decays to twice fp32's precision: 64 roundings one after the other leave 2e-6, and all on one side where
+// the decay is a fixed one, against one of a token's own in a walk.
+struct GcDecay {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void times(float a) {
+    const float h = __fmul_rn(hi, a), l = fmaf(lo, a, fmaf(hi, a, -h));
+    hi = __fadd_rn(h, l);
+    lo = __fadd_rn(l, -__fadd_rn(hi, -h));
+  }
+  // x times the product, rounded once
+  __device__ __forceinline__ float of(float x) const {
+    const float h = __fmul_rn(x, hi);
+    return __fadd_rn(h, fmaf(x, lo, fmaf(x, hi, -h)));
+  }
+};
 
 // ------------------------------------------------------------------------------------------ the chunks' own part of S
 template <typename TQ, typename T>
@@ -138,7 +165,7 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
   extern __shared__ __align__(16) float gsm[];
   float* ks = gsm;                              // [GC_T][GC_PITCH]
   float* vs = ks + GC_T * GC_PITCH;             // [GC_T][GC_PITCH]
-  __shared__ float tail[GC_W];
+  __shared__ float2 tail[GC_W];
   const int col_tiles = (a.dv + GC_W - 1) / GC_W;
   const int r0 = (blockIdx.z / col_tiles) * GC_W, j0 = (blockIdx.z % col_tiles) * GC_W, head = blockIdx.y;
   GcPlace at;
@@ -148,7 +175,7 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
   const int tid = threadIdx.x, ch = tid & (GC_W - 1), half = tid >> 7;
   const bool mine = r0 + ch < a.dk;
   // k times the decays of the tokens behind it: 32 tokens per thread from the end, then the later half's whole decay
-  float p = 1.f;
+  GcDecay p;
 #pragma unroll 8
   for (int t = half * 32 + 31; t >= half * 32; --t) {
     float kv = 0.f, al = 1.f;
@@ -156,10 +183,10 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
       kv = gc_key<TQ>(a, head, m0 + t, r0 + ch);
       al = gc_alpha(a, head, m0 + t, r0 + ch);
     }
-    ks[t * GC_PITCH + ch] = kv * p;
-    p *= al;
+    ks[t * GC_PITCH + ch] = p.of(kv);
+    p.times(al);
   }
-  if (half == 1) tail[ch] = p;
+  if (half == 1) tail[ch] = make_float2(p.hi, p.lo);
   for (int i = tid; i < GC_T * GC_W; i += GC_THREADS) {
     const int t = i >> 7, j = j0 + (i & (GC_W - 1));
     vs[t * GC_PITCH + (i & (GC_W - 1))] = t < n && j < a.dv ? gc_value<T>(a, head, m0 + t, j) : 0.f;
@@ -167,9 +194,9 @@ __global__ void __launch_bounds__(GC_THREADS) gla_fold_kernel(const GlaArgs a) {
   __syncthreads();
   float* unit = gc_unit(a, blockIdx.x, head);
   if (half == 0) {
-    const float f = tail[ch];
-    for (int t = 0; t < 32; ++t) ks[t * GC_PITCH + ch] *= f;
-    if (j0 == 0 && mine) unit[r0 + ch] = p * f;
+    const float2 f = tail[ch];
+    for (int t = 0; t < 32; ++t) ks[t * GC_PITCH + ch] *= f.x;
+    if (j0 == 0 && mine) unit[r0 + ch] = (float)(((double)p.hi + p.lo) * ((double)f.x + f.y));
   }
   __syncthreads();
   const int tx = tid & 15, ty = tid >> 4;
@@ -247,9 +274,15 @@ __global__ void __launch_bounds__(GC_THREADS) gla_carry_kernel(const GlaArgs a) 
 }
 
 // ------------------------------------------------------------------------------------------ the outputs
-// acc[4][4] (rows 4 ty.., two columns each: 4 tx.. and 64 + 4 tx..) += rows [.][k] times mat [k][columns], `depth` of k
+// acc[4][4] (rows 4 ty.., two columns each: 4 tx.. and 64 + 4 tx..) += rows [.][k] times mat [k][columns], `depth` of k,
+// GC_CHAIN at most, as a sum of their own
 __device__ __forceinline__ void gc_product(uint64_t (&acc)[4][4], const float* rows, int pitch, const float* mat, int depth,
                                            int tx) {
+  uint64_t sum[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[i][j] = 0;
 #pragma unroll 2
   for (int k = 0; k < depth; k += 4) {
     float4 r[4];
@@ -262,24 +295,31 @@ __device__ __forceinline__ void gc_product(uint64_t (&acc)[4][4], const float* r
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint64_t w = gc_pack(kk == 0 ? r[i].x : kk == 1 ? r[i].y : kk == 2 ? r[i].z : r[i].w);
-        gc_fma2(acc[i][0], w, b0.x);
-        gc_fma2(acc[i][1], w, b0.y);
-        gc_fma2(acc[i][2], w, b1.x);
-        gc_fma2(acc[i][3], w, b1.y);
+        gc_fma2(sum[i][0], w, b0.x);
+        gc_fma2(sum[i][1], w, b0.y);
+        gc_fma2(sum[i][2], w, b1.x);
+        gc_fma2(sum[i][3], w, b1.y);
       }
     }
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) gc_add2(acc[i][j], sum[i][j]);
 }
 
-template <typename TQ, typename T>
+// SCALAR: the decay is one number per token for all channels (tok_gates, head_decay).  Then it is left out of the products: the
+// state's part of a token is multiplied by D_t behind them and a pair's weight by the product of the decays between its two
+// tokens, so that no quotient is taken and no decay is too small.
+template <typename TQ, typename T, bool SCALAR>
 __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a) {
   mi_pdl_enter();
   extern __shared__ __align__(16) float gsm[];
-  float* qs = gsm;                              // [GC_T][GC_PITCH]  q D
-  float* ks = qs + GC_T * GC_PITCH;             // [GC_T][GC_PITCH]  k / D
+  float* qs = gsm;                              // [GC_T][GC_PITCH]  q D (SCALAR: q)
+  float* ks = qs + GC_T * GC_PITCH;             // [GC_T][GC_PITCH]  k / D (SCALAR: k)
   float* slab = ks + GC_T * GC_PITCH;           // [GC_SLAB][GC_PITCH]
   float* ps = slab + GC_SLAB * GC_PITCH;        // [GC_T][GC_PP]
-  __shared__ float tail[GC_W];
+  __shared__ float tail[SCALAR ? 1 : GC_W], decay[SCALAR ? GC_T : 1], from_start[SCALAR ? GC_T : 1];
   const int j0 = blockIdx.z * GC_W, head = blockIdx.y;
   GcPlace at;
   if (!gc_find(a, blockIdx.x, false, at)) return;
@@ -290,59 +330,84 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
   const TQ* q = reinterpret_cast<const TQ*>(a.q);
 
   uint64_t acc[4][4];
-  float pair[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      acc[i][j] = 0;
-      pair[i][j] = 0.f;
-    }
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
   for (int i = tid; i < GC_T * GC_PP; i += GC_THREADS) ps[i] = 0.f;
+  if (SCALAR && tid < GC_T) decay[tid] = tid < n ? gc_alpha(a, head, m0 + tid, 0) : 1.f;
 
   for (int c0 = 0; c0 < a.dk; c0 += GC_W) {      // 128 key channels at a time
     const bool mine = c0 + ch < a.dk;
     if (c0) __syncthreads();
-    // D of every token: 32 tokens per thread, then the earlier half's whole decay
-    float p = 1.f;
+    bool quotient = true;
+    if (SCALAR) {
 #pragma unroll 8
-    for (int t = half * 32; t < half * 32 + 32; ++t) {
-      if (mine && t < n) p *= gc_alpha(a, head, m0 + t, c0 + ch);
-      qs[t * GC_PITCH + ch] = p;
-    }
-    if (half == 0) tail[ch] = p;
-    __syncthreads();
-    const float f = half ? tail[ch] : 1.f;
-    const bool quotient = __syncthreads_and(p * f >= GC_SMALLEST) != 0;
-#pragma unroll 8
-    for (int t = half * 32; t < half * 32 + 32; ++t) {
-      float qv = 0.f, kv = 0.f;
-      const float d = qs[t * GC_PITCH + ch] * f;
-      if (mine && t < n) {
-        qv = mi_to_float(q[(m0 + t) * a.qk_stride + head * a.dk + c0 + ch]) * a.q_scale;
-        kv = gc_key<TQ>(a, head, m0 + t, c0 + ch);
+      for (int t = half * 32; t < half * 32 + 32; ++t) {
+        float qv = 0.f, kv = 0.f;
+        if (mine && t < n) {
+          qv = mi_to_float(q[(m0 + t) * a.qk_stride + head * a.dk + c0 + ch]) * a.q_scale;
+          kv = gc_key<TQ>(a, head, m0 + t, c0 + ch);
+        }
+        qs[t * GC_PITCH + ch] = qv;
+        ks[t * GC_PITCH + ch] = kv;
       }
-      qs[t * GC_PITCH + ch] = qv * d;
-      ks[t * GC_PITCH + ch] = quotient ? kv / d : kv;
+    } else {
+      // D of every token: 32 tokens per thread, then the earlier half's whole decay
+      GcDecay p;
+#pragma unroll 8
+      for (int t = half * 32; t < half * 32 + 32; ++t) {
+        if (mine && t < n) p.times(gc_alpha(a, head, m0 + t, c0 + ch));
+        qs[t * GC_PITCH + ch] = p.hi;
+      }
+      if (half == 0) tail[ch] = p.hi;
+      __syncthreads();
+      const float f = half ? tail[ch] : 1.f;
+      quotient = __syncthreads_and(p.hi * f >= GC_SMALLEST) != 0;
+#pragma unroll 8
+      for (int t = half * 32; t < half * 32 + 32; ++t) {
+        float qv = 0.f, kv = 0.f;
+        const float d = qs[t * GC_PITCH + ch] * f;
+        if (mine && t < n) {
+          qv = mi_to_float(q[(m0 + t) * a.qk_stride + head * a.dk + c0 + ch]) * a.q_scale;
+          kv = gc_key<TQ>(a, head, m0 + t, c0 + ch);
+        }
+        qs[t * GC_PITCH + ch] = qv * d;
+        ks[t * GC_PITCH + ch] = quotient ? kv / d : kv;
+      }
     }
     __syncthreads();
-    // the pairs' weights
+    // the pairs' weights (a pair's weight counts from the key's token on), GC_CHAIN channels at a time
     if (quotient) {
+      for (int k0 = 0; k0 < GC_W; k0 += GC_CHAIN) {
+        float pair[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) pair[i][j] = 0.f;
 #pragma unroll 2
-      for (int k = 0; k < GC_W; k += 4) {
-        float4 r[4], c[4];
+        for (int k = k0; k < k0 + GC_CHAIN; k += 4) {
+          float4 r[4], c[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * GC_PITCH + k);
+          for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * GC_PITCH + k);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * GC_PITCH + k);
+          for (int j = 0; j < 4; ++j) c[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * GC_PITCH + k);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              pair[i][j] = fmaf(r[i].x, c[j].x, pair[i][j]);
+              pair[i][j] = fmaf(r[i].y, c[j].y, pair[i][j]);
+              pair[i][j] = fmaf(r[i].z, c[j].z, pair[i][j]);
+              pair[i][j] = fmaf(r[i].w, c[j].w, pair[i][j]);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            pair[i][j] = fmaf(r[i].x, c[j].x, pair[i][j]);
-            pair[i][j] = fmaf(r[i].y, c[j].y, pair[i][j]);
-            pair[i][j] = fmaf(r[i].z, c[j].z, pair[i][j]);
-            pair[i][j] = fmaf(r[i].w, c[j].w, pair[i][j]);
+            const int t = ty * 4 + i, s = tx + 16 * j;
+            if (s <= t) ps[t * GC_PP + s] += pair[i][j];
           }
       }
     } else {
@@ -376,17 +441,29 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
         slab[r * GC_PITCH + j] = (k0 + r < depth && j0 + j < a.dv) ? S[(size_t)(c0 + k0 + r) * a.dv + j0 + j] : 0.f;
       }
       __syncthreads();
-      gc_product(acc, qs + (ty * 4) * GC_PITCH + k0, GC_PITCH, slab, GC_SLAB, tx);
+      for (int u = 0; u < GC_SLAB; u += GC_CHAIN)
+        gc_product(acc, qs + (ty * 4) * GC_PITCH + k0 + u, GC_PITCH, slab + u * GC_PITCH, GC_CHAIN, tx);
     }
   }
-  // the chunk's own keys (a pair's weight counts from the key's token on)
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int t = ty * 4 + i, s = tx + 16 * j;
-      ps[t * GC_PP + s] = s <= t ? ps[t * GC_PP + s] + pair[i][j] : 0.f;
+  if (SCALAR) {
+    __syncthreads();
+    if (tid <= GC_T) {       // thread s: the decays behind key s, thread 64: those from the chunk's beginning on
+      GcDecay p;
+      for (int t = tid < GC_T ? tid + 1 : 0; t < n; ++t) {
+        p.times(decay[t]);
+        if (tid < GC_T) ps[t * GC_PP + tid] *= p.hi;
+        else from_start[t] = p.hi;
+      }
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t d = gc_pack(ty * 4 + i < n ? from_start[ty * 4 + i] : 0.f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) gc_mul2(acc[i][j], d);
+    }
+  }
+  // the chunk's own keys
   for (int s0 = 0; s0 < n; s0 += GC_SLAB) {
     __syncthreads();
     for (int i = tid; i < GC_SLAB * GC_W; i += GC_THREADS) {
@@ -395,7 +472,8 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
     }
     __syncthreads();
     // (rows of four tokens see no key behind their last)
-    gc_product(acc, ps + (ty * 4) * GC_PP + s0, GC_PP, slab, max(0, min(GC_SLAB, ty * 4 + 4 - s0)), tx);
+    for (int u = 0; u < GC_SLAB; u += GC_CHAIN)
+      gc_product(acc, ps + (ty * 4) * GC_PP + s0 + u, GC_PP, slab + u * GC_PITCH, max(0, min(GC_CHAIN, ty * 4 + 4 - s0 - u)), tx);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -428,7 +506,7 @@ static cudaError_t gla_chunks_launch(const GlaArgs& a, int total_chunks, int n_l
   const size_t fold_smem = (size_t)2 * GC_T * GC_PITCH * sizeof(float);
   const size_t out_smem = ((size_t)(2 * GC_T + GC_SLAB) * GC_PITCH + (size_t)GC_T * GC_PP) * sizeof(float);
   auto fold = gla_fold_kernel<TQ, T>;
-  auto out = gla_out_kernel<TQ, T>;
+  auto out = a.tok_gates || a.head_decay ? gla_out_kernel<TQ, T, true> : gla_out_kernel<TQ, T, false>;
   cudaError_t e = cudaFuncSetAttribute(fold, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fold_smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
   if (e != cudaSuccess) return e;

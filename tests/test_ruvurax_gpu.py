@@ -379,6 +379,41 @@ def test_linear_attention_in_chunks(heads, dk, dv, portions, decays):
     assert ((state[1].cpu().double() - S).abs() <= rounds * 2.0 ** -24 * size + 1e-30).all()
 
 
+@pytest.mark.parametrize("heads,dk,dv", [(3, 128, 128), (2, 64, 200), (2, 200, 64)])
+@pytest.mark.parametrize("decays", ["channel", "head", "token", "token_dead", "steep"])
+def test_chunks_are_no_further_from_64_bits_than_the_walk(heads, dk, dv, decays, monkeypatch):
+    """800 tokens, every one rounded once per state element in the walk, with decays near 1 (per channel as gates of
+    temperature 16 give them, fixed ones, one per token, some of these 0) and steep ones.  Products over 64 tokens carry the roundings
+    of their decays to every element and take longer sums: neither may show.  (The state's chain of 64 products is allowed 5
+    parts in a hundred: two of its terms' factors are rounded where the walk rounds one.)"""
+    o, n = ops(), 800
+    q, k, v = rnd(n, heads * dk, seed=70).bfloat16(), rnd(n, heads * dk, seed=71, scale=dk ** -0.5).bfloat16(), rnd(n, heads * dv, seed=72).bfloat16()
+    z = rnd(n, heads * dk, seed=73) + 1 if decays == "channel" else rnd(n, heads * dk, seed=73) * 3 - 2 if decays == "steep" else None
+    tau = 16.0 if decays == "channel" else 1.0
+    hd = torch.tensor([0.96875, 0.99, 0.999][:heads]) if decays == "head" else None
+    tg = None
+    if decays.startswith("token"):
+        tg = torch.stack([torch.sigmoid(rnd(n, heads, seed=74) + 3), torch.sigmoid(rnd(n, heads, seed=75)), torch.zeros(n, heads)], dim=-1)
+        if decays == "token_dead":
+            tg[::23, :, 0] = 0.0
+    alpha = (torch.sigmoid(z.double()).reshape(n, heads, dk) ** (1 / tau) if z is not None else
+             hd.double()[None, :, None].expand(n, heads, dk) if hd is not None else tg[..., :1].double().expand(n, heads, dk))
+    kk = k.double().reshape(n, heads, dk) * (tg[..., 1:2].double() if tg is not None else 1.0)
+    S, want = torch.zeros(heads, dk, dv, dtype=torch.float64), torch.empty(n, heads * dv, dtype=torch.float64)
+    for t in range(n):
+        S = alpha[t][:, :, None] * S + kk[t][:, :, None] * v[t].double().reshape(heads, 1, dv)
+        want[t] = torch.einsum("hkv,hk->hv", S, q[t].double().reshape(heads, dk)).flatten()
+    dev = lambda x: None if x is None else x.contiguous().to(DEV)
+    off = {}
+    for form, limit in (("walk", n), ("chunks", 0)):
+        monkeypatch.setattr(o, "GLA_LONG", limit)
+        state = torch.zeros(1, heads, dk, dv, device=DEV)
+        out = o.gla_scan(dev(q), dev(k), dev(v), dev(z), None, tau, 1.0, heads, dk, dv, state, ctx_for([n], [0]), head_decay=dev(hd),
+                         tok_gates=dev(tg))
+        off[form] = float((out.cpu().double() - want).norm()), float((state[0].cpu().double() - S).norm())
+    assert all(c <= 1.1 * w for c, w in zip(off["chunks"], off["walk"])), off
+
+
 @pytest.mark.parametrize("lens", [[1, 200, 33, 1, 64, 129, 5], [65, 64, 63], [1] * 300 + [150] + [2] * 20 + [64, 70]])
 @pytest.mark.parametrize("longer_than", [None, 32])
 @pytest.mark.parametrize("decays", ["channel", "head", "token"])
