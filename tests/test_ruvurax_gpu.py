@@ -414,6 +414,27 @@ def test_chunks_are_no_further_from_64_bits_than_the_walk(heads, dk, dv, decays,
     assert all(c <= 1.1 * w for c, w in zip(off["chunks"], off["walk"])), off
 
 
+def test_steep_decays_in_chunks_take_no_longer_than_the_walk(monkeypatch):
+    """Channels that all but die within a chunk go pair by pair (743 us where the walk takes 1026; the gates evaluated anew
+    for every pair took 2635): 1.5 times the walk's time is the bound, for the noise of a timer."""
+    o, n, heads, d = ops(), 2000, 32, 128
+    q, k, v = (rnd(n, heads * d, seed=i).bfloat16().to(DEV) for i in (70, 71, 72))
+    z, state, ctx = (rnd(n, heads * d, seed=73) * 3 - 2).to(DEV), torch.zeros(1, heads, d, d, device=DEV), ctx_for([n], [0])
+
+    def time(limit):
+        monkeypatch.setattr(o, "GLA_LONG", limit)
+        best = math.inf
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            o.gla_scan(q, k, v, z, None, 1.0, 1.0, heads, d, d, state, ctx)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+    assert time(0) <= 1.5 * time(n)
+
+
 @pytest.mark.parametrize("lens", [[1, 200, 33, 1, 64, 129, 5], [65, 64, 63], [1] * 300 + [150] + [2] * 20 + [64, 70]])
 @pytest.mark.parametrize("longer_than", [None, 32])
 @pytest.mark.parametrize("decays", ["channel", "head", "token"])
