@@ -275,16 +275,18 @@ __global__ void __launch_bounds__(GC_THREADS) gla_carry_kernel(const GlaArgs a) 
 
 // ------------------------------------------------------------------------------------------ the outputs
 // acc[4][4] (rows 4 ty.., two columns each: 4 tx.. and 64 + 4 tx..) += rows [.][k] times mat [k][columns], `depth` of k,
-// GC_CHAIN at most, as a sum of their own
+// GC_CHAIN at most, as a sum of their own; with `own` four more k, row i taking the first i + 1 of them (a token's own key
+// and those before it: what a later token brings must not reach it, not even as zero times an infinity)
+struct GcNo { static constexpr bool value = false; };
+struct GcYes { static constexpr bool value = true; };
 __device__ __forceinline__ void gc_product(uint64_t (&acc)[4][4], const float* rows, int pitch, const float* mat, int depth,
-                                           int tx) {
+                                           bool own, int tx) {
   uint64_t sum[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) sum[i][j] = 0;
-#pragma unroll 2
-  for (int k = 0; k < depth; k += 4) {
+  auto four = [&](int k, auto triangle) {
     float4 r[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(rows + i * pitch + k);
@@ -293,7 +295,7 @@ __device__ __forceinline__ void gc_product(uint64_t (&acc)[4][4], const float* r
       const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(mat + (k + kk) * GC_PITCH + tx * 4);
       const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(mat + (k + kk) * GC_PITCH + 64 + tx * 4);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = decltype(triangle)::value ? kk : 0; i < 4; ++i) {
         const uint64_t w = gc_pack(kk == 0 ? r[i].x : kk == 1 ? r[i].y : kk == 2 ? r[i].z : r[i].w);
         gc_fma2(sum[i][0], w, b0.x);
         gc_fma2(sum[i][1], w, b0.y);
@@ -301,7 +303,10 @@ __device__ __forceinline__ void gc_product(uint64_t (&acc)[4][4], const float* r
         gc_fma2(sum[i][3], w, b1.y);
       }
     }
-  }
+  };
+#pragma unroll 2
+  for (int k = 0; k < depth; k += 4) four(k, GcNo());
+  if (own) four(depth, GcYes());
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -461,7 +466,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
       }
       __syncthreads();
       for (int u = 0; u < GC_SLAB; u += GC_CHAIN)
-        gc_product(acc, qs + (ty * 4) * GC_PITCH + k0 + u, GC_PITCH, slab + u * GC_PITCH, GC_CHAIN, tx);
+        gc_product(acc, qs + (ty * 4) * GC_PITCH + k0 + u, GC_PITCH, slab + u * GC_PITCH, GC_CHAIN, false, tx);
     }
   }
   if (SCALAR) {
@@ -490,9 +495,11 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_out_kernel(const GlaArgs a)
       slab[r * GC_PITCH + j] = (s0 + r < n && j0 + j < a.dv) ? gc_value<T>(a, head, m0 + s0 + r, j0 + j) : 0.f;
     }
     __syncthreads();
-    // (rows of four tokens see no key behind their last)
-    for (int u = 0; u < GC_SLAB; u += GC_CHAIN)
-      gc_product(acc, ps + (ty * 4) * GC_PP + s0 + u, GC_PP, slab + u * GC_PITCH, max(0, min(GC_CHAIN, ty * 4 + 4 - s0 - u)), tx);
+    for (int u = 0; u < GC_SLAB; u += GC_CHAIN) {
+      const int before = ty * 4 - s0 - u;      // keys of this chain in front of the rows' own four
+      if (before >= 0)
+        gc_product(acc, ps + (ty * 4) * GC_PP + s0 + u, GC_PP, slab + u * GC_PITCH, min(GC_CHAIN, before), before < GC_CHAIN, tx);
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

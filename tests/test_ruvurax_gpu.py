@@ -414,6 +414,30 @@ def test_chunks_are_no_further_from_64_bits_than_the_walk(heads, dk, dv, decays,
     assert all(c <= 1.1 * w for c, w in zip(off["chunks"], off["walk"])), off
 
 
+@pytest.mark.parametrize("decays", ["channel", "head", "steep"])
+@pytest.mark.parametrize("what", ["v", "k", "q"])
+def test_what_a_token_brings_does_not_reach_the_tokens_before_it(decays, what, monkeypatch):
+    """An infinity or a NaN in one token's row: every token before it keeps its output to the bit, wherever in a chunk it
+    lies (in the chunks' products a later key has the weight 0, and 0 times an infinity is NaN)."""
+    o, n, heads, d = ops(), 130, 2, 48
+    monkeypatch.setattr(o, "GLA_LONG", 0)
+    rows = {x: rnd(n, heads * d, seed=70 + i).bfloat16() for i, x in enumerate("qkv")}
+    z = None if decays == "head" else rnd(n, heads * d, seed=73) * 3 - 2 if decays == "steep" else rnd(n, heads * d, seed=73) + 1
+    hd = torch.tensor([0.9, 0.99]).to(DEV) if decays == "head" else None
+
+    def run(rows):
+        state = torch.zeros(1, heads, d, d, device=DEV)
+        return o.gla_scan(*(rows[x].to(DEV) for x in "qkv"), None if z is None else z.to(DEV), None, 1.0, 1.0, heads, d, d, state,
+                          ctx_for([n], [0]), head_decay=hd).cpu()
+    clean = run(rows)
+    assert torch.isfinite(clean).all()
+    for at, bad in ((1, math.inf), (2, math.nan), (3, math.inf), (19, -math.inf), (34, math.nan), (63, math.inf), (66, math.inf), (129, math.nan)):
+        spoilt = dict(rows)
+        spoilt[what] = rows[what].clone()
+        spoilt[what][at] = bad
+        assert torch.equal(run(spoilt)[:at], clean[:at]), at
+
+
 def test_steep_decays_in_chunks_take_no_longer_than_the_walk(monkeypatch):
     """Channels that all but die within a chunk go pair by pair (743 us where the walk takes 1026; the gates evaluated anew
     for every pair took 2635): 1.5 times the walk's time is the bound, for the noise of a timer."""
