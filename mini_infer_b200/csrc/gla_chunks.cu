@@ -22,7 +22,7 @@
 // channel, 752 and 92 with one per head; 32 heads of 128 x 128 1026 and 600, 870 and 459.  Inputs fetched 16 tokens ahead into
 // registers: 194 for 176 us of folds, 329 for 307 of outputs; the halves of a chunk's decays one after the other instead of side
 // by side: 814 for 588.  Where decays differ by channel the quotient D_t / D_s is taken as (q D_t) (k / D_s) if no
-// channel of the chunk falls below 1e-30 (|log alpha| up to 1.08 per token on average); a chunk where one does multiplies
+// channel of the chunk falls below 1e-20 (|log alpha| up to 0.72 per token on average); a chunk where one does multiplies
 // its pairs' decays out one by one.
 #include "common.cuh"
 
@@ -38,7 +38,7 @@ MI_DEFINE_ERROR_API()
 // 2.0, 1.9, 1.9e-7; 2.2, 1.4, 1.3, 1.3e-7 (by the walk 2.0, 3.4 and 1.2e-7), at 107, 107, 109 and 112 us.
 #define GC_CHAIN 16
 #define GC_THREADS 256
-#define GC_SMALLEST 1e-30f
+#define GC_SMALLEST 1e-20f     // leaves 1e18 on either side for k / D and q D before fp32 ends
 
 struct GlaArgs {
   const void *q, *k, *v;

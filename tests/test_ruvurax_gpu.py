@@ -438,6 +438,24 @@ def test_what_a_token_brings_does_not_reach_the_tokens_before_it(decays, what, m
         assert torch.equal(run(spoilt)[:at], clean[:at]), at
 
 
+@pytest.mark.parametrize("scale", [1e15, 1e-15])
+@pytest.mark.parametrize("fall", [20.0, 40.0, 60.0, 75.0])
+def test_large_and_small_keys_beside_strong_decays(scale, fall, monkeypatch):
+    """Keys and queries far from 1, decays that fall by e^-fall within a chunk: k / D and q D stay inside fp32 in every form that a
+    chunk may take.  Against the token loop in float64, 200 roundings of the largest terms."""
+    o, n, d = ops(), 100, 16
+    monkeypatch.setattr(o, "GLA_LONG", 0)
+    q, k, v = rnd(n, d, seed=70).bfloat16() / scale, rnd(n, d, seed=71).bfloat16() * scale, rnd(n, d, seed=72).bfloat16()
+    z = torch.full((n, d), -math.log(math.expm1(fall / 64)))          # sigmoid(z) = e^(-fall / 64)
+    alpha, S, size = torch.sigmoid(z.double()), torch.zeros(d, d, dtype=torch.float64), torch.zeros(d, d, dtype=torch.float64)
+    state = torch.zeros(1, 1, d, d, device=DEV)
+    got = o.gla_scan(q.to(DEV), k.to(DEV), v.to(DEV), z.to(DEV), None, 1.0, 1.0, 1, d, d, state, ctx_for([n], [0])).cpu().double()
+    for t in range(n):
+        add = k[t].double()[:, None] * v[t].double()[None, :]
+        S, size = alpha[t][:, None] * S + add, alpha[t][:, None] * size + add.abs()
+        assert ((got[t] - q[t].double() @ S).abs() <= 200 * 2.0 ** -24 * (q[t].double().abs() @ size)).all(), t
+
+
 def test_steep_decays_in_chunks_take_no_longer_than_the_walk(monkeypatch):
     """Channels that all but die within a chunk go pair by pair (743 us where the walk takes 1026; the gates evaluated anew
     for every pair took 2635): 1.5 times the walk's time is the bound, for the noise of a timer."""
