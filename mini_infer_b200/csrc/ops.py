@@ -290,7 +290,7 @@ def _sig_recurrent(lib: ctypes.CDLL) -> None:
                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_rglru_scan.argtypes = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int,
                                   c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, ll, c_int,
-                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
+                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_rglru_scan_long.argtypes = lib.mi_rglru_scan.argtypes
     lib.mi_gla_scan.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
                                 c_void_p, ll, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -1545,7 +1545,12 @@ def _portions_over(ctx, n: int) -> list[int]:
     return [] if ctx.decode_only else [k for k in ctx.host_q_len if k > n]
 
 
-RGLRU_LONG = 32      # portions up to this long are walked by one thread per channel
+# Every portion by itself: up to this long it is walked by one thread per channel, longer ones by 32.  Walk, 32 threads, and two
+# passes over chunks of 64 (which they took the place of), us, 4096 channels: one request of 17 tokens 17, 11 and 18, 64 54, 12
+# and 57, 128 105, 12 and 94; 8 requests of 33 30, 60 and 33, 64 55, 61 and 64, 128 148, 63 and 148; 32 requests of 33 56, 226
+# and 56, 65 122, 249 and 202, 128 239, 259 and 231.  32 threads per channel cost every request a whole block per 16 channels: the
+# line lies where a step full of such portions begins to gain.
+RGLRU_LONG = 128
 
 
 def rglru_scan(gates: torch.Tensor, gate_bias_r: torch.Tensor, gate_bias_i: torch.Tensor, lam: torch.Tensor,
@@ -1574,22 +1579,17 @@ def rglru_scan(gates: torch.Tensor, gate_bias_r: torch.Tensor, gate_bias_i: torc
     if stride < taps * C:
         raise KernelError("rglru: state row too short")
     lib = _lib("recurrent")
-    longest = _max_q_len(ctx)
-    if u.dtype == torch.bfloat16 and longest > RGLRU_LONG:
-        # long portions: a channel's tokens side by side (the float32 path keeps the plain walk, whose sums do
-        # not depend on where a portion starts)
-        rc = lib.mi_rglru_scan_long(_ptr(gates), M, bw, _ptr(gate_bias_r), _ptr(gate_bias_i), _ptr(lam),
-                                    float(decay_scale), _ptr(u), u.stride(0), _ptr(y), y.stride(0), _ptr(y_bias),
-                                    _ptr(x_in), x_in.stride(0), _ptr(x_in_bias), _ptr(state), stride, int(taps),
-                                    _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(out),
-                                    out.stride(0), ctx.n_requests, C, _code(u.dtype), _stream())
+    # (the float32 path keeps the plain walk for every portion: its sums do not depend on where a portion starts)
+    n_long = len(_portions_over(ctx, RGLRU_LONG)) if u.dtype == torch.bfloat16 else 0
+    args = (_ptr(gates), M, bw, _ptr(gate_bias_r), _ptr(gate_bias_i), _ptr(lam), float(decay_scale), _ptr(u), u.stride(0),
+            _ptr(y), y.stride(0), _ptr(y_bias), _ptr(x_in), x_in.stride(0), _ptr(x_in_bias), _ptr(state), stride, int(taps),
+            _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(out), out.stride(0), ctx.n_requests, C)
+    if n_long < ctx.n_requests:
+        rc = lib.mi_rglru_scan(*args, RGLRU_LONG if n_long else 2 ** 31 - 1, _code(u.dtype), _stream())
         _finish(lib, rc, "rglru")
-        return
-    rc = lib.mi_rglru_scan(_ptr(gates), M, bw, _ptr(gate_bias_r), _ptr(gate_bias_i), _ptr(lam), float(decay_scale),
-                           _ptr(u), u.stride(0), _ptr(y), y.stride(0), _ptr(y_bias), _ptr(x_in), x_in.stride(0),
-                           _ptr(x_in_bias), _ptr(state), stride, int(taps), _ptr(ctx.q_start), _ptr(ctx.q_len),
-                           _ptr(ctx.state_slot), _ptr(out), out.stride(0), ctx.n_requests, C, _code(u.dtype), _stream())
-    _finish(lib, rc, "rglru")
+    if n_long:
+        rc = lib.mi_rglru_scan_long(*args, RGLRU_LONG, _code(u.dtype), _stream())
+        _finish(lib, rc, "rglru")
 
 
 # Every portion by itself: up to this long it is walked token by token, longer ones are taken in chunks of 64.  Walk and

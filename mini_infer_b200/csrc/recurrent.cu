@@ -3,8 +3,8 @@
 // Every request of a step brings q_len[b] consecutive tokens (rows q_start[b] .. of the packed
 // activations) and owns row state_slot[b] of a state arena (fp32, zeroed when the request is
 // admitted).  All recurrences run in fp32, token by token in the order of the positions, so a
-// result never depends on how a prompt was cut into steps or on what else is in the batch (long bfloat16
-// portions are taken in chunks, here and in gla_chunks.cu, which moves the fp32 rounding).
+// result never depends on what else is in the batch, nor on how a prompt was cut into steps (but bfloat16 portions longer than a
+// limit are taken in chunks, here and in gla_chunks.cu, which moves the fp32 rounding; each portion by its own length).
 //
 //   mi_causal_conv     per channel: out[t] = b + sum_j w[j] * in[t - (taps-1-j)], in = x + x_bias,
 //                      with the taps-1 inputs before the portion taken from the state (zeros before
@@ -234,12 +234,14 @@ __global__ void rglru_scan_kernel(const float* __restrict__ gates, int M, int bw
                                   const T* __restrict__ xin, int xin_stride, const float* __restrict__ xin_bias,
                                   float* __restrict__ state, long long state_stride, int taps,
                                   const int* __restrict__ q_start, const int* __restrict__ q_len,
-                                  const int* __restrict__ state_slot, T* __restrict__ out, int out_stride, int C) {
+                                  const int* __restrict__ state_slot, T* __restrict__ out, int out_stride, int C,
+                                  int up_to) {
   mi_pdl_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int req = blockIdx.y;
   if (c >= C) return;
   const int len = q_len[req], row0 = q_start[req];
+  if (len > up_to) return;              // rglru_long_kernel takes it
   float* st = state + (size_t)state_slot[req] * state_stride;
   float* Sp = st + (size_t)(taps - 1) * C + c;
   float S = *Sp;
@@ -277,12 +279,13 @@ __global__ void rglru_scan_kernel(const float* __restrict__ gates, int M, int bw
   }
 }
 
+// Portions longer than up_to are left alone.
 extern "C" int mi_rglru_scan(const float* gates, int M, int bw, const float* br, const float* bi, const float* lam,
                              float decay_scale, const void* u, int u_stride, const void* y, int y_stride,
                              const float* y_bias, const void* xin, int xin_stride, const float* xin_bias,
                              float* state, long long state_stride, int taps, const int* q_start, const int* q_len,
-                             const int* state_slot, void* out, int out_stride, int n_requests, int C, int dtype,
-                             cudaStream_t stream) {
+                             const int* state_slot, void* out, int out_stride, int n_requests, int C, int up_to,
+                             int dtype, cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (taps < 1 || taps > MAX_TAPS) MI_REFUSE("rglru: %d taps (1 to %d are taken)", taps, MAX_TAPS);
   if (bw <= 0 || C % bw) MI_REFUSE("rglru: %d channels are no whole number of blocks of %d", C, bw);
@@ -292,11 +295,11 @@ extern "C" int mi_rglru_scan(const float* gates, int M, int bw, const float* br,
   if (dtype == MI_DTYPE_F32)
     MI_LAUNCH((rglru_scan_kernel<float>), grid, threads, 0, stream, gates, M, bw, br, bi, lam, decay_scale,
               (const float*)u, u_stride, (const float*)y, y_stride, y_bias, (const float*)xin, xin_stride, xin_bias,
-              state, state_stride, taps, q_start, q_len, state_slot, (float*)out, out_stride, C);
+              state, state_stride, taps, q_start, q_len, state_slot, (float*)out, out_stride, C, up_to);
   else if (dtype == MI_DTYPE_BF16)
     MI_LAUNCH((rglru_scan_kernel<bf16>), grid, threads, 0, stream, gates, M, bw, br, bi, lam, decay_scale,
               (const bf16*)u, u_stride, (const bf16*)y, y_stride, y_bias, (const bf16*)xin, xin_stride, xin_bias,
-              state, state_stride, taps, q_start, q_len, state_slot, (bf16*)out, out_stride, C);
+              state, state_stride, taps, q_start, q_len, state_slot, (bf16*)out, out_stride, C, up_to);
   else
     MI_REFUSE("rglru: unknown dtype %d", dtype);
   MI_RETURN_LAUNCH_STATUS();
@@ -335,12 +338,13 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
                   const T* __restrict__ xin, int xin_stride, const float* __restrict__ xin_bias,
                   float* __restrict__ state, long long state_stride, int taps, const int* __restrict__ q_start,
                   const int* __restrict__ q_len, const int* __restrict__ state_slot, T* __restrict__ out, int out_stride,
-                  int C) {
+                  int C, int longer_than) {
   mi_pdl_enter();
   __shared__ float fold_a[RU_SEG][RU_CH + 1], fold_b[RU_SEG][RU_CH + 1];   // then: the state a thread begins with (b)
   __shared__ float carry[RU_CH];
   const int tid = threadIdx.x, cl = tid % RU_CH, seg = tid / RU_CH, c = blockIdx.x * RU_CH + cl, req = blockIdx.y;
   const int len = q_len[req], row0 = q_start[req];
+  if (len <= longer_than) return;
   const bool in = c < C;
   float* st = state + (size_t)state_slot[req] * state_stride;
   const int blk = in ? c / bw : 0, cj = c - blk * bw;
@@ -432,12 +436,14 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
   }
 }
 
+// The portions longer than longer_than.
 extern "C" int mi_rglru_scan_long(const float* gates, int M, int bw, const float* br, const float* bi,
                                   const float* lam, float decay_scale, const void* u, int u_stride, const void* y,
                                   int y_stride, const float* y_bias, const void* xin, int xin_stride,
                                   const float* xin_bias, float* state, long long state_stride, int taps,
                                   const int* q_start, const int* q_len, const int* state_slot, void* out,
-                                  int out_stride, int n_requests, int C, int dtype, cudaStream_t stream) {
+                                  int out_stride, int n_requests, int C, int longer_than, int dtype,
+                                  cudaStream_t stream) {
   if (n_requests <= 0) return 0;
   if (taps < 1 || taps > MAX_TAPS) MI_REFUSE("rglru: %d taps (1 to %d are taken)", taps, MAX_TAPS);
   if (bw <= 0 || C % bw) MI_REFUSE("rglru: %d channels are no whole number of blocks of %d", C, bw);
@@ -446,7 +452,7 @@ extern "C" int mi_rglru_scan_long(const float* gates, int M, int bw, const float
   dim3 grid((C + RU_CH - 1) / RU_CH, n_requests);
   MI_LAUNCH((rglru_long_kernel<bf16>), grid, RU_THREADS, 0, stream, gates, M, bw, br, bi, lam, decay_scale, (const bf16*)u,
             u_stride, (const bf16*)y, y_stride, y_bias, (const bf16*)xin, xin_stride, xin_bias, state, state_stride, taps,
-            q_start, q_len, state_slot, (bf16*)out, out_stride, C);
+            q_start, q_len, state_slot, (bf16*)out, out_stride, C, longer_than);
   MI_RETURN_LAUNCH_STATUS();
 }
 

@@ -570,6 +570,39 @@ def test_convolution_and_recurrent_unit_in_long_portions(C, bw, taps, act, porti
     assert torch.equal(state[1, :taps - 1].cpu(), (x.float() + xb)[Tn - (taps - 1):])
 
 
+def unit_inputs(lens, C, bw, seed=80):
+    n = sum(lens)
+    g = {"gates": rnd(C // bw, n, 2 * bw, seed=seed)}
+    g.update({k: rnd(n, C, seed=seed + i).bfloat16() for i, k in enumerate(("u", "y", "x"), 1)})
+    g.update({k: rnd(C, seed=seed + i) * 0.1 for i, k in enumerate(("br", "bi", "lam", "yb", "xb"), 5)})
+    return g
+
+
+def run_unit(g, lens, which, S0, taps):
+    starts = np.concatenate([[0], np.cumsum(lens)])
+    a, b = starts[which[0]], starts[which[-1] + 1]
+    d = {k: (v[:, a:b] if k == "gates" else v[a:b] if v.dim() == 2 else v).contiguous().to(DEV) for k, v in g.items()}
+    state, out = S0[which].to(DEV), torch.empty(b - a, S0.shape[2], dtype=torch.bfloat16, device=DEV)
+    ops().rglru_scan(d["gates"], d["br"], d["bi"], d["lam"], 8.0, d["u"], d["y"], d["yb"], d["x"], d["xb"], taps, state,
+                     ctx_for([lens[i] for i in which], list(range(len(which)))), out)
+    return out.cpu(), state.cpu()
+
+
+@pytest.mark.parametrize("lens", [[1, 200, 33, 1, 64, 129, 5], [1] * 40 + [300] + [2] * 5])
+@pytest.mark.parametrize("longer_than", [None, 32])
+def test_recurrent_unit_of_unequal_portions_in_one_step(lens, longer_than, monkeypatch):
+    """A portion's numbers are to the bit those it gets alone, whatever shares the step."""
+    if longer_than is not None:
+        monkeypatch.setattr(ops(), "RGLRU_LONG", longer_than)
+    C, bw, taps = 40, 20, 4
+    g, S0 = unit_inputs(lens, C, bw), rnd(len(lens), taps, C, seed=95)
+    out, state = run_unit(g, lens, list(range(len(lens))), S0, taps)
+    starts = np.concatenate([[0], np.cumsum(lens)])
+    for i in sorted({lens.index(n) for n in set(lens)}):
+        alone, alone_state = run_unit(g, lens, [i], S0, taps)
+        assert torch.equal(alone, out[starts[i]:starts[i + 1]]) and torch.equal(alone_state[0], state[i]), i
+
+
 @pytest.mark.parametrize("K", [64, 256, 520, 1024, 2816, 8192])
 def test_experts_of_few_rows_sum_as_fp32_would(K):
     """The fp32 result of the streaming product of few rows against float64.  Summing K products one by one in fp32 is off
