@@ -309,7 +309,9 @@ extern "C" int mi_rglru_scan(const float* gates, int M, int bw, const float* br,
 // The same recurrence for long portions.  A block owns 16 channels of a request and takes its tokens 256 at a time: 32
 // threads per channel hold eight tokens' (a, b) each in registers and fold them into S_end = A S_begin + B, a warp per
 // channel scans the 32 folds, and every thread walks its eight tokens from the state it then knows.  (Blocks of twice the
-// threads leave room for one per SM: 160 blocks of 2560 channels then run in two turns.)  What bounds it is
+// threads leave room for one per SM: 160 blocks of 2560 channels then run in two turns.)  Folds and scan are fp64: in fp32 a
+// state that has gone through them is further from 64 bits than one walked token by token (7.8 and 7.2e-8 after 1000
+// tokens, 7.1 so; 68 and 71 us).  What bounds it is
 // the arithmetic of the gates (five exponentials, two divisions, a root per token and channel), which is done
 // once; two passes of one thread per 64 tokens did it twice and stood still for their loads (2000 tokens of 2560
 // channels: 60 + 90 us; 118 with a round's loads where they are used, 68 with all of them first).
@@ -340,8 +342,8 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
                   const int* __restrict__ q_len, const int* __restrict__ state_slot, T* __restrict__ out, int out_stride,
                   int C, int longer_than) {
   mi_pdl_enter();
-  __shared__ float fold_a[RU_SEG][RU_CH + 1], fold_b[RU_SEG][RU_CH + 1];   // then: the state a thread begins with (b)
-  __shared__ float carry[RU_CH];
+  __shared__ double fold_a[RU_SEG][RU_CH + 1], fold_b[RU_SEG][RU_CH + 1];   // then: the state a thread begins with (b)
+  __shared__ double carry[RU_CH];
   const int tid = threadIdx.x, cl = tid % RU_CH, seg = tid / RU_CH, c = blockIdx.x * RU_CH + cl, req = blockIdx.y;
   const int len = q_len[req], row0 = q_start[req];
   if (len <= longer_than) return;
@@ -379,11 +381,12 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
       const int t = first + i;
       uv[i] = (in && t < len) ? y[(size_t)(row0 + t) * y_stride + c] : T(0.f);
     }
-    float A = 1.f, B = 0.f;
+    double A = 1.0, B = 0.0;
 #pragma unroll
     for (int i = 0; i < RU_TOK; ++i) {
-      B = fmaf(k[i].a, B, k[i].b);
-      A *= k[i].a;
+      const double ka = k[i].a;
+      B = fma(ka, B, (double)k[i].b);
+      A *= ka;
     }
     fold_a[seg][cl] = A;
     fold_b[seg][cl] = B;
@@ -391,24 +394,24 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
     // warp w, lane l: fold l of channel w
     const int warp = tid >> 5, lane = tid & 31;
     if (warp < RU_CH) {
-      float sa = fold_a[lane][warp], sb = fold_b[lane][warp];      // then: all folds up to here as one
+      double sa = fold_a[lane][warp], sb = fold_b[lane][warp];      // then: all folds up to here as one
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
-        const float pa = __shfl_up_sync(0xffffffffu, sa, off), pb = __shfl_up_sync(0xffffffffu, sb, off);
+        const double pa = __shfl_up_sync(0xffffffffu, sa, off), pb = __shfl_up_sync(0xffffffffu, sb, off);
         if (lane >= off) {
-          sb = fmaf(sa, pb, sb);
+          sb = fma(sa, pb, sb);
           sa *= pa;
         }
       }
-      const float S0 = carry[warp];
-      const float end = fmaf(sa, S0, sb);                 // the state behind this lane's fold
-      const float before = __shfl_up_sync(0xffffffffu, end, 1);
+      const double S0 = carry[warp];
+      const double end = fma(sa, S0, sb);                 // the state behind this lane's fold
+      const double before = __shfl_up_sync(0xffffffffu, end, 1);
       fold_b[lane][warp] = lane ? before : S0;
       __syncwarp();
       if (lane == 31) carry[warp] = end;
     }
     __syncthreads();
-    float S = fold_b[seg][cl];
+    float S = (float)fold_b[seg][cl];
 #pragma unroll
     for (int i = 0; i < RU_TOK; ++i) {
       const int t = first + i;
@@ -418,7 +421,7 @@ rglru_long_kernel(const float* __restrict__ gates, int M, int bw, const float* _
     __syncthreads();                                      // the folds are read before the next round's
   }
   if (seg != 0 || !in) return;
-  st[(size_t)(taps - 1) * C + c] = carry[cl];
+  st[(size_t)(taps - 1) * C + c] = (float)carry[cl];
   if (taps > 1) {
     const float xb = xin_bias ? xin_bias[c] : 0.f;
     float keep[MAX_TAPS];

@@ -603,6 +603,26 @@ def test_recurrent_unit_of_unequal_portions_in_one_step(lens, longer_than, monke
         assert torch.equal(alone, out[starts[i]:starts[i + 1]]) and torch.equal(alone_state[0], state[i]), i
 
 
+@pytest.mark.parametrize("n", [65, 256, 300, 1000])
+def test_recurrent_unit_of_long_portions_is_no_further_from_64_bits_than_the_walk(n, monkeypatch):
+    """The state behind the portion, walked token by token in fp32 and by folds and a scan, both against float64."""
+    C, bw, taps = 640, 64, 4
+    g, S0 = unit_inputs([n], C, bw), rnd(1, taps, C, seed=95)
+    r = torch.sigmoid(torch.cat(list(g["gates"][:, :, :bw].double()), dim=1) + g["br"].double())
+    i = torch.sigmoid(torch.cat(list(g["gates"][:, :, bw:].double()), dim=1) + g["bi"].double())
+    log_a = -8.0 * r * torch.nn.functional.softplus(g["lam"].double() - 3)
+    a, inp = log_a.exp(), torch.sqrt(-torch.expm1(2 * log_a)) * i * g["u"].double()
+    S = S0[0, taps - 1].double()
+    for t in range(n):
+        S = a[t] * S + inp[t]
+    g["lam"] = g["lam"] - 3
+    off = {}
+    for form, limit in (("walk", n), ("scan", 0)):
+        monkeypatch.setattr(ops(), "RGLRU_LONG", limit)
+        off[form] = float((run_unit(g, [n], [0], S0, taps)[1][0, taps - 1].double() - S).norm())
+    assert off["scan"] <= 1.02 * off["walk"], off
+
+
 @pytest.mark.parametrize("K", [64, 256, 520, 1024, 2816, 8192])
 def test_experts_of_few_rows_sum_as_fp32_would(K):
     """The fp32 result of the streaming product of few rows against float64.  Summing K products one by one in fp32 is off
