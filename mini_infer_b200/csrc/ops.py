@@ -121,6 +121,8 @@ def recover_from_wait_failure(device: torch.device) -> None:
             buf.zero_()
         for _partials, counters in _tma_ws.get(idx, []):
             counters.zero_()
+        for _part_o, _part_ml, counters in _balanced_ws.get(idx, []):
+            counters.zero_()
     torch.cuda.synchronize(device)
 
 

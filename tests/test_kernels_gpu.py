@@ -636,6 +636,19 @@ def test_attention_decode_balanced(nq, nkv, d, page):
         assert (got - want).abs().max().item() <= BF16_BOUND
 
 
+def test_decode_attention_after_a_recovery():
+    """Counters as an interrupted balanced decode leaves them (some stretches of a unit counted in, the others not): the recovery
+    clears them, and the next call merges every unit's stretches, none of them early."""
+    args = ([1] * 3, [2048, 700, 129], 8, 2, 64, 16, torch.bfloat16)
+    run_attention(*args, seed=11, kernel="balanced")
+    for _, _, counters in ops()._balanced_ws[0]:
+        counters[::3] = 1
+        counters[1::3] = 7
+    ops().recover_from_wait_failure(torch.device(DEV))
+    got, want = run_attention(*args, seed=11, kernel="balanced")
+    assert torch.isfinite(got).all() and (got - want).abs().max().item() <= BF16_BOUND
+
+
 @pytest.mark.parametrize("unit_cost", [0, 1, 2, 5, 40])
 def test_attention_decode_balanced_whatever_a_unit_is_reckoned_to_cost(unit_cost):
     """The balanced kernel lengthens every unit by a number of positions that stand for no chunk

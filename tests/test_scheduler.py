@@ -397,6 +397,24 @@ def test_a_kernel_that_gave_up_waiting_cancels_the_step_and_raises():
     assert res.finish_reason == "length" and len(res.tokens) == 3
 
 
+def test_the_recovery_clears_the_counters_of_every_kernel_that_counts(monkeypatch):
+    """What an interrupted kernel may have left non-zero and the next call starts from: of the split decode, of the balanced
+    decode and of the streaming product, in every buffer that was ever handed out for the device."""
+    import torch
+
+    from mini_infer_b200.csrc import ops
+
+    word, left = torch.ones(1, dtype=torch.int32), lambda: torch.full((5,), 3, dtype=torch.int32)
+    split, balanced, product = [left(), left()], [(left(), left(), left()) for _ in range(2)], [(left(), left())]
+    monkeypatch.setattr(ops, "_decode_counter_bufs", {0: split})
+    monkeypatch.setattr(ops, "_balanced_ws", {0: balanced})
+    monkeypatch.setattr(ops, "_tma_ws", {0: product})
+    monkeypatch.setattr(ops, "status_word", lambda device: word)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
+    ops.recover_from_wait_failure(torch.device("cuda", 0))
+    assert int(word) == 0 and all(int(c.abs().sum()) == 0 for c in split + [w[2] for w in balanced] + [w[1] for w in product])
+
+
 def test_streaming_callback_may_call_back_into_the_scheduler():
     """Callbacks run outside the scheduler's lock: one that cancels its own request, asks for
     the load and submits another request does not deadlock."""
