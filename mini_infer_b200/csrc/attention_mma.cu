@@ -699,12 +699,21 @@ __device__ __noinline__ void balanced_merge_unit(const float* __restrict__ part_
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 v[8];
   float4 o[8];
+  const bool pieces = (reinterpret_cast<uintptr_t>(part_o) & 15) == 0;      // (scratch may come in at any float)
   auto load = [&](int gb) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int g = min(gb + k, g_last);
-      v[k] = __ldcg(ml + (size_t)g * DEC_HEADS);
-      o[k] = __ldcg(reinterpret_cast<const float4*>(part_o + (((size_t)unit + g) * DEC_HEADS + r) * d + c4));
+    for (int k = 0; k < 8; ++k) v[k] = __ldcg(ml + (size_t)min(gb + k, g_last) * DEC_HEADS);
+    const float* first = part_o + ((size_t)unit * DEC_HEADS + r) * d + c4;
+    if (pieces) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        o[k] = __ldcg(reinterpret_cast<const float4*>(first + (size_t)min(gb + k, g_last) * DEC_HEADS * d));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float* p = first + (size_t)min(gb + k, g_last) * DEC_HEADS * d;
+        o[k] = make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+      }
     }
   };
   load(g_first);
@@ -1177,7 +1186,12 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
         dst[1] = pack_bf16(acc.z * inv, acc.w * inv);
       } else {
         const size_t slot = ((size_t)unit + blockIdx.x) * DEC_HEADS + r;
-        *reinterpret_cast<float4*>(part_o + slot * d + c4) = acc;
+        float* po = part_o + slot * d + c4;
+        if ((reinterpret_cast<uintptr_t>(part_o) & 15) == 0) {
+          *reinterpret_cast<float4*>(po) = acc;
+        } else {
+          po[0] = acc.x; po[1] = acc.y; po[2] = acc.z; po[3] = acc.w;
+        }
         if (c4 == 0) *reinterpret_cast<float2*>(part_ml + slot * 2) = make_float2(m, L);
       }
     }
@@ -1709,8 +1723,8 @@ extern "C" int mi_attention_decode_balanced(const void* q, int q_stride, void* o
     MI_REFUSE("attention: rotating inside the decode kernel needs a head size of 64, 128 or 256, got %d", d);
   if (int rc = check_common(q, q_stride, out, out_stride, kcache, vcache, nq, nkv, d, page_size, window)) return rc;
   if (grid <= 0 || !part_o || !part_ml || !counters) MI_REFUSE("attention: the balanced kernel needs its grid and scratch");
-  if (!mi_aligned(part_o, 16) || !mi_aligned(part_ml, 8) || !mi_aligned(counters, 4))
-    MI_REFUSE("attention: scratch must be aligned (part_o to 16 bytes, part_ml to 8, counters to 4)");
+  if (!mi_aligned(part_o, 4) || !mi_aligned(part_ml, 8) || !mi_aligned(counters, 4))
+    MI_REFUSE("attention: scratch must be aligned (part_o and counters to 4 bytes, part_ml to 8)");
   if (B > 16384) MI_REFUSE("attention: %d requests in one decode step", B);
   const int page_shift = shift_of(page_size);
   const size_t smem = balanced_smem_bytes(B, d);

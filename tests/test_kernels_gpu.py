@@ -636,6 +636,20 @@ def test_attention_decode_balanced(nq, nkv, d, page):
         assert (got - want).abs().max().item() <= BF16_BOUND
 
 
+def test_balanced_decode_with_scratch_at_any_float(monkeypatch):
+    """The entry point takes partial results at any 4-byte address, and gives the same bits at each."""
+    args = ([1] * 3, [2048, 700, 129], 8, 2, 64, 16, torch.bfloat16)
+    want, _ = run_attention(*args, seed=11, kernel="balanced")
+    real = ops()._balanced_workspace
+    for off in (1, 2, 3):
+        def shifted(device, o_floats, ml_floats, counters, off=off):
+            part_o, part_ml, count = real(device, o_floats + 4, ml_floats, counters)
+            return part_o[off:], part_ml, count
+        monkeypatch.setattr(ops(), "_balanced_workspace", shifted)
+        got, _ = run_attention(*args, seed=11, kernel="balanced")
+        assert torch.equal(got, want), off
+
+
 def test_decode_attention_after_a_recovery():
     """Counters as an interrupted balanced decode leaves them (some stretches of a unit counted in, the others not): the recovery
     clears them, and the next call merges every unit's stretches, none of them early."""
