@@ -30,9 +30,9 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 // ------------------------------------------------------------------------------------------
 // Few rows.  A block owns 16 columns of the result (rows of W); 64 threads per part of k stream their part of
 // them, with the rows of A beside it, through a ring of stages filled by cp.async, 16 x 4 threads, RM rows of A each.  One
-// element's sum is a chain of K / 4 multiply-adds (4 cycles each: 1.1 us at K = 2048).  The first stages of W are asked for
-// before the wait for the kernel before.  2 x 3072 x 2048 behind one another: 19 us with one part (a chain four times
+// element's sum is a chain of K / 4 multiply-adds (4 cycles each: 1.1 us at K = 2048).  2 x 3072 x 2048 behind one another: 19 us with one part (a chain four times
 // as long behind a ring four times as narrow), 322 us with 128 columns per block and no ring; 3.9 us of bytes.
+// w_constant: no kernel before this one writes W, so that its first stages are asked for before the wait for that kernel.
 // ------------------------------------------------------------------------------------------
 #define RB_COLS 16
 #define RB_K 32
@@ -42,7 +42,7 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 template <int RM, int STAGES>
 __global__ void __launch_bounds__(64 * PARTS) gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                                    float* __restrict__ C, int M, int N, int K, int lda,
-                                                                   int ldw, int ldc) {
+                                                                   int ldw, int ldc, int w_constant) {
   extern __shared__ __align__(16) float rsm[];
   constexpr int ROWS = 4 * RM;
   constexpr int STAGE = (RB_COLS + ROWS) * RB_PITCH;
@@ -71,8 +71,9 @@ __global__ void __launch_bounds__(64 * PARTS) gemm_f32_rows_kernel(const float* 
     }
   };
   const int ahead = min(STAGES - 1, chunks);
-  for (int s = 0; s < ahead; ++s) load_w(s);      // weights depend on no kernel before this one
-  mi_pdl_wait();
+  if (!w_constant) mi_pdl_wait();
+  for (int s = 0; s < ahead; ++s) load_w(s);
+  if (w_constant) mi_pdl_wait();
   for (int s = 0; s < STAGES - 1; ++s) {
     if (s < chunks) load_a(s);
     asm volatile("cp.async.commit_group;\n" ::: "memory");   // (W's first stages ride in the first group)
@@ -273,12 +274,13 @@ __global__ void __launch_bounds__(256) gemm_f32_any_kernel(const float* __restri
 
 template <int RM, int STAGES>
 static cudaError_t launch_rows(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
-                               cudaStream_t stream) {
+                               int w_constant, cudaStream_t stream) {
   const size_t smem = (size_t)PARTS * STAGES * (RB_COLS + 4 * RM) * RB_PITCH * sizeof(float);
   auto kern = gemm_f32_rows_kernel<RM, STAGES>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return MI_LAUNCH(kern, (N + RB_COLS - 1) / RB_COLS, 64 * PARTS, smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
+  return MI_LAUNCH(kern, (N + RB_COLS - 1) / RB_COLS, 64 * PARTS, smem, stream, A, W, C, M, N, K, lda, ldw, ldc,
+                   w_constant);
 }
 
 template <int TM>
@@ -292,9 +294,10 @@ static cudaError_t launch_tile(const float* A, const float* W, float* C, int M, 
                    K, lda, ldw, ldc);
 }
 
+// w_constant: W is not written by any kernel that may still run (a loaded weight).
 // Zero-padded tails of a part add exact zeros at the end of its sum, so they do not change it.
 extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
-                           int ldw, int ldc, cudaStream_t stream) {
+                           int ldw, int ldc, int w_constant, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) MI_REFUSE("gemm_f32: K must be positive, got %d", K);
   if (lda < K || ldw < K || ldc < N) MI_REFUSE("gemm_f32: leading dimensions too small");
@@ -305,10 +308,10 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
     MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
               lda, ldw, ldc);
   } else if (M <= RB_MAX_ROWS) {
-    e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, stream)
-        : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, stream)
-        : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, stream)
-                  : launch_rows<8, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+        : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+        : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+                  : launch_rows<8, 4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream);
   } else {
     e = launch_tile<4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
   }

@@ -166,7 +166,7 @@ def _sig_elementwise(lib: ctypes.CDLL) -> None:
 
 def _sig_gemm_f32(lib: ctypes.CDLL) -> None:
     lib.mi_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                c_int, c_void_p]
+                                c_int, c_int, c_void_p]
 
 
 def _sig_attention_generic(lib: ctypes.CDLL) -> None:
@@ -578,8 +578,9 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None, pairs: bool
     return out
 
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``a [M, K] @ w [N, K]^T`` in true fp32 (CUDA cores, fixed summation order)."""
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, w_constant: bool = False) -> torch.Tensor:
+    """``a [M, K] @ w [N, K]^T`` in true fp32 (CUDA cores, fixed summation order).  With ``w_constant`` the kernel may read
+    ``w`` while kernels before it still run: for weights, never for what such a kernel writes."""
     _cuda(a, w, out)
     if a.dtype != torch.float32 or w.dtype != torch.float32:
         raise KernelError("gemm_f32: operands must be float32")
@@ -595,7 +596,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
         raise KernelError("gemm_f32: bad output tensor")
     lib = _lib("gemm_f32")
     rc = lib.mi_gemm_f32(_ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0) if M > 1 else K,
-                         w.stride(0) if N > 1 else K, out.stride(0) if M > 1 else N, _stream())
+                         w.stride(0) if N > 1 else K, out.stride(0) if M > 1 else N, 1 if w_constant else 0, _stream())
     _finish(lib, rc, "gemm_f32")
     return out
 
@@ -1253,12 +1254,12 @@ GLU_ACT = {"silu": 1, "gelu_tanh": 2}
 
 
 def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, row_stats: "RowStats | None" = None,
-                  act: str = "silu") -> torch.Tensor:
+                  act: str = "silu", w_constant: bool = False) -> torch.Tensor:
     """``act(x Wg^T) * (x Wu^T)`` for a merged projection whose rows alternate gate, up
     (``w_pairs [2 I, K]``); ``act`` is ``"silu"`` or ``"gelu_tanh"``.  Decode-sized bfloat16 inputs
     run the product and the activation as one kernel (gemm_rows with its gate/up epilogue);
     everything else runs ``linear`` and an activation-and-multiply kernel on the interleaved
-    result.  ``row_stats``: see ``RowStats``."""
+    result.  ``row_stats``: see ``RowStats``; ``w_constant``: see ``linear``."""
     if act not in GLU_ACT:
         raise KernelError(f"linear_swiglu: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
@@ -1267,23 +1268,24 @@ def linear_swiglu(x: torch.Tensor, w_pairs: torch.Tensor, row_stats: "RowStats |
     if row_stats is not None:
         raise KernelError("linear_swiglu: row statistics need the streaming product (ask linear_fusable first)")
     if act == "silu":
-        return silu_mul(linear(x, w_pairs), pairs=True)
-    return glu_mul_pairs(linear(x, w_pairs), act)
+        return silu_mul(linear(x, w_pairs, w_constant=w_constant), pairs=True)
+    return glu_mul_pairs(linear(x, w_pairs, w_constant=w_constant), act)
 
 
 UNARY_ACT = {"xielu": 3, "relu2": 4}      # the streaming product's epilogue numbers
 
 
-def linear_activated(x: torch.Tensor, w: torch.Tensor, act: str, numbers: tuple[float, float]) -> torch.Tensor:
+def linear_activated(x: torch.Tensor, w: torch.Tensor, act: str, numbers: tuple[float, float],
+                     w_constant: bool = False) -> torch.Tensor:
     """``act(x w^T)`` value by value in fp32; ``"xielu"`` with ``numbers = (a, b)``: ``a z^2 + z / 2`` for ``z > 0``,
     ``b (e^z - 1 - z) + z / 2`` for ``z <= 0``; ``"relu2"``: the square of ``max(z, 0)``.  Decode-sized bfloat16 inputs run the activation in the streaming
-    product's epilogue, everything else runs ``linear`` and the activation in place."""
+    product's epilogue, everything else runs ``linear`` (``w_constant``: see there) and the activation in place."""
     if act not in UNARY_ACT:
         raise KernelError(f"linear_activated: unknown activation {act!r}")
     if (x.dtype == torch.bfloat16 and USE_TMA_GEMM and x.shape[0] <= TMA_GEMM_DISPATCH_ROWS
             and w.dtype == torch.bfloat16 and gemm_tma_ok(x, w)):
         return _few_rows_product(x, w, torch.bfloat16, act=(act, numbers))
-    y = linear(x, w)
+    y = linear(x, w, w_constant=w_constant)
     lib = _lib("stream")
     if act == "relu2":
         rc = lib.mi_relu2_map(_ptr(y), _ptr(y), y.numel(), _code(y.dtype), _stream())
@@ -1297,7 +1299,7 @@ _MM_OUT_DTYPE: bool | None = None
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
-           row_stats: "RowStats | None" = None) -> torch.Tensor:
+           row_stats: "RowStats | None" = None, w_constant: bool = False) -> torch.Tensor:
     """``x [M, K] @ w [N, K]^T``.
 
     float32 operands run the true-fp32 CUDA-core kernel (never a library product, which
@@ -1306,7 +1308,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     kernel before it still runs; other bfloat16 operands use the library product with fp32
     accumulation, as the reference does for every linear layer (``distributed/linear.py:167``).
     ``out_dtype=float32`` keeps the accumulator's precision in the result (used for logits).
-    ``row_stats`` (streaming product only): see ``RowStats``.
+    ``row_stats`` (streaming product only): see ``RowStats``.  ``w_constant`` (float32): see ``gemm_f32``; the
+    bfloat16 kernels for few rows take every ``w`` as constant.
     """
     global _MM_OUT_DTYPE, launch_count
     if row_stats is not None:
@@ -1316,7 +1319,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
     if x.dtype == torch.float32:
         if w.dtype != torch.float32:
             raise KernelError("linear: fp32 activations need fp32 weights")
-        return gemm_f32(x, w)
+        return gemm_f32(x, w, w_constant=w_constant)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"linear: unsupported dtypes {x.dtype} x {w.dtype}")
     _cuda(x, w)

@@ -63,7 +63,7 @@ class Linear:
             if x.kind != "rms":
                 raise ValueError(f"this product cannot finish a norm of kind {x.kind!r}")
             return ops.linear(x.x, self.weight, out_dtype, row_stats=x.stats)
-        return ops.linear(x, self.weight, out_dtype)
+        return ops.linear(x, self.weight, out_dtype, w_constant=True)
 
     def fusable(self, n_rows: int, kind: str = "rms") -> bool:
         return kind == "rms" and ops.linear_fusable(n_rows, self.weight)
@@ -603,7 +603,7 @@ class SwiGLU(FeedForward):
                 raise ValueError(f"this product cannot finish a norm of kind {x.kind!r}")
             h = ops.linear_swiglu(x.x, self.gate_up_proj.weight, row_stats=x.stats, act=self.activation)
         else:
-            h = ops.linear_swiglu(x, self.gate_up_proj.weight, act=self.activation)
+            h = ops.linear_swiglu(x, self.gate_up_proj.weight, act=self.activation, w_constant=True)
         return self.down_proj(h) if into is None else self.down_proj.into_stream(h, into)
 
 
@@ -664,7 +664,7 @@ class ActivatedMLP(FeedForward):
             self.act_params = (p, 0.5 + q)
 
     def forward(self, x, ctx):
-        return self.down(ops.linear_activated(x, self.up, self.activation, self.act_params))
+        return self.down(ops.linear_activated(x, self.up, self.activation, self.act_params, w_constant=True))
 
 
 # ----------------------------------------------------------------------------- embedding / head

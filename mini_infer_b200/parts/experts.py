@@ -129,7 +129,7 @@ class RoutedExperts(FeedForward):
     def forward(self, x, ctx):
         shared = None
         if self.shared_pairs is not None:
-            shared = self.shared_out(ops.linear_swiglu(x, self.shared_pairs, act="silu"))
+            shared = self.shared_out(ops.linear_swiglu(x, self.shared_pairs, act="silu", w_constant=True))
         elif self.shared_in is not None:
             shared = self.shared_out(ops.clamped_glu(self.shared_in(x), self.shared_limit, self.alpha, self.up_offset))
         ids, weights, logits = ops.moe_route(x, self.router, self.top, scores=self.scores, groups=self.groups,

@@ -209,6 +209,21 @@ def test_gemm_f32_gives_the_same_bits_from_every_kernel(N, K):
     assert torch.equal(ops().gemm_f32(a.to(DEV), odd[:, 1:]), full)
 
 
+@pytest.mark.parametrize("M", [1, 4, 8, 16, 32, 33])
+def test_gemm_f32_of_a_matrix_that_the_kernel_before_writes(M):
+    """W is the result of a long product of this library right in front of the call: unless the caller says that it is constant,
+    no kernel may read it before that product is done."""
+    a, b, x = (rnd(n, 2048, seed=15 + n).to(DEV) for n in (256, 2048, M))
+    w = torch.full((256, 2048), float("nan"), device=DEV)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        ops().gemm_f32(a, b, out=w)
+        got, lin = ops().gemm_f32(x, w), ops().linear(x, w)
+        assert torch.equal(got, ops().gemm_f32(x, w.clone())) and torch.equal(lin, got) and torch.isfinite(got).all()
+        assert torch.equal(ops().linear(x, w, w_constant=True), got)
+        w.fill_(float("nan"))
+
+
 def test_gemm_f32_is_not_reduced_precision():
     # products that a 10-bit (TF32) or 8-bit (bf16) mantissa would lose
     a = torch.tensor([[1.0 + 2.0 ** -20, 1.0]], device=DEV)
