@@ -37,7 +37,11 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 #define RB_COLS 16
 #define RB_K 32
 #define RB_PITCH (RB_K + 4)      // floats per staged row: eight rows' 16-byte pieces touch every bank once
+// Rows and tiles, us: N x K = 3072 x 2048 with 1 row 11 and 40, 16 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
+// and 52, 32 29 and 53; 6144 x 2048 16 28 and 58, 17 49 and 57, 32 56 and 58; 32000 x 2048 8 81 and 121, 16 115 and 121, 17
+// 222 and 121, 32 256 and 123 (a block's 16 columns then come round fourteen times, each with all rows).
 #define RB_MAX_ROWS 32
+#define RB_MAX_COLS 8192          // above 16 rows
 
 template <int RM, int STAGES>
 __global__ void __launch_bounds__(64 * PARTS) gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
@@ -307,7 +311,7 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
   if (!vec) {
     MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
               lda, ldw, ldc);
-  } else if (M <= RB_MAX_ROWS) {
+  } else if (M <= 16 || (M <= RB_MAX_ROWS && N <= RB_MAX_COLS)) {
     e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
         : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
         : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)

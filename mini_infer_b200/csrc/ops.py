@@ -1066,12 +1066,11 @@ def sample(
 
 
 TMA_GEMM_MAX_ROWS = 128            # what gemm_tma.cu takes
-# ``linear`` routes inputs of up to this many rows, all that gemm_rows takes, to it; the library takes larger ones.
-# Measured on a B200 inside a captured decode step (Llama 3.1 8B sizes, milliseconds per step, own
-# product (gemm_tma) against the library's): up to 16 rows the own product is ahead, because it marks the weights
-# to leave the L2 first and does the block's additions and norms in its epilogues (batch 8: 3.74 vs 4.05;
-# batch 16: 4.17 vs 4.42; gemm_rows is another 16 us per layer ahead); from 32 rows on the library is (5.23 vs
-# 5.15; 64 rows: 7.34 vs 6.63).
+# ``linear`` routes inputs of up to this many rows, all that gemm_rows takes, to it; the library takes larger ones.  The four
+# products of a layer in a captured graph, us, gemm_rows and the library's: Llama 3.1 8B sizes 1 row 67.5 and 84.9, 8 70.7 and
+# 85.3, 16 77.9 and 84.0; 2048 wide 14.8 and 34.1, 17.6 and 30.4, 21.1 and 25.4.  (Beyond, gemm_tma and the library's: 8B sizes 17
+# rows 90.5 and 84.2, 32 93.2 and 90.2; 2048 wide 44.1 and 25.3, 45.9 and 25.8.)  The own product also does the block's
+# additions and norms in its epilogues.
 TMA_GEMM_DISPATCH_ROWS = 16
 USE_TMA_GEMM = os.environ.get("MINI_INFER_TMA_GEMM", "1") != "0"
 _tma_ws: dict[int, list[tuple[torch.Tensor, torch.Tensor]]] = {}

@@ -2,7 +2,7 @@
 
     python -m mini_infer_b200.microbench attention_decode --batch 8 --context 2048
     python -m mini_infer_b200.microbench attention_prefill --tokens 2048 [--impl mma]
-    python -m mini_infer_b200.microbench gemm_tma --rows 8 --n 28672 --k 4096 [--epilogue stream|stats]
+    python -m mini_infer_b200.microbench gemm_rows --rows 8 --n 28672 --k 4096 [--epilogue stream|stats]
     python -m mini_infer_b200.microbench add_rmsnorm --rows 8 --width 4096
     python -m mini_infer_b200.microbench norm_add --rows 16384 --width 2048
     python -m mini_infer_b200.microbench mlstm_gates --rows 2048 --heads 4
@@ -174,7 +174,8 @@ def attention_prefill(args, ops, device, flush) -> tuple[float, str]:
     return us, f"{flops / us / 1e6:.1f} TFLOP/s (causal flops)"
 
 
-def gemm_tma(args, ops, device, flush) -> tuple[float, str]:
+def few_rows_product(args, ops, device, flush) -> tuple[float, str]:
+    product = getattr(ops, args.kernel)
     x = torch.randn(args.rows, args.k, device=device, dtype=torch.bfloat16)
     w = torch.randn(args.n, args.k, device=device, dtype=torch.bfloat16)
     if args.epilogue == "stream":      # the product added to the fp32 stream, gain and statistics for the next norm
@@ -182,15 +183,18 @@ def gemm_tma(args, ops, device, flush) -> tuple[float, str]:
         gain = torch.ones(args.n, device=device)
 
         def run():
-            ops.gemm_tma(x, w, residual=stream, gain=gain, eps=1e-5)
-    elif args.epilogue == "stats":     # every row scaled by the statistics the product before left
-        stats = ops.RowStats(torch.rand(-(-args.k // 128), 16, device=device) * 128, args.k, 1e-5)
+            product(x, w, residual=stream, gain=gain, eps=1e-5)
+    elif args.epilogue == "stats":     # every row scaled by the statistics that a product of k features left
+        stream, one = torch.zeros(args.rows, args.k, device=device), torch.ones(args.k, device=device)
+        w_before = torch.randn(args.k, 64, device=device, dtype=torch.bfloat16)
+        _, stats = product(torch.randn(args.rows, 64, device=device, dtype=torch.bfloat16), w_before, residual=stream,
+                           gain=one, eps=1e-5)
 
         def run():
-            ops.gemm_tma(x, w, row_stats=stats)
+            product(x, w, row_stats=stats)
     else:
         def run():
-            ops.gemm_tma(x, w)
+            product(x, w)
 
     us = _time(run, args.iters, args.warmup, flush)
     status = ops.gemm_tma_status()
@@ -287,7 +291,8 @@ def sample(args, ops, device, flush) -> tuple[float, str]:
 KERNELS = {
     "attention_decode": attention_decode,
     "attention_prefill": attention_prefill,
-    "gemm_tma": gemm_tma,
+    "gemm_rows": few_rows_product,
+    "gemm_tma": few_rows_product,
     "add_rmsnorm": add_rmsnorm,
     "norm_add": norm_add,
     "mlstm_gates": mlstm_gates,
@@ -322,7 +327,7 @@ def main(argv=None) -> int:
                          "keys spread evenly over persistent blocks (default) or equal slices per request; "
                          "library: FlashInfer's paged prefill wrapper on the same shapes, for comparison")
     ap.add_argument("--epilogue", choices=["plain", "stream", "stats"], default="plain",
-                    help="gemm_tma: the plain product, or one of its fused forms for up to 16 rows")
+                    help="gemm_rows, gemm_tma: the plain product, or one of its fused forms for up to 16 rows")
     ap.add_argument("--rope", action="store_true",
                     help="attention_decode: give the kernel un-rotated q, k, v and the rotary table (it rotates and stores itself)")
     ap.add_argument("--skew", type=float, default=0.0,

@@ -209,6 +209,15 @@ def test_gemm_f32_gives_the_same_bits_from_every_kernel(N, K):
     assert torch.equal(ops().gemm_f32(a.to(DEV), odd[:, 1:]), full)
 
 
+@pytest.mark.parametrize("N", [8192, 8193, 8224])
+def test_gemm_f32_of_17_to_32_rows_on_either_side_of_the_widths_limit(N):
+    """The kernel for few rows up to 8192 columns, tiles above: the same bits."""
+    a, w = rnd(40, 72, seed=17).to(DEV), rnd(N, 72, seed=18).to(DEV)
+    full = ops().gemm_f32(a, w)
+    for M in (16, 17, 24, 32, 33):
+        assert torch.equal(ops().gemm_f32(a[:M], w), full[:M]), M
+
+
 @pytest.mark.parametrize("M", [1, 4, 8, 16, 32, 33])
 def test_gemm_f32_of_a_matrix_that_the_kernel_before_writes(M):
     """W is the result of a long product of this library right in front of the call: unless the caller says that it is constant,
