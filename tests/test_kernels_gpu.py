@@ -679,9 +679,10 @@ def test_decode_attention_after_a_recovery():
     clears them, and the next call merges every unit's stretches, none of them early."""
     args = ([1] * 3, [2048, 700, 129], 8, 2, 64, 16, torch.bfloat16)
     run_attention(*args, seed=11, kernel="balanced")
-    for _, _, counters in ops()._balanced_ws[0]:
-        counters[::3] = 1
-        counters[1::3] = 7
+    with torch.inference_mode():           # (a step may have made the buffers, in inference mode)
+        for _, _, counters in ops()._balanced_ws[0]:
+            counters[::3] = 1
+            counters[1::3] = 7
     ops().recover_from_wait_failure(torch.device(DEV))
     got, want = run_attention(*args, seed=11, kernel="balanced")
     assert torch.isfinite(got).all() and (got - want).abs().max().item() <= BF16_BOUND
