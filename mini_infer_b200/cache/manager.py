@@ -129,6 +129,11 @@ class AppendPlan:
         return np.concatenate([np.asarray(p, dtype=np.int64) for p in parts]) if parts else []
 
 
+# Portions longer than this get their slots as an array: 4, 32, 64 and 256 tokens take 3.4, 3.7, 3.8 and 4.8 us that way and
+# 1.0, 2.7, 4.7 and 16.3 as a list, page by page (pages of 16, the copy into the step's buffer included).
+ARRAY_PORTION = 48
+
+
 def group_needs(needs: Sequence) -> list[GroupSpec]:
     """Partition cache layers by what they keep per token."""
     order: list[tuple] = []
@@ -378,10 +383,16 @@ class CacheManager:
                     updates.extend((req.slot, len(table), page))
                     table.append(page)
                 parts = plan.slot_parts[gi]
-                if n_new == 1:
+                if n_new <= ARRAY_PORTION:
                     if not parts or not isinstance(parts[-1], list):
                         parts.append([])
-                    parts[-1].append(table[start // ps] * ps + start % ps)
+                    slots = parts[-1]
+                    if n_new == 1:
+                        slots.append(table[start // ps] * ps + start % ps)
+                    else:
+                        for idx in range(start // ps, -(-total // ps)):      # page by page
+                            base = table[idx] * ps
+                            slots.extend(range(base + max(0, start - idx * ps), base + min(ps, total - idx * ps)))
                 else:                                                    # all pages at once
                     first = start // ps
                     pages = np.array(table[first:-(-total // ps)], dtype=np.int64)

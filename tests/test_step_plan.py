@@ -56,6 +56,41 @@ def _timed(runner, entries):
     return time.perf_counter() - t0
 
 
+def test_slots_of_short_and_long_portions(monkeypatch):
+    """Lists up to ARRAY_PORTION tokens, arrays beyond, in any order, give every token the slot that its page and place make;
+    and short portions are not the slower for it (as arrays they cost 3 us each)."""
+    from mini_infer_b200.cache import manager
+
+    n = manager.ARRAY_PORTION
+    lens = [1, 2, 15, 16, 17, n - 1, n, n + 1, 3, 200, 1, n + 17, 5]
+
+    def plan(lens, first=5):
+        runner, cache = runner_for(n_layers=1, pages=2000)
+        for i in range(len(lens)):
+            cache.add_request(i)
+            cache.plan_append([(i, first)])
+        return cache, lambda: runner.host_plan([StepEntry(i, list(range(k)), []) for i, k in enumerate(lens)])
+
+    cache, go = plan(lens)
+    got, at = view(go(), "slots0"), 0
+    for i, k in enumerate(lens):
+        table = cache.table(i)
+        assert got[at:at + k] == [table[p // 16] * 16 + p % 16 for p in range(5, 5 + k)], i
+        at += k
+
+    def best():
+        times = []
+        for _ in range(30):
+            _, go = plan([17] * 48)
+            t0 = time.perf_counter()
+            go()
+            times.append(time.perf_counter() - t0)
+        return min(times)
+    lists = best()
+    monkeypatch.setattr(manager, "ARRAY_PORTION", 1)
+    assert lists < best()
+
+
 def test_layout_of_a_mixed_step_and_of_a_captured_one():
     runner, cache = runner_for(n_layers=2, pages=64, max_requests=4)
     for r in "ab":
