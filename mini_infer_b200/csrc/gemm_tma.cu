@@ -1,7 +1,8 @@
 // y[M, N] = x[M, K] * W[N, K]^T for few rows of x (decode): two weight-streaming products.
 // The engine's steps of up to 16 rows run gemm_rows_kernel, whose blocks exchange nothing (its
 // comment, further down, has both sides measured).  The other, gemm_tma_kernel, takes up to 128
-// rows on the fifth-generation tensor cores, as an entry point of its own:
+// rows on the fifth-generation tensor cores: for models whose sums of decode steps keep their
+// order, and as an entry point of its own:
 //
 // With a handful of tokens the product is bound by reading W once, so the kernel is built
 // around that stream.  The operands are swapped: 128 rows of W are the M side of the MMA and

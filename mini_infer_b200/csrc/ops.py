@@ -134,12 +134,12 @@ KEPT_MIN_CHUNKS = 4      # chunks of 64 keys that a block of decode attention ta
 def kept_sums():
     """Inside, and in this thread only, bfloat16 work of decode steps adds up in one order that does not change from one
     version of the kernels to the next: products of up to 16 rows run ``gemm_tma``, experts with few rows the streaming
-    kernel on CUDA cores, decode attention cuts its keys into stretches of four chunks or more.  Everywhere else the faster kernels run,
-    which are as close to the exact sums or closer.
+    kernel on CUDA cores, decode attention cuts its keys into stretches of four chunks or more.  Everywhere else the
+    faster kernels run, which are as close to the exact sums or closer.
 
     It is for models that turn a difference in the last bit into another answer: a router that first picks groups of experts
-    and is undecided between two groups changes several experts with large weights at once (a quarter of such a token's logits'
-    size, against a hundredth for an undecided last expert), and so much of what the model said before."""
+    and is undecided between two groups changes several experts with large weights at once (up to 0.4 of such a token's logits
+    in the 2-norm, against 0.08 where only the last expert is undecided), and so much of what the model said before."""
     before = getattr(_sums, "kept", False)
     _sums.kept = True
     try:
