@@ -151,10 +151,10 @@ struct GcDecay {
     hi = __fadd_rn(h, l);
     lo = __fadd_rn(l, -__fadd_rn(hi, -h));
   }
-  // x times the product, rounded once
+  // x times the product, rounded once (an infinite x stays infinite: its remainder would be inf - inf)
   __device__ __forceinline__ float of(float x) const {
     const float h = __fmul_rn(x, hi);
-    return __fadd_rn(h, fmaf(x, lo, fmaf(x, hi, -h)));
+    return isinf(h) ? h : __fadd_rn(h, fmaf(x, lo, fmaf(x, hi, -h)));
   }
 };
 

@@ -438,6 +438,29 @@ def test_what_a_token_brings_does_not_reach_the_tokens_before_it(decays, what, m
         assert torch.equal(run(spoilt)[:at], clean[:at]), at
 
 
+@pytest.mark.parametrize("decays", ["channel", "head", "token"])
+@pytest.mark.parametrize("at", [0, 31, 40, 63, 64, 100, 129])
+def test_an_infinite_key_leaves_what_it_leaves_in_the_walk(decays, at, monkeypatch):
+    """One channel of one key is infinite: that row of the state becomes infinite with the values' signs, the outputs from that
+    token on with the query's too, and nothing becomes NaN; the rest is finite.  Chunks and walk agree in each."""
+    o, n, heads, d = ops(), 130, 2, 48
+    q, k, v = (rnd(n, heads * d, seed=70 + i).bfloat16() for i in range(3))
+    k[at, 5], k[at, d + 7] = math.inf, -math.inf
+    z = (rnd(n, heads * d, seed=73) + 4).to(DEV) if decays == "channel" else None
+    hd = torch.tensor([0.9, 0.99]).to(DEV) if decays == "head" else None
+    tg = torch.sigmoid(rnd(n, heads, 3, seed=74) + 4).to(DEV) if decays == "token" else None
+    got = {}
+    for form, limit in (("walk", n), ("chunks", 0)):
+        monkeypatch.setattr(o, "GLA_LONG", limit)
+        state = torch.zeros(1, heads, d, d, device=DEV)
+        out = o.gla_scan(q.to(DEV), k.to(DEV), v.to(DEV), z, None, 1.0, 1.0, heads, d, d, state, ctx_for([n], [0]), head_decay=hd,
+                         tok_gates=tg)
+        got[form] = out.cpu(), state.cpu()
+    for walk, chunks in zip(*got.values()):
+        assert walk.isinf().any() and not walk.isnan().any() and not chunks.isnan().any()
+        assert torch.equal(walk.isinf(), chunks.isinf()) and torch.equal(walk[walk.isinf()], chunks[walk.isinf()])
+
+
 @pytest.mark.parametrize("scale", [1e15, 1e-15])
 @pytest.mark.parametrize("fall", [20.0, 40.0, 60.0, 75.0])
 def test_large_and_small_keys_beside_strong_decays(scale, fall, monkeypatch):
