@@ -152,6 +152,11 @@ def _sums_kept() -> bool:
     return getattr(_sums, "kept", False)
 
 
+def sums_kept() -> bool:
+    """Whether this thread is inside ``kept_sums``."""
+    return _sums_kept()
+
+
 def _sig_elementwise(lib: ctypes.CDLL) -> None:
     lib.mi_embedding.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_add_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1826,13 +1831,14 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     ``up_offset`` 0 is the plain ``silu(g) * u``).  Weights are stacked per expert:
     ``w_gate_up [E, 2 ff, H]`` (an expert's gate rows, then its up rows), ``w_down [E, H, ff]``.
     ``shared_gate`` (fp32, one number per token, any row stride): its sigmoid multiplies ``shared[t]``.
+    ``shared`` may also be a function that returns it, called when the experts' products are launched.
     Entries are sorted by expert on the device; nothing is read back.  Three routes: a step that
     brings an expert only a few rows streams the weights (bfloat16); large bfloat16 steps gather
     each expert's rows and use the library's grouped product (as the dense layers use the library's
     product for many rows); everything else walks 64-row tiles with this module's own kernels
     (tensor cores for bfloat16, CUDA cores with a fixed summation order for float32)."""
     global launch_count
-    _cuda(x, ids, weights, w_gate_up, w_down, shared)
+    _cuda(x, ids, weights, w_gate_up, w_down)
     _cols(x, "moe")
     M, H = x.shape
     E, ff2, _ = w_gate_up.shape
@@ -1844,10 +1850,15 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     if ids.dtype != torch.int32 or weights.dtype != torch.float32 or ids.shape != weights.shape or ids.shape[0] != M \
             or not ids.is_contiguous() or not weights.is_contiguous():
         raise KernelError("moe: ids int32 [M, top] and weights fp32 [M, top]")
-    if shared is not None:
+
+    def check_shared():
+        _cuda(shared)
         _cols(shared, "moe")
         if shared.shape != (M, H) or shared.dtype != x.dtype:
             raise KernelError("moe: the shared expert's output must be [M, H] in x's dtype")
+
+    if isinstance(shared, torch.Tensor):
+        check_shared()
     n = M * top
     lib = _lib("moe")
     pieces = (x.dtype == torch.bfloat16 and H % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0
@@ -1879,6 +1890,9 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
         rc = lib.mi_moe_down(_ptr(act), _ptr(w_down), H * ff, _ptr(plan), E, _ptr(y), n, H, ff, tile,
                              1 if _sums_kept() else 0, _code(x.dtype), _stream())
         _finish(lib, rc, "moe_down")
+    if callable(shared) and not isinstance(shared, torch.Tensor):
+        shared = shared()
+        check_shared()
     out = torch.empty((M, H), dtype=x.dtype, device=dev)
     if shared_gate is not None and (shared is None or shared_gate.dtype != torch.float32 or shared_gate.shape[0] != M
                                     or shared_gate.dim() > 2 or (shared_gate.dim() == 2 and shared_gate.shape[1] != 1)):

@@ -39,6 +39,7 @@ from .base import (
     register_position,
     register_stream_part,
 )
+from .streams import beside
 
 
 def _as_compute(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -800,17 +801,21 @@ class ParallelBlock(Arrangement):
             return self.mixer.forward(a, ctx, cache, self.position), stream
         if isinstance(n2, SameNorm):             # one norm, read by both branches
             a, stream = n1.forward(x, residual)
-            m = self.mixer.forward(a, ctx, cache, self.position)
-            return BranchSum((m, ff.forward(a, ctx))), stream
+            return BranchSum(self._branches(a, a, ctx, cache)), stream
         if isinstance(n1, LayerNorm) and isinstance(n2, LayerNorm) and n1.eps == n2.eps:
             a, b, stream = n1.forward_with(n2, x, residual)
         else:
             a, stream = n1.forward(x, residual)
             zero = torch.zeros_like(a)          # any pair of norms: the second one sees the same stream
             b, _ = n2.forward(zero, stream.clone())
-        m = self.mixer.forward(a, ctx, cache, self.position)
-        f = ff.forward(b, ctx)
-        return BranchSum((m, f)), stream
+        return BranchSum(self._branches(a, b, ctx, cache)), stream
+
+    def _branches(self, a, b, ctx, cache):
+        """Neither branch reads what the other writes."""
+        with beside() as side:
+            f = side.run(lambda: self.feed_forward.forward(b, ctx))
+            m = self.mixer.forward(a, ctx, cache, self.position)
+            return m, f()
 
 
 class BranchNormBlock(Arrangement):

@@ -9,6 +9,7 @@ import torch
 from ..csrc import ops
 from .base import FeedForward, ParamDecl, register_feed_forward
 from .builtin import Linear, _as_compute
+from .streams import beside
 
 
 class RoutedExperts(FeedForward):
@@ -126,19 +127,21 @@ class RoutedExperts(FeedForward):
                 self.shared_in = Linear(torch.cat([gate, up], dim=0).contiguous())
             self.shared_out = Linear(_as_compute(tensors["shared.down"], dtype).contiguous())
 
-    def forward(self, x, ctx):
-        shared = None
+    def _shared_expert(self, x):
         if self.shared_pairs is not None:
-            shared = self.shared_out(ops.linear_swiglu(x, self.shared_pairs, act="silu", w_constant=True))
-        elif self.shared_in is not None:
-            shared = self.shared_out(ops.clamped_glu(self.shared_in(x), self.shared_limit, self.alpha, self.up_offset))
-        ids, weights, logits = ops.moe_route(x, self.router, self.top, scores=self.scores, groups=self.groups,
-                                             keep_groups=self.keep_groups, scale=self.route_scale,
-                                             correction=self.choice_correction, group_top2=self.group_score == "top2",
-                                             experts=self.experts, return_logits=True, bias=self.logit_bias)
-        gate = logits[:, self.experts:self.experts + 1] if self.shared_gate else None
-        return ops.moe_experts(x, ids, weights, self.w_gate_up, self.w_down, self.limit, self.alpha, shared,
-                               up_offset=self.up_offset, shared_gate=gate)
+            return self.shared_out(ops.linear_swiglu(x, self.shared_pairs, act="silu", w_constant=True))
+        return self.shared_out(ops.clamped_glu(self.shared_in(x), self.shared_limit, self.alpha, self.up_offset))
+
+    def forward(self, x, ctx):
+        with beside() as side:      # the shared expert beside the router and the routed ones
+            shared = side.run(lambda: self._shared_expert(x)) if self.shared_ff else None
+            ids, weights, logits = ops.moe_route(x, self.router, self.top, scores=self.scores, groups=self.groups,
+                                                 keep_groups=self.keep_groups, scale=self.route_scale,
+                                                 correction=self.choice_correction, group_top2=self.group_score == "top2",
+                                                 experts=self.experts, return_logits=True, bias=self.logit_bias)
+            gate = logits[:, self.experts:self.experts + 1] if self.shared_gate else None
+            return ops.moe_experts(x, ids, weights, self.w_gate_up, self.w_down, self.limit, self.alpha, shared,
+                                   up_offset=self.up_offset, shared_gate=gate)
 
 
 register_feed_forward("routed_experts", RoutedExperts, replace=True)

@@ -15,12 +15,16 @@ columns.
 
 from __future__ import annotations
 
+import copy
+import functools
+
 import torch
 
 from ..csrc import ops
 from .base import KVNeed, LayerCache, Mixer, ParamDecl, PlanNeeds, StateNeed, StepContext, build_part, register_mixer
 from .builtin import InterleavedRotary, Linear, RotaryPosition, _as_compute
 from .spec import PartSpec
+from .streams import beside
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -758,15 +762,25 @@ class SideBySide(Mixer):
         proj32 = self._in32(x, out_dtype=torch.float32) if self._in32 is not None else None
         out = torch.empty((ctx.n_tokens, sum(c.out_width for c in self.children)), dtype=x.dtype, device=x.device)
         i0 = o0 = p0 = 0
-        for c, scale in zip(self.children, self.scales):
+        # Each has its own columns of both, and at most one keys and values and at most one a state; what the second one
+        # leaves for the layers behind it, in a dictionary of its own, is theirs when both are through.
+        second = copy.copy(ctx)
+        second.scratch = dict(ctx.scratch)
+        mixes = []
+        for c, scale, cx in zip(self.children, self.scales, (ctx, second)):
             kw = {}
             if c.in32_width:
                 kw["proj32"] = proj32[:, p0:p0 + c.in32_width]
                 p0 += c.in32_width
-            c.mix(proj[:, i0:i0 + c.in_width], out[:, o0:o0 + c.out_width], scale, ctx, cache,
-                  position if c.takes_position else None, **kw)
+            mixes.append(functools.partial(c.mix, proj[:, i0:i0 + c.in_width], out[:, o0:o0 + c.out_width], scale, cx, cache,
+                                           position if c.takes_position else None, **kw))
             i0 += c.in_width
             o0 += c.out_width
+        with beside() as side:
+            side.run(mixes[1])
+            mixes[0]()
+        for key, value in second.scratch.items():
+            ctx.scratch.setdefault(key, value)
         return self._out(out)
 
 

@@ -1,0 +1,69 @@
+"""Independent pieces of a layer side by side in a captured step.
+
+A step of a few tokens is a chain of short kernels, each of which leaves most of the chip idle at its ends.  Where a layer
+has two chains that only meet at an addition or an output projection (a mixer and a feed-forward that read the same stream,
+two mixers of one layer, a shared expert and the routed ones), the second one is recorded on a stream of its own, and the
+step's graph has two branches.  What a step computes does not depend on it, and neither do its kernels.
+
+Replays of decode steps of 8 requests, us, one branch and two: Ruvurax 4096 wide 851 and 802 (its experts' weights alone take
+400 at the copy bandwidth), Lilulix 2048 wide 335 and 298; Ruvurax 2048 wide, one request, 277 and 210.  With the mixer's
+branch on a stream of higher priority 821, 318 and 238: its kernels, launched ahead of their inputs, then hold the SMs
+while they wait.  Steps that are launched kernel by kernel stay one chain: they are bound by the host (two prompt steps of Ruvurax
+with two branches 4.9 ms where one takes 4.0), and so nothing is allocated on one stream and freed on another outside a capture.
+"""
+
+from __future__ import annotations
+
+import torch
+
+from ..csrc import ops
+
+# The stream beside each stream that steps are recorded on, per device (from the library's pool of a few dozen).
+_beside: dict[tuple[int, int], torch.cuda.Stream] = {}
+
+
+class beside:
+    """``with beside() as side:``  ``result = side.run(f)`` launches what ``f()`` launches on a stream beside the
+    current one, behind everything launched before; ``result()`` is what ``f`` returned (a tensor or None), and what is
+    launched after that call, or after the block, starts behind ``f``'s kernels.  In between neither ``f`` nor the rest touches
+    what the other writes.
+
+    The caller keeps every tensor that ``f`` reads alive until the block's end.  Only a captured step has the second
+    stream, and under ``ops.kept_sums`` not even that: ``gemm_tma``, which runs the products there, has one workspace per device."""
+
+    def __init__(self) -> None:
+        self.joined = True
+        self.on = torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing() and not ops.sums_kept()
+        if self.on:
+            self.here = torch.cuda.current_stream()
+            key = (self.here.device_index, self.here.cuda_stream)
+            self.stream = _beside.get(key)
+            if self.stream is None:
+                self.stream = _beside[key] = torch.cuda.Stream(self.here.device)
+
+    def __enter__(self) -> "beside":
+        return self
+
+    def run(self, f):
+        if not self.on:
+            value = f()
+            return lambda: value
+        self.stream.wait_stream(self.here)
+        self.joined = False
+        with torch.cuda.stream(self.stream):
+            value = f()
+
+        def result():
+            self._join()
+            if value is not None:
+                value.record_stream(self.here)      # its memory belongs to the stream beside
+            return value
+        return result
+
+    def _join(self) -> None:
+        if not self.joined:
+            self.joined = True
+            self.here.wait_stream(self.stream)
+
+    def __exit__(self, *error) -> None:
+        self._join()                   # behind an error as well: a capture ends with one stream

@@ -1,0 +1,48 @@
+"""Captured steps whose layers have two branches (``parts/streams.py``): the same bits as the steps launched kernel by
+kernel, which are one chain, over many replays back to back."""
+
+import importlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("model,which", [("ruvurax", "P"), ("ruvurax", "M"), ("lilulix", "A")])
+def test_two_branches_give_the_bits_of_one_chain(model, which, dtype):
+    from mini_infer_b200.engine import StepEntry
+    from mini_infer_b200.parts import streams
+
+    module = importlib.import_module(f"test_{model}_gpu")
+    cfg, n_new = module.CONFIGS[which], 40
+    tokens = [module.prompt(cfg, n + n_new, salt=30 + n) for n in (3, 11, 7)]
+    rows, used = {}, []
+    real = streams.beside.run
+
+    def run(self, f):
+        used.append(self.on)
+        return real(self, f)
+
+    streams.beside.run = run
+    try:
+        for graph in (False, True):
+            runner = module.make_runner(which, dtype, num_blocks=64, cuda_graph=graph)
+            for i in range(3):
+                runner.add_request(i)
+            runner.step([StepEntry(i, t[:len(t) - n_new]) for i, t in enumerate(tokens)])
+            got = []
+            for j in range(n_new):
+                step = runner.step([StepEntry(i, [t[len(t) - n_new + j]], [0]) for i, t in enumerate(tokens)])
+                got.append(step.logits.clone())
+            rows[graph] = torch.stack(got)
+            if graph:
+                assert any(used), "no branch was recorded"
+                assert all(s.replays == n_new - 1 for s in runner.stepper._graphs.values())
+            else:
+                assert used and not any(used)
+    finally:
+        streams.beside.run = real
+    assert torch.isfinite(rows[True]).all()
+    assert torch.equal(rows[True], rows[False])
