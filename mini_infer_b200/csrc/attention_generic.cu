@@ -37,10 +37,11 @@ MI_DEFINE_ERROR_API()
 #define BK 32
 #define NTHREADS 128
 
-// whether the instance for values of up to DMAX fetches these rows a chunk ahead
-template <int DMAX>
+// whether the instance for values of up to DMAX fetches these rows a chunk ahead (float32 rows of these sizes have
+// attention_f32_kernel)
+template <typename T, int DMAX>
 __host__ __device__ __forceinline__ bool rows_ahead(int d, int dv, int v_prefix) {
-  return DMAX <= 128 && d <= DMAX && (d & 3) == 0 && (dv & 3) == 0 && !v_prefix;
+  return sizeof(T) == 2 && DMAX <= 128 && d <= DMAX && (d & 3) == 0 && (dv & 3) == 0 && !v_prefix;
 }
 
 template <typename T, int DMAX>
@@ -63,8 +64,8 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
   float* Ss = Ks + BK * (d + 1);          // [BQ][BK]
   // With 16-byte pieces and heads of up to 128 the next chunk's rows come into registers while this one is worked on
   // (a chunk of 32 keys took 18 us when every one began with a round trip to the block table and one to its rows).
-  constexpr int PRE = DMAX <= 128 ? DMAX / 16 : 0;
-  const bool ahead = PRE > 0 && rows_ahead<DMAX>(d, dv, v_prefix);
+  constexpr int PRE = sizeof(T) == 2 && DMAX <= 128 ? DMAX / 16 : 0;
+  const bool ahead = PRE > 0 && rows_ahead<T, DMAX>(d, dv, v_prefix);
   // per key row of the chunk at hand (and of the next): element offset / d (-1: none) and chunk permutation
   int* rowbase2 = reinterpret_cast<int*>(Ss + BQ * BK);  // [1 or 2][BK]
   int* rowswz2 = rowbase2 + (ahead ? 2 : 1) * BK;        // [1 or 2][BK]
@@ -278,6 +279,323 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ 
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// float32, keys and values of up to 128 in whole 16-byte pieces: the 32-bit path's kernel.
+//
+// What bounds it: for prompts the reads of shared memory (16 bytes a lane, 4 cycles a warp: 8 of them for 64 multiply-adds of
+// the scores, 5 for 64 of the values), for single tokens the chain of a chunk (128 multiply-adds per score, then 32 per
+// column).  So the four warps of a block (16 query tokens of one head) walk the keys side by side: warp w takes the chunks of
+// 32 whose number is w modulo 4, with a running maximum, sum and output of its own, and the four are merged in the order of
+// the warps.  Which warp adds what, and in which order, depends on a key's position alone, so a row has the same bits
+// however the work is cut.  A warp copies its next keys (cp.async) while it works on the values, and the values while it
+// works on the scores.  A tile of one token spreads keys and columns over all 32 lanes instead of 4 rows per lane; its
+// sums run in the same order.  2 requests of 131 tokens, 16 heads over 4 of 128, in the kernel above and here: four
+// launches for the prompts and 16 for single tokens 1.10 and 0.36 ms (here 50 and 10 us each).
+// ------------------------------------------------------------------------------------------
+#define F32_WARPS 4
+#define F32_PPITCH 20        // floats per key of the weights (16 rows)
+
+__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool in) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(dst);
+  const int n = in ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(a), "l"(src), "r"(n) : "memory");
+}
+
+// the largest number of the lanes whose indices differ in the bits from lo to hi
+__device__ __forceinline__ float lanes_max(float v, int lo, int hi) {
+  for (int o = lo; o <= hi; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+template <int DMAX>
+__global__ void __launch_bounds__(32 * F32_WARPS)
+attention_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride,
+                     const float* __restrict__ kcache, const float* __restrict__ vcache,
+                     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ table_rows, int page_size,
+                     const int* __restrict__ q_start, const int* __restrict__ q_len, const int* __restrict__ kv_len,
+                     const int* __restrict__ tile_req, const int* __restrict__ tile_tok0, int nq, int nkv, int d, int dv,
+                     float scale, int window, int chunk, const float* __restrict__ sinks, const float* __restrict__ slopes,
+                     int keep, float softcap) {
+  mi_pdl_enter();   // inputs come from the kernels before this one
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kp = d + 4;                                  // pitch of query and key rows: eight rows touch every bank once
+  float* Qs = smem;                                      // [BQ][kp]
+  float* Ks = Qs + BQ * kp + warp * BK * (kp + dv);      // this warp's keys [BK][kp] ...
+  float* Vs = Ks + BK * kp;                              // ... values [BK][dv] ...
+  float* Ps = smem + BQ * kp + F32_WARPS * BK * (kp + dv) + warp * BK * F32_PPITCH;   // ... and weights [BK][16 rows]
+  __shared__ float merge_m[F32_WARPS][BQ], merge_l[F32_WARPS][BQ];
+
+  const int tile = blockIdx.x / nq, h = blockIdx.x - tile * nq;   // all heads of a tile, then the next tile (the caller lists long tiles first)
+  const int kvh = h / (nq / nkv);
+  const int b = tile_req[tile], tok0 = tile_tok0[tile];
+  const int ql = q_len[b], kl = kv_len[b], qs = q_start[b];
+  const int* table = block_table + (size_t)(table_rows ? table_rows[b] : b) * bt_stride;
+  const int rows = min(BQ, ql - tok0);
+  const int p0 = kl - ql + tok0, j_end = p0 + rows;      // the first query's position, one past the last visible key
+  int j_lo = window > 0 ? max(0, p0 - window + 1) : 0;   // the first row's bound is the lowest of the tile
+  if (chunk > 0) j_lo = max(j_lo, (p0 / chunk) * chunk);
+  const float slope = slopes ? slopes[h] : 0.f;
+  const MiKeyWalk<true> walk(j_lo, keep, BK);
+  const int n_chunks = walk.count(j_end, BK);
+  const int swz_k = mi_swizzle_mask_rows(d, 4), swz_v = mi_swizzle_mask_rows(dv, 4);
+
+  // the rows of a chunk: lane j holds key j's row in the caches (-1: not visible to any query) and its offset in the page
+  auto locate = [&](int c, int& base, int& off) {
+    const int j = c * BK + lane;
+    base = -1;
+    off = j % page_size;
+    if ((j >= j_lo || j < keep) && j < j_end) base = (table[j / page_size] * nkv + kvh) * page_size + off;
+  };
+  auto copy = [&](float* dst, int pitch, const float* cache, int width, int mask, int base, int off) {
+    const int pieces = width >> 2;
+    if (32 % pieces == 0) {          // a lane's piece is the same in every row
+      const int step = 32 / pieces, piece = lane % pieces;
+      int row = lane / pieces;
+#pragma unroll 8
+      for (int i = 0; i < pieces; ++i, row += step) {
+        const int rb = __shfl_sync(0xffffffffu, base, row), ro = __shfl_sync(0xffffffffu, off, row);
+        cp_async16_zfill(dst + row * pitch + piece * 4, cache + (size_t)max(rb, 0) * width + ((piece ^ (ro & mask)) << 2), rb >= 0);
+      }
+    } else {
+      for (int i = lane; i < BK * pieces; i += 32) {       // (every lane takes as many turns: BK is 32)
+        const int row = i / pieces, piece = i - row * pieces;
+        const int rb = __shfl_sync(0xffffffffu, base, row), ro = __shfl_sync(0xffffffffu, off, row);
+        cp_async16_zfill(dst + row * pitch + piece * 4, cache + (size_t)max(rb, 0) * width + ((piece ^ (ro & mask)) << 2), rb >= 0);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto next_of = [&](int i) {        // the first chunk of the walk from i on that is this warp's
+    while (i < n_chunks && (walk.chunk(i) & (F32_WARPS - 1)) != warp) ++i;
+    return i;
+  };
+
+  int ci = next_of(0), base = -1, off = 0;
+  if (ci < n_chunks) {
+    locate(walk.chunk(ci), base, off);
+    copy(Ks, kp, kcache, d, swz_k, base, off);
+    copy(Vs, dv, vcache, dv, swz_v, base, off);
+  }
+  for (int idx = tid; idx < (rows == 1 ? d : BQ * d); idx += 32 * F32_WARPS) {
+    const int r = idx / d, k = idx - r * d;
+    Qs[r * kp + k] = r < rows ? q[(size_t)(qs + tok0 + r) * q_stride + h * d + k] : 0.f;
+  }
+  __syncthreads();
+
+  const int rg = lane >> 3, c8 = lane & 7;
+  // many rows: row rg * 4 + i, keys c8 + 8 jj, columns c8 * 4 + 32 e ..; one row: key `lane`, columns lane * 4 ..
+  constexpr int NE = DMAX / 32;
+  float m_i[4], l_i[4], acc[4][NE * 4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m_i[i] = -INFINITY;
+    l_i[i] = 0.f;
+#pragma unroll
+    for (int e = 0; e < NE * 4; ++e) acc[i][e] = 0.f;
+  }
+  auto masked = [&](float s, int row, int j) {
+    const int p = p0 + row;
+    int lo = window > 0 ? max(0, p - window + 1) : 0;
+    if (chunk > 0) lo = max(lo, (p / chunk) * chunk);
+    // (every rounding is named: the two forms below must not contract it differently)
+    float v = __fmul_rn(s, scale);
+    if (softcap > 0.f) v = __fmul_rn(softcap, tanhf(v / softcap));
+    return row < rows && j <= p && (j >= lo || j < keep) ? fmaf(-slope, (float)(p - j), v) : -INFINITY;
+  };
+  const bool one = rows == 1;
+
+  while (ci < n_chunks) {
+    const int j0 = walk.chunk(ci) * BK;
+    const int cn = next_of(ci + 1);
+    int base_n = -1, off_n = 0;
+    if (cn < n_chunks) locate(walk.chunk(cn), base_n, off_n);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");       // the keys are there; the values may be under way
+    __syncwarp();
+    if (one) {
+      float s = 0.f;
+      const float4* kr = reinterpret_cast<const float4*>(Ks + lane * kp);
+      const float4* qr = reinterpret_cast<const float4*>(Qs);
+#pragma unroll 8
+      for (int k = 0; k < (d >> 2); ++k) {
+        const float4 kv = kr[k], qv = qr[k];
+        s = fmaf(qv.w, kv.w, fmaf(qv.z, kv.z, fmaf(qv.y, kv.y, fmaf(qv.x, kv.x, s))));
+      }
+      s = masked(s, 0, j0 + lane);
+      __syncwarp();
+      if (cn < n_chunks) copy(Ks, kp, kcache, d, swz_k, base_n, off_n);
+      else asm volatile("cp.async.commit_group;\n" ::: "memory");
+      const float m_new = fmaxf(m_i[0], lanes_max(s, 1, 16));
+      float alpha = 1.f, p = 0.f;
+      if (m_new != -INFINITY) {
+        alpha = expf(m_i[0] - m_new);
+        p = expf(s - m_new);
+      }
+      Ps[lane] = p;
+      p += __shfl_xor_sync(0xffffffffu, p, 8);
+      p += __shfl_xor_sync(0xffffffffu, p, 16);
+#pragma unroll
+      for (int o = 1; o <= 4; o <<= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+      l_i[0] = fmaf(l_i[0], alpha, p);
+      m_i[0] = m_new;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[0][e] = __fmul_rn(acc[0][e], alpha);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");     // the values
+      __syncwarp();
+      if (lane * 4 < dv) {
+#pragma unroll 8
+        for (int j = 0; j < BK; ++j) {
+          const float pj = Ps[j];
+          const float4 v = *reinterpret_cast<const float4*>(Vs + j * dv + lane * 4);
+          acc[0][0] = fmaf(pj, v.x, acc[0][0]);
+          acc[0][1] = fmaf(pj, v.y, acc[0][1]);
+          acc[0][2] = fmaf(pj, v.z, acc[0][2]);
+          acc[0][3] = fmaf(pj, v.w, acc[0][3]);
+        }
+      }
+    } else {
+      float s[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) s[i][jj] = 0.f;
+      if (rg * 4 < rows) {
+        const float* qr = Qs + rg * 4 * kp;
+        const float* kr = Ks + c8 * kp;
+#pragma unroll 2
+        for (int k = 0; k < d; k += 4) {
+          float4 qv[4], kv[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const float4*>(qr + i * kp + k);
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) kv[jj] = *reinterpret_cast<const float4*>(kr + 8 * jj * kp + k);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj)
+              s[i][jj] = fmaf(qv[i].w, kv[jj].w, fmaf(qv[i].z, kv[jj].z, fmaf(qv[i].y, kv[jj].y, fmaf(qv[i].x, kv[jj].x, s[i][jj]))));
+        }
+      }
+      __syncwarp();
+      if (cn < n_chunks) copy(Ks, kp, kcache, d, swz_k, base_n, off_n);
+      else asm volatile("cp.async.commit_group;\n" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          s[i][jj] = masked(s[i][jj], rg * 4 + i, j0 + c8 + 8 * jj);
+          mx = fmaxf(mx, s[i][jj]);
+        }
+        const float m_new = fmaxf(m_i[i], lanes_max(mx, 1, 4));
+        float alpha = 1.f;
+        if (m_new != -INFINITY) {
+          alpha = expf(m_i[i] - m_new);
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) s[i][jj] = expf(s[i][jj] - m_new);
+        } else {
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) s[i][jj] = 0.f;
+        }
+        float psum = (s[i][0] + s[i][1]) + (s[i][2] + s[i][3]);      // (the order of one row's butterfly)
+#pragma unroll
+        for (int o = 1; o <= 4; o <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
+        l_i[i] = fmaf(l_i[i], alpha, psum);
+        m_i[i] = m_new;
+#pragma unroll
+        for (int e = 0; e < NE * 4; ++e) acc[i][e] = __fmul_rn(acc[i][e], alpha);
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+        *reinterpret_cast<float4*>(Ps + (c8 + 8 * jj) * F32_PPITCH + rg * 4) = make_float4(s[0][jj], s[1][jj], s[2][jj], s[3][jj]);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");     // the values
+      __syncwarp();
+      if (rg * 4 < rows) {
+#pragma unroll 4
+        for (int j = 0; j < BK; ++j) {
+          const float4 p = *reinterpret_cast<const float4*>(Ps + j * F32_PPITCH + rg * 4);
+          const float pr[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+          for (int e = 0; e < NE; ++e) {
+            if (c8 * 4 + 32 * e >= dv) continue;
+            const float4 v = *reinterpret_cast<const float4*>(Vs + j * dv + c8 * 4 + 32 * e);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              acc[i][4 * e] = fmaf(pr[i], v.x, acc[i][4 * e]);
+              acc[i][4 * e + 1] = fmaf(pr[i], v.y, acc[i][4 * e + 1]);
+              acc[i][4 * e + 2] = fmaf(pr[i], v.z, acc[i][4 * e + 2]);
+              acc[i][4 * e + 3] = fmaf(pr[i], v.w, acc[i][4 * e + 3]);
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (cn < n_chunks) copy(Vs, dv, vcache, dv, swz_v, base_n, off_n);
+    ci = cn;
+  }
+
+  // the warps' shares, over their own keys' memory, then row by row in the order of the warps
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncwarp();
+  float* share = Ks;      // [rows][dv]
+  if (one) {
+    if (lane * 4 < dv) *reinterpret_cast<float4*>(share + lane * 4) = make_float4(acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
+    if (lane == 0) {
+      merge_m[warp][0] = m_i[0];
+      merge_l[warp][0] = l_i[0];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = rg * 4 + i;
+#pragma unroll
+      for (int e = 0; e < NE; ++e)
+        if (c8 * 4 + 32 * e < dv)
+          *reinterpret_cast<float4*>(share + row * dv + c8 * 4 + 32 * e) =
+              make_float4(acc[i][4 * e], acc[i][4 * e + 1], acc[i][4 * e + 2], acc[i][4 * e + 3]);
+      if (c8 == 0) {
+        merge_m[warp][row] = m_i[i];
+        merge_l[warp][row] = l_i[i];
+      }
+    }
+  }
+  __syncthreads();
+  const float* shares = smem + BQ * kp;
+  for (int idx = tid; idx < rows * dv; idx += 32 * F32_WARPS) {
+    const int row = idx / dv, col = idx - row * dv;
+    const float sink = sinks ? sinks[h] : -INFINITY;     // joins the denominator without a key or a value
+    float m = sink;
+#pragma unroll
+    for (int w = 0; w < F32_WARPS; ++w) m = fmaxf(m, merge_m[w][row]);
+    float l = 0.f, o = 0.f;
+#pragma unroll
+    for (int w = 0; w < F32_WARPS; ++w) {
+      const float f = merge_m[w][row] == -INFINITY ? 0.f : expf(merge_m[w][row] - m);
+      l = fmaf(merge_l[w][row], f, l);
+      o = fmaf(shares[w * BK * (kp + dv) + row * dv + col], f, o);
+    }
+    if (sinks) l += expf(sink - m);
+    if (l > 0.f) out[(size_t)(qs + tok0 + row) * out_stride + h * dv + col] = o * (1.f / l);
+  }
+}
+
+template <int DMAX>
+static int launch_f32(const void* q, int q_stride, void* out, int out_stride, const void* kcache, const void* vcache,
+                      const int* block_table, int bt_stride, const int* table_rows, int page_size, const int* q_start,
+                      const int* q_len, const int* kv_len, const int* tile_req, const int* tile_tok0, int n_tiles, int nq,
+                      int nkv, int d, int dv, float scale, int window, int chunk, const float* sinks, const float* slopes,
+                      int keep, float softcap, cudaStream_t stream) {
+  const size_t smem = ((size_t)BQ * (d + 4) + (size_t)F32_WARPS * BK * (d + 4 + dv) + F32_WARPS * BK * F32_PPITCH) * sizeof(float);
+  auto kern = attention_f32_kernel<DMAX>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  MI_LAUNCH((kern), (unsigned)(n_tiles * nq), 32 * F32_WARPS, smem, stream, (const float*)q, q_stride, (float*)out, out_stride,
+            (const float*)kcache, (const float*)vcache, block_table, bt_stride, table_rows, page_size, q_start, q_len, kv_len,
+            tile_req, tile_tok0, nq, nkv, d, dv, scale, window, chunk, sinks, slopes, keep, softcap);
+  return 0;
+}
+
 template <typename T, int DMAX>
 static int launch(const void* q, int q_stride, void* out, int out_stride, const void* kcache,
                   const void* vcache, const int* block_table, int bt_stride, const int* table_rows, int page_size,
@@ -286,7 +604,7 @@ static int launch(const void* q, int q_stride, void* out, int out_stride, const 
                   int chunk, const float* sinks, const float* slopes, int v_prefix, int keep, float softcap,
                   cudaStream_t stream) {
   const size_t smem = ((v_prefix ? 0 : (size_t)BK * ((dv + 3) & ~3)) + (size_t)BQ * d + (size_t)BK * (d + 1) + BQ * BK) *
-                          sizeof(float) + (rows_ahead<DMAX>(d, dv, v_prefix) ? 4 : 2) * BK * sizeof(int);
+                          sizeof(float) + (rows_ahead<T, DMAX>(d, dv, v_prefix) ? 4 : 2) * BK * sizeof(int);
   auto kern = attention_generic_kernel<T, DMAX>;
   if (smem > 227 * 1024) return MI_REFUSED - 1;
   if (smem > 48 * 1024) {
@@ -324,6 +642,18 @@ extern "C" int mi_attention_generic_capped(const void* q, int q_stride, void* ou
   if (page_size <= 0 || window < 0) MI_REFUSE("attention: bad page size %d or window %d", page_size, window);
   if (!mi_aligned(kcache, 16) || !mi_aligned(vcache, 16)) MI_REFUSE("attention: cache must be 16-byte aligned");
   int rc;
+  // One rule for every step of a model: its rows must not change kernels with the cutting.
+  if (dtype == MI_DTYPE_F32 && !v_prefix && d <= 128 && dv <= 128 && d % 4 == 0 && dv % 4 == 0) {
+#define MI_F32(DMAX)                                                                                                       \
+  rc = launch_f32<DMAX>(q, q_stride, out, out_stride, kcache, vcache, block_table, bt_stride, table_rows, page_size, q_start, \
+                        q_len, kv_len, tile_req, tile_tok0, n_tiles, nq, nkv, d, dv, scale, window, chunk, sinks, slopes, \
+                        keep, softcap, stream)
+    if (dv <= 64) MI_F32(64);
+    else MI_F32(128);
+#undef MI_F32
+    if (rc) return rc;
+    MI_RETURN_LAUNCH_STATUS();
+  }
 #define MI_GO(T, DMAX)                                                                              \
   rc = launch<T, DMAX>(q, q_stride, out, out_stride, kcache, vcache, block_table, bt_stride,        \
                        table_rows, page_size, q_start, q_len, kv_len, tile_req, tile_tok0, n_tiles, nq, nkv, d, dv, \

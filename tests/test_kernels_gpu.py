@@ -535,6 +535,34 @@ def test_attention_finds_a_far_key_among_hundreds(dtype):
         assert (got - want).abs().max().item() <= tol(dtype, fp32=2e-5, bf16=1 / 64)
 
 
+@pytest.mark.parametrize("window", [0, 5, 70])
+@pytest.mark.parametrize("nq,nkv,d,page,kl,n", [(4, 2, 128, 16, 300, 45), (3, 1, 16, 4, 131, 17), (2, 2, 48, 8, 33, 33),
+                                                (5, 5, 112, 32, 129, 1), (1, 1, 64, 16, 32, 31)])
+def test_float32_attention_has_the_same_bits_however_it_is_cut(nq, nkv, d, page, kl, n, window):
+    """A portion of ``n`` tokens in tiles of up to 16, in pairs and token by token (the warps' chunks, one row and many)."""
+    o = ops()
+    kc, vc, bt, ks, vs = build_paged([kl], nkv, d, page, torch.float32, seed=d)
+    kc, vc = as_pages(kc, page).to(DEV), as_pages(vc, page).to(DEV)
+    q = rnd(n, nq * d, seed=d + 1).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    rows = {}
+    for size in (n, 2, 1):
+        starts = list(range(0, n, size))
+        lens = [min(size, n - s) for s in starts]
+        tiles = [(b, t) for b, m in enumerate(lens) for t in range(0, m, o.ATTENTION_TILE_TOKENS)]
+        out = torch.full_like(q, float("nan"))
+        o.attention_generic(q, nq * d, out, kc, vc, bt.to(DEV), page, i32(starts), i32(lens),
+                            i32([kl - n + s + m for s, m in zip(starts, lens)]), i32([b for b, _ in tiles]),
+                            i32([t for _, t in tiles]), len(tiles), nq, nkv, d, d ** -0.5, window,
+                            table_rows=i32([0] * len(starts)))
+        rows[size] = out
+    want = P.causal_attention(q.cpu().double().view(n, nq, d), ks[0].double(), vs[0].double(), d ** -0.5, window or None,
+                              q_offset=kl - n)
+    assert torch.equal(rows[1], rows[n]) and torch.equal(rows[2], rows[n])
+    # scores of up to d products and sums over up to kl keys, rounded to 2^-24 each
+    assert (rows[n].cpu().double().view(n, nq, d) - want).abs().max().item() <= (d + kl) * 2.0 ** -24 * 8
+
+
 BF16_BOUND = 1 / 64      # probabilities and outputs are rounded to bfloat16 (2^-9 each)
 
 
