@@ -32,11 +32,11 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fP
 # library name -> (sources, extra headers that invalidate the cache, extra flags)
 LIBRARIES: dict[str, tuple[list[str], list[str], list[str]]] = {
     "elementwise": (["elementwise.cu"], ["common.cuh"], []),
-    "gemm_f32": (["gemm_f32.cu"], ["common.cuh"], []),
+    "gemm_f32": (["gemm_f32.cu"], ["common.cuh", "bulk_copy.cuh"], []),
     "attention_generic": (["attention_generic.cu"], ["common.cuh"], []),
     "sampling": (["sampling.cu"], ["common.cuh"], []),
     "attention_mma": (["attention_mma.cu"], ["common.cuh", "attention_noalloc.h"], []),
-    "gemm_tma": (["gemm_tma.cu"], ["common.cuh"], []),
+    "gemm_tma": (["gemm_tma.cu"], ["common.cuh", "bulk_copy.cuh"], []),
     "attention_tc": (["attention_tc.cu"], ["common.cuh"], []),
     "layernorm": (["layernorm.cu"], ["common.cuh"], []),
     "rope_norm": (["rope_norm.cu"], ["common.cuh"], []),

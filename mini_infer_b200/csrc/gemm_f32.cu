@@ -4,12 +4,14 @@
 // multiple of 32, the last one shorter), each accumulated from its first k on with fused multiply-adds, whatever kernel and
 // tile it falls in, so a row's result does not depend on which other rows share the call.
 //
-//   gemm_f32_rows_kernel   up to 32 rows (decode): bound by one reading of W
+//   gemm_f32_stream_kernel up to 4 rows (decode): bound by one reading of W
+//   gemm_f32_rows_kernel   up to 32 rows
 //   gemm_f32_tile_kernel   more rows: bound by the fused multiply-adds
 //   gemm_f32_any_kernel    operands without 16-byte rows
-#include "common.cuh"
+#include "bulk_copy.cuh"
 
 MI_DEFINE_ERROR_API()
+MI_DEFINE_STATUS_API(mi_gemm_f32_status)
 
 #define PARTS 4
 // where part p of k begins (a multiple of 32, so that a staged piece lies in one part)
@@ -28,6 +30,124 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) 
 __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync %0, 64;\n" ::"r"(part + 1) : "memory"); }
 
 // ------------------------------------------------------------------------------------------
+// Up to 4 rows.  What bounds it: the stream of W.  A block per SM owns N / 148 columns of the result (rows of W) over the
+// whole of k, in tiles of up to 32 columns, a lane each; warps 0 to 3 have a part of k each, and warp 4 feeds them by TMA,
+// 32 k of every part per stage, through a ring that is full of W before the wait for the kernel before and does not run
+// empty between tiles.  Two rows, 32000 x 2048: 67 us in blocks of 16 columns whose ring starts anew with
+// every block (the kernel below), 50 here (41 of bytes); a step of a four-layer model of that width (16 products of 3072 to
+// 6144 x 2048, the head) 290 us of products and 240.  Behind the stream stand the reads of A from shared memory, RM of them beside
+// one of W.
+// ------------------------------------------------------------------------------------------
+#define ST_K 32                     // k per part and stage: 128 bytes, one swizzle row
+#define ST_COLS 32                  // most columns per tile
+#define ST_MAX_ROWS 4
+#define ST_MAX_STAGES 16
+#define ST_THREADS (32 * (PARTS + 1))
+#define ST_BUDGET (200 * 1024)
+
+template <int RM>
+__global__ void __launch_bounds__(ST_THREADS, 1)
+gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* __restrict__ C,
+                       int M, int N, int K, int ldc, int cols, int n_tiles, int stages, int w_constant) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[ST_MAX_STAGES], empty[ST_MAX_STAGES];
+  __shared__ float sums[2][PARTS][RM][ST_COLS];
+  __shared__ int give_up;
+  // per stage and part a box of W (cols rows of 128 bytes) and one of A (M rows), each from a multiple of 1024 on
+  const uint32_t w_bytes = (uint32_t)cols * ST_K * 4, a_bytes = (uint32_t)M * ST_K * 4;
+  const uint32_t w_box = (w_bytes + 1023) & ~1023u, part_bytes = w_box + 1024, stage_bytes = PARTS * part_bytes;
+  mi_pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first = blockIdx.x * cols * n_tiles;
+  const int tiles = min(n_tiles, (N - first + cols - 1) / cols);
+  const int chunks = (part_begin(K, 1) + ST_K - 1) / ST_K;      // of the longest part; shorter ones read zeros from where they end
+  volatile int* gu = &give_up;
+
+  if (warp == PARTS) {
+    if (lane < stages) {
+      mbar_init(&full[lane], 2 * PARTS);       // the boxes of W and A
+      mbar_init(&empty[lane], PARTS);
+    }
+    if (lane == 0) give_up = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    __syncwarp();
+    asm volatile("bar.arrive 1, 160;\n" ::: "memory");
+    const int units = tiles * chunks, first_turn = min(stages, units);
+    const uint64_t policy = l2_policy_evict_first(), policy_a = l2_policy_evict_normal();
+    // lane p: W's box of part p; lane PARTS + p: A's.  A chunk behind the end of its part is asked for at K (a multiple of 4
+    // here): zeros.
+    const int part = lane & (PARTS - 1), k0 = part_begin(K, part), k1 = part_begin(K, part + 1);
+    auto load = [&](bool of_w, int st, int u) {
+      const int tile = u / chunks, k = k0 + (u - tile * chunks) * ST_K, x = k < k1 ? k : K;
+      unsigned char* dst = smem + (size_t)st * stage_bytes + part * part_bytes + (of_w ? 0u : w_box);
+      mbar_expect_tx(&full[st], of_w ? w_bytes : a_bytes);
+      tma_load_2d_hint(dst, of_w ? &map_w : &map_a, x, of_w ? first + tile * cols : 0, &full[st], of_w ? policy : policy_a);
+    };
+    if (!w_constant) mi_pdl_wait();
+    if (lane < PARTS)
+      for (int u = 0; u < first_turn; ++u) load(true, u, u);
+    if (w_constant) mi_pdl_wait();
+    if (lane >= PARTS && lane < 2 * PARTS)
+      for (int u = 0; u < first_turn; ++u) load(false, u, u);
+    __syncwarp();
+    if (lane < 2 * PARTS) {
+      int st = 0, round = 0;
+      for (int u = first_turn; u < units; ++u) {
+        if (!mbar_wait(&empty[st], round & 1, gu)) break;
+        load(lane < PARTS, st, u);
+        if (++st == stages) { st = 0; ++round; }
+      }
+    }
+    return;
+  }
+
+  asm volatile("bar.sync 1, 160;\n" ::: "memory");      // the barriers are initialised
+  mi_pdl_wait();                                        // the kernels before may read C
+  const int row = min(lane, cols - 1), sw = row & 7;
+  int st = 0, round = 0;
+  bool ok = true;
+  for (int tile = 0; tile < tiles; ++tile) {
+    float acc[RM];
+#pragma unroll
+    for (int i = 0; i < RM; ++i) acc[i] = 0.f;
+    for (int kc = 0; kc < chunks; ++kc) {
+      if (ok && !mbar_wait(&full[st], round & 1, gu)) ok = false;
+      if (ok) {
+        const unsigned char* ws = smem + (size_t)st * stage_bytes + warp * part_bytes + row * 128;
+        const unsigned char* as = smem + (size_t)st * stage_bytes + warp * part_bytes + w_box;
+        float4 w[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) w[c] = *reinterpret_cast<const float4*>(ws + ((c ^ sw) << 4));
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+#pragma unroll
+          for (int i = 0; i < RM; ++i) {      // (rows beyond M: whatever lies behind the box; nothing stores them)
+            const float4 a = *reinterpret_cast<const float4*>(as + i * 128 + ((c ^ i) << 4));
+            acc[i] = fmaf(a.w, w[c].w, fmaf(a.z, w[c].z, fmaf(a.y, w[c].y, fmaf(a.x, w[c].x, acc[i]))));
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+      if (++st == stages) { st = 0; ++round; }
+    }
+#pragma unroll
+    for (int i = 0; i < RM; ++i) sums[tile & 1][warp][i][lane] = acc[i];
+    asm volatile("bar.sync 2, 128;\n" ::: "memory");     // (the next tile writes the other half)
+    const int n = first + tile * cols + lane;
+    if (ok && lane < cols && n < N) {
+      for (int m = warp; m < M; m += PARTS) {
+        float v = sums[tile & 1][0][m][lane];
+#pragma unroll
+        for (int p = 1; p < PARTS; ++p) v += sums[tile & 1][p][m][lane];
+        C[(size_t)m * ldc + n] = v;
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------
 // Few rows.  A block owns 16 columns of the result (rows of W); 64 threads per part of k stream their part of
 // them, with the rows of A beside it, through a ring of stages filled by cp.async, 16 x 4 threads, RM rows of A each.  One
 // element's sum is a chain of K / 4 multiply-adds (4 cycles each: 1.1 us at K = 2048).  2 x 3072 x 2048 behind one another: 19 us with one part (a chain four times
@@ -37,7 +157,7 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 #define RB_COLS 16
 #define RB_K 32
 #define RB_PITCH (RB_K + 4)      // floats per staged row: eight rows' 16-byte pieces touch every bank once
-// Rows and tiles, us: N x K = 3072 x 2048 with 1 row 11 and 40, 16 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
+// Rows and tiles, us: N x K = 3072 x 2048 with 16 rows 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
 // and 52, 32 29 and 53; 6144 x 2048 16 28 and 58, 17 49 and 57, 32 56 and 58; 32000 x 2048 8 81 and 121, 16 115 and 121, 17
 // 222 and 121, 32 256 and 123 (a block's 16 columns then come round fourteen times, each with all rows).
 #define RB_MAX_ROWS 32
@@ -298,11 +418,46 @@ static cudaError_t launch_tile(const float* A, const float* W, float* C, int M, 
                    K, lda, ldw, ldc);
 }
 
+// A float32 matrix [rows, cols] with `ld` elements between rows, in boxes of box_rows x 32 with the 128-byte swizzle.
+static bool make_map_f32(CUtensorMap* map, const float* base, int rows, int cols, long long ld, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {ST_K, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int RM>
+static int launch_stream(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                         int w_constant, int sms, cudaStream_t stream) {
+  const int tiles = (N + ST_COLS * sms - 1) / (ST_COLS * sms), per = sms * tiles, cols = (N + per - 1) / per;
+  const int grid = (N + cols * tiles - 1) / (cols * tiles);
+  const int chunks = (part_begin(K, 1) + ST_K - 1) / ST_K;
+  const int stage_bytes = PARTS * (((cols * ST_K * 4 + 1023) & ~1023) + 1024);
+  int stages = ST_BUDGET / stage_bytes;
+  if (stages > ST_MAX_STAGES) stages = ST_MAX_STAGES;
+  if (stages > chunks * tiles) stages = chunks * tiles;
+  const size_t smem = (size_t)stages * stage_bytes + 1024;
+  CUtensorMap map_w, map_a;
+  if (!make_map_f32(&map_w, W, N, K, ldw, cols) || !make_map_f32(&map_a, A, M, K, lda, M))
+    MI_REFUSE("gemm_f32: the driver refused a tensor map (M %d, N %d, K %d)", M, N, K);
+  auto kern = gemm_f32_stream_kernel<RM>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  MI_LAUNCH(kern, grid, ST_THREADS, smem, stream, map_w, map_a, C, M, N, K, ldc, cols, tiles, stages, w_constant);
+  return 0;
+}
+
 // w_constant: W is not written by any kernel that may still run (a loaded weight).
 // Zero-padded tails of a part add exact zeros at the end of its sum, so they do not change it.
 extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
-                           int ldw, int ldc, int w_constant, cudaStream_t stream) {
+                           int ldw, int ldc, int w_constant, int sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
+  if (sms <= 0) MI_REFUSE("gemm_f32: bad number of SMs %d", sms);
   if (K <= 0) MI_REFUSE("gemm_f32: K must be positive, got %d", K);
   if (lda < K || ldw < K || ldc < N) MI_REFUSE("gemm_f32: leading dimensions too small");
   if ((M + 15) / 16 > 65535) MI_REFUSE("gemm_f32: too many rows (%d)", M);
@@ -311,9 +466,13 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
   if (!vec) {
     MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
               lda, ldw, ldc);
+  } else if (M <= ST_MAX_ROWS) {
+    const int rc = M == 1   ? launch_stream<1>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
+                   : M == 2 ? launch_stream<2>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
+                            : launch_stream<4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream);
+    if (rc) return rc;
   } else if (M <= 16 || (M <= RB_MAX_ROWS && N <= RB_MAX_COLS)) {
-    e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
-        : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+    e = M <= 8    ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
         : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
                   : launch_rows<8, 4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream);
   } else {

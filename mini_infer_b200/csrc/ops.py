@@ -68,7 +68,7 @@ _configured: set[str] = set()
 # Libraries whose kernels have bounded waits.  Their give-ups are reported into one int32 word
 # per device (``status_word``), which the engine copies to the host with every step's result;
 # on their own the libraries would each keep a word that only a synchronising call can read.
-_WAITING_LIBRARIES = ("attention_mma", "attention_tc", "gemm_tma")
+_WAITING_LIBRARIES = ("attention_mma", "attention_tc", "gemm_tma", "gemm_f32")
 _status_words: dict[int, torch.Tensor] = {}
 _status_shared: set[tuple[str, int]] = set()
 
@@ -171,7 +171,9 @@ def _sig_elementwise(lib: ctypes.CDLL) -> None:
 
 def _sig_gemm_f32(lib: ctypes.CDLL) -> None:
     lib.mi_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                c_int, c_int, c_void_p]
+                                c_int, c_int, c_int, c_void_p]
+    lib.mi_gemm_f32_status.argtypes = [c_int]
+    lib.mi_set_status_word.argtypes = [c_void_p]
 
 
 def _sig_attention_generic(lib: ctypes.CDLL) -> None:
@@ -599,9 +601,10 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, 
         out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     elif out.shape != (M, N) or out.dtype != torch.float32 or out.stride(1) != 1:
         raise KernelError("gemm_f32: bad output tensor")
-    lib = _lib("gemm_f32")
+    lib = _waiting_lib("gemm_f32", a.device)
     rc = lib.mi_gemm_f32(_ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0) if M > 1 else K,
-                         w.stride(0) if N > 1 else K, out.stride(0) if M > 1 else N, 1 if w_constant else 0, _stream())
+                         w.stride(0) if N > 1 else K, out.stride(0) if M > 1 else N, 1 if w_constant else 0,
+                         _sms(a.device), _stream())
     _finish(lib, rc, "gemm_f32")
     return out
 

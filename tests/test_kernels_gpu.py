@@ -209,6 +209,19 @@ def test_gemm_f32_gives_the_same_bits_from_every_kernel(N, K):
     assert torch.equal(ops().gemm_f32(a.to(DEV), odd[:, 1:]), full)
 
 
+@pytest.mark.parametrize("N,K", [(5, 4), (148, 132), (4736, 64), (4737, 100), (9500, 516), (33000, 36)])
+def test_gemm_f32_of_up_to_4_rows_in_tiles_of_columns(N, K):
+    """One to seven tiles per block, rings longer and shorter than the sum, parts of k without a term: the bits of the tiles of
+    40 rows, also into a wider result and for one row alone."""
+    a, w = rnd(40, K, seed=21).to(DEV), rnd(N, K, seed=22).to(DEV)
+    full = ops().gemm_f32(a, w)
+    for M in (1, 2, 3, 4):
+        assert torch.equal(ops().gemm_f32(a[:M], w, w_constant=M % 2 == 0), full[:M]), M
+    wide = torch.full((3, N + 7), float("nan"), device=DEV)
+    ops().gemm_f32(a[37:], w, out=wide[:, :N])
+    assert torch.equal(wide[:, :N], full[37:]) and torch.isnan(wide[:, N:]).all()
+
+
 @pytest.mark.parametrize("N", [8192, 8193, 8224])
 def test_gemm_f32_of_17_to_32_rows_on_either_side_of_the_widths_limit(N):
     """The kernel for few rows up to 8192 columns, tiles above: the same bits."""
