@@ -913,9 +913,9 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
     // pages and, once the other warps have come to the chunk's copy, over the copy's row of that position.  Blocks
     // that read the same chunk (other head groups of the key/value head) write the same bytes.
     if (!store_kv) return;
-    mi_pdl_wait();
     const int half = d >> 1, n_rot = half >> 3, cpr = d >> 3, per_unit = n_rot + cpr;
     int it = 0, n_new = 0;
+    bool waited = false;
     for (long long i = i0; i < i1;) {
       int b, u, c_rel, seg, n_b;
       const int len = balanced_part(i, i1, cum, B, U, ov, b, u, c_rel, seg, n_b);
@@ -924,6 +924,8 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
         const int kvh = u / hblocks, kl = kv_len[b], tok = q_start[b], pos = kl - 1, st = (it - 1) % DEC_STAGES;
         const int* table = block_table + (size_t)(table_rows ? table_rows[b] : b) * bt_stride;
         const int page = table[page_shift >= 0 ? (pos >> page_shift) : (pos / page_size)];
+        if (!waited) mi_pdl_wait();      // the plan's numbers are there before the kernel ahead is through, its product is not
+        waited = true;
         const int off = inpage_of(pos, page_size, page_shift), swz = off & swz_mask;
         const bf16* krow = q + (size_t)tok * q_stride + (size_t)(nq + kvh) * d;
         const bf16* vrow = krow + (size_t)nkv * d;
@@ -972,6 +974,14 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
     return;
   }
 
+  // the first unit's place in the plan, asked for ahead of the wait like the pages
+  int tok_first = 0, kl_first = 0;
+  if (i0 < i1) {
+    int b, u, c_rel, seg, n_b;
+    balanced_part(i0, i1, cum, B, U, ov, b, u, c_rel, seg, n_b);
+    tok_first = q_start[b];
+    kl_first = kv_len[b];
+  }
   mi_pdl_wait();   // the queries come from the kernel before this one
   const int ksteps = d >> 4;
   const float sc = scale * LOG2E;
@@ -991,7 +1001,7 @@ attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16*
     const int kvh = u / hblocks, hb = u - kvh * hblocks;
     const int heads_here = min(DEC_HEADS, g - hb * DEC_HEADS);
     const int head0 = kvh * g + hb * DEC_HEADS;
-    const int kl = kv_len[b], tok = q_start[b];
+    const int kl = i == i0 ? kl_first : kv_len[b], tok = i == i0 ? tok_first : q_start[b];
     const int lo = first_visible(kl - 1, window);
     const MiKeyWalk<EXT> walk(lo, keep, KCHUNK);
 
