@@ -12,6 +12,8 @@
 // gather list is given, else i.  Gains and biases are fp32.
 #include "common.cuh"
 
+#include <initializer_list>
+
 MI_DEFINE_ERROR_API()
 
 template <typename T>
@@ -101,6 +103,96 @@ __global__ void add_layernorm_kernel(const float* __restrict__ stream, const T* 
   }
 }
 
+// The same for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays in registers, and the gains and
+// biases, which no kernel writes, are asked for before the wait.  Every piece is read and written once, in one round trip: 8
+// rows of 4096 with two norms 8.3 us in the kernel above, 3.5 here; 2048 rows of 2048 24
+// and 15 us (10 of bytes).
+template <typename T, int NV>
+__global__ void __launch_bounds__(512)
+add_layernorm4_kernel(const float* __restrict__ stream, const T* __restrict__ add1, const T* __restrict__ add2,
+                      float* __restrict__ stream_out, const int* __restrict__ rows, const float* __restrict__ w1,
+                      const float* __restrict__ b1, T* __restrict__ out1, const float* __restrict__ w2,
+                      const float* __restrict__ b2, T* __restrict__ out2, int H, float eps) {
+  mi_pdl_launch_dependents();
+  __shared__ float red[32];
+  float g1[NV][4], c1[NV][4], g2[NV][4], c2[NV][4], r[NV][4], f[4];
+  Vec4<float> v;
+  Vec4<T> a;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int k = 4 * (threadIdx.x + n * blockDim.x);
+    if (k < H) {
+      v.load(w1 + k); v.get(g1[n]);
+      v.load(b1 + k); v.get(c1[n]);
+      if (out2) {
+        v.load(w2 + k); v.get(g2[n]);
+        v.load(b2 + k); v.get(c2[n]);
+      }
+    }
+  }
+  mi_pdl_wait();
+  const size_t i = blockIdx.x, src = rows ? rows[i] : i;
+  float sum = 0.f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int k = 4 * (threadIdx.x + n * blockDim.x);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) r[n][e] = 0.f;
+    if (k < H) {
+      v.load(stream + src * H + k);
+      v.get(r[n]);
+      if (add1) {
+        a.load(add1 + src * H + k);
+        a.get(f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+      }
+      if (add2) {
+        a.load(add2 + src * H + k);
+        a.get(f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+      }
+      sum += (r[n][0] + r[n][1]) + (r[n][2] + r[n][3]);
+    }
+  }
+  const float mean = mi_block_sum(sum, red) / (float)H;
+  float sq = 0.f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+    if (4 * (threadIdx.x + n * blockDim.x) < H) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float dlt = r[n][e] - mean;
+        sq += dlt * dlt;
+      }
+    }
+  const float rstd = 1.f / sqrtf(mi_block_sum(sq, red) / (float)H + eps);
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int k = 4 * (threadIdx.x + n * blockDim.x);
+    if (k >= H) continue;
+    if (stream_out) {
+      v.set(r[n]);
+      v.store(stream_out + i * H + k);
+    }
+    float y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      f[e] = (r[n][e] - mean) * rstd;
+      y[e] = f[e] * g1[n][e] + c1[n][e];
+    }
+    a.set(y);
+    a.store(out1 + i * H + k);
+    if (out2) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = f[e] * g2[n][e] + c2[n][e];
+      a.set(y);
+      a.store(out2 + i * H + k);
+    }
+  }
+}
+
 extern "C" int mi_add_layernorm(const float* stream, const void* add1, const void* add2, float* stream_out,
                                 const int* rows, const float* w1, const float* b1, void* out1,
                                 const float* w2, const float* b2, void* out2, int M, int H, float eps,
@@ -111,6 +203,29 @@ extern "C" int mi_add_layernorm(const float* stream, const void* add1, const voi
   const size_t smem = (32 + (size_t)H) * sizeof(float);
   if (smem > 200 * 1024) MI_REFUSE("layernorm: a row of %d floats does not fit in shared memory", H);
   const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
+  bool pieces = H % 4 == 0 && H <= 16 * threads;
+  for (const void* ptr : {(const void*)stream, add1, add2, (const void*)stream_out, (const void*)w1, (const void*)b1,
+                          (const void*)out1, (const void*)w2, (const void*)b2, (const void*)out2})
+    pieces = pieces && mi_aligned(ptr, 16);
+  if (pieces) {
+#define MI_GO4(T, NV)                                                                                               \
+  MI_LAUNCH((add_layernorm4_kernel<T, NV>), M, threads, 0, stream_, stream, (const T*)add1, (const T*)add2, stream_out, \
+            rows, w1, b1, (T*)out1, w2, b2, (T*)out2, H, eps)
+#define MI_GO4_T(T)                          \
+  if (H <= 4 * threads) MI_GO4(T, 1);        \
+  else if (H <= 8 * threads) MI_GO4(T, 2);   \
+  else MI_GO4(T, 4)
+    if (dtype == MI_DTYPE_F32) {
+      MI_GO4_T(float);
+    } else if (dtype == MI_DTYPE_BF16) {
+      MI_GO4_T(bf16);
+    } else {
+      MI_REFUSE("layernorm: unknown dtype %d", dtype);
+    }
+#undef MI_GO4_T
+#undef MI_GO4
+    MI_RETURN_LAUNCH_STATUS();
+  }
 #define MI_GO(T)                                                                                       \
   do {                                                                                                 \
     auto kern = add_layernorm_kernel<T>;                                                               \

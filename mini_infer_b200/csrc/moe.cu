@@ -49,6 +49,9 @@ __device__ __forceinline__ float mi_clamped_glu_value(float g, float u, float li
 #define ROUTE_MAX_PER_LANE 8
 #define ROUTE_WARPS 4
 
+// PER: experts (and groups) per lane, known to the compiler: 8 tokens of 32 experts took
+// 5.3 us with eight of them, 3.3 with one.
+template <int PER>
 __global__ void __launch_bounds__(32 * ROUTE_WARPS)
 moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict__ ids,
                   float* __restrict__ weights, int M, int E, int top, int mode, int n_groups,
@@ -56,15 +59,15 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
                   const float* __restrict__ bias) {
   // bias [E]: added to the logits before anything else; correction [E] (mode 2): to the choice scores alone
   mi_pdl_enter();
-  __shared__ float choice_sh[ROUTE_WARPS][32 * ROUTE_MAX_PER_LANE];
+  __shared__ float choice_sh[ROUTE_WARPS][32 * PER];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x * ROUTE_WARPS + warp;
   if (t >= M) return;
   const float* z = logits + (size_t)t * stride;
-  float lg[ROUTE_MAX_PER_LANE];       // choice scores; minus infinity: out of the race
-  float sc[ROUTE_MAX_PER_LANE];       // mode 2: the scores that become weights
+  float lg[PER];       // choice scores; minus infinity: out of the race
+  float sc[PER];       // mode 2: the scores that become weights
 #pragma unroll
-  for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
     lg[i] = e < E ? z[e] + (bias ? bias[e] : 0.f) : -INFINITY;
     sc[i] = 0.f;
@@ -76,10 +79,10 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
   float zmax = -INFINITY, zsum = 0.f;
   if (mode == 1) {
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i) zmax = fmaxf(zmax, lg[i]);
+    for (int i = 0; i < PER; ++i) zmax = fmaxf(zmax, lg[i]);
     zmax = mi_warp_max(zmax);
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i)
+    for (int i = 0; i < PER; ++i)
       if (lane + 32 * i < E) zsum += expf(lg[i] - zmax);
     zsum = mi_warp_sum(zsum);
   }
@@ -89,12 +92,12 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
     const int per = E / n_groups;
     float* mine = choice_sh[warp];
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i)
+    for (int i = 0; i < PER; ++i)
       if (lane + 32 * i < E) mine[lane + 32 * i] = lg[i];
     __syncwarp();
-    float gs[ROUTE_MAX_PER_LANE];
+    float gs[PER];
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i) {
+    for (int i = 0; i < PER; ++i) {
       const int g = lane + 32 * i;
       gs[i] = -INFINITY;
       if (g < n_groups) {
@@ -112,7 +115,7 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
       float best = -INFINITY;
       int best_g = 0x7fffffff;
 #pragma unroll
-      for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i) {
+      for (int i = 0; i < PER; ++i) {
         const int g = lane + 32 * i;
         if (g < n_groups && !((kept_mask >> i) & 1u) && (gs[i] > best || (gs[i] == best && g < best_g))) {
           best = gs[i];
@@ -132,7 +135,7 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
       if ((best_g & 31) == lane) kept_mask |= 1u << (best_g >> 5);
     }
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i) {
+    for (int i = 0; i < PER; ++i) {
       const int e = lane + 32 * i;
       const int g = e < E ? e / per : 0;
       const unsigned owner_mask = __shfl_sync(0xffffffffu, kept_mask, g & 31);   // every lane takes part
@@ -145,7 +148,7 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
     float best = -INFINITY;
     int best_e = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i) {
+    for (int i = 0; i < PER; ++i) {
       const int e = lane + 32 * i;
       if (e < E && (lg[i] > best || (lg[i] == best && e < best_e)) && lg[i] != -INFINITY) {
         best = lg[i];
@@ -163,7 +166,7 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
     }
     float score = 0.f;
 #pragma unroll
-    for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i)
+    for (int i = 0; i < PER; ++i)
       if (best_e == lane + 32 * i) {
         lg[i] = -INFINITY;   // taken
         score = sc[i];
@@ -197,8 +200,13 @@ extern "C" int mi_moe_select(const float* logits, int stride, int* ids, float* w
     if (keep <= 0 || keep > n_groups) MI_REFUSE("moe: %d of %d groups kept", keep, n_groups);
     if (keep * (E / n_groups) < top) MI_REFUSE("moe: %d groups of %d experts cannot give %d experts", keep, E / n_groups, top);
   }
-  MI_LAUNCH((moe_select_kernel), (M + ROUTE_WARPS - 1) / ROUTE_WARPS, 32 * ROUTE_WARPS, 0, stream, logits, stride, ids,
-            weights, M, E, top, mode, n_groups, keep, scale, correction, group_top2, bias);
+#define MI_SELECT(PER)                                                                                                    \
+  MI_LAUNCH((moe_select_kernel<PER>), (M + ROUTE_WARPS - 1) / ROUTE_WARPS, 32 * ROUTE_WARPS, 0, stream, logits, stride, ids, \
+            weights, M, E, top, mode, n_groups, keep, scale, correction, group_top2, bias)
+  if (E <= 32) MI_SELECT(1);
+  else if (E <= 64) MI_SELECT(2);
+  else MI_SELECT(ROUTE_MAX_PER_LANE);
+#undef MI_SELECT
   MI_RETURN_LAUNCH_STATUS();
 }
 

@@ -347,7 +347,7 @@ def _sig_stream(lib: ctypes.CDLL) -> None:
                                            c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, ll, ll, c_int,
                                            c_void_p]
     lib.mi_add_rmsnorm_multi.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                         c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
+                                         c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_int, c_void_p]
     lib.mi_glu_mul_pairs.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_embedding_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
                                          c_void_p]
@@ -2021,7 +2021,8 @@ def add_rmsnorm_multi(stream: torch.Tensor | None, adds, gain: torch.Tensor, eps
     lib = _lib("stream")
     rc = lib.mi_add_rmsnorm_multi(_ptr(stream), _ptr(adds[0] if adds else None), _ptr(adds[1] if len(adds) > 1 else None),
                                   _ptr(add32), _ptr(row_add), _ptr(new_stream), _ptr(rows), _ptr(gain), _ptr(out),
-                                  M, H, float(eps), _code(dtype), _stream())
+                                  M, H, float(eps), 1 if _sums_kept() else 0,
+                                  _code(dtype), _stream())
     _finish(lib, rc, "rmsnorm")
     return out, new_stream
 

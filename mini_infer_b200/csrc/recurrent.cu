@@ -982,6 +982,44 @@ __global__ void headnorm_gate_kernel(const float* __restrict__ o, int o_stride, 
   }
 }
 
+// The same for heads of PER * 32 without a normaliser: a head, its gate and the gain are asked for at once and stay in registers.
+// The sums run in the order of the kernel above.  8 tokens of 16 heads of 128: 3.5 and
+// 2.1 us.
+template <typename T, int PER>
+__global__ void __launch_bounds__(128)
+headnorm_gate_lanes_kernel(const float* __restrict__ o, int o_stride, const float* __restrict__ w, const T* __restrict__ g,
+                           int g_stride, T* __restrict__ out, int out_stride, int M, int heads, float eps, int act,
+                           float scale, int w_head) {
+  mi_pdl_enter();
+  constexpr int dv = 32 * PER;
+  const int lane = threadIdx.x & 31;
+  const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (unit >= (long long)M * heads) return;
+  const int t = (int)(unit / heads), h = (int)(unit - (long long)t * heads);
+  const float* src = o + (size_t)t * o_stride + (size_t)h * dv + lane;
+  float v[PER], gv[PER], gain[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    v[j] = src[32 * j];
+    gv[j] = act ? mi_to_float(g[(size_t)t * g_stride + h * dv + lane + 32 * j]) : 0.f;
+    gain[j] = w[(size_t)h * w_head + lane + 32 * j];
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) ss += v[j] * v[j];
+  ss = mi_warp_sum(ss);
+  const float mult = 1.f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    float a = 1.f;
+    if (act) {
+      const float sg = 1.f / (1.f + expf(-gv[j]));
+      a = act == 2 ? gv[j] * sg : sg;
+    }
+    out[(size_t)t * out_stride + h * dv + lane + 32 * j] = mi_from_float<T>(v[j] * mult * gain[j] * a * scale);
+  }
+}
+
 extern "C" int mi_headnorm_gate(const float* o, int o_stride, const float* w, const void* g, int g_stride,
                                 void* out, int out_stride, int M, int heads, int dv, float eps, int act,
                                 float scale, int w_head, const float* tok_gates, float den_eps, int dtype,
@@ -991,6 +1029,23 @@ extern "C" int mi_headnorm_gate(const float* o, int o_stride, const float* w, co
   const long long units = (long long)M * heads;
   const long long blocks = (units + 3) / 4;
   if (blocks > 0x7fffffffLL) MI_REFUSE("headnorm_gate: too many blocks for one launch");
+  if (!tok_gates && (dv == 64 || dv == 128 || dv == 256) && (dtype == MI_DTYPE_F32 || dtype == MI_DTYPE_BF16)) {
+#define MI_LANES(T, PER)                                                                                           \
+  MI_LAUNCH((headnorm_gate_lanes_kernel<T, PER>), (unsigned)blocks, 128, 0, stream, o, o_stride, w, (const T*)g, g_stride, \
+            (T*)out, out_stride, M, heads, eps, act, scale, w_head)
+#define MI_LANES_T(T)               \
+  if (dv == 64) MI_LANES(T, 2);     \
+  else if (dv == 128) MI_LANES(T, 4); \
+  else MI_LANES(T, 8)
+    if (dtype == MI_DTYPE_F32) {
+      MI_LANES_T(float);
+    } else {
+      MI_LANES_T(bf16);
+    }
+#undef MI_LANES_T
+#undef MI_LANES
+    MI_RETURN_LAUNCH_STATUS();
+  }
   if (dtype == MI_DTYPE_F32)
     MI_LAUNCH((headnorm_gate_kernel<float>), (unsigned)blocks, 128, 0, stream, o, o_stride, w, (const float*)g,
               g_stride, (float*)out, out_stride, M, heads, dv, eps, act, scale, w_head, tok_gates, den_eps);

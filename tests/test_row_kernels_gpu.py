@@ -1,0 +1,170 @@
+"""The forms of the small row kernels that take whole aligned pieces against those that take any row: the same call on a
+tensor that starts four bytes off, or with a width that is no multiple of a piece, reaches the other form."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+DTYPES = [torch.float32, torch.bfloat16]
+
+
+def ops():
+    from mini_infer_b200.csrc import ops as o
+    return o
+
+
+def rnd(*shape, dtype=torch.float32, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(dtype).to(DEV)
+
+
+def shifted(t):
+    """The same numbers at an address that is no multiple of 16."""
+    flat = torch.empty(t.numel() + 2, dtype=t.dtype, device=t.device)[2:]
+    flat.copy_(t.reshape(-1))
+    return flat.view(t.shape)
+
+
+def bound(dtype, want):
+    # a norm of fp32 sums over up to 8192 numbers in two orders: some ulps; a bfloat16 result may round the other way
+    return (2.0 ** -7 if dtype == torch.bfloat16 else 1e-5) * want.abs().max().clamp(min=1.0).item()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,H", [(1, 4), (3, 516), (8, 2048), (5, 2052), (2, 4096), (3, 8192), (2, 8196), (4, 4099)])
+def test_layer_norm_in_registers(dtype, M, H):
+    o = ops()
+    stream, a1, a2 = rnd(M, H, seed=1), rnd(M, H, dtype=dtype, seed=2), rnd(M, H, dtype=dtype, seed=3)
+    w1, b1, w2, b2 = (rnd(H, seed=s) for s in (4, 5, 6, 7))
+    r = stream.double() + a1.double() + a2.double()
+    n = (r - r.mean(dim=1, keepdim=True)) * torch.rsqrt(r.var(dim=1, unbiased=False, keepdim=True) + 1e-6)
+    for adds in ((a1, a2), (shifted(a1), a2)):
+        new = stream.clone()
+        out1, out2 = o.add_layernorm(new, adds, [(w1, b1), (w2, b2)], 1e-6, dtype)
+        assert (new.double() - r).abs().max().item() <= 1e-6 * r.abs().max().item()
+        for got, w, b in ((out1, w1, b1), (out2, w2, b2)):
+            want = n * w.double() + b.double()
+            assert (got.double() - want).abs().max().item() <= bound(dtype, want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,H", [(1, 8), (3, 516), (8, 2048), (2, 4096), (3, 8192), (2, 8196), (4, 4099)])
+def test_norm_of_several_addends_in_registers(dtype, M, H):
+    o = ops()
+    stream, add32, row_add, gain = rnd(M, H, seed=1), rnd(M, H, seed=2), rnd(H, seed=3), rnd(H, seed=4)
+    a1, a2 = rnd(M, H, dtype=dtype, seed=5), rnd(M, H, dtype=dtype, seed=6)
+    for adds, extra in (((a1, a2), True), ((shifted(a1), a2), True), ((a1,), False), ((), True)):
+        kw = dict(add32=add32, row_add=row_add) if extra else {}
+        r = stream.double() + sum(a.double() for a in adds) + ((add32.double() + row_add.double()) if extra else 0.0)
+        want = gain.double() * r * torch.rsqrt((r * r).mean(dim=1, keepdim=True) + 1e-6)
+        out, new = o.add_rmsnorm_multi(stream, adds, gain, 1e-6, dtype, **kw)
+        assert (new.double() - r).abs().max().item() <= 1e-6 * r.abs().max().item()
+        assert (out.double() - want).abs().max().item() <= bound(dtype, want)
+        with o.kept_sums():                   # the order that kept sums have: close, and the same stream
+            kept, stream_kept = o.add_rmsnorm_multi(stream, adds, gain, 1e-6, dtype, **kw)
+        assert torch.equal(stream_kept, new) and (kept.double() - want).abs().max().item() <= bound(dtype, want)
+
+
+@pytest.mark.parametrize("act", ["sigmoid", "silu"])
+@pytest.mark.parametrize("M,C,per", [(1, 8, 1), (3, 264, 1), (70, 1024, 1), (5, 256, 128), (5, 96, 8), (4, 96, 4), (3, 100, 1)])
+def test_gate_in_pieces_has_the_bits_of_single_elements(M, C, per, act):
+    o = ops()
+    x, g = rnd(M, C + 24, dtype=torch.bfloat16, seed=1)[:, 8:8 + C], rnd(M, C // per, dtype=torch.bfloat16, seed=2)
+    out, single = (torch.empty(M, C, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    o.gate_mul(x, g, out, act, 0.5, per=per)
+    o.gate_mul(shifted(x.contiguous()), g, single, act, 0.5, per=per)
+    assert torch.equal(out, single)
+    z = g.double().repeat_interleave(per, dim=1)
+    want = x.double() * torch.sigmoid(z) * (z if act == "silu" else 1.0) * 0.5
+    assert (out.double() - want).abs().max().item() <= 2.0 ** -8 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M", [3, 70])
+@pytest.mark.parametrize("d,rot", [(64, 64), (64, 0), (128, 128), (128, 64), (128, 0), (256, 256), (256, 128), (128, 32), (96, 96)])
+def test_normed_and_rotated_heads_in_registers(dtype, M, d, rot):
+    """Heads whose pairs lie in one lane, and (the last two) those that go through shared memory, against float64."""
+    o, nq, nkv, page = ops(), 5, 2, 8
+    x = rnd(M, (nq + 2 * nkv) * d, dtype=dtype, seed=1)
+    qg, kg = rnd(d, seed=2), rnd(d, seed=3)
+    positions = torch.arange(M, dtype=torch.int32, device=DEV) * 37 + 5
+    freq = 10000.0 ** (-torch.arange(0, max(rot, 2), 2, dtype=torch.float64, device=DEV) / max(rot, 2))
+    caches = [torch.zeros(-(-M // page), nkv, page, d, dtype=dtype, device=DEV) for _ in range(2)]
+    packed = x.clone()
+    o.qk_norm_rope_store(packed, 0, nq * d, (nq + nkv) * d, nq, nkv, d, d, q_gain=qg, k_gain=kg, eps=1e-6, rot=rot,
+                         positions=positions, freq=freq if rot else None, slots=torch.arange(M, dtype=torch.int32, device=DEV),
+                         kcache=caches[0], vcache=caches[1])
+    heads = x.double().view(M, -1, d)
+    for first, n, gain in ((0, nq, qg), (nq, nkv, kg)):
+        h = heads[:, first:first + n]
+        y = h * torch.rsqrt((h * h).mean(dim=-1, keepdim=True) + 1e-6) * gain.double()
+        if rot:
+            ang = positions.double()[:, None, None] * freq
+            u, v = y[..., :rot // 2].clone(), y[..., rot // 2:rot].clone()
+            y[..., :rot // 2], y[..., rot // 2:rot] = u * ang.cos() - v * ang.sin(), v * ang.cos() + u * ang.sin()
+        got = packed.double().view(M, -1, d)[:, first:first + n]
+        assert (got - y).abs().max().item() <= bound(dtype, y)
+    rows = o.unpack_cache_pages(caches[0])[:M].reshape(M, -1)
+    assert torch.equal(rows, packed[:, nq * d:(nq + nkv) * d])
+    assert torch.equal(o.unpack_cache_pages(caches[1])[:M].reshape(M, -1), x[:, (nq + nkv) * d:])
+
+
+def cache_pair(M, nkv, d, page, dtype):
+    return [torch.zeros(-(-M // page), nkv, page, d, dtype=dtype, device=DEV) for _ in range(2)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M", [2, 70])
+@pytest.mark.parametrize("nq,nkv,d,rot", [(3, 1, 2, 2), (32, 8, 128, 64), (5, 2, 100, 10), (2, 1, 256, 256)])
+def test_rotated_unit_heads_in_pairs_have_the_bits_of_single_elements(dtype, M, nq, nkv, d, rot):
+    o, page = ops(), 8
+    width = (nq + 2 * nkv) * d
+    x = rnd(M, width, dtype=dtype, seed=1)
+    inv = 1000.0 ** (-torch.arange(0, rot, 2, dtype=torch.float32, device=DEV) / rot)
+    slots = torch.arange(M, dtype=torch.int32, device=DEV)
+    results = []
+    for off in (0, 1):               # from the second column on a pair is no aligned access
+        wide = torch.zeros(M, width + 2, dtype=dtype, device=DEV)
+        packed = wide[:, off:off + width]
+        packed.copy_(x)
+        k, v = cache_pair(M, nkv, d, page, dtype)
+        o.rope_norm_store(packed, 0, nq * d, (nq + nkv) * d, nq, nkv, d, d, positions=slots * 37 + 5, inv_freq=inv, rot=rot,
+                          unit_norm=True, eps=1e-6, slots=slots, kcache=k, vcache=v)
+        results.append((packed.clone(), k, v))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    h = x.double().view(M, -1, d)[:, :nq + nkv]
+    ang = (slots * 37 + 5).float()[:, None, None] * inv
+    y, u, w = h.clone(), h[..., 0:rot:2], h[..., 1:rot:2]
+    y[..., 0:rot:2] = u * ang.double().cos() - w * ang.double().sin()
+    y[..., 1:rot:2] = w * ang.double().cos() + u * ang.double().sin()
+    y = y * torch.rsqrt((y * y).mean(dim=-1, keepdim=True) + 1e-6)
+    assert (results[0][0].double().view(M, -1, d)[:, :nq + nkv] - y).abs().max().item() <= bound(dtype, y)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M", [2, 70])
+@pytest.mark.parametrize("own", [False, True])
+@pytest.mark.parametrize("d", [4, 64, 128, 132, 256])
+def test_biased_and_normed_heads_in_pieces(dtype, M, own, d):
+    o, nq, nkv, page = ops(), 6, 2, 8
+    width = (nq + (2 if own else 1) * nkv) * d
+    x, slots = rnd(M, width, dtype=dtype, seed=1), torch.arange(M, dtype=torch.int32, device=DEV)
+    qb, kb, qg, kg = rnd(nq * d, seed=2), rnd(nkv * d, seed=3), rnd(d, seed=4), rnd(d, seed=5)
+    h = x.double().view(M, -1, d)[:, :nq + nkv] + torch.cat([qb, kb]).double().view(-1, d)
+    want = h * torch.rsqrt((h * h).mean(dim=-1, keepdim=True) + 1e-6)
+    want = want * torch.cat([qg.expand(nq, d), kg.expand(nkv, d)]).double()
+    for off in (0, 1):
+        wide = torch.zeros(M, width + 4, dtype=dtype, device=DEV)
+        packed = wide[:, off:off + width]
+        packed.copy_(x)
+        k, v = cache_pair(M, nkv, d, page, dtype)
+        o.qk_bias_norm_store(packed, 0, nq * d, (nq + nkv) * d if own else nq * d, nq, nkv, d, d, q_bias=qb, k_bias=kb, q_gain=qg,
+                             k_gain=kg, eps=1e-6, values_are_keys=not own, slots=slots, kcache=k, vcache=v)
+        got = packed.double().reshape(M, -1, d)[:, :nq + nkv]
+        assert (got - want).abs().max().item() <= bound(dtype, want)
+        assert torch.equal(o.unpack_cache_pages(k)[:M].reshape(M, -1), packed[:, nq * d:(nq + nkv) * d])
+        values = o.unpack_cache_pages(v)[:M]
+        if own:
+            assert torch.equal(values.reshape(M, -1), x[:, (nq + nkv) * d:])
+        else:
+            assert (values.double() - h[:, nq:]).abs().max().item() <= bound(dtype, h)
