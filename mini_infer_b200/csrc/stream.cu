@@ -140,13 +140,14 @@ __global__ void add_rmsnorm_multi_kernel(const float* __restrict__ stream_in, co
 }
 
 // The same for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays in registers, the gain, which no
-// kernel writes, is asked for before the wait, and every operand is one round trip.  8 rows of 2048 and 2 addends 4.2 us
+// kernel writes, is asked for before the wait (what kernels do write is not `__restrict__`: the compiler may move loads through
+// such pointers over the wait), and every operand is one round trip.  8 rows of 2048 and 2 addends 4.2 us
 // above, 2.1 here; 2048 rows of 4096 25 and 23 us (18 of bytes).
 template <typename T, int NV>
 __global__ void __launch_bounds__(512)
-add_rmsnorm_multi4_kernel(const float* __restrict__ stream_in, const T* __restrict__ add1, const T* __restrict__ add2,
-                          const float* __restrict__ add32, const float* __restrict__ row_add, float* __restrict__ stream_out,
-                          const int* __restrict__ rows, const float* __restrict__ gain, T* __restrict__ out, int H, float eps) {
+add_rmsnorm_multi4_kernel(const float* stream_in, const T* add1, const T* add2, const float* add32, const float* row_add,
+                          float* stream_out, const int* rows, const float* __restrict__ gain, T* __restrict__ out, int H,
+                          float eps) {
   mi_pdl_launch_dependents();
   __shared__ float red[32];
   float g[NV][4], r[NV][4], f[4], h[4];

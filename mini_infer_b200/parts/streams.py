@@ -18,8 +18,10 @@ import torch
 
 from ..csrc import ops
 
-# The stream beside each stream that steps are recorded on, per device (from the library's pool of a few dozen).
-_beside: dict[tuple[int, int], torch.cuda.Stream] = {}
+# The streams beside each stream that steps are recorded on, one per block that is open at a time, and how many are open; per
+# device (from the library's pool of a few dozen).
+_beside: dict[tuple[int, int], list[torch.cuda.Stream]] = {}
+_open: dict[tuple[int, int], int] = {}
 
 
 class beside:
@@ -36,12 +38,16 @@ class beside:
         self.on = torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing() and not ops.sums_kept()
         if self.on:
             self.here = torch.cuda.current_stream()
-            key = (self.here.device_index, self.here.cuda_stream)
-            self.stream = _beside.get(key)
-            if self.stream is None:
-                self.stream = _beside[key] = torch.cuda.Stream(self.here.device)
+            self.key = (self.here.device_index, self.here.cuda_stream)
 
     def __enter__(self) -> "beside":
+        if self.on:       # (only one thread records on a stream at a time)
+            depth = _open.get(self.key, 0)
+            streams = _beside.setdefault(self.key, [])
+            if depth == len(streams):
+                streams.append(torch.cuda.Stream(self.here.device))
+            self.stream = streams[depth]
+            _open[self.key] = depth + 1
         return self
 
     def run(self, f):
@@ -67,3 +73,5 @@ class beside:
 
     def __exit__(self, *error) -> None:
         self._join()                   # behind an error as well: a capture ends with one stream
+        if self.on:
+            _open[self.key] -= 1
