@@ -309,7 +309,7 @@ def _sig_recurrent(lib: ctypes.CDLL) -> None:
     lib.mi_delta_scan.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                   c_int, c_float, c_float, c_void_p, ll, ll, c_void_p, c_void_p, c_void_p, c_void_p,
                                   c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int,
-                                  c_void_p]
+                                  c_int, c_void_p]
     lib.mi_headnorm_gate.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                      c_int, c_float, c_int, c_float, c_int, c_void_p, c_float, c_int, c_void_p]
 
@@ -1716,7 +1716,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
                            int(state_offset), _ptr(ctx.q_start), _ptr(ctx.q_len), _ptr(ctx.state_slot), _ptr(o),
                            o.stride(0), ctx.n_requests, heads, kv_heads, dk, dv, _ptr(conv_in),
                            conv_in.stride(0) if conv_in is not None else 0, C, int(taps) if conv_in is not None else 1,
-                           _code(q.dtype), _stream())
+                           _max_q_len(ctx), _code(q.dtype), _stream())
     _finish(lib, rc, "delta")
     return o
 

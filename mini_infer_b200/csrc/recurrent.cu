@@ -728,7 +728,12 @@ extern "C" int mi_mlstm_gates(const float* zi, const float* zf, int z_stride, co
 // the column's lanes by three exchanges, in an order that depends on nothing but the sizes.  Tokens are staged
 // in groups of DELTA_L = DELTA_W, one per warp: the warp makes q and k unit vectors, computes g, beta and k . q,
 // and leaves them in shared memory (rows padded to 8 R with k = q = 0, g = 1) for the walk.
-// A block has DELTA_W warps, so it owns DELTA_W * DELTA_NC value columns of one head of one request.
+// A block owns DELTA_W * DELTA_NC value columns of one head of one request.
+// SPLIT (long portions, dk <= 128): four warps walk, two columns a lane, and DELTA_W more stage the next group into
+// a second buffer meanwhile.  Staging (three sums over a warp, exponentials, a square root) took a group as long as
+// the walk, and the walk is bound by its reads of shared memory, of which two columns a lane need half.  The
+// sums' order stays.  2000 tokens of 32 heads of 128: 946 us with the walkers staging, 703 with eight walkers of one
+// column a lane beside eight staging, 576 so; two columns a lane with the walkers staging: 1432.
 // state row of a request: [taps-1][C] convolution inputs (oldest first), then S [heads][dk][dv].
 // ------------------------------------------------------------------------------------------
 #define DELTA_L 8   // tokens per group: one per warp
@@ -737,8 +742,8 @@ extern "C" int mi_mlstm_gates(const float* zi, const float* zf, int z_stride, co
 #define DELTA_W 8
 #define DELTA_COLS (DELTA_NC * DELTA_W)
 
-template <typename T, int R>
-__global__ void __launch_bounds__(32 * DELTA_W)
+template <typename T, int R, bool SPLIT>
+__global__ void __launch_bounds__(32 * (SPLIT ? DELTA_W + DELTA_W / 2 : DELTA_W))
 delta_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int stride,
                   const float* __restrict__ z, int z_stride, const float* __restrict__ dt_bias,
                   const float* __restrict__ a_log, const T* __restrict__ b, int b_stride, float q_scale,
@@ -751,29 +756,38 @@ delta_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
   constexpr int RS = DKP / 32;           // rows a lane stages per token
   constexpr int NG = R / 4;              // groups of four rows per lane
   extern __shared__ __align__(16) float dsm[];
+  constexpr int BUF = 3 * DELTA_L * DKP + DELTA_L * DELTA_COLS + 2 * DELTA_L;   // floats of a staged group
   float* ks = dsm;                       // [DELTA_L][DKP]
   float* qs = ks + DELTA_L * DKP;        // [DELTA_L][DKP]
   float* gs = qs + DELTA_L * DKP;        // [DELTA_L][DKP]
   float* vs = gs + DELTA_L * DKP;        // [DELTA_L][DELTA_COLS]
   float* bs = vs + DELTA_L * DELTA_COLS; // [DELTA_L] beta
   float* kqs = bs + DELTA_L;             // [DELTA_L] k . q
-  const int lane = threadIdx.x, warp = threadIdx.y, tid = warp * 32 + lane;
+  const int lane = threadIdx.x, tid = threadIdx.y * 32 + lane;
+  constexpr int CPL = SPLIT ? 2 : 1;         // columns per lane: DELTA_NC apart
+  constexpr int WALKERS = DELTA_W / CPL;
+  const bool stager = SPLIT && threadIdx.y >= WALKERS;
+  const int warp = stager ? threadIdx.y - WALKERS : threadIdx.y;
   const int part = lane / DELTA_NC, col = lane % DELTA_NC;
   const int head = blockIdx.y, req = blockIdx.z;
   const int kvh = head / (heads / kv_heads);
   const int len = q_len[req], row0 = q_start[req];
   float* st = state + (size_t)state_slot[req] * state_stride;
   float* S = st + s_off + (size_t)head * dk * dv;
-  const int j = blockIdx.x * DELTA_COLS + warp * DELTA_NC + col;   // this lane's column
+  const int c0 = warp * DELTA_NC * CPL + col, j0 = blockIdx.x * DELTA_COLS + c0;   // this lane's first column
   const float A = expf(a_log[head]);
-  float s[R];
+  float s[CPL][R];
+  if (!stager) {
 #pragma unroll
-  for (int i = 0; i < NG; ++i)
+    for (int c = 0; c < CPL; ++c)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int kk = 4 * (part + DELTA_PARTS * i) + e;
-      s[4 * i + e] = (kk < dk && j < dv) ? S[(size_t)kk * dv + j] : 0.f;
-    }
+      for (int i = 0; i < NG; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int kk = 4 * (part + DELTA_PARTS * i) + e, j = j0 + DELTA_NC * c;
+          s[c][4 * i + e] = (kk < dk && j < dv) ? S[(size_t)kk * dv + j] : 0.f;
+        }
+  }
   // Warp w stages token w of a group.  What it needs from global memory (its token's k, q, pre-activations of
   // the decay, beta and the block's values) is fetched into registers one group ahead, before the walk
   // over the group at hand, so that the walk hides the fetch.
@@ -805,89 +819,157 @@ delta_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
     pb = b[m * b_stride + head];
     if (jj < dv) pv = v[m * stride + head * dv + jj];
   };
-  fetch(warp);
-  for (int t0 = 0; t0 < len; t0 += DELTA_L) {
-    const int n = min(DELTA_L, len - t0);
-    __syncthreads();   // the group before is consumed
-    if (warp < n) {
-      const int l = warp;
-      float kv_[RS], qv_[RS], ssk = 0.f, ssq = 0.f;
+  // token l = warp of a group, in the buffer that begins at float `at`
+  auto stage = [&](int at) {
+    const int l = warp;
+    float kv_[RS], qv_[RS], ssk = 0.f, ssq = 0.f;
 #pragma unroll
-      for (int i = 0; i < RS; ++i) {
-        kv_[i] = mi_to_float(pk[i]);
-        qv_[i] = mi_to_float(pq_[i]);
-        ssk = fmaf(kv_[i], kv_[i], ssk);
-        ssq = fmaf(qv_[i], qv_[i], ssq);
-      }
-      ssk = mi_warp_sum(ssk);
-      ssq = mi_warp_sum(ssq);
-      const float mk = 1.f / sqrtf(ssk + unit_eps), mq = q_scale / sqrtf(ssq + unit_eps);
-      float kq = 0.f;
-#pragma unroll
-      for (int i = 0; i < RS; ++i) {
-        const int kk = lane + 32 * i;
-        float kn = 0.f, qn = 0.f, g = 1.f;
-        if (kk < dk) {
-          kn = kv_[i] * mk;
-          qn = qv_[i] * mq;
-          g = expf(-A * mi_softplus(pz[i] + dtb[i]));
-        }
-        ks[l * DKP + kk] = kn;
-        qs[l * DKP + kk] = qn;
-        gs[l * DKP + kk] = g;
-        kq = fmaf(kn, qn, kq);
-      }
-      kq = mi_warp_sum(kq);
-      if (lane == 0) {
-        kqs[l] = kq;
-        bs[l] = mi_sigmoid(mi_to_float(pb));
-      }
-      vs[l * DELTA_COLS + lane] = jj < dv ? mi_to_float(pv) : 0.f;
+    for (int i = 0; i < RS; ++i) {
+      kv_[i] = mi_to_float(pk[i]);
+      qv_[i] = mi_to_float(pq_[i]);
+      ssk = fmaf(kv_[i], kv_[i], ssk);
+      ssq = fmaf(qv_[i], qv_[i], ssq);
     }
-    __syncthreads();
-    fetch(t0 + DELTA_L + warp);
+    ssk = mi_warp_sum(ssk);
+    ssq = mi_warp_sum(ssq);
+    const float mk = 1.f / sqrtf(ssk + unit_eps), mq = q_scale / sqrtf(ssq + unit_eps);
+    float kq = 0.f;
+#pragma unroll
+    for (int i = 0; i < RS; ++i) {
+      const int kk = lane + 32 * i;
+      float kn = 0.f, qn = 0.f, g = 1.f;
+      if (kk < dk) {
+        kn = kv_[i] * mk;
+        qn = qv_[i] * mq;
+        g = expf(-A * mi_softplus(pz[i] + dtb[i]));
+      }
+      ks[at + l * DKP + kk] = kn;
+      qs[at + l * DKP + kk] = qn;
+      gs[at + l * DKP + kk] = g;
+      kq = fmaf(kn, qn, kq);
+    }
+    kq = mi_warp_sum(kq);
+    if (lane == 0) {
+      kqs[at + l] = kq;
+      bs[at + l] = mi_sigmoid(mi_to_float(pb));
+    }
+    vs[at + l * DELTA_COLS + lane] = jj < dv ? mi_to_float(pv) : 0.f;
+  };
+  auto walk = [&](int t0, int n, int at) {
+    // SPLIT: a token's words are asked for ahead of the exchanges of the token before (the other form has no registers for them)
+    float4 g4[NG], k4[NG], q4[NG];
+    auto words = [&](const float* from, int l, float4 (&to)[NG]) {
+#pragma unroll
+      for (int i = 0; i < NG; ++i)
+        to[i] = *reinterpret_cast<const float4*>(from + at + l * DKP + 4 * (part + DELTA_PARTS * i));
+    };
+    if (SPLIT) {
+      words(gs, 0, g4);
+      words(ks, 0, k4);
+      words(qs, 0, q4);
+    }
     for (int l = 0; l < n; ++l) {
-      float kreg[R];
-      float r0 = 0.f, r1 = 0.f, p0 = 0.f, p1 = 0.f;
+      float4 kreg[NG];
+      float r[CPL], pq[CPL], val[CPL];
 #pragma unroll
-      for (int i = 0; i < NG; ++i) {
-        const int at = l * DKP + 4 * (part + DELTA_PARTS * i);
-        const float4 g4 = *reinterpret_cast<const float4*>(gs + at);
-        const float4 k4 = *reinterpret_cast<const float4*>(ks + at);
-        const float4 q4 = *reinterpret_cast<const float4*>(qs + at);
-        float* si = s + 4 * i;
-        float* ki = kreg + 4 * i;
-        ki[0] = k4.x; ki[1] = k4.y; ki[2] = k4.z; ki[3] = k4.w;
-        si[0] *= g4.x; si[1] *= g4.y; si[2] *= g4.z; si[3] *= g4.w;
-        r0 = fmaf(si[0], k4.x, r0); r1 = fmaf(si[1], k4.y, r1);
-        r0 = fmaf(si[2], k4.z, r0); r1 = fmaf(si[3], k4.w, r1);
-        p0 = fmaf(si[0], q4.x, p0); p1 = fmaf(si[1], q4.y, p1);
-        p0 = fmaf(si[2], q4.z, p0); p1 = fmaf(si[3], q4.w, p1);
+      for (int c = 0; c < CPL; ++c) {
+        float r0 = 0.f, r1 = 0.f, p0 = 0.f, p1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+          if (!SPLIT) {
+            const int word = at + l * DKP + 4 * (part + DELTA_PARTS * i);
+            g4[i] = *reinterpret_cast<const float4*>(gs + word);
+            k4[i] = *reinterpret_cast<const float4*>(ks + word);
+            q4[i] = *reinterpret_cast<const float4*>(qs + word);
+          }
+          float* si = s[c] + 4 * i;
+          kreg[i] = k4[i];
+          si[0] *= g4[i].x; si[1] *= g4[i].y; si[2] *= g4[i].z; si[3] *= g4[i].w;
+          r0 = fmaf(si[0], k4[i].x, r0); r1 = fmaf(si[1], k4[i].y, r1);
+          r0 = fmaf(si[2], k4[i].z, r0); r1 = fmaf(si[3], k4[i].w, r1);
+          p0 = fmaf(si[0], q4[i].x, p0); p1 = fmaf(si[1], q4[i].y, p1);
+          p0 = fmaf(si[2], q4[i].z, p0); p1 = fmaf(si[3], q4[i].w, p1);
+        }
+        r[c] = r0 + r1;
+        pq[c] = p0 + p1;
+        val[c] = vs[at + l * DELTA_COLS + c0 + DELTA_NC * c];
       }
-      float r = r0 + r1, pq = p0 + p1;
-#pragma unroll
-      for (int off = DELTA_NC; off < 32; off <<= 1) {
-        r += __shfl_xor_sync(0xffffffffu, r, off);
-        pq += __shfl_xor_sync(0xffffffffu, pq, off);
+      const float beta = bs[at + l], kq = kqs[at + l];
+      if (SPLIT && l + 1 < n) {
+        words(gs, l + 1, g4);
+        words(ks, l + 1, k4);
+        words(qs, l + 1, q4);
       }
-      const float u = bs[l] * (vs[l * DELTA_COLS + warp * DELTA_NC + col] - r);
 #pragma unroll
-      for (int i = 0; i < R; ++i) s[i] = fmaf(kreg[i], u, s[i]);
-      if (part == 0 && j < dv) o[(size_t)(row0 + t0 + l) * o_stride + head * dv + j] = fmaf(u, kqs[l], pq);
+      for (int off = DELTA_NC; off < 32; off <<= 1)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          r[c] += __shfl_xor_sync(0xffffffffu, r[c], off);
+          pq[c] += __shfl_xor_sync(0xffffffffu, pq[c], off);
+        }
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const float u = beta * (val[c] - r[c]);
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+          float* si = s[c] + 4 * i;
+          si[0] = fmaf(kreg[i].x, u, si[0]); si[1] = fmaf(kreg[i].y, u, si[1]);
+          si[2] = fmaf(kreg[i].z, u, si[2]); si[3] = fmaf(kreg[i].w, u, si[3]);
+        }
+        const int j = j0 + DELTA_NC * c;
+        if (part == 0 && j < dv) o[(size_t)(row0 + t0 + l) * o_stride + head * dv + j] = fmaf(u, kq, pq[c]);
+      }
+    }
+  };
+  if (SPLIT) {
+    // Barriers 1 and 2: buffer 0 or 1 is full; 3 and 4: it is free again.  All warps take part in each.
+    constexpr int ALL = 32 * (WALKERS + DELTA_W);
+    int buf = 0;
+    if (stager) {
+      fetch(warp);
+      for (int t0 = 0; t0 < len; t0 += DELTA_L, buf ^= 1) {
+        if (t0 >= 2 * DELTA_L) asm volatile("bar.sync %0, %1;\n" ::"r"(3 + buf), "n"(ALL) : "memory");
+        if (t0 + warp < len) stage(buf * BUF);
+        __syncwarp();
+        asm volatile("bar.arrive %0, %1;\n" ::"r"(1 + buf), "n"(ALL) : "memory");
+        fetch(t0 + DELTA_L + warp);
+      }
+    } else {
+      for (int t0 = 0; t0 < len; t0 += DELTA_L, buf ^= 1) {
+        asm volatile("bar.sync %0, %1;\n" ::"r"(1 + buf), "n"(ALL) : "memory");
+        walk(t0, min(DELTA_L, len - t0), buf * BUF);
+        __syncwarp();
+        if (t0 + 2 * DELTA_L < len) asm volatile("bar.arrive %0, %1;\n" ::"r"(3 + buf), "n"(ALL) : "memory");
+      }
+    }
+  } else {
+    fetch(warp);
+    for (int t0 = 0; t0 < len; t0 += DELTA_L) {
+      const int n = min(DELTA_L, len - t0);
+      __syncthreads();   // the group before is consumed
+      if (warp < n) stage(0);
+      __syncthreads();
+      fetch(t0 + DELTA_L + warp);
+      walk(t0, n, 0);
     }
   }
+  if (!stager) {
 #pragma unroll
-  for (int i = 0; i < NG; ++i)
+    for (int c = 0; c < CPL; ++c)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int kk = 4 * (part + DELTA_PARTS * i) + e;
-      if (kk < dk && j < dv) S[(size_t)kk * dv + j] = s[4 * i + e];
-    }
+      for (int i = 0; i < NG; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int kk = 4 * (part + DELTA_PARTS * i) + e, j = j0 + DELTA_NC * c;
+          if (kk < dk && j < dv) S[(size_t)kk * dv + j] = s[c][4 * i + e];
+        }
+  }
   // the convolution's next tail (the request's blocks share its channels): the last taps-1 of (old tail,
   // this portion's inputs); the convolution itself ran before this kernel and nothing else reads the tail here
   if (taps > 1) {
     const int n_blocks = gridDim.x * gridDim.y, block_id = blockIdx.y * gridDim.x + blockIdx.x;
-    for (int c = block_id * 32 * DELTA_W + tid; c < C; c += n_blocks * 32 * DELTA_W) {
+    const int threads = 32 * blockDim.y;
+    for (int c = block_id * threads + tid; c < C; c += n_blocks * threads) {
       float keep[MAX_TAPS];
 #pragma unroll
       for (int j = 0; j < MAX_TAPS - 1; ++j) {
@@ -909,18 +991,26 @@ extern "C" int mi_delta_scan(const void* q, const void* k, const void* v, int st
                              float unit_eps, float* state, long long state_stride, long long s_off,
                              const int* q_start, const int* q_len, const int* state_slot, float* o, int o_stride,
                              int n_requests, int heads, int kv_heads, int dk, int dv, const void* xin, int xin_stride,
-                             int C, int taps, int dtype, cudaStream_t stream) {
+                             int C, int taps, int longest, int dtype, cudaStream_t stream) {
+  // longest: the longest portion of the step (chooses the kernel's form; any value is correct)
   if (n_requests <= 0) return 0;
   if (dk <= 0 || dk > 256 || dv <= 0) MI_REFUSE("delta: key size %d must lie in [1, 256], value size %d above 0", dk, dv);
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads) MI_REFUSE("delta: %d heads cannot share %d key heads", heads, kv_heads);
   if (heads > 65535 || n_requests > 65535) MI_REFUSE("delta: too many heads or requests for one launch");
   if (taps < 1 || taps > MAX_TAPS) MI_REFUSE("delta: %d taps (1 to %d are taken)", taps, MAX_TAPS);
-  dim3 grid((dv + DELTA_COLS - 1) / DELTA_COLS, heads, n_requests), block(32, DELTA_W);
+  dim3 grid((dv + DELTA_COLS - 1) / DELTA_COLS, heads, n_requests);
+  // Warps of their own for staging for portions of more than DELTA_SPLIT_ABOVE tokens: short ones are bound by the
+  // state's way in and out, and smaller blocks leave room for more of it.  64 requests of 16 tokens, 16 heads of 128:
+  // 179 us without, 201 with; 16 of 32, 32 heads: 158 and 160; 8 of 100, 16 heads: 129 and 119.  A head of more than
+  // 128 rows leaves a lane no registers for a second column.
+  constexpr int DELTA_SPLIT_ABOVE = 32;
+  const bool split = longest > DELTA_SPLIT_ABOVE && dk <= 128;
+  const dim3 block(32, split ? DELTA_W + DELTA_W / 2 : DELTA_W);
   const int dkp = dk <= 32 ? 32 : dk <= 64 ? 64 : dk <= 128 ? 128 : 256;   // DELTA_PARTS * R of the instance below
-  const size_t smem = ((size_t)3 * DELTA_L * dkp + DELTA_L * DELTA_COLS + 2 * DELTA_L) * sizeof(float);
-#define MI_GO(T, R)                                                                                                  \
+  const size_t smem = ((size_t)3 * DELTA_L * dkp + DELTA_L * DELTA_COLS + 2 * DELTA_L) * sizeof(float) * (split ? 2 : 1);
+#define MI_GO(T, R, SPLIT)                                                                                           \
   do {                                                                                                               \
-    auto kern = delta_scan_kernel<T, R>;                                                                             \
+    auto kern = delta_scan_kernel<T, R, SPLIT>;                                                                      \
     if (smem > 48 * 1024) {                                                                                          \
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
       if (e != cudaSuccess) return (int)e;                                                                           \
@@ -931,10 +1021,14 @@ extern "C" int mi_delta_scan(const void* q, const void* k, const void* v, int st
   } while (0)
 #define MI_GO_R(T)                  \
   do {                              \
-    if (dk <= 32) MI_GO(T, 4);       \
-    else if (dk <= 64) MI_GO(T, 8);  \
-    else if (dk <= 128) MI_GO(T, 16);\
-    else MI_GO(T, 32);               \
+    if (split) {                     \
+      if (dk <= 32) MI_GO(T, 4, true); \
+      else if (dk <= 64) MI_GO(T, 8, true); \
+      else MI_GO(T, 16, true);       \
+    } else if (dk <= 32) MI_GO(T, 4, false); \
+    else if (dk <= 64) MI_GO(T, 8, false);   \
+    else if (dk <= 128) MI_GO(T, 16, false); \
+    else MI_GO(T, 32, false);        \
   } while (0)
   if (dtype == MI_DTYPE_F32) MI_GO_R(float);
   else if (dtype == MI_DTYPE_BF16) MI_GO_R(bf16);

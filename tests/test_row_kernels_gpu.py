@@ -168,3 +168,38 @@ def test_biased_and_normed_heads_in_pieces(dtype, M, own, d):
             assert torch.equal(values.reshape(M, -1), x[:, (nq + nkv) * d:])
         else:
             assert (values.double() - h[:, nq:]).abs().max().item() <= bound(dtype, h)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kvh,dk,dv", [(2, 1, 20, 33), (3, 3, 32, 8), (4, 2, 64, 64), (2, 2, 100, 37), (1, 1, 128, 40),
+                                             (2, 1, 128, 128)])
+@pytest.mark.parametrize("lens", [(33, 41), (32, 15), (34, 1), (130, 8), (16, 56)])
+def test_delta_rule_with_warps_that_stage(dtype, heads, kvh, dk, dv, lens):
+    """A long portion, staged by warps of its own, against the same tokens in portions too short for that: one order of
+    sums, so the outputs, the states and the convolution's tails are equal bit by bit."""
+    from types import SimpleNamespace
+    gk, taps = kvh * dk, 3
+    C = 2 * gk + heads * dv
+    s_off = (taps - 1) * C
+    n = sum(lens)
+    u, x, z = rnd(n, C, dtype=dtype, seed=1), rnd(n, C, dtype=dtype, seed=2), rnd(n, heads * dk, seed=3)
+    b, dt, a_log = rnd(n, heads, dtype=dtype, seed=4), rnd(heads * dk, seed=5), rnd(heads, seed=6) - 0.5
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def scan(starts, portions, slots, state):
+        ctx = SimpleNamespace(q_start=i32(*starts), q_len=i32(*portions), state_slot=i32(*slots), n_requests=len(portions),
+                              decode_only=max(portions) == 1, host_q_len=list(portions))
+        return ops().delta_scan(u[:, :gk], u[:, gk:2 * gk], u[:, 2 * gk:], z, dt, a_log, b, dk ** -0.5, 1e-6, heads, kvh,
+                                dk, dv, state, s_off, ctx, conv_in=x, taps=taps)
+
+    begin = rnd(3, s_off + heads * dk * dv, seed=7)
+    whole, cut = begin.clone(), begin.clone()
+    got = scan((0, lens[0]), lens, (2, 0), whole)
+    want = torch.empty_like(got)
+    for start, length, slot in ((0, lens[0], 2), (lens[0], lens[1], 0)):
+        for t in range(0, length, 7):
+            m = min(7, length - t)
+            want[start + t:start + t + m] = scan((start + t,), (m,), (slot,), cut)[start + t:start + t + m]
+    assert torch.isfinite(got).all()
+    assert torch.equal(got, want) and torch.equal(whole, cut)
+    assert torch.equal(whole[1], begin[1])
