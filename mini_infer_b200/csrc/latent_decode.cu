@@ -131,6 +131,7 @@ latent_value_kernel(const float* __restrict__ part_o, const float* __restrict__ 
   extern __shared__ __align__(16) float lat[];       // [rank]
   __shared__ float weight[V_MAX_SPLITS];
   __shared__ float inv_l;
+  __shared__ int last;
   constexpr float LOG2E = 1.4426950408889634f;
   const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, lane8 = tid & 7;
   const int pieces = rank >> 3;
@@ -169,23 +170,31 @@ latent_value_kernel(const float* __restrict__ part_o, const float* __restrict__ 
       const float sink2 = sinks ? sinks[h] * LOG2E : -INFINITY;
       const float mf = fmaxf(mi_warp_max(fmaxf(ml[0].x, ml[1].x)), sink2);
       float l = 0.f;
+      int runs = 0;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
+        const unsigned joined = __ballot_sync(0xffffffffu, ml[k].x != -INFINITY);
+        if (joined) runs = 32 * k + 32 - __clz(joined);
         const float ws = ml[k].x == -INFINITY ? 0.f : exp2f(ml[k].x - mf);
         weight[tid + 32 * k] = ws;
         l += mi_warp_sum(ml[k].y * ws);
       }
       if (sinks) l += exp2f(sink2 - mf);
-      if (tid == 0) inv_l = l > 0.f ? 1.f / l : 0.f;
+      if (tid == 0) {
+        inv_l = l > 0.f ? 1.f / l : 0.f;
+        last = runs;
+      }
     }
     __syncthreads();
     const float inv = inv_l;
+    const int runs = last;           // the runs behind the last one that a key joined have left no sums
     for (int c = tid; c < rank; c += V_THREADS) {
       float sum = 0.f;
-      for (int s0 = 0; s0 < n_splits; s0 += V_RUNS) {     // added in order
+      for (int s0 = 0; s0 < runs; s0 += V_RUNS) {         // added in order
         if (s0 || c != tid) ask(s0, c);
 #pragma unroll
-        for (int u = 0; u < V_RUNS; ++u) sum = fmaf(v[u], s0 + u < V_MAX_SPLITS ? weight[s0 + u] : 0.f, sum);
+        for (int u = 0; u < V_RUNS; ++u)
+          if (s0 + u < runs) sum = fmaf(v[u], weight[s0 + u], sum);
       }
       lat[c] = sum * inv;
     }

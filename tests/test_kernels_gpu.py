@@ -924,3 +924,42 @@ def test_sample_draws_follow_softmax_and_ignore_the_batch():
     alone = sample_rows(logits[:1], [0.9], None, None, [42], [1234])
     mixed = sample_rows(logits[:3], [0.9, 0.0, 0.9], None, None, [7, 8, 42], [0, 0, 1234])
     assert alone[0] == mixed[2]
+
+
+@pytest.mark.parametrize("lens", [[1, 64, 65, 700], [130], [1, 0, 2049]])
+@pytest.mark.parametrize("n,rd,rank,sink", [(16, 16, 64, False), (20, 16, 512, True)])
+def test_runs_without_keys_leave_no_sums(lens, n, rd, rank, sink, monkeypatch):
+    """Steps planned for more keys than a request holds: the runs behind its last key leave their sums as the scratch
+    was (here NaN), and both kernels that add runs up stop before them.  A request without keys gives zeros."""
+    from types import SimpleNamespace
+    o = ops()
+    real = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: real(*a, **k).fill_(float("nan"))
+                        if k.get("dtype") in (torch.float32, torch.bfloat16) else real(*a, **k))
+    i32 = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    page, d, M, scale = 16, rank + rd, len(lens), 0.6
+    per = -(-max(lens) // page)
+    rows = rnd(M, per * page, 1, d, dtype=torch.bfloat16, seed=1).cuda()
+    kc = o.pack_cache_pages(rows.reshape(M * per * page, 1, d), page)
+    table = torch.arange(M * per, dtype=torch.int32, device="cuda").reshape(M, per)
+    ctx = SimpleNamespace(groups=[SimpleNamespace(block_table=table, page_size=page, table_rows=i32(range(M)))],
+                          decode_only=True, n_tokens=M, q_start=i32(range(M)), q_len=i32([1] * M), kv_len=i32(lens),
+                          max_kv_len=64 * 64, tiles={1: (None, None, M)}, q_tiles=lambda tt: (None, None, M))
+    q = rnd(M, n * d, dtype=torch.bfloat16, seed=2, scale=d ** -0.5).cuda()
+    sinks = torch.linspace(-2.0, 3.0, n, device="cuda") if sink else None
+    cache = SimpleNamespace(group=0, k=kc, v=None)
+    runs = o.attention_latent_runs(q, cache, ctx, n, d, rank, scale, sinks=sinks)
+    assert runs[2] == 64 and torch.isnan(runs[0]).any()
+    eye = torch.eye(rank, dtype=torch.bfloat16, device="cuda").expand(n, rank, rank).contiguous()
+    fused, merged = (torch.zeros(M, n * rank, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    o.latent_value(runs, sinks, eye, fused, n)
+    o.attention_ext(q, merged, cache, ctx, n, 1, d, rank, scale, sinks=sinks, values_in_keys=True)
+    for i, x in enumerate(lens):
+        c = rows[i, :x, 0].double()
+        s = torch.einsum("nd,jd->nj", q[i].double().view(n, d), c) * scale
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None]], dim=1)
+        want = (torch.softmax(s, dim=1)[:, :x] @ c[:, :rank]).reshape(-1)
+        # weights and results rounded to bfloat16: 2^-8 of the largest value each, twice over for the sums
+        for got in (fused[i], merged[i]):
+            assert (got.double() - want).abs().max() <= 2.0 ** -6 * max(1.0, want.abs().max().item() if x else 1.0), (i, x)
