@@ -769,10 +769,10 @@ extern "C" int mi_moe_gate_up(const void* x, int x_stride, const void* w_gate, c
     dim3 g(stream_it ? stream_blocks(ff, per_warp) : (ff + 15) / 16, max_tiles(n_entries, E, FEW_ROWS));
     if (g.y > 65535) MI_REFUSE("moe: too many row tiles for one launch");
     if (stream_it)
-      MI_LAUNCH((moe_stream_kernel<true>), g, 32 * MS_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
+      MI_LAUNCH_BEHIND((moe_stream_kernel<true>), g, 32 * MS_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
                 (const bf16*)w_up, w_expert_stride, perm, top, plan, E, act, ff, H, per_warp, limit, alpha, offset);
     else
-      MI_LAUNCH((moe_rows_kernel<true>), g, 32 * MR_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
+      MI_LAUNCH_BEHIND((moe_rows_kernel<true>), g, 32 * MR_WARPS, 0, stream, (const bf16*)x, x_stride, (const bf16*)w_gate,
                 (const bf16*)w_up, w_expert_stride, perm, top, plan, E, act, ff, H, limit, alpha, offset);
     MI_RETURN_LAUNCH_STATUS();
   }
@@ -802,10 +802,10 @@ extern "C" int mi_moe_down(const void* act, const void* w_down, long long w_expe
     dim3 g(stream_it ? stream_blocks((H + 1) / 2, per_warp) : (H + 31) / 32, max_tiles(n_entries, E, FEW_ROWS));
     if (g.y > 65535) MI_REFUSE("moe: too many row tiles for one launch");
     if (stream_it)
-      MI_LAUNCH((moe_stream_kernel<false>), g, 32 * MS_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
+      MI_LAUNCH_BEHIND((moe_stream_kernel<false>), g, 32 * MS_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
                 (const bf16*)nullptr, w_expert_stride, (const int*)nullptr, 1, plan, E, (void*)y, H, ff, per_warp, 0.f, 0.f, 0.f);
     else
-      MI_LAUNCH((moe_rows_kernel<false>), g, 32 * MR_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
+      MI_LAUNCH_BEHIND((moe_rows_kernel<false>), g, 32 * MR_WARPS, 0, stream, (const bf16*)act, ff, (const bf16*)w_down,
                 (const bf16*)nullptr, w_expert_stride, (const int*)nullptr, 1, plan, E, (void*)y, H, ff, 0.f, 0.f, 0.f);
     MI_RETURN_LAUNCH_STATUS();
   }

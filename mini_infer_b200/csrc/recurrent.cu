@@ -177,7 +177,7 @@ static bool conv_in_pieces(const T* x, int x_stride, const float* x_bias, const 
   dim3 grid((C / N + 127) / 128, (max_q_len + tile - 1) / tile, n_requests);
   if (grid.y > 65535 || grid.z > 65535) return false;
 #define MI_GO(TAPS)                                                                                                    \
-  MI_LAUNCH((causal_conv_pieces_kernel<T, TAPS>), grid, 128, 0, stream, x, x_stride, x_bias, w, b, state, state_stride, \
+  MI_LAUNCH_BEHIND((causal_conv_pieces_kernel<T, TAPS>), grid, 128, 0, stream, x, x_stride, x_bias, w, b, state, state_stride, \
             q_start, q_len, state_slot, out, out_stride, C, tile, act)
   if (taps == 2) MI_GO(2);
   else if (taps == 3) MI_GO(3);
@@ -204,10 +204,10 @@ extern "C" int mi_causal_conv(const void* x, int x_stride, const float* x_bias, 
   dim3 grid((C + 127) / 128, (max_q_len + tile - 1) / tile, n_requests);
   if (grid.y > 65535 || grid.z > 65535) MI_REFUSE("causal_conv: too many tiles for one launch");
   if (dtype == MI_DTYPE_F32)
-    MI_LAUNCH((causal_conv_kernel<float>), grid, 128, 0, stream, (const float*)x, x_stride, x_bias, w, b, state,
+    MI_LAUNCH_BEHIND((causal_conv_kernel<float>), grid, 128, 0, stream, (const float*)x, x_stride, x_bias, w, b, state,
               state_stride, q_start, q_len, state_slot, (float*)out, out_stride, C, taps, tile, act);
   else if (dtype == MI_DTYPE_BF16)
-    MI_LAUNCH((causal_conv_kernel<bf16>), grid, 128, 0, stream, (const bf16*)x, x_stride, x_bias, w, b, state,
+    MI_LAUNCH_BEHIND((causal_conv_kernel<bf16>), grid, 128, 0, stream, (const bf16*)x, x_stride, x_bias, w, b, state,
               state_stride, q_start, q_len, state_slot, (bf16*)out, out_stride, C, taps, tile, act);
   else
     MI_REFUSE("causal_conv: unknown dtype %d", dtype);
