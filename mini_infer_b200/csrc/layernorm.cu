@@ -103,24 +103,23 @@ __global__ void add_layernorm_kernel(const float* __restrict__ stream, const T* 
   }
 }
 
-// The same for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays in registers, and the gains and
+// The same bits for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays on chip, and the gains and
 // biases, which no kernel writes, are asked for before the wait (what kernels do write is not `__restrict__`: the compiler may
-// move loads through such pointers over the wait).  Every piece is read and written once, in one round trip: 8
-// rows of 4096 with two norms 8.3 us in the kernel above, 3.5 here; 2048 rows of 2048 24
-// and 15 us (10 of bytes).
+// move loads through such pointers over the wait).  Every piece is read and written once, in one round trip.  The sums run in
+// the order of the kernel above, a thread's elements blockDim apart: the row goes through shared memory for them.  8 rows of 4096 with two
+// norms 6.0 us in the kernel above, 3.0 here (2.9 with the four of a piece added up first, which gives other bits); 2048 rows of
+// 2048 17.6, 13.2 and 12.1 (10 of bytes).
 template <typename T, int NV>
-__global__ void __launch_bounds__(512)
-add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* stream_out, const int* rows,
-                      const float* __restrict__ w1,
-                      const float* __restrict__ b1, T* __restrict__ out1, const float* __restrict__ w2,
-                      const float* __restrict__ b2, T* __restrict__ out2, int H, float eps) {
+__global__ void __launch_bounds__(512, NV == 4 ? 1 : NV == 2 ? 2 : 3)
+add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* stream_out, const int* rows, const float* w1,
+                      const float* b1, T* __restrict__ out1, const float* w2, const float* b2, T* __restrict__ out2, int H, float eps) {
   mi_pdl_launch_dependents();
   __shared__ float red[32];
-  float g1[NV][4], c1[NV][4], g2[NV][4], c2[NV][4], r[NV][4], f[4];
+  __shared__ __align__(16) float row[NV * 4 * 512];
+  float g1[NV][4], c1[NV][4], g2[NV][4], c2[NV][4], r[4], f[4];
   Vec4<float> v;
   Vec4<T> a;
-#pragma unroll
-  for (int n = 0; n < NV; ++n) {
+  auto gains = [&](int n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k < H) {
       v.load(w1 + k); v.get(g1[n]);
@@ -130,57 +129,61 @@ add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* 
         v.load(b2 + k); v.get(c2[n]);
       }
     }
-  }
+  };
+#pragma unroll
+  for (int n = 0; n < NV; ++n) gains(n);
   mi_pdl_wait();
   const size_t i = blockIdx.x, src = rows ? rows[i] : i;
-  float sum = 0.f;
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) r[n][e] = 0.f;
     if (k < H) {
       v.load(stream + src * H + k);
-      v.get(r[n]);
+      v.get(r);
       if (add1) {
         a.load(add1 + src * H + k);
         a.get(f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+        for (int e = 0; e < 4; ++e) r[e] += f[e];
       }
       if (add2) {
         a.load(add2 + src * H + k);
         a.get(f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+        for (int e = 0; e < 4; ++e) r[e] += f[e];
       }
-      sum += (r[n][0] + r[n][1]) + (r[n][2] + r[n][3]);
+      v.set(r);
+      v.store(row + k);
     }
+  }
+  __syncthreads();
+  float own[NV * 4], sum = 0.f;
+#pragma unroll
+  for (int j = 0; j < NV * 4; ++j) {
+    const int k = threadIdx.x + j * blockDim.x;
+    own[j] = k < H ? row[k] : 0.f;
+    sum += own[j];
   }
   const float mean = mi_block_sum(sum, red) / (float)H;
   float sq = 0.f;
 #pragma unroll
-  for (int n = 0; n < NV; ++n)
-    if (4 * (threadIdx.x + n * blockDim.x) < H) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float dlt = r[n][e] - mean;
-        sq += dlt * dlt;
-      }
+  for (int j = 0; j < NV * 4; ++j)
+    if (threadIdx.x + j * blockDim.x < H) {
+      const float dlt = own[j] - mean;
+      sq += dlt * dlt;
     }
   const float rstd = 1.f / sqrtf(mi_block_sum(sq, red) / (float)H + eps);
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k >= H) continue;
-    if (stream_out) {
-      v.set(r[n]);
-      v.store(stream_out + i * H + k);
-    }
+    v.load(row + k);
+    v.get(r);
+    if (stream_out) v.store(stream_out + i * H + k);
     float y[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      f[e] = (r[n][e] - mean) * rstd;
+      f[e] = (r[e] - mean) * rstd;
       y[e] = f[e] * g1[n][e] + c1[n][e];
     }
     a.set(y);
@@ -210,8 +213,8 @@ extern "C" int mi_add_layernorm(const float* stream, const void* add1, const voi
     pieces = pieces && mi_aligned(ptr, 16);
   if (pieces) {
 #define MI_GO4(T, NV)                                                                                               \
-  MI_LAUNCH((add_layernorm4_kernel<T, NV>), M, threads, 0, stream_, stream, (const T*)add1, (const T*)add2, stream_out, \
-            rows, w1, b1, (T*)out1, w2, b2, (T*)out2, H, eps)
+  MI_LAUNCH((add_layernorm4_kernel<T, NV>), M, threads, 0, stream_, \
+            stream, (const T*)add1, (const T*)add2, stream_out, rows, w1, b1, (T*)out1, w2, b2, (T*)out2, H, eps)
 #define MI_GO4_T(T)                          \
   if (H <= 4 * threads) MI_GO4(T, 1);        \
   else if (H <= 8 * threads) MI_GO4(T, 2);   \

@@ -135,7 +135,7 @@ def kept_sums():
     """Inside, and in this thread only, bfloat16 work of decode steps adds up in one order that does not change from one
     version of the kernels to the next: products of up to 16 rows run ``gemm_tma``, experts with few rows the streaming
     kernel on CUDA cores, decode attention cuts its keys into stretches of four chunks or more.  Everywhere else the
-    faster kernels run, which are as close to the exact sums or closer.
+    faster kernels run, which are as close to the exact sums or closer.  (Norms have one order for all, inside and outside.)
 
     It is for models that turn a difference in the last bit into another answer: a router that first picks groups of experts
     and is undecided between two groups changes several experts with large weights at once (up to 0.4 of such a token's logits
@@ -347,7 +347,7 @@ def _sig_stream(lib: ctypes.CDLL) -> None:
                                            c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, ll, ll, c_int,
                                            c_void_p]
     lib.mi_add_rmsnorm_multi.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                         c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_int, c_void_p]
+                                         c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
     lib.mi_glu_mul_pairs.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_embedding_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
                                          c_void_p]
@@ -2021,8 +2021,7 @@ def add_rmsnorm_multi(stream: torch.Tensor | None, adds, gain: torch.Tensor, eps
     lib = _lib("stream")
     rc = lib.mi_add_rmsnorm_multi(_ptr(stream), _ptr(adds[0] if adds else None), _ptr(adds[1] if len(adds) > 1 else None),
                                   _ptr(add32), _ptr(row_add), _ptr(new_stream), _ptr(rows), _ptr(gain), _ptr(out),
-                                  M, H, float(eps), 1 if _sums_kept() else 0,
-                                  _code(dtype), _stream())
+                                  M, H, float(eps), _code(dtype), _stream())
     _finish(lib, rc, "rmsnorm")
     return out, new_stream
 

@@ -111,8 +111,10 @@ qk_bias_norm_store_kernel(T* __restrict__ packed, int stride, int q_off, int k_o
   }
 }
 
-// The same for heads of whole aligned pieces of four, up to 256 wide: a lane has NV pieces of a head, so that a head is one
-// access per operand.  2048 tokens of 32 queries and 8 keys of 128: 30 us in the kernel above, 21 here.
+// The same bits for heads of whole aligned pieces of four, up to 256 wide: a lane has NV pieces of a head, so that a head is one
+// access per operand.  The sum of squares runs in the order of the kernel above, a lane's elements 32 apart: the head goes
+// through shared memory for it.  2048 tokens of 32 queries and 8 keys of 128: 41 us in the kernel above, 19 here (17 with the
+// four of a piece added up first, which gives other bits).
 template <typename T, int NV>
 __global__ void __launch_bounds__(128)
 qk_bias_norm_store4_kernel(T* __restrict__ packed, int stride, int q_off, int k_off, int v_off, int nq, int nkv, int d,
@@ -121,6 +123,7 @@ qk_bias_norm_store4_kernel(T* __restrict__ packed, int stride, int q_off, int k_
                            int values_are_keys, const int* __restrict__ slots, T* __restrict__ kcache,
                            T* __restrict__ vcache, int page_size, int writes) {
   mi_pdl_enter();
+  __shared__ __align__(16) float heads[4][128 * NV];       // a warp's head
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   T* row = packed + (size_t)t * stride;
@@ -148,7 +151,6 @@ qk_bias_norm_store4_kernel(T* __restrict__ packed, int stride, int q_off, int k_
     const float* bias = is_q ? q_bias : k_bias;
     const float* gain = is_q ? q_gain : k_gain;
     float val[NV][4], g[NV][4], f[4];
-    float ss = 0.f;
     Vec4<float> v;
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
@@ -160,14 +162,18 @@ qk_bias_norm_store4_kernel(T* __restrict__ packed, int stride, int q_off, int k_
           v.get(g[n]);
         }
         a.get(val[n]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f[e] = 0.f;
         if (bias) {
           v.load(bias + hh * d + k);
           v.get(f);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) val[n][e] += f[e];
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ss += val[n][e] * val[n][e];
+        for (int e = 0; e < 4; ++e) val[n][e] += f[e];
+        if (gain) {
+          v.set(val[n]);
+          v.store(heads[warp] + k);
+        }
       }
     }
     const size_t at = ((size_t)(page * nkv + hh) * page_size + offset) * d;
@@ -184,6 +190,14 @@ qk_bias_norm_store4_kernel(T* __restrict__ packed, int stride, int q_off, int k_
     }
     float mult = 1.f;
     if (gain) {
+      __syncwarp();
+      float ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4 * NV; ++j) {
+        const float x1 = lane + 32 * j < d ? heads[warp][lane + 32 * j] : 0.f;
+        ss += x1 * x1;
+      }
+      __syncwarp();               // (the next head may take this one's place)
       ss = mi_warp_sum(ss);
       mult = 1.f / sqrtf(ss / (float)d + eps);
     }

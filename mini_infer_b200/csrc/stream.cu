@@ -139,102 +139,110 @@ __global__ void add_rmsnorm_multi_kernel(const float* __restrict__ stream_in, co
   }
 }
 
-// The same for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays in registers, the gain, which no
+// The same bits for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays on chip, the gain, which no
 // kernel writes, is asked for before the wait (what kernels do write is not `__restrict__`: the compiler may move loads through
-// such pointers over the wait), and every operand is one round trip.  8 rows of 2048 and 2 addends 4.2 us
-// above, 2.1 here; 2048 rows of 4096 25 and 23 us (18 of bytes).
+// such pointers over the wait), and every operand is one round trip.  The sum of squares runs in the order of the kernel above,
+// a thread's elements blockDim apart: the row goes through shared memory for it.  8 rows of 2048 and 2 addends 3.1 us above, 1.8
+// here; 2048 rows of 4096 36 and 23 (18 of bytes).
 template <typename T, int NV>
 __global__ void __launch_bounds__(512)
 add_rmsnorm_multi4_kernel(const float* stream_in, const T* add1, const T* add2, const float* add32, const float* row_add,
-                          float* stream_out, const int* rows, const float* __restrict__ gain, T* __restrict__ out, int H,
+                          float* stream_out, const int* rows, const float* gain, T* __restrict__ out, int H,
                           float eps) {
   mi_pdl_launch_dependents();
   __shared__ float red[32];
-  float g[NV][4], r[NV][4], f[4], h[4];
+  __shared__ __align__(16) float row[NV * 4 * 512];
+  float g[NV][4], r[4], f[4];
   Vec4<float> v;
   Vec4<T> a;
-#pragma unroll
-  for (int n = 0; n < NV; ++n) {
+  auto gains = [&](int n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k < H) {
       v.load(gain + k);
       v.get(g[n]);
     }
-  }
+  };
+#pragma unroll
+  for (int n = 0; n < NV; ++n) gains(n);
   mi_pdl_wait();
   const size_t i = blockIdx.x, src = rows ? rows[i] : i;
-  float sq = 0.f;
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k >= H) continue;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[n][e] = f[e] = 0.f;
+    for (int e = 0; e < 4; ++e) r[e] = 0.f;
     if (add1) {
       a.load(add1 + src * H + k);
-      a.get(f);
+      a.get(r);
     }
     if (add2) {
       a.load(add2 + src * H + k);
-      a.get(h);
+      a.get(f);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) f[e] += h[e];
+      for (int e = 0; e < 4; ++e) r[e] += f[e];
     }
     if (stream_in) {
       v.load(stream_in + src * H + k);
-      v.get(r[n]);
-    }
+      v.get(f);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+      for (int e = 0; e < 4; ++e) r[e] = f[e] + r[e];
+    }
     if (add32) {
       v.load(add32 + src * H + k);
       v.get(f);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+      for (int e = 0; e < 4; ++e) r[e] += f[e];
     }
     if (row_add) {
       v.load(row_add + k);
       v.get(f);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) r[n][e] += f[e];
+      for (int e = 0; e < 4; ++e) r[e] += f[e];
     }
+    v.set(r);
+    v.store(row + k);
+  }
+  __syncthreads();
+  float own[NV * 4], sq = 0.f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) sq += r[n][e] * r[n][e];
+  for (int j = 0; j < NV * 4; ++j) {
+    const int k = threadIdx.x + j * blockDim.x;
+    own[j] = k < H ? row[k] : 0.f;
+    sq += own[j] * own[j];
   }
   const float rstd = 1.f / sqrtf(mi_block_sum(sq, red) / (float)H + eps);
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k >= H) continue;
-    if (stream_out) {
-      v.set(r[n]);
-      v.store(stream_out + i * H + k);
-    }
+    v.load(row + k);
+    v.get(r);
+    if (stream_out) v.store(stream_out + i * H + k);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = r[n][e] * rstd * g[n][e];
+    for (int e = 0; e < 4; ++e) f[e] = r[e] * rstd * g[n][e];
     a.set(f);
     a.store(out + i * H + k);
   }
 }
 
-// kept: the sum of squares in the order that the first kernel has (models whose sums are kept).
 extern "C" int mi_add_rmsnorm_multi(const float* stream_in, const void* add1, const void* add2, const float* add32,
                                     const float* row_add, float* stream_out, const int* rows, const float* gain,
-                                    void* out, int M, int H, float eps, int kept, int dtype, cudaStream_t stream) {
+                                    void* out, int M, int H, float eps, int dtype, cudaStream_t stream) {
   if (M <= 0) return 0;
   if (H <= 0) MI_REFUSE("rmsnorm: bad width %d", H);
   if (rows && stream_out) MI_REFUSE("rmsnorm: a gathered norm does not write the stream");
   const size_t smem = (32 + (size_t)H) * sizeof(float);
   if (smem > 200 * 1024) MI_REFUSE("rmsnorm: a row of %d floats does not fit in shared memory", H);
   const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
-  bool pieces = !kept && H % 4 == 0 && H <= 16 * threads;
+  bool pieces = H % 4 == 0 && H <= 16 * threads;
   for (const void* ptr : {(const void*)stream_in, add1, add2, (const void*)add32, (const void*)row_add, (const void*)stream_out,
                           (const void*)gain, (const void*)out})
     pieces = pieces && mi_aligned(ptr, 16);
   if (pieces) {
 #define MI_GO4(T, NV)                                                                                                   \
-  MI_LAUNCH((add_rmsnorm_multi4_kernel<T, NV>), M, threads, 0, stream, stream_in, (const T*)add1, (const T*)add2, add32, row_add, \
-            stream_out, rows, gain, (T*)out, H, eps)
+  MI_LAUNCH((add_rmsnorm_multi4_kernel<T, NV>), M, threads, 0, stream, \
+            stream_in, (const T*)add1, (const T*)add2, add32, row_add, stream_out, rows, gain, (T*)out, H, eps)
 #define MI_GO4_T(T)                          \
   if (H <= 4 * threads) MI_GO4(T, 1);        \
   else if (H <= 8 * threads) MI_GO4(T, 2);   \

@@ -203,3 +203,43 @@ def test_delta_rule_with_warps_that_stage(dtype, heads, kvh, dk, dv, lens):
     assert torch.isfinite(got).all()
     assert torch.equal(got, want) and torch.equal(whole, cut)
     assert torch.equal(whole[1], begin[1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,H", [(1, 4), (3, 100), (3, 508), (3, 516), (2, 1028), (8, 2048), (5, 2052), (2, 4096), (2, 4100), (3, 8192)])
+def test_norms_in_registers_have_the_bits_of_the_form_for_any_row(dtype, M, H):
+    """One order of sums whatever the address, the kept sums of models with groups of experts among them."""
+    o = ops()
+    stream, a1, a2, add32 = rnd(M, H, seed=1), rnd(M, H, dtype=dtype, seed=2), rnd(M, H, dtype=dtype, seed=3), rnd(M, H, seed=8)
+    w1, b1, w2, b2 = (rnd(H, seed=s) for s in (4, 5, 6, 7))
+    rows = torch.tensor([M - 1, 0], dtype=torch.int32, device=DEV)
+    for adds in ((a1, a2), (a1,), ()):
+        got = []
+        for w in (w1, shifted(w1)):           # a gain at any address takes the other form
+            new = stream.clone()
+            outs = o.add_layernorm(new, adds, [(w, b1), (w2, b2)], 1e-6, dtype)
+            got.append([*outs, new, *o.add_layernorm(stream, adds, [(w, b1)], 1e-6, dtype, rows=rows)])
+            for s, kw in ((stream, {}), (stream, dict(add32=add32, row_add=b1)), (None, dict(add32=add32))):
+                got[-1] += o.add_rmsnorm_multi(s, adds, w, 1e-6, dtype, **kw)
+            got[-1].append(o.add_rmsnorm_multi(stream, adds, w, 1e-6, dtype, rows=rows)[0])
+        assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M", [2, 70])
+@pytest.mark.parametrize("d", [4, 20, 64, 100, 128, 132, 252, 256])
+def test_biased_heads_in_pieces_have_the_bits_of_single_elements(dtype, M, d):
+    o, nq, nkv, page = ops(), 6, 2, 8
+    width = (nq + nkv) * d
+    x, slots = rnd(M, width, dtype=dtype, seed=1), torch.arange(M, dtype=torch.int32, device=DEV)
+    qb, kb, qg, kg = rnd(nq * d, seed=2), rnd(nkv * d, seed=3), rnd(d, seed=4), rnd(d, seed=5)
+    for bias in (True, False):
+        got = []
+        for off in (0, 1):               # from the second column on a piece is no aligned access
+            packed = torch.zeros(M, width + 4, dtype=dtype, device=DEV)[:, off:off + width]
+            packed.copy_(x)
+            k, v = cache_pair(M, nkv, d, page, dtype)
+            o.qk_bias_norm_store(packed, 0, nq * d, nq * d, nq, nkv, d, d, q_bias=qb if bias else None, k_bias=kb if bias else None,
+                                 q_gain=qg, k_gain=kg, eps=1e-6, values_are_keys=True, slots=slots, kcache=k, vcache=v)
+            got.append((packed, k, v))
+        assert all(torch.equal(a, b) for a, b in zip(*got))
