@@ -4,12 +4,15 @@
 //                     (ties: the lower index; optionally among the experts of the best groups only) and
 //                     their weights (the softmax over those alone, or their share of the softmax over all
 //                     experts, times a factor, or their sigmoids times a factor, chosen with a correction
-//                     added per expert) -> ids [M, top] int32, weights [M, top] fp32
+//                     added per expert) -> ids [M, top] int32, weights [M, top] fp32.  Where a token has fewer
+//                     candidates than `top` (logits that are NaN or minus infinity) the others of its ids are
+//                     valid ones and their weights NaN
 //   mi_moe_plan       sorts the M*top (token, choice) entries by expert: perm[pos] = entry, inv[entry] =
 //                     pos, offsets[E + 1], and the list of row tiles (expert, first row, rows) that the
 //                     grouped products walk.  Nothing comes back to the host: the products are launched
 //                     for the largest possible number of tiles and the surplus blocks leave at once.
-//                     Tiles have 64 rows, or 8 for steps that bring an expert only a few rows.
+//                     Tiles have 64 rows, or 8 for steps that bring an expert only a few rows.  An entry whose id
+//                     is no expert's stands behind all others, in no tile, with inv = -1, and its token comes out NaN.
 //   mi_moe_gate_up    act[pos, :] = glu(W_gate[e] x_token, W_up[e] x_token) for the entries of each expert
 //   mi_moe_down       y[pos, :] = W_down[e] act[pos, :]   (fp32)
 //   mi_moe_gather     xs[pos, :] = x[token of pos, :], for steps whose products are a library's grouped product
@@ -164,6 +167,8 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
         best_e = oe;
       }
     }
+    const bool none = best_e >= E;       // no candidate is left
+    if (none) best_e = k;
     float score = 0.f;
 #pragma unroll
     for (int i = 0; i < PER; ++i)
@@ -175,6 +180,7 @@ moe_select_kernel(const float* __restrict__ logits, int stride, int* __restrict_
     float p;
     if (mode == 2) p = __shfl_sync(0xffffffffu, score, best_e & 31);
     else p = mode == 1 ? expf(best - zmax) / zsum : expf(best - first);
+    if (none) p = __int_as_float(0x7fc00000);
     denom += p;
     if (lane == k) {
       my_val = p;
@@ -220,11 +226,12 @@ __global__ void moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* 
                                 int* __restrict__ inv, int* __restrict__ plan, int tile_rows) {
   mi_pdl_enter();
   extern __shared__ int sh[];
-  int* counts = sh;            // [E]
-  int* cursor = sh + E;        // [E]
-  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
+  int* counts = sh;            // [E + 1]: the last one counts the ids that are no expert's
+  int* cursor = sh + E + 1;    // [E + 1]
+  auto expert = [&](int i) { const unsigned e = (unsigned)ids[i]; return e < (unsigned)E ? (int)e : E; };
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) counts[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&counts[ids[i]], 1);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&counts[expert(i)], 1);
   __syncthreads();
   // rows and tiles in front of every expert: a warp scan per 32 experts, carried on from one to the next by one warp
   if (threadIdx.x < 32) {
@@ -259,14 +266,15 @@ __global__ void moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* 
     }
     if (lane == 0) {
       offsets[E] = run;
+      cursor[E] = run;
       plan[0] = nt;
     }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int pos = atomicAdd(&cursor[ids[i]], 1);
+    const int e = expert(i), pos = atomicAdd(&cursor[e], 1);
     perm[pos] = i;
-    inv[i] = pos;
+    inv[i] = e < E ? pos : -1;
   }
 }
 
@@ -279,7 +287,7 @@ extern "C" int mi_moe_plan(const int* ids, int n, int E, int* perm, int* inv, in
   if (n <= 0) return 0;
   if (E <= 0 || E > 4096) MI_REFUSE("moe: %d experts", E);
   if (tile_rows != TILE_M && tile_rows != FEW_ROWS) MI_REFUSE("moe: tiles of %d rows", tile_rows);
-  MI_LAUNCH((moe_plan_kernel), 1, 1024, 2 * E * sizeof(int), stream, ids, n, E, perm, inv, plan, tile_rows);
+  MI_LAUNCH((moe_plan_kernel), 1, 1024, 2 * (E + 1) * sizeof(int), stream, ids, n, E, perm, inv, plan, tile_rows);
   MI_RETURN_LAUNCH_STATUS();
 }
 
@@ -867,8 +875,10 @@ __global__ void moe_combine_kernel(const YT* __restrict__ y, const int* __restri
   const float sg = (shared && shared_gate) ? 1.f / (1.f + expf(-shared_gate[(size_t)t * gate_stride])) : 1.f;
   for (int c = threadIdx.x; c < H; c += blockDim.x) {
     float acc = 0.f;
-    for (int k = 0; k < top; ++k)
-      acc = fmaf(weights[(size_t)t * top + k], mi_to_float(y[(size_t)inv[(size_t)t * top + k] * H + c]), acc);
+    for (int k = 0; k < top; ++k) {
+      const int row = inv[(size_t)t * top + k];
+      acc = row < 0 ? __int_as_float(0x7fc00000) : fmaf(weights[(size_t)t * top + k], mi_to_float(y[(size_t)row * H + c]), acc);
+    }
     if (shared) acc = fmaf(sg, mi_to_float(shared[(size_t)t * shared_stride + c]), acc);
     out[(size_t)t * H + c] = mi_from_float<T>(acc);
   }
@@ -885,8 +895,9 @@ __global__ void moe_combine4_kernel(const YT* __restrict__ y, const int* __restr
   __shared__ float wts[32];
   const int t = blockIdx.x;
   if (threadIdx.x < top) {
-    rows[threadIdx.x] = inv[(size_t)t * top + threadIdx.x];
-    wts[threadIdx.x] = weights[(size_t)t * top + threadIdx.x];
+    const int row = inv[(size_t)t * top + threadIdx.x];      // (a weight of NaN for an id that is no expert's)
+    rows[threadIdx.x] = max(row, 0);
+    wts[threadIdx.x] = row < 0 ? __int_as_float(0x7fc00000) : weights[(size_t)t * top + threadIdx.x];
   }
   const float sg = (shared && shared_gate) ? 1.f / (1.f + expf(-shared_gate[(size_t)t * gate_stride])) : 1.f;
   __syncthreads();
