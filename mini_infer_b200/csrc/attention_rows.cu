@@ -174,13 +174,14 @@ attention_rows_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict
   const int chunks_all = walk.count(j_end, CHUNK), chunks_mine = (chunks_all + n_splits - 1) / n_splits;
   const int i_begin = split * chunks_mine, i_stop = min(chunks_all, (split + 1) * chunks_mine);
   const float cap_k = EXT && softcap > 0.f ? scale / softcap : 0.f;
-  // A run without keys leaves its maxima and denominators only: the runs with keys come first, and whoever adds them up
-  // stops at the last one that any key joined.  (A captured step has the runs of the longest request it may meet: 50
+  // A run without keys leaves its maxima and denominators only, the latter -1: the runs with keys come first, and whoever adds
+  // them up stops behind the last one with a denominator of its own (keys of NaN leave a maximum of minus infinity too, and
+  // sums that are to be seen).  (A captured step has the runs of the longest request it may meet: 50
   // for 3200 keys, of which a request of 700 fills 11; the others wrote zeros, 32 KB for 16 rows of 512, to be read
   // again.  8 requests of 16 heads: the merge with the values 9.8 us to 7.1, a step of three such layers 276 to 268.)
   if (n_splits > 1 && i_begin >= i_stop) {
     float2* pml = reinterpret_cast<float2*>(part_ml) + ((size_t)(blockIdx.x / n_splits) * n_splits + split) * R;
-    for (int r = tid; r < R; r += NT) pml[r] = make_float2(-INFINITY, 0.f);
+    for (int r = tid; r < R; r += NT) pml[r] = make_float2(-INFINITY, -1.f);
     return;
   }
 
@@ -455,17 +456,17 @@ attention_rows_merge_kernel(const float* __restrict__ part_o, const float* __res
     const float sink2 = sinks ? sinks[head] * LOG2E : -INFINITY;
     const float mf = fmaxf(m, sink2);
     float l = 0.f;
-    int runs = 0;                                   // one past the last run that a key joined
+    int runs = 0;                                   // one past the last run with keys
     for (int s0 = 0; s0 < n_splits; s0 += 32) {     // runs in ascending order: lanes, then the warp's fixed tree
       const int s = s0 + lane;
       float w = 0.f, part = 0.f;
       bool any = false;
       if (s < n_splits) {
-        const float ms = pml[(size_t)s * R * 2];
+        const float ms = pml[(size_t)s * R * 2], ls = pml[(size_t)s * R * 2 + 1];
         w = ms == -INFINITY ? 0.f : exp2f(ms - mf);
-        part = pml[(size_t)s * R * 2 + 1] * w;
+        part = ls * w;
         weight[s] = w;
-        any = ms != -INFINITY;
+        any = !(ls < 0.f);
       }
       l += mi_warp_sum(part);
       const unsigned joined = __ballot_sync(0xffffffffu, any);
@@ -482,7 +483,7 @@ attention_rows_merge_kernel(const float* __restrict__ part_o, const float* __res
   const int runs = last;
   bf16* o = out + (size_t)(q_start[b] + tok0 + rows.token(r)) * out_stride + head * dv;
   const float* po = part_o + ((size_t)unit * n_splits * R + r) * dv;
-  // four columns per thread, eight runs in flight; the runs behind the last with a key have left no sums
+  // four columns per thread, eight runs in flight; the runs behind the last one with keys have left no sums
   for (int c = threadIdx.x * 4; c < dv; c += blockDim.x * 4) {
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     int s = 0;

@@ -165,7 +165,7 @@ latent_value_kernel(const float* __restrict__ part_o, const float* __restrict__ 
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int s = tid + 32 * k;
-        ml[k] = s < n_splits ? *reinterpret_cast<const float2*>(pml + (size_t)s * RUN_ROWS * 2) : make_float2(-INFINITY, 0.f);
+        ml[k] = s < n_splits ? *reinterpret_cast<const float2*>(pml + (size_t)s * RUN_ROWS * 2) : make_float2(-INFINITY, -1.f);
       }
       const float sink2 = sinks ? sinks[h] * LOG2E : -INFINITY;
       const float mf = fmaxf(mi_warp_max(fmaxf(ml[0].x, ml[1].x)), sink2);
@@ -173,7 +173,7 @@ latent_value_kernel(const float* __restrict__ part_o, const float* __restrict__ 
       int runs = 0;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const unsigned joined = __ballot_sync(0xffffffffu, ml[k].x != -INFINITY);
+        const unsigned joined = __ballot_sync(0xffffffffu, !(ml[k].y < 0.f));
         if (joined) runs = 32 * k + 32 - __clz(joined);
         const float ws = ml[k].x == -INFINITY ? 0.f : exp2f(ml[k].x - mf);
         weight[tid + 32 * k] = ws;
@@ -187,7 +187,7 @@ latent_value_kernel(const float* __restrict__ part_o, const float* __restrict__ 
     }
     __syncthreads();
     const float inv = inv_l;
-    const int runs = last;           // the runs behind the last one that a key joined have left no sums
+    const int runs = last;           // the runs behind the last one with keys (a denominator of -1) have left no sums
     for (int c = tid; c < rank; c += V_THREADS) {
       float sum = 0.f;
       for (int s0 = 0; s0 < runs; s0 += V_RUNS) {         // added in order

@@ -963,3 +963,35 @@ def test_runs_without_keys_leave_no_sums(lens, n, rd, rank, sink, monkeypatch):
         # weights and results rounded to bfloat16: 2^-8 of the largest value each, twice over for the sums
         for got in (fused[i], merged[i]):
             assert (got.double() - want).abs().max() <= 2.0 ** -6 * max(1.0, want.abs().max().item() if x else 1.0), (i, x)
+
+
+@pytest.mark.parametrize("lens,runs", [([65, 1, 130, 3], 64), ([65, 1, 130, 3], 3)])
+def test_requests_whose_keys_are_all_nan_come_out_nan(lens, runs):
+    """A fault stays visible: a request with nothing but NaN in its keys and values gives NaN, cut into runs of keys or not, and
+    the requests beside it what they give without it."""
+    from types import SimpleNamespace
+    o = ops()
+    i32 = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    page, n, rd, rank, M, scale = 16, 16, 16, 64, len(lens), 0.6
+    d, per = rank + rd, -(-max(lens) // page)
+    rows = rnd(M, per * page, 1, d, dtype=torch.bfloat16, seed=1).cuda()
+    q = rnd(M, n * d, dtype=torch.bfloat16, seed=2, scale=d ** -0.5).cuda()
+    table = torch.arange(M * per, dtype=torch.int32, device="cuda").reshape(M, per)
+    eye = torch.eye(rank, dtype=torch.bfloat16, device="cuda").expand(n, rank, rank).contiguous()
+    results = []
+    for broken in ((), (1, 2)):
+        rows[list(broken)] = float("nan")
+        kc = o.pack_cache_pages(rows.reshape(M * per * page, 1, d), page)
+        ctx = SimpleNamespace(groups=[SimpleNamespace(block_table=table, page_size=page, table_rows=i32(range(M)))],
+                              decode_only=True, n_tokens=M, q_start=i32(range(M)), q_len=i32([1] * M), kv_len=i32(lens),
+                              max_kv_len=64 * runs, tiles={1: (None, None, M)}, q_tiles=lambda tt: (None, None, M))
+        cache = SimpleNamespace(group=0, k=kc, v=None)
+        parts = o.attention_latent_runs(q, cache, ctx, n, d, rank, scale)
+        assert parts[2] == runs
+        fused, merged = (torch.zeros(M, n * rank, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        o.latent_value(parts, None, eye, fused, n)
+        o.attention_ext(q, merged, cache, ctx, n, 1, d, rank, scale, values_in_keys=True)
+        results.append((fused, merged))
+    for good, got in zip(*results):
+        assert torch.isfinite(good).all() and torch.isnan(got[[1, 2]]).all()
+        assert torch.equal(got[[0, 3]], good[[0, 3]])
