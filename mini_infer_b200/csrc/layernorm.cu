@@ -103,16 +103,16 @@ __global__ void add_layernorm_kernel(const float* __restrict__ stream, const T* 
   }
 }
 
-// The same bits for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays on chip, and the gains and
-// biases, which no kernel writes, are asked for before the wait (what kernels do write is not `__restrict__`: the compiler may
-// move loads through such pointers over the wait).  Every piece is read and written once, in one round trip.  The sums run in
+// The same bits for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays on chip.  AHEAD: no
+// kernel that may still run writes the gains and biases (a model's own), and they are asked for before the wait; without it 8 rows
+// of 4096 with two norms 3.0 us become 3.4.  Every piece is read and written once, in one round trip.  The sums run in
 // the order of the kernel above, a thread's elements blockDim apart: the row goes through shared memory for them.  8 rows of 4096 with two
 // norms 6.0 us in the kernel above, 3.0 here (2.9 with the four of a piece added up first, which gives other bits); 2048 rows of
 // 2048 17.6, 13.2 and 12.1 (10 of bytes).
-template <typename T, int NV>
+template <typename T, int NV, bool AHEAD>
 __global__ void __launch_bounds__(512, NV == 4 ? 1 : NV == 2 ? 2 : 3)
 add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* stream_out, const int* rows, const float* w1,
-                      const float* b1, T* __restrict__ out1, const float* w2, const float* b2, T* __restrict__ out2, int H, float eps) {
+                      const float* b1, T* out1, const float* w2, const float* b2, T* out2, int H, float eps) {
   mi_pdl_launch_dependents();
   __shared__ float red[32];
   __shared__ __align__(16) float row[NV * 4 * 512];
@@ -130,8 +130,10 @@ add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* 
       }
     }
   };
+  if (AHEAD) {
 #pragma unroll
-  for (int n = 0; n < NV; ++n) gains(n);
+    for (int n = 0; n < NV; ++n) gains(n);
+  }
   mi_pdl_wait();
   const size_t i = blockIdx.x, src = rows ? rows[i] : i;
 #pragma unroll
@@ -177,6 +179,7 @@ add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* 
   for (int n = 0; n < NV; ++n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k >= H) continue;
+    if (!AHEAD) gains(n);
     v.load(row + k);
     v.get(r);
     if (stream_out) v.store(stream_out + i * H + k);
@@ -197,9 +200,10 @@ add_layernorm4_kernel(const float* stream, const T* add1, const T* add2, float* 
   }
 }
 
+// w_constant: no kernel that may still run writes the gains and biases
 extern "C" int mi_add_layernorm(const float* stream, const void* add1, const void* add2, float* stream_out,
                                 const int* rows, const float* w1, const float* b1, void* out1,
-                                const float* w2, const float* b2, void* out2, int M, int H, float eps,
+                                const float* w2, const float* b2, void* out2, int M, int H, float eps, int w_constant,
                                 int dtype, cudaStream_t stream_) {
   if (M <= 0) return 0;
   if (H <= 0) MI_REFUSE("layernorm: bad width %d", H);
@@ -212,8 +216,9 @@ extern "C" int mi_add_layernorm(const float* stream, const void* add1, const voi
                           (const void*)out1, (const void*)w2, (const void*)b2, (const void*)out2})
     pieces = pieces && mi_aligned(ptr, 16);
   if (pieces) {
+    const bool ahead = w_constant != 0;
 #define MI_GO4(T, NV)                                                                                               \
-  MI_LAUNCH((add_layernorm4_kernel<T, NV>), M, threads, 0, stream_, \
+  MI_LAUNCH((ahead ? add_layernorm4_kernel<T, NV, true> : add_layernorm4_kernel<T, NV, false>), M, threads, 0, stream_, \
             stream, (const T*)add1, (const T*)add2, stream_out, rows, w1, b1, (T*)out1, w2, b2, (T*)out2, H, eps)
 #define MI_GO4_T(T)                          \
   if (H <= 4 * threads) MI_GO4(T, 1);        \

@@ -282,7 +282,7 @@ def _sig_expanded(lib: ctypes.CDLL) -> None:
 def _sig_layernorm(lib: ctypes.CDLL) -> None:
     lib.mi_embedding_scaled.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p]
     lib.mi_add_layernorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                     c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
+                                     c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_int, c_void_p]
 
 
 def _sig_rope_norm(lib: ctypes.CDLL) -> None:
@@ -347,7 +347,7 @@ def _sig_stream(lib: ctypes.CDLL) -> None:
                                            c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, ll, ll, c_int,
                                            c_void_p]
     lib.mi_add_rmsnorm_multi.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                         c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
+                                         c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_int, c_void_p]
     lib.mi_glu_mul_pairs.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_embedding_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
                                          c_void_p]
@@ -1370,11 +1370,13 @@ def embedding_scaled(table: torch.Tensor, ids: torch.Tensor, scale: float) -> to
 
 
 def add_layernorm(stream: torch.Tensor, adds, norms, eps: float, dtype: torch.dtype, *,
-                  rows: torch.Tensor | None = None, update_stream: bool = True):
+                  rows: torch.Tensor | None = None, update_stream: bool = True, w_constant: bool = False):
     """Layer norm(s) of ``r = stream + sum(adds)`` (fp32; ``adds``: up to two ``[M, H]`` tensors
     of ``dtype``).  ``norms``: one or two ``(gain, bias)`` pairs (fp32 ``[H]``); one output in
     ``dtype`` per pair.  Without ``rows`` and with ``update_stream`` the stream is replaced by
-    ``r`` in place; with ``rows`` (int32) only those rows are normalised and the stream stays."""
+    ``r`` in place; with ``rows`` (int32) only those rows are normalised and the stream stays.  With
+    ``w_constant`` the kernel may read gains and biases while kernels before it still run: for a model's
+    own, never for what such a kernel writes."""
     adds = [a for a in adds if a is not None]
     if len(adds) > 2 or not 1 <= len(norms) <= 2:
         raise KernelError("layernorm: at most two addends and one or two norms")
@@ -1400,7 +1402,8 @@ def add_layernorm(stream: torch.Tensor, adds, norms, eps: float, dtype: torch.dt
     rc = lib.mi_add_layernorm(_ptr(stream), _ptr(a1), _ptr(a2),
                               _ptr(stream if (rows is None and update_stream and adds) else None), _ptr(rows),
                               _ptr(norms[0][0]), _ptr(norms[0][1]), _ptr(outs[0]), _ptr(w2), _ptr(b2),
-                              _ptr(outs[1] if len(outs) > 1 else None), M, H, float(eps), _code(dtype), _stream())
+                              _ptr(outs[1] if len(outs) > 1 else None), M, H, float(eps), 1 if w_constant else 0,
+                              _code(dtype), _stream())
     _finish(lib, rc, "layernorm")
     return outs
 
@@ -1991,12 +1994,14 @@ def embedding_rmsnorm(table: torch.Tensor, ids: torch.Tensor, gain: torch.Tensor
 
 def add_rmsnorm_multi(stream: torch.Tensor | None, adds, gain: torch.Tensor, eps: float, dtype: torch.dtype, *,
                       add32: torch.Tensor | None = None, row_add: torch.Tensor | None = None,
-                      rows: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor | None]:
+                      rows: torch.Tensor | None = None,
+                      w_constant: bool = False) -> tuple[torch.Tensor, torch.Tensor | None]:
     """RMS norm of ``r = stream + sum(adds) + add32 + row_add`` in fp32: ``stream`` the fp32 stream
     ``[M, H]``, ``adds`` up to two ``[M, H]`` tensors of ``dtype`` (branch outputs), ``add32`` an fp32
     ``[M, H]`` tensor, ``row_add`` an fp32 ``[H]`` vector added to every row; each may be missing.
     Returns ``(gain * r * rsqrt(mean(r^2) + eps)`` in ``dtype``, the new fp32 stream ``r``)``; with
-    ``rows`` (int32) only those rows are normalised and no stream is returned."""
+    ``rows`` (int32) only those rows are normalised and no stream is returned.  ``w_constant``: see
+    ``add_layernorm`` (the gain)."""
     adds = [a for a in adds if a is not None]
     if len(adds) > 2:
         raise KernelError("rmsnorm: at most two addends in the compute dtype")
@@ -2021,7 +2026,7 @@ def add_rmsnorm_multi(stream: torch.Tensor | None, adds, gain: torch.Tensor, eps
     lib = _lib("stream")
     rc = lib.mi_add_rmsnorm_multi(_ptr(stream), _ptr(adds[0] if adds else None), _ptr(adds[1] if len(adds) > 1 else None),
                                   _ptr(add32), _ptr(row_add), _ptr(new_stream), _ptr(rows), _ptr(gain), _ptr(out),
-                                  M, H, float(eps), _code(dtype), _stream())
+                                  M, H, float(eps), 1 if w_constant else 0, _code(dtype), _stream())
     _finish(lib, rc, "rmsnorm")
     return out, new_stream
 

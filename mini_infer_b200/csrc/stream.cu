@@ -139,15 +139,15 @@ __global__ void add_rmsnorm_multi_kernel(const float* __restrict__ stream_in, co
   }
 }
 
-// The same bits for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays on chip, the gain, which no
-// kernel writes, is asked for before the wait (what kernels do write is not `__restrict__`: the compiler may move loads through
-// such pointers over the wait), and every operand is one round trip.  The sum of squares runs in the order of the kernel above,
+// The same bits for rows of whole aligned pieces of four that fit NV pieces a thread: the row stays on chip, and every
+// operand is one round trip.  AHEAD: no kernel that may still run writes the gain (a model's own), and it is asked for before the
+// wait; without it 8 rows of 4096 2.4 us become 2.8.  The sum of squares runs in the order of the kernel above,
 // a thread's elements blockDim apart: the row goes through shared memory for it.  8 rows of 2048 and 2 addends 3.1 us above, 1.8
 // here; 2048 rows of 4096 36 and 23 (18 of bytes).
-template <typename T, int NV>
+template <typename T, int NV, bool AHEAD>
 __global__ void __launch_bounds__(512)
 add_rmsnorm_multi4_kernel(const float* stream_in, const T* add1, const T* add2, const float* add32, const float* row_add,
-                          float* stream_out, const int* rows, const float* gain, T* __restrict__ out, int H,
+                          float* stream_out, const int* rows, const float* gain, T* out, int H,
                           float eps) {
   mi_pdl_launch_dependents();
   __shared__ float red[32];
@@ -162,8 +162,10 @@ add_rmsnorm_multi4_kernel(const float* stream_in, const T* add1, const T* add2, 
       v.get(g[n]);
     }
   };
+  if (AHEAD) {
 #pragma unroll
-  for (int n = 0; n < NV; ++n) gains(n);
+    for (int n = 0; n < NV; ++n) gains(n);
+  }
   mi_pdl_wait();
   const size_t i = blockIdx.x, src = rows ? rows[i] : i;
 #pragma unroll
@@ -216,6 +218,7 @@ add_rmsnorm_multi4_kernel(const float* stream_in, const T* add1, const T* add2, 
   for (int n = 0; n < NV; ++n) {
     const int k = 4 * (threadIdx.x + n * blockDim.x);
     if (k >= H) continue;
+    if (!AHEAD) gains(n);
     v.load(row + k);
     v.get(r);
     if (stream_out) v.store(stream_out + i * H + k);
@@ -226,9 +229,10 @@ add_rmsnorm_multi4_kernel(const float* stream_in, const T* add1, const T* add2, 
   }
 }
 
+// w_constant: no kernel that may still run writes the gain
 extern "C" int mi_add_rmsnorm_multi(const float* stream_in, const void* add1, const void* add2, const float* add32,
                                     const float* row_add, float* stream_out, const int* rows, const float* gain,
-                                    void* out, int M, int H, float eps, int dtype, cudaStream_t stream) {
+                                    void* out, int M, int H, float eps, int w_constant, int dtype, cudaStream_t stream) {
   if (M <= 0) return 0;
   if (H <= 0) MI_REFUSE("rmsnorm: bad width %d", H);
   if (rows && stream_out) MI_REFUSE("rmsnorm: a gathered norm does not write the stream");
@@ -240,8 +244,9 @@ extern "C" int mi_add_rmsnorm_multi(const float* stream_in, const void* add1, co
                           (const void*)gain, (const void*)out})
     pieces = pieces && mi_aligned(ptr, 16);
   if (pieces) {
+    const bool ahead = w_constant != 0;
 #define MI_GO4(T, NV)                                                                                                   \
-  MI_LAUNCH((add_rmsnorm_multi4_kernel<T, NV>), M, threads, 0, stream, \
+  MI_LAUNCH((ahead ? add_rmsnorm_multi4_kernel<T, NV, true> : add_rmsnorm_multi4_kernel<T, NV, false>), M, threads, 0, stream, \
             stream_in, (const T*)add1, (const T*)add2, add32, row_add, stream_out, rows, gain, (T*)out, H, eps)
 #define MI_GO4_T(T)                          \
   if (H <= 4 * threads) MI_GO4(T, 1);        \

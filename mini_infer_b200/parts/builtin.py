@@ -141,7 +141,8 @@ class RMSNorm(Norm):
         branches (compute dtype), an fp32 tensor and an fp32 row that a stream part left
         (``BranchSum.stream_add``, ``row_add``); before the first layer an fp32 ``x`` is the stream
         itself.  The stream that comes in is left as it is; a new one is returned."""
-        if getattr(self, "_gain32", None) is None:
+        there = getattr(self, "_gain32", None) is not None
+        if not there:
             self._gain32 = self.weight.to(torch.float32).contiguous()
         adds, add32, row_add = (), None, None
         if isinstance(x, BranchSum):
@@ -151,7 +152,7 @@ class RMSNorm(Norm):
         else:
             adds = (x,)
         return ops.add_rmsnorm_multi(residual, adds, self._gain32, self.eps, self.dtype, add32=add32,
-                                     row_add=row_add, rows=rows)
+                                     row_add=row_add, rows=rows, w_constant=there)
 
 
 class SameNorm(Norm):
@@ -191,14 +192,14 @@ class LayerNorm(Norm):
 
     def forward(self, x, residual, rows=None):
         stream, adds = self.stream_and_addends(x, residual)
-        out, = ops.add_layernorm(stream, adds, [(self.weight, self.bias)], self.eps, self.dtype, rows=rows)
+        out, = ops.add_layernorm(stream, adds, [(self.weight, self.bias)], self.eps, self.dtype, rows=rows, w_constant=True)
         return out, (None if rows is not None else stream)
 
     def forward_with(self, other: "LayerNorm", x, residual):
         """This norm and ``other`` of the same stream in one pass: ``(out_self, out_other, stream)``."""
         stream, adds = self.stream_and_addends(x, residual)
         a, b = ops.add_layernorm(stream, adds, [(self.weight, self.bias), (other.weight, other.bias)],
-                                 self.eps, self.dtype)
+                                 self.eps, self.dtype, w_constant=True)
         return a, b, stream
 
 

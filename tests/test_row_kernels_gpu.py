@@ -243,3 +243,25 @@ def test_biased_heads_in_pieces_have_the_bits_of_single_elements(dtype, M, d):
                                  q_gain=qg, k_gain=kg, eps=1e-6, values_are_keys=True, slots=slots, kcache=k, vcache=v)
             got.append((packed, k, v))
         assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_gains_that_the_kernel_before_writes(dtype):
+    """Gain and bias are results of a long product of this library right in front of the norm: unless the caller says that they are
+    constant, no kernel may read them before that product is done."""
+    o, M, H, K = ops(), 3, 2048, 8192
+    x, w, stream, add = rnd(1, K, seed=1), rnd(H, K, seed=2), rnd(M, H, seed=3), rnd(M, H, dtype=dtype, seed=4)
+    gain = torch.full((1, H), float("nan"), device=DEV)
+    norms = [lambda g, **kw: o.add_layernorm(stream, [add], [(g, g)], 1e-6, dtype, update_stream=False, **kw)[0],
+             lambda g, **kw: o.add_layernorm(stream, [add], [(g, g), (g, g)], 1e-6, dtype, update_stream=False, **kw)[1],
+             lambda g, **kw: o.add_rmsnorm_multi(stream, [add], g, 1e-6, dtype, **kw)[0]]
+    for norm in norms:
+        for _ in range(5):
+            gain.fill_(float("nan"))
+            torch.cuda.synchronize()
+            o.gemm_f32(x, w, out=gain)
+            got = norm(gain[0])
+            torch.cuda.synchronize()
+            want = norm(gain[0].clone())
+            assert torch.isfinite(want).all() and torch.equal(got, want)
+        assert torch.equal(norm(gain[0], w_constant=True), want)
