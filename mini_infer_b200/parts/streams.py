@@ -72,6 +72,8 @@ class beside:
             self.here.wait_stream(self.stream)
 
     def __exit__(self, *error) -> None:
-        self._join()                   # behind an error as well: a capture ends with one stream
-        if self.on:
-            _open[self.key] -= 1
+        try:
+            self._join()               # behind an error as well: a capture ends with one stream
+        finally:
+            if self.on:
+                _open[self.key] -= 1
