@@ -84,6 +84,8 @@ class ConvAttention(PagedSoftmax):
     tensors: ``q``, ``k``, ``v``, ``q.conv``, ``k.conv``, ``v.conv`` (``[channels, conv_taps]``), ``o``.
     """
 
+    alone = True
+
     def __init__(self, spec):
         super().__init__(spec)
         g = self.spec.params.get
@@ -148,6 +150,8 @@ class DifferentialAttention(PagedSoftmax):
     ``head_gate`` (default False).
     tensors: ``q``, ``k``, ``v``, ``o``, ``lq1``, ``lk1``, ``lq2``, ``lk2`` and, with the gate, ``g``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)

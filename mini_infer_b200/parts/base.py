@@ -149,7 +149,7 @@ class StepContext:
     # block tables before its first kernel (the step runner's business, not a part's)
     table_updates: list = field(default_factory=list)
     # what parts of different layers share within one step (a table that depends on the step's
-    # positions only, say): filled by whoever needs it first
+    # positions only, say): filled by whoever needs it first (two parts side by side, ``Part.alone``: each for itself)
     scratch: dict = field(default_factory=dict)
 
     def q_tiles(self, tokens: int) -> tuple[torch.Tensor, torch.Tensor, int]:
@@ -176,6 +176,16 @@ class Part:
     # Whether a difference in the last bit can change this part's output a great deal: a step of its model then
     # runs under ``ops.kept_sums``.
     keeps_sums: bool = False
+    # Whether ``forward`` (a projected mixer's ``mix``) may run beside the layer's other part in a captured step, on a stream of
+    # its own: it reads nothing that the other part leaves in ``StepContext.scratch`` or changes, and changes nothing that the
+    # other reads.  What both need from the dictionary each then fills for itself.  Parts that do not say so run one after the
+    # other, the mixer first (of two mixers the left one).  A class says it for itself: one derived from it says it again.
+    alone: bool = False
+
+    def __init_subclass__(cls, **kwargs) -> None:
+        super().__init_subclass__(**kwargs)
+        if "alone" not in cls.__dict__:
+            cls.alone = False
 
     def __init__(self, spec: PartSpec) -> None:
         self.spec = spec

@@ -39,7 +39,7 @@ from .base import (
     register_position,
     register_stream_part,
 )
-from .streams import beside
+from .streams import pair
 
 
 def _as_compute(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -394,6 +394,8 @@ class RotaryPosition(Position):
     such a kernel forms the angle in double precision).
     """
 
+    alone = True
+
     def bind(self, tensors, dtype, device):
         d = int(self.param("head_dim"))
         self.rotary_dim = int(self.spec.params.get("rotary_dim") or d)
@@ -463,6 +465,8 @@ class InterleavedRotary(Position):
     params: ``head_dim``, ``theta``, optional ``rotary_dim`` (default ``head_dim``).
     """
 
+    alone = True
+
     def bind(self, tensors, dtype, device):
         d = int(self.param("head_dim"))
         self.rotary_dim = int(self.spec.params.get("rotary_dim") or d)
@@ -493,6 +497,8 @@ class GroupedQueryAttention(Mixer):
     (default ``head_dim ** -0.5``).
     tensors: ``q_proj.weight``, ``k_proj.weight``, ``v_proj.weight``, ``o_proj.weight``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -573,6 +579,8 @@ class SwiGLU(FeedForward):
     tensors: ``gate_proj.weight``, ``up_proj.weight``, ``down_proj.weight``.
     """
 
+    alone = True
+
     def __init__(self, spec):
         super().__init__(spec)
         self.activation = str(self.spec.params.get("activation", "silu"))
@@ -618,6 +626,8 @@ class ClampedGLU(FeedForward):
     ``up_offset`` (default 1).  tensors: ``gate``, ``up``, ``down``.
     """
 
+    alone = True
+
     def param_decls(self):
         H, I = int(self.param("hidden_size")), int(self.param("intermediate_size"))
         return {"gate": ParamDecl((I, H)), "up": ParamDecl((I, H)), "down": ParamDecl((H, I))}
@@ -643,6 +653,8 @@ class ActivatedMLP(FeedForward):
     params: ``hidden_size``, ``intermediate_size``, ``activation``.  tensors: ``up``, ``down`` and, for
     ``"xielu"``, ``act [2]``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -812,11 +824,8 @@ class ParallelBlock(Arrangement):
         return BranchSum(self._branches(a, b, ctx, cache)), stream
 
     def _branches(self, a, b, ctx, cache):
-        """Neither branch reads what the other writes."""
-        with beside() as side:
-            f = side.run(lambda: self.feed_forward.forward(b, ctx))
-            m = self.mixer.forward(a, ctx, cache, self.position)
-            return m, f()
+        return pair(ctx, self.mixer, lambda c: self.mixer.forward(a, c, cache, self.position),
+                    self.feed_forward, lambda c: self.feed_forward.forward(b, c), self.position)
 
 
 class BranchNormBlock(Arrangement):

@@ -37,6 +37,8 @@ class RoutedExperts(FeedForward):
     shared expert, ``shared.gate``, ``shared.up``, ``shared.down`` and, with its gate, ``shared.sg``.
     """
 
+    alone = True
+
     def __init__(self, spec):
         super().__init__(spec)
         g = self.spec.params.get

@@ -55,6 +55,8 @@ class LatentAttention(ProjectedMixer):
     asked, ``sink``, ``g``.
     """
 
+    alone = True
+
     def __init__(self, spec):
         super().__init__(spec)
         g = self.spec.params.get
@@ -233,6 +235,8 @@ class DistanceBiasAttention(ProjectedMixer):
     (default False), ``slope_span`` (default 8; None: no distance bias), ``sink`` (None, ``"learned"``, ``"zero"``).
     tensors: ``q``, ``k``, ``o``; as asked ``v``, ``q.b``, ``k.b``, ``q.norm``, ``k.norm``, ``sink``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)

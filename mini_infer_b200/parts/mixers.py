@@ -15,7 +15,6 @@ columns.
 
 from __future__ import annotations
 
-import copy
 import functools
 
 import torch
@@ -24,7 +23,7 @@ from ..csrc import ops
 from .base import KVNeed, LayerCache, Mixer, ParamDecl, PlanNeeds, StateNeed, StepContext, build_part, register_mixer
 from .builtin import InterleavedRotary, Linear, RotaryPosition, _as_compute
 from .spec import PartSpec
-from .streams import beside
+from .streams import pair
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -83,6 +82,8 @@ class GatedWindowAttention(ProjectedMixer):
     (default False) with ``eps``, ``gate`` (None or ``"sigmoid"`` / ``"silu"``).
     tensors: ``q``, ``k``, ``v``, ``o`` and, with a gate, ``g``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -207,6 +208,8 @@ class ChunkAttention(ProjectedMixer):
     tensors: ``q``, ``k``, ``v``, ``o`` and, as asked, ``q.norm``, ``k.norm``, ``vmix``, ``g``, ``q.b``, ``k.b``,
     ``v.b``, ``sink``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -361,6 +364,8 @@ class GatedLinearAttention(ProjectedMixer):
     tensors: ``q``, ``k``, ``v``, ``g``, ``o``, ``norm``, ``a1``, ``a2``, ``a2.b``.
     """
 
+    alone = True
+
     def __init__(self, spec):
         super().__init__(spec)
         self.hidden = int(self.param("hidden_size"))
@@ -425,6 +430,8 @@ class Retention(ProjectedMixer):
     params: ``hidden_size``, ``num_heads``, ``key_dim``, ``value_dim``, ``decay`` (one number per head), ``eps``.
     tensors: ``q``, ``k``, ``v``, ``g``, ``o``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -496,6 +503,8 @@ class ChannelDeltaRule(ProjectedMixer):
     tensors: ``q``, ``q.conv``, ``k``, ``k.conv``, ``v``, ``v.conv``, ``b``, ``A_log``, ``norm``, ``a1``, ``a2``,
     ``dt_bias``, ``g1``, ``g2``, ``o``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -592,6 +601,7 @@ class MatrixMemory(ProjectedMixer):
     tensors: ``q``, ``k``, ``v``, ``g``, ``o``, ``norm``, ``i``, ``i.b``, ``f``, ``f.b``.
     """
 
+    alone = True
     takes_position = False
 
     def __init__(self, spec):
@@ -657,6 +667,8 @@ class RealGatedLinearRecurrence(ProjectedMixer):
     params: ``hidden_size``, ``width``, ``blocks``, ``conv_taps``, optional ``decay_scale`` (default 8).
     tensors: ``y``, ``y.b``, ``x``, ``x.b``, ``conv``, ``conv.b``, ``ra``, ``ra.b``, ``ri``, ``ri.b``, ``lam``, ``o``.
     """
+
+    alone = True
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -734,6 +746,7 @@ class SideBySide(Mixer):
         if sum(c.cache_need() is not None for c in self.children) > 1 or \
                 sum(c.state_need() is not None for c in self.children) > 1:
             raise ValueError("side by side, at most one mixer may keep keys and values and one a state")
+        self.alone = all(c.alone for c in self.children)
 
     def param_decls(self):
         return {c.spec.prefix + local: decl for c in self.children for local, decl in c.param_decls().items()}
@@ -762,26 +775,22 @@ class SideBySide(Mixer):
         proj32 = self._in32(x, out_dtype=torch.float32) if self._in32 is not None else None
         out = torch.empty((ctx.n_tokens, sum(c.out_width for c in self.children)), dtype=x.dtype, device=x.device)
         i0 = o0 = p0 = 0
-        # Each has its own columns of both, and at most one keys and values and at most one a state; what the second one
-        # leaves for the layers behind it, in a dictionary of its own, is theirs when both are through.
-        second = copy.copy(ctx)
-        second.scratch = dict(ctx.scratch)
-        mixes = []
-        for c, scale, cx in zip(self.children, self.scales, (ctx, second)):
+        mixes = []      # each has its own columns of both, and at most one keys and values and at most one a state
+        for c, scale in zip(self.children, self.scales):
             kw = {}
             if c.in32_width:
                 kw["proj32"] = proj32[:, p0:p0 + c.in32_width]
                 p0 += c.in32_width
-            mixes.append(functools.partial(c.mix, proj[:, i0:i0 + c.in_width], out[:, o0:o0 + c.out_width], scale, cx, cache,
-                                           position if c.takes_position else None, **kw))
+            mixes.append(functools.partial(self._mix, c, proj[:, i0:i0 + c.in_width], out[:, o0:o0 + c.out_width], scale, cache,
+                                           position if c.takes_position else None, kw))
             i0 += c.in_width
             o0 += c.out_width
-        with beside() as side:
-            side.run(mixes[1])
-            mixes[0]()
-        for key, value in second.scratch.items():
-            ctx.scratch.setdefault(key, value)
+        pair(ctx, self.children[0], mixes[0], self.children[1], mixes[1], position)
         return self._out(out)
+
+    @staticmethod
+    def _mix(child, proj, out, scale, cache, position, kw, ctx):
+        child.mix(proj, out, scale, ctx, cache, position, **kw)
 
 
 register_mixer("gated_window_attention", GatedWindowAttention, replace=True)

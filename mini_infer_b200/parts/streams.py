@@ -3,7 +3,8 @@
 A step of a few tokens is a chain of short kernels, each of which leaves most of the chip idle at its ends.  Where a layer
 has two chains that only meet at an addition or an output projection (a mixer and a feed-forward that read the same stream,
 two mixers of one layer, a shared expert and the routed ones), the second one is recorded on a stream of its own, and the
-step's graph has two branches.  What a step computes does not depend on it, and neither do its kernels.
+step's graph has two branches.  What a step computes does not depend on it, and neither do its kernels.  Parts of a layer are
+recorded so only where they say that they may be (``Part.alone``).
 
 Replays of decode steps of 8 requests, us, one branch and two: Ruvurax 4096 wide 851 and 802 (its experts' weights alone take
 400 at the copy bandwidth), Lilulix 2048 wide 335 and 298; Ruvurax 2048 wide, one request, 277 and 210.  With the mixer's
@@ -13,6 +14,8 @@ with two branches 4.9 ms where one takes 4.0), and so nothing is allocated on on
 """
 
 from __future__ import annotations
+
+import copy
 
 import torch
 
@@ -77,3 +80,23 @@ class beside:
         finally:
             if self.on:
                 _open[self.key] -= 1
+
+
+def pair(ctx, part, run, other, run_other, position=None):
+    """``(run(ctx), run_other(ctx))`` of a layer's two parts (tensors or None), the second one beside the first in a captured step
+    where both, and the ``position`` part they may call, say that they can.  It then has a ``ctx.scratch`` of its own, as it was
+    in front of both; what it leaves there, and the first one does not, is the layers' behind them when both are through."""
+    parts = (part, other) if position is None else (part, other, position)
+    if not all(getattr(p, "alone", False) for p in parts):
+        return run(ctx), run_other(ctx)
+    with beside() as side:
+        if not side.on:
+            mine = run(ctx)
+            return mine, side.run(lambda: run_other(ctx))()
+        own = copy.copy(ctx)
+        own.scratch = dict(ctx.scratch)
+        theirs = side.run(lambda: run_other(own))
+        both = run(ctx), theirs()
+    for key, value in own.scratch.items():
+        ctx.scratch.setdefault(key, value)
+    return both
