@@ -157,6 +157,24 @@ def sums_kept() -> bool:
     return _sums_kept()
 
 
+_branches = threading.local()
+
+
+def open_branches() -> list:
+    """The blocks of two branches (``parts/streams.py``) that this thread is recording, outermost first."""
+    if not hasattr(_branches, "open"):
+        _branches.open = []
+    return _branches.open
+
+
+def _claim_workspace(name: str) -> None:
+    """Scratch that exists once per device is written by one branch of a captured step alone."""
+    for block in open_branches():
+        if block.workspaces.setdefault(name, block.second) != block.second:
+            raise KernelError(f"{name}: both branches of a captured layer use the device's one workspace; parts that do must "
+                              "name it in device_scratch, or not say that they stand alone")
+
+
 def _sig_elementwise(lib: ctypes.CDLL) -> None:
     lib.mi_embedding.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_add_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -819,6 +837,7 @@ def _decode_counters(device: torch.device, n: int) -> torch.Tensor:
 
 
 def attention_decode(q, q_stride, out, kcache, vcache, block_table, page_size, q_start, kv_len,
+    _claim_workspace("decode_attention")
                      n_requests, nq, nkv, head_dim, scale, window=0, n_splits=1, slice_chunks=None,
                      table_rows=None) -> None:
     """bfloat16 decode attention: one query token per request, keys cut into ``n_splits``
@@ -864,6 +883,7 @@ def _balanced_workspace(device: torch.device, o_floats: int, ml_floats: int, cou
                       torch.zeros(max(counters, 4096), dtype=torch.int32, device=device)))
     return stack[-1]
 
+    _claim_workspace("decode_attention")
 
 def attention_decode_balanced(q, q_stride, out, kcache, vcache, block_table, page_size, q_start, kv_len,
                               n_requests, nq, nkv, head_dim, scale, window=0, table_rows=None,
@@ -1095,6 +1115,7 @@ def _tma_workspace(device: torch.device, floats: int, counters: int) -> tuple[to
             torch.zeros(max(counters, 4096), dtype=torch.int32, device=device),
         ))
     return stack[-1]
+    _claim_workspace("gemm_tma")
 
 
 def gemm_tma_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
