@@ -4,7 +4,7 @@
 // multiple of 32, the last one shorter), each accumulated from its first k on with fused multiply-adds, whatever kernel and
 // tile it falls in, so a row's result does not depend on which other rows share the call.
 //
-//   gemm_f32_stream_kernel up to 4 rows of a wide result (decode): bound by one reading of W
+//   gemm_f32_stream_kernel up to 4 rows (decode): bound by one reading of W
 //   gemm_f32_rows_kernel   up to 32 rows
 //   gemm_f32_tile_kernel   more rows: bound by the fused multiply-adds
 //   gemm_f32_any_kernel    operands without 16-byte rows
@@ -45,8 +45,7 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 #define ST_THREADS (32 * (PARTS + 1))
 #define ST_BUDGET (200 * 1024)
 
-// LIMIT: polls of a copy's barrier before a warp gives up (0 in a test's instance).
-template <int RM, int LIMIT>
+template <int RM>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* __restrict__ C,
                        int M, int N, int K, int ldc, int cols, int n_tiles, int stages, int w_constant) {
@@ -107,18 +106,13 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   mi_pdl_wait();                                        // the kernels before may read C
   const int row = min(lane, cols - 1), sw = row & 7;
   int st = 0, round = 0;
-  // After a wait that ran out (ok) a warp computes no more but goes on waiting for every copy and handing its stage on, so that
-  // none is under way when the block leaves; a copy that does not come then either (there) ends that too.
-  bool ok = true, there = true;
+  bool ok = true;
   for (int tile = 0; tile < tiles; ++tile) {
     float acc[RM];
 #pragma unroll
     for (int i = 0; i < RM; ++i) acc[i] = 0.f;
     for (int kc = 0; kc < chunks; ++kc) {
-      if (there && !mbar_wait(&full[st], round & 1, gu, LIMIT)) {
-        ok = false;
-        there = mbar_drain(&full[st], round & 1);
-      }
+      if (ok && !mbar_wait(&full[st], round & 1, gu)) ok = false;
       if (ok) {
         const unsigned char* ws = smem + (size_t)st * stage_bytes + warp * part_bytes + row * 128;
         const unsigned char* as = smem + (size_t)st * stage_bytes + warp * part_bytes + w_box;
@@ -135,7 +129,7 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
       }
       __syncwarp();
-      if (lane == 0 && there) mbar_arrive(&empty[st]);
+      if (lane == 0) mbar_arrive(&empty[st]);
       if (++st == stages) { st = 0; ++round; }
     }
 #pragma unroll
@@ -163,7 +157,7 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #define RB_COLS 16
 #define RB_K 32
 #define RB_PITCH (RB_K + 4)      // floats per staged row: eight rows' 16-byte pieces touch every bank once
-// Rows and tiles, us: N x K = 3072 x 2048 with 1 row 11 and 40, 16 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
+// Rows and tiles, us: N x K = 3072 x 2048 with 16 rows 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
 // and 52, 32 29 and 53; 6144 x 2048 16 28 and 58, 17 49 and 57, 32 56 and 58; 32000 x 2048 8 81 and 121, 16 115 and 121, 17
 // 222 and 121, 32 256 and 123 (a block's 16 columns then come round fourteen times, each with all rows).
 #define RB_MAX_ROWS 32
@@ -437,7 +431,7 @@ static bool make_map_f32(CUtensorMap* map, const float* base, int rows, int cols
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int RM, int LIMIT = SPIN_LIMIT>
+template <int RM>
 static int launch_stream(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
                          int w_constant, int sms, cudaStream_t stream) {
   const int tiles = (N + ST_COLS * sms - 1) / (ST_COLS * sms), per = sms * tiles, cols = (N + per - 1) / per;
@@ -451,32 +445,17 @@ static int launch_stream(const float* A, const float* W, float* C, int M, int N,
   CUtensorMap map_w, map_a;
   if (!make_map_f32(&map_w, W, N, K, ldw, cols) || !make_map_f32(&map_a, A, M, K, lda, M))
     MI_REFUSE("gemm_f32: the driver refused a tensor map (M %d, N %d, K %d)", M, N, K);
-  auto kern = gemm_f32_stream_kernel<RM, LIMIT>;
+  auto kern = gemm_f32_stream_kernel<RM>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   MI_LAUNCH(kern, grid, ST_THREADS, smem, stream, map_w, map_a, C, M, N, K, ldc, cols, tiles, stages, w_constant);
   return 0;
 }
 
-// Which of the two kernels takes up to 4 rows, from their times in us, streaming kernel and kernel for few rows, weights out of memory.
-// A block per SM has few of its 32 lanes at work in narrow results, and three and four rows of A read from shared memory stand
-// longer beside one of W:
-//   rows, K       N = 256        1024         2048         4096         6144         8192         32000
-//   1, 2048     7.5   6.7    7.9   6.8    7.9   9.7    8.0  10.5   14.2  17.3   14.8  21.0   48.4  66.5
-//   2, 256      2.5   2.0    2.6   2.2    2.6   2.4    2.5   2.5    3.6   4.4    3.7   4.8    9.0  14.5
-//   2, 2048     9.0   6.7    9.4   6.8    9.4   9.7    9.4  10.5   14.7  17.6   15.3  21.4   49.7  66.7
-//   4, 1024     6.4   3.9    6.6   4.1    6.7   5.6    7.2   6.3   11.6  10.2   11.9  12.8   34.0  38.2
-//   4, 4096    18.2  12.1   18.6  13.2   18.6  17.4   19.1  19.0   34.4  30.4   34.8  37.4    110   121
-static bool takes_stream(int M, int N, int K) {
-  if (M <= 2) return N >= 2048 && (long long)N * K >= 1 << 20;
-  return M <= ST_MAX_ROWS && N >= 8192;
-}
-
-// w_constant: W is not written by any kernel that may still run (a loaded weight).  no_wait: the streaming kernel gives up
-// at its first copy, as after a wait that ran out; C is then not to be trusted, and the status word says so.
+// w_constant: W is not written by any kernel that may still run (a loaded weight).
 // Zero-padded tails of a part add exact zeros at the end of its sum, so they do not change it.
 extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
-                           int ldw, int ldc, int w_constant, int sms, int no_wait, cudaStream_t stream) {
+                           int ldw, int ldc, int w_constant, int sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (sms <= 0) MI_REFUSE("gemm_f32: bad number of SMs %d", sms);
   if (K <= 0) MI_REFUSE("gemm_f32: K must be positive, got %d", K);
@@ -487,15 +466,13 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
   if (!vec) {
     MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
               lda, ldw, ldc);
-  } else if (takes_stream(M, N, K)) {
-    const int rc = no_wait  ? launch_stream<ST_MAX_ROWS, 0>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
-                   : M == 1 ? launch_stream<1>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
+  } else if (M <= ST_MAX_ROWS) {
+    const int rc = M == 1   ? launch_stream<1>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
                    : M == 2 ? launch_stream<2>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
                             : launch_stream<4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream);
     if (rc) return rc;
   } else if (M <= 16 || (M <= RB_MAX_ROWS && N <= RB_MAX_COLS)) {
-    e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
-        : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+    e = M <= 8    ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
         : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
                   : launch_rows<8, 4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream);
   } else {

@@ -157,24 +157,6 @@ def sums_kept() -> bool:
     return _sums_kept()
 
 
-_branches = threading.local()
-
-
-def open_branches() -> list:
-    """The blocks of two branches (``parts/streams.py``) that this thread is recording, outermost first."""
-    if not hasattr(_branches, "open"):
-        _branches.open = []
-    return _branches.open
-
-
-def _claim_workspace(name: str) -> None:
-    """Scratch that exists once per device is written by one branch of a captured step alone."""
-    for block in open_branches():
-        if block.workspaces.setdefault(name, block.second) != block.second:
-            raise KernelError(f"{name}: both branches of a captured layer use the device's one workspace; parts that do must "
-                              "name it in device_scratch, or not say that they stand alone")
-
-
 def _sig_elementwise(lib: ctypes.CDLL) -> None:
     lib.mi_embedding.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_add_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -189,7 +171,7 @@ def _sig_elementwise(lib: ctypes.CDLL) -> None:
 
 def _sig_gemm_f32(lib: ctypes.CDLL) -> None:
     lib.mi_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                c_int, c_int, c_int, c_int, c_void_p]
+                                c_int, c_int, c_int, c_void_p]
     lib.mi_gemm_f32_status.argtypes = [c_int]
     lib.mi_set_status_word.argtypes = [c_void_p]
 
@@ -603,11 +585,9 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None, pairs: bool
     return out
 
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, w_constant: bool = False, *,
-             no_wait: bool = False) -> torch.Tensor:
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, w_constant: bool = False) -> torch.Tensor:
     """``a [M, K] @ w [N, K]^T`` in true fp32 (CUDA cores, fixed summation order).  With ``w_constant`` the kernel may read
-    ``w`` while kernels before it still run: for weights, never for what such a kernel writes.  ``no_wait``: the
-    kernel for few rows and wide results behaves as if its first wait ran out (it sets the status word; for tests)."""
+    ``w`` while kernels before it still run: for weights, never for what such a kernel writes."""
     _cuda(a, w, out)
     if a.dtype != torch.float32 or w.dtype != torch.float32:
         raise KernelError("gemm_f32: operands must be float32")
@@ -624,15 +604,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, 
     lib = _waiting_lib("gemm_f32", a.device)
     rc = lib.mi_gemm_f32(_ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0) if M > 1 else K,
                          w.stride(0) if N > 1 else K, out.stride(0) if M > 1 else N, 1 if w_constant else 0,
-                         _sms(a.device), 1 if no_wait else 0, _stream())
+                         _sms(a.device), _stream())
     _finish(lib, rc, "gemm_f32")
     return out
-
-
-def gemm_f32_status(reset: bool = True) -> int:
-    """1 when a block of the float32 product gave up a bounded wait since the last reset (its output is then wrong).
-    Synchronises the device."""
-    return int(_lib("gemm_f32").mi_gemm_f32_status(1 if reset else 0))
 
 
 def cache_swizzle_mask(head_dim: int, dtype: torch.dtype) -> int:
@@ -837,7 +811,6 @@ _decode_counter_bufs: dict[int, list[torch.Tensor]] = {}
 
 
 def _decode_counters(device: torch.device, n: int) -> torch.Tensor:
-    _claim_workspace("decode_attention")
     idx = device.index if device.index is not None else torch.cuda.current_device()
     stack = _decode_counter_bufs.setdefault(idx, [])
     if not stack or stack[-1].numel() < n:
@@ -883,7 +856,6 @@ _balanced_ws: dict[int, list[tuple[torch.Tensor, torch.Tensor, torch.Tensor]]] =
 
 
 def _balanced_workspace(device: torch.device, o_floats: int, ml_floats: int, counters: int):
-    _claim_workspace("decode_attention")
     idx = _device_index(device)
     stack = _balanced_ws.setdefault(idx, [])
     if not stack or stack[-1][0].numel() < o_floats or stack[-1][1].numel() < ml_floats or stack[-1][2].numel() < counters:
@@ -1115,7 +1087,6 @@ _tma_ws: dict[int, list[tuple[torch.Tensor, torch.Tensor]]] = {}
 def _tma_workspace(device: torch.device, floats: int, counters: int) -> tuple[torch.Tensor, torch.Tensor]:
     """Partial tiles and per-tile arrival counters (zero between calls) of the streaming
     product, per device; never freed once handed out (a captured graph may hold the address)."""
-    _claim_workspace("gemm_tma")
     idx = device.index if device.index is not None else torch.cuda.current_device()
     stack = _tma_ws.setdefault(idx, [])
     if not stack or stack[-1][0].numel() < floats or stack[-1][1].numel() < counters:

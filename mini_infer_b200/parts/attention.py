@@ -85,7 +85,6 @@ class ConvAttention(PagedSoftmax):
     """
 
     alone = True
-    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -153,7 +152,6 @@ class DifferentialAttention(PagedSoftmax):
     """
 
     alone = True
-    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)

@@ -56,7 +56,6 @@ class LatentAttention(ProjectedMixer):
     """
 
     alone = True
-    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -238,7 +237,6 @@ class DistanceBiasAttention(ProjectedMixer):
     """
 
     alone = True
-    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
