@@ -157,6 +157,24 @@ def sums_kept() -> bool:
     return _sums_kept()
 
 
+_branches = threading.local()
+
+
+def open_branches() -> list:
+    """The blocks of two branches (``parts/streams.py``) that this thread is recording, outermost first."""
+    if not hasattr(_branches, "open"):
+        _branches.open = []
+    return _branches.open
+
+
+def _claim_workspace(name: str) -> None:
+    """Scratch that exists once per device is written by one branch of a captured step alone."""
+    for block in open_branches():
+        if block.workspaces.setdefault(name, block.second) != block.second:
+            raise KernelError(f"{name}: both branches of a captured layer use the device's one workspace; parts that do must "
+                              "name it in device_scratch, or not say that they stand alone")
+
+
 def _sig_elementwise(lib: ctypes.CDLL) -> None:
     lib.mi_embedding.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_add_rmsnorm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -811,6 +829,7 @@ _decode_counter_bufs: dict[int, list[torch.Tensor]] = {}
 
 
 def _decode_counters(device: torch.device, n: int) -> torch.Tensor:
+    _claim_workspace("decode_attention")
     idx = device.index if device.index is not None else torch.cuda.current_device()
     stack = _decode_counter_bufs.setdefault(idx, [])
     if not stack or stack[-1].numel() < n:
@@ -856,6 +875,7 @@ _balanced_ws: dict[int, list[tuple[torch.Tensor, torch.Tensor, torch.Tensor]]] =
 
 
 def _balanced_workspace(device: torch.device, o_floats: int, ml_floats: int, counters: int):
+    _claim_workspace("decode_attention")
     idx = _device_index(device)
     stack = _balanced_ws.setdefault(idx, [])
     if not stack or stack[-1][0].numel() < o_floats or stack[-1][1].numel() < ml_floats or stack[-1][2].numel() < counters:
@@ -1087,6 +1107,7 @@ _tma_ws: dict[int, list[tuple[torch.Tensor, torch.Tensor]]] = {}
 def _tma_workspace(device: torch.device, floats: int, counters: int) -> tuple[torch.Tensor, torch.Tensor]:
     """Partial tiles and per-tile arrival counters (zero between calls) of the streaming
     product, per device; never freed once handed out (a captured graph may hold the address)."""
+    _claim_workspace("gemm_tma")
     idx = device.index if device.index is not None else torch.cuda.current_device()
     stack = _tma_ws.setdefault(idx, [])
     if not stack or stack[-1][0].numel() < floats or stack[-1][1].numel() < counters:

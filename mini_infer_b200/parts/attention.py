@@ -85,6 +85,7 @@ class ConvAttention(PagedSoftmax):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -152,6 +153,7 @@ class DifferentialAttention(PagedSoftmax):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)

@@ -181,6 +181,9 @@ class Part:
     # other reads.  What both need from the dictionary each then fills for itself.  Parts that do not say so run one after the
     # other, the mixer first (of two mixers the left one).  A class says it for itself: one derived from it says it again.
     alone: bool = False
+    # the scratch memory that ``ops`` keeps one of per device and that ``forward`` may use ("decode_attention", "gemm_tma"): two
+    # parts with one of these in common run one after the other too
+    device_scratch: frozenset[str] = frozenset()
 
     def __init_subclass__(cls, **kwargs) -> None:
         super().__init_subclass__(**kwargs)

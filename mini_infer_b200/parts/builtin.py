@@ -499,6 +499,7 @@ class GroupedQueryAttention(Mixer):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)

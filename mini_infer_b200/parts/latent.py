@@ -56,6 +56,7 @@ class LatentAttention(ProjectedMixer):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -237,6 +238,7 @@ class DistanceBiasAttention(ProjectedMixer):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)

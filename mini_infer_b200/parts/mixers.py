@@ -84,6 +84,7 @@ class GatedWindowAttention(ProjectedMixer):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -210,6 +211,7 @@ class ChunkAttention(ProjectedMixer):
     """
 
     alone = True
+    device_scratch = frozenset({"decode_attention"})
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -747,6 +749,7 @@ class SideBySide(Mixer):
                 sum(c.state_need() is not None for c in self.children) > 1:
             raise ValueError("side by side, at most one mixer may keep keys and values and one a state")
         self.alone = all(c.alone for c in self.children)
+        self.device_scratch = frozenset().union(*(c.device_scratch for c in self.children))
 
     def param_decls(self):
         return {c.spec.prefix + local: decl for c in self.children for local, decl in c.param_decls().items()}

@@ -34,7 +34,8 @@ class beside:
     what the other writes.
 
     The caller keeps every tensor that ``f`` reads alive until the block's end.  Only a captured step has the second
-    stream, and under ``ops.kept_sums`` not even that: ``gemm_tma``, which runs the products there, has one workspace per device."""
+    stream, and under ``ops.kept_sums`` not even that: ``gemm_tma``, which runs the products there, has one workspace per device
+    (``ops`` raises where both sides of a block ask for such a workspace)."""
 
     def __init__(self) -> None:
         self.joined = True
@@ -51,6 +52,8 @@ class beside:
                 streams.append(torch.cuda.Stream(self.here.device))
             self.stream = streams[depth]
             _open[self.key] = depth + 1
+            ops.open_branches().append(self)
+            self.second, self.workspaces = False, {}
         return self
 
     def run(self, f):
@@ -59,8 +62,12 @@ class beside:
             return lambda: value
         self.stream.wait_stream(self.here)
         self.joined = False
-        with torch.cuda.stream(self.stream):
-            value = f()
+        self.second = True
+        try:
+            with torch.cuda.stream(self.stream):
+                value = f()
+        finally:
+            self.second = False
 
         def result():
             self._join()
@@ -80,6 +87,7 @@ class beside:
         finally:
             if self.on:
                 _open[self.key] -= 1
+                ops.open_branches().remove(self)
 
 
 def pair(ctx, part, run, other, run_other, position=None):
@@ -87,7 +95,7 @@ def pair(ctx, part, run, other, run_other, position=None):
     where both, and the ``position`` part they may call, say that they can.  It then has a ``ctx.scratch`` of its own, as it was
     in front of both; what it leaves there, and the first one does not, is the layers' behind them when both are through."""
     parts = (part, other) if position is None else (part, other, position)
-    if not all(getattr(p, "alone", False) for p in parts):
+    if not all(getattr(p, "alone", False) for p in parts) or part.device_scratch & other.device_scratch:
         return run(ctx), run_other(ctx)
     with beside() as side:
         if not side.on:

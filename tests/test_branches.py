@@ -1,11 +1,12 @@
-"""A layer's two parts in order or side by side (``parts/streams.py``), on the host: who runs first and what each finds in the
-step's shared dictionary."""
+"""A layer's two parts in order or side by side (``parts/streams.py``), on the host: who runs first, what each finds in the
+step's shared dictionary, and which scratch memory both may ask for."""
 
 from types import SimpleNamespace
 
 import pytest
 import torch
 
+from mini_infer_b200.csrc import ops
 from mini_infer_b200.parts import streams
 from mini_infer_b200.parts.base import FeedForward, Mixer
 from mini_infer_b200.parts.builtin import ParallelBlock, SameNorm
@@ -135,8 +136,14 @@ class AloneProjected(ToyProjected):
     alone = True
 
 
+class AttendingProjected(ToyProjected):
+    alone = True
+    device_scratch = frozenset({"decode_attention"})
+
+
 @pytest.mark.parametrize("kinds,apart", [((ToyProjected, ToyProjected), False), ((AloneProjected, ToyProjected), False),
-                                         ((AloneProjected, AloneProjected), True)])
+                                         ((AloneProjected, AttendingProjected), True),
+                                         ((AttendingProjected, AttendingProjected), False)])
 @pytest.mark.parametrize("recorded", [False, True])
 def test_two_mixers_of_a_layer(kinds, apart, recorded, monkeypatch):
     if recorded:
@@ -154,6 +161,26 @@ def test_two_mixers_of_a_layer(kinds, apart, recorded, monkeypatch):
         assert ToyProjected.saw[0][0] == "left"
 
 
+def test_one_workspace_per_device_is_one_branchs_alone(monkeypatch):
+    Recording(monkeypatch)
+    with streams.beside() as side:
+        ops._claim_workspace("a")
+        side.run(lambda: ops._claim_workspace("b"))
+        ops._claim_workspace("a")
+        with pytest.raises(ops.KernelError, match="a: both branches"):
+            side.run(lambda: ops._claim_workspace("a"))
+        with pytest.raises(ops.KernelError, match="b: both branches"):
+            ops._claim_workspace("b")
+        with streams.beside() as inner:       # an inner block's branches are one branch of the outer block
+            inner.run(lambda: ops._claim_workspace("c"))
+        ops._claim_workspace("c")
+        with pytest.raises(ops.KernelError, match="c: both branches"):
+            side.run(lambda: ops._claim_workspace("c"))
+    assert not ops.open_branches()
+    ops._claim_workspace("a")
+    ops._claim_workspace("b")
+
+
 def test_a_block_whose_join_fails_is_closed(monkeypatch):
     rec = Recording(monkeypatch)
     here = rec.now[-1]
@@ -166,5 +193,5 @@ def test_a_block_whose_join_fails_is_closed(monkeypatch):
                     raise RuntimeError("capture")
                 here.wait_stream = fail
         del here.wait_stream
-        assert not any(streams._open.values())
+        assert not any(streams._open.values()) and not ops.open_branches()
     assert len(streams._beside[(0, here.cuda_stream)]) == 1

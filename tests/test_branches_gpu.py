@@ -46,3 +46,20 @@ def test_two_branches_give_the_bits_of_one_chain(model, which, dtype):
         streams.beside.run = real
     assert torch.isfinite(rows[True]).all()
     assert torch.equal(rows[True], rows[False])
+
+
+def test_both_branches_asking_for_one_workspace_is_an_error():
+    """Found while the step is recorded: nothing runs."""
+    from mini_infer_b200.csrc import ops
+    from mini_infer_b200.parts import streams
+
+    x, w = (torch.randn(*s, device="cuda", dtype=torch.bfloat16) for s in ((4, 128), (256, 128)))
+    want = ops.gemm_tma(x, w).clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with pytest.raises(ops.KernelError, match="both branches"):
+        with torch.cuda.graph(graph):
+            with streams.beside() as side:
+                side.run(lambda: ops.gemm_tma(x, w))
+                ops.gemm_tma(x, w)
+    assert not ops.open_branches() and torch.equal(ops.gemm_tma(x, w), want)
