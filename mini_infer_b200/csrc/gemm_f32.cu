@@ -4,7 +4,7 @@
 // multiple of 32, the last one shorter), each accumulated from its first k on with fused multiply-adds, whatever kernel and
 // tile it falls in, so a row's result does not depend on which other rows share the call.
 //
-//   gemm_f32_stream_kernel up to 4 rows (decode): bound by one reading of W
+//   gemm_f32_stream_kernel up to 4 rows of a wide result (decode): bound by one reading of W
 //   gemm_f32_rows_kernel   up to 32 rows
 //   gemm_f32_tile_kernel   more rows: bound by the fused multiply-adds
 //   gemm_f32_any_kernel    operands without 16-byte rows
@@ -157,7 +157,7 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #define RB_COLS 16
 #define RB_K 32
 #define RB_PITCH (RB_K + 4)      // floats per staged row: eight rows' 16-byte pieces touch every bank once
-// Rows and tiles, us: N x K = 3072 x 2048 with 16 rows 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
+// Rows and tiles, us: N x K = 3072 x 2048 with 1 row 11 and 40, 16 18 and 36, 17 33 and 37, 32 38 and 37; 2048 x 3072 16 rows 25
 // and 52, 32 29 and 53; 6144 x 2048 16 28 and 58, 17 49 and 57, 32 56 and 58; 32000 x 2048 8 81 and 121, 16 115 and 121, 17
 // 222 and 121, 32 256 and 123 (a block's 16 columns then come round fourteen times, each with all rows).
 #define RB_MAX_ROWS 32
@@ -452,6 +452,20 @@ static int launch_stream(const float* A, const float* W, float* C, int M, int N,
   return 0;
 }
 
+// Which of the two kernels takes up to 4 rows, from their times in us, streaming kernel and kernel for few rows, weights out of memory.
+// A block per SM has few of its 32 lanes at work in narrow results, and three and four rows of A read from shared memory stand
+// longer beside one of W:
+//   rows, K       N = 256        1024         2048         4096         6144         8192         32000
+//   1, 2048     7.5   6.7    7.9   6.8    7.9   9.7    8.0  10.5   14.2  17.3   14.8  21.0   48.4  66.5
+//   2, 256      2.5   2.0    2.6   2.2    2.6   2.4    2.5   2.5    3.6   4.4    3.7   4.8    9.0  14.5
+//   2, 2048     9.0   6.7    9.4   6.8    9.4   9.7    9.4  10.5   14.7  17.6   15.3  21.4   49.7  66.7
+//   4, 1024     6.4   3.9    6.6   4.1    6.7   5.6    7.2   6.3   11.6  10.2   11.9  12.8   34.0  38.2
+//   4, 4096    18.2  12.1   18.6  13.2   18.6  17.4   19.1  19.0   34.4  30.4   34.8  37.4    110   121
+static bool takes_stream(int M, int N, int K) {
+  if (M <= 2) return N >= 2048 && (long long)N * K >= 1 << 20;
+  return M <= ST_MAX_ROWS && N >= 8192;
+}
+
 // w_constant: W is not written by any kernel that may still run (a loaded weight).
 // Zero-padded tails of a part add exact zeros at the end of its sum, so they do not change it.
 extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
@@ -466,13 +480,14 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
   if (!vec) {
     MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
               lda, ldw, ldc);
-  } else if (M <= ST_MAX_ROWS) {
+  } else if (takes_stream(M, N, K)) {
     const int rc = M == 1   ? launch_stream<1>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
                    : M == 2 ? launch_stream<2>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
                             : launch_stream<4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream);
     if (rc) return rc;
   } else if (M <= 16 || (M <= RB_MAX_ROWS && N <= RB_MAX_COLS)) {
-    e = M <= 8    ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+    e = M <= 4    ? launch_rows<1, 8>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
+        : M <= 8  ? launch_rows<2, 6>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
         : M <= 16 ? launch_rows<4, 5>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream)
                   : launch_rows<8, 4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, stream);
   } else {

@@ -222,6 +222,15 @@ def test_gemm_f32_of_up_to_4_rows_in_tiles_of_columns(N, K):
     assert torch.equal(wide[:, :N], full[37:]) and torch.isnan(wide[:, N:]).all()
 
 
+@pytest.mark.parametrize("N,K", [(2047, 516), (2048, 508), (2048, 512), (2052, 2048), (8188, 64), (8191, 132), (8192, 132), (8193, 128)])
+def test_gemm_f32_of_up_to_4_rows_on_either_side_of_the_limits(N, K):
+    """Narrow results go to the kernel for few rows, wide ones to the streaming kernel: the bits of the tiles of 40 rows."""
+    a, w = rnd(40, K, seed=23).to(DEV), rnd(N, K, seed=24).to(DEV)
+    full = ops().gemm_f32(a, w)
+    for M in (1, 2, 3, 4, 5):
+        assert torch.equal(ops().gemm_f32(a[:M], w, w_constant=M % 2 == 1), full[:M]), M
+
+
 @pytest.mark.parametrize("N", [8192, 8193, 8224])
 def test_gemm_f32_of_17_to_32_rows_on_either_side_of_the_widths_limit(N):
     """The kernel for few rows up to 8192 columns, tiles above: the same bits."""
