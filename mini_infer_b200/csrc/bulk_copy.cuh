@@ -36,14 +36,26 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* give_up) {
-  for (int it = 0; it < SPIN_LIMIT; ++it) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* give_up, int limit = SPIN_LIMIT) {
+  for (int it = 0; it < limit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 1023) == 1023 && *give_up) return false;   // another role of this block gave up
   }
   report_give_up();
   *give_up = 1;
   return false;
+}
+
+// After a wait that ran out: whether the copy lands all the same within some ms.
+__device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity) {
+  uint32_t landed = 0;
+  for (int it = 0; it < (1 << 18) && !landed; ++it)
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(landed)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  return landed != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {

@@ -45,7 +45,8 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 #define ST_THREADS (32 * (PARTS + 1))
 #define ST_BUDGET (200 * 1024)
 
-template <int RM>
+// LIMIT: polls of a copy's barrier before a warp gives up (0 in a test's instance).
+template <int RM, int LIMIT>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* __restrict__ C,
                        int M, int N, int K, int ldc, int cols, int n_tiles, int stages, int w_constant) {
@@ -106,13 +107,18 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   mi_pdl_wait();                                        // the kernels before may read C
   const int row = min(lane, cols - 1), sw = row & 7;
   int st = 0, round = 0;
-  bool ok = true;
+  // After a wait that ran out (ok) a warp computes no more but goes on waiting for every copy and handing its stage on, so that
+  // none is under way when the block leaves; a copy that does not come then either (there) ends that too.
+  bool ok = true, there = true;
   for (int tile = 0; tile < tiles; ++tile) {
     float acc[RM];
 #pragma unroll
     for (int i = 0; i < RM; ++i) acc[i] = 0.f;
     for (int kc = 0; kc < chunks; ++kc) {
-      if (ok && !mbar_wait(&full[st], round & 1, gu)) ok = false;
+      if (there && !mbar_wait(&full[st], round & 1, gu, LIMIT)) {
+        ok = false;
+        there = mbar_drain(&full[st], round & 1);
+      }
       if (ok) {
         const unsigned char* ws = smem + (size_t)st * stage_bytes + warp * part_bytes + row * 128;
         const unsigned char* as = smem + (size_t)st * stage_bytes + warp * part_bytes + w_box;
@@ -129,7 +135,7 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[st]);
+      if (lane == 0 && there) mbar_arrive(&empty[st]);
       if (++st == stages) { st = 0; ++round; }
     }
 #pragma unroll
@@ -431,7 +437,7 @@ static bool make_map_f32(CUtensorMap* map, const float* base, int rows, int cols
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int RM>
+template <int RM, int LIMIT = SPIN_LIMIT>
 static int launch_stream(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
                          int w_constant, int sms, cudaStream_t stream) {
   const int tiles = (N + ST_COLS * sms - 1) / (ST_COLS * sms), per = sms * tiles, cols = (N + per - 1) / per;
@@ -445,7 +451,7 @@ static int launch_stream(const float* A, const float* W, float* C, int M, int N,
   CUtensorMap map_w, map_a;
   if (!make_map_f32(&map_w, W, N, K, ldw, cols) || !make_map_f32(&map_a, A, M, K, lda, M))
     MI_REFUSE("gemm_f32: the driver refused a tensor map (M %d, N %d, K %d)", M, N, K);
-  auto kern = gemm_f32_stream_kernel<RM>;
+  auto kern = gemm_f32_stream_kernel<RM, LIMIT>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   MI_LAUNCH(kern, grid, ST_THREADS, smem, stream, map_w, map_a, C, M, N, K, ldc, cols, tiles, stages, w_constant);
@@ -466,10 +472,11 @@ static bool takes_stream(int M, int N, int K) {
   return M <= ST_MAX_ROWS && N >= 8192;
 }
 
-// w_constant: W is not written by any kernel that may still run (a loaded weight).
+// w_constant: W is not written by any kernel that may still run (a loaded weight).  no_wait: the streaming kernel gives up
+// at its first copy, as after a wait that ran out; C is then not to be trusted, and the status word says so.
 // Zero-padded tails of a part add exact zeros at the end of its sum, so they do not change it.
 extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda,
-                           int ldw, int ldc, int w_constant, int sms, cudaStream_t stream) {
+                           int ldw, int ldc, int w_constant, int sms, int no_wait, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (sms <= 0) MI_REFUSE("gemm_f32: bad number of SMs %d", sms);
   if (K <= 0) MI_REFUSE("gemm_f32: K must be positive, got %d", K);
@@ -481,7 +488,8 @@ extern "C" int mi_gemm_f32(const float* A, const float* W, float* C, int M, int 
     MI_LAUNCH((gemm_f32_any_kernel), dim3((N + AB_T - 1) / AB_T, (M + AB_T - 1) / AB_T), 256, 0, stream, A, W, C, M, N, K,
               lda, ldw, ldc);
   } else if (takes_stream(M, N, K)) {
-    const int rc = M == 1   ? launch_stream<1>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
+    const int rc = no_wait  ? launch_stream<ST_MAX_ROWS, 0>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
+                   : M == 1 ? launch_stream<1>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
                    : M == 2 ? launch_stream<2>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream)
                             : launch_stream<4>(A, W, C, M, N, K, lda, ldw, ldc, w_constant, sms, stream);
     if (rc) return rc;

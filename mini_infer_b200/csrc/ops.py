@@ -189,7 +189,7 @@ def _sig_elementwise(lib: ctypes.CDLL) -> None:
 
 def _sig_gemm_f32(lib: ctypes.CDLL) -> None:
     lib.mi_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                c_int, c_int, c_int, c_void_p]
+                                c_int, c_int, c_int, c_int, c_void_p]
     lib.mi_gemm_f32_status.argtypes = [c_int]
     lib.mi_set_status_word.argtypes = [c_void_p]
 
@@ -603,9 +603,11 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor | None = None, pairs: bool
     return out
 
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, w_constant: bool = False) -> torch.Tensor:
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, w_constant: bool = False, *,
+             no_wait: bool = False) -> torch.Tensor:
     """``a [M, K] @ w [N, K]^T`` in true fp32 (CUDA cores, fixed summation order).  With ``w_constant`` the kernel may read
-    ``w`` while kernels before it still run: for weights, never for what such a kernel writes."""
+    ``w`` while kernels before it still run: for weights, never for what such a kernel writes.  ``no_wait``: the
+    kernel for few rows and wide results behaves as if its first wait ran out (it sets the status word; for tests)."""
     _cuda(a, w, out)
     if a.dtype != torch.float32 or w.dtype != torch.float32:
         raise KernelError("gemm_f32: operands must be float32")
@@ -622,9 +624,15 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, 
     lib = _waiting_lib("gemm_f32", a.device)
     rc = lib.mi_gemm_f32(_ptr(a), _ptr(w), _ptr(out), M, N, K, a.stride(0) if M > 1 else K,
                          w.stride(0) if N > 1 else K, out.stride(0) if M > 1 else N, 1 if w_constant else 0,
-                         _sms(a.device), _stream())
+                         _sms(a.device), 1 if no_wait else 0, _stream())
     _finish(lib, rc, "gemm_f32")
     return out
+
+
+def gemm_f32_status(reset: bool = True) -> int:
+    """1 when a block of the float32 product gave up a bounded wait since the last reset (its output is then wrong).
+    Synchronises the device."""
+    return int(_lib("gemm_f32").mi_gemm_f32_status(1 if reset else 0))
 
 
 def cache_swizzle_mask(head_dim: int, dtype: torch.dtype) -> int:

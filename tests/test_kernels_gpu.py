@@ -231,6 +231,20 @@ def test_gemm_f32_of_up_to_4_rows_on_either_side_of_the_limits(N, K):
         assert torch.equal(ops().gemm_f32(a[:M], w, w_constant=M % 2 == 1), full[:M]), M
 
 
+def test_gemm_f32_whose_wait_runs_out_reports_it_and_the_next_one_is_right():
+    """Every block gives up at its first copy, leaves with none under way, and sets the status word."""
+    a, w = rnd(2, 2048, seed=25).to(DEV), rnd(9500, 2048, seed=26).to(DEV)
+    want = ops().gemm_f32(a, w)
+    word = ops().status_word(torch.device(DEV))
+    assert ops().gemm_f32_status() == 0 and int(word) == 0
+    for M in (1, 2):
+        ops().gemm_f32(a[:M], w, no_wait=True)
+        assert int(word) == 1
+        ops().recover_from_wait_failure(torch.device(DEV))
+        assert ops().gemm_f32_status() == 0
+        assert torch.equal(ops().gemm_f32(a[:M], w), want[:M]) and int(word) == 0
+
+
 @pytest.mark.parametrize("N", [8192, 8193, 8224])
 def test_gemm_f32_of_17_to_32_rows_on_either_side_of_the_widths_limit(N):
     """The kernel for few rows up to 8192 columns, tiles above: the same bits."""
