@@ -351,14 +351,14 @@ __device__ __forceinline__ void decode_merge_when_last(const float* __restrict__
 
 template <int DMAX>
 __global__ void __launch_bounds__(DEC_THREADS)
-attention_decode_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out, int out_stride,
-                        const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
+attention_decode_kernel(const bf16* q, int q_stride, bf16* out, int out_stride,
+                        const bf16* kcache, const bf16* vcache,
                         const int* __restrict__ block_table, int bt_stride, const int* __restrict__ table_rows,
                         int page_size, int page_shift,
                         const int* __restrict__ q_start, const int* __restrict__ kv_len, int nq, int nkv,
                         int d, float scale, int window, int n_splits, const int* __restrict__ slice_chunks,
-                        float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters,
-                        int* __restrict__ status) {
+                        float* part_o, float* part_ml, int* counters,
+                        int* status) {
   // The next kernel's blocks may be scheduled.  This kernel reads the batch description and
   // the keys and values of earlier positions before it waits for the kernels ahead of it: the
   // description was uploaded before the step's first kernel, and the step's own kernels write
@@ -752,14 +752,14 @@ __device__ __noinline__ void balanced_merge_unit(const float* __restrict__ part_
 // DMAX, known to the compiler: the loops over it lose their conditions, of which a chunk's instructions were a good part.
 template <int DMAX, bool ROPE, bool EXT, bool EXACT>
 __global__ void __launch_bounds__(ROPE ? BAL_THREADS : DEC_THREADS, DMAX <= 128 ? 2 : 1)
-attention_decode_balanced_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restrict__ out, int out_stride,
-                                 const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
+attention_decode_balanced_kernel(const bf16* q, int q_stride, bf16* out, int out_stride,
+                                 const bf16* kcache, const bf16* vcache,
                                  const int* __restrict__ block_table, int bt_stride,
                                  const int* __restrict__ table_rows, int page_size, int page_shift,
                                  const int* __restrict__ q_start, const int* __restrict__ kv_len, int B, int nq,
                                  int nkv, int d_any, float scale, int window, int min_chunks, int unit_cost,
-                                 float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters,
-                                 int* __restrict__ status, const float* __restrict__ rope_cs, int store_kv,
+                                 float* part_o, float* part_ml, int* counters,
+                                 int* status, const float* rope_cs, int store_kv,
                                  const float* __restrict__ sinks, int keep_any, float cap_k, float cap_h,
                                  const float* __restrict__ slopes) {
   const int keep = EXT ? keep_any : 0;

@@ -47,7 +47,9 @@ typedef __nv_bfloat16 bf16;
 // the launch latency and lets a kernel do work that does not depend on its predecessors (set
 // up barriers, stream weights into shared memory) ahead of time.  The contract: a kernel calls
 // mi_pdl_wait() before it reads or writes anything that an earlier kernel may write or read;
-// before that it touches only immutable data (weights) and its own shared or tensor memory.
+// before that it touches only immutable data (weights that the caller calls constant, the step's plan) and its own shared or
+// tensor memory.  A kernel that does such work marks only that data `__restrict__`: through a pointer marked so the compiler may
+// move a load over the wait, and an operand that an earlier kernel writes would be read before it is there.
 // mi_pdl_launch_dependents() lets the next kernel's blocks be scheduled; it is called first
 // thing, so the look-ahead is limited only by what fits on the SMs.  Kernels launched by
 // other libraries take part as ordinary stream work: they start after everything before them

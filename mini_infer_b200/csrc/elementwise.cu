@@ -66,8 +66,8 @@ extern "C" int mi_embedding(const void* table, const int* ids, void* out, int M,
 // dependents start only when its writes are done and visible, not at its beginning as the
 // other kernels do.
 // ---------------------------------------------------------------------------
-__global__ void table_update_kernel(int* __restrict__ table, int stride, int rows,
-                                    const int* __restrict__ updates, const int* __restrict__ count,
+__global__ void table_update_kernel(int* table, int stride, int rows,
+                                    const int* updates, const int* count,
                                     int capacity) {
   mi_pdl_wait();
   const int n = min(*count, capacity);

@@ -48,7 +48,7 @@ __device__ __forceinline__ void part_barrier(int part) { asm volatile("bar.sync 
 // LIMIT: polls of a copy's barrier before a warp gives up (0 in a test's instance).
 template <int RM, int LIMIT>
 __global__ void __launch_bounds__(ST_THREADS, 1)
-gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* __restrict__ C,
+gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* C,
                        int M, int N, int K, int ldc, int cols, int n_tiles, int stages, int w_constant) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -170,8 +170,8 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #define RB_MAX_COLS 8192          // above 16 rows
 
 template <int RM, int STAGES>
-__global__ void __launch_bounds__(64 * PARTS) gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                                   float* __restrict__ C, int M, int N, int K, int lda,
+__global__ void __launch_bounds__(64 * PARTS) gemm_f32_rows_kernel(const float* A, const float* __restrict__ W,
+                                                                   float* C, int M, int N, int K, int lda,
                                                                    int ldw, int ldc, int w_constant) {
   extern __shared__ __align__(16) float rsm[];
   constexpr int ROWS = 4 * RM;

@@ -150,8 +150,8 @@ struct EpilogueFusion {
 template <typename OutT, bool kFused, int kAct>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                OutT* __restrict__ y, int ldy, int M, int N, int K, int n_tok, int stages, int kb, int chunked, int swiglu,
-                float* __restrict__ partials, int* __restrict__ counters, const EpilogueFusion fus, int w_evict_first) {
+                OutT* y, int ldy, int M, int N, int K, int n_tok, int stages, int kb, int chunked, int swiglu,
+                float* partials, int* counters, const EpilogueFusion fus, int w_evict_first) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // stage s: kb W boxes [128][64] bf16 (16 KB each), then kb x boxes [n_tok][64] bf16
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -525,7 +525,7 @@ __device__ __forceinline__ void gr_ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) 
 template <typename OutT, int NT, bool kFused, int kAct>
 __global__ void __launch_bounds__(GR_THREADS, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                 OutT* __restrict__ y, int ldy, int M, int N, int K, int tile_rows, int n_row_tiles, int stages, int kb,
+                 OutT* y, int ldy, int M, int N, int K, int tile_rows, int n_row_tiles, int stages, int kb,
                  int chunked, int swiglu, const EpilogueFusion fus, int w_evict_first) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);

@@ -32,9 +32,9 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
 
 // grid = (heads, blocks of Q_ROWS rows of W, then one more for the rotation)
 __global__ void __launch_bounds__(128)
-latent_query_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restrict__ uk_t, int M, int n, int d, int rank,
+latent_query_kernel(const bf16* q, int q_stride, const bf16* __restrict__ uk_t, int M, int n, int d, int rank,
                     int rd, int rot, int interleaved, const int* __restrict__ positions,
-                    const double* __restrict__ freq, bf16* __restrict__ qfull) {
+                    const double* __restrict__ freq, bf16* qfull) {
   mi_pdl_launch_dependents();
   __shared__ __align__(16) float qs[Q_MAX_TOKENS][Q_MAX_D];
   const int h = blockIdx.x, tid = threadIdx.x, dk = rank + rd, qh = d + rd;
@@ -123,10 +123,10 @@ extern "C" int mi_latent_query(const void* q, int q_stride, const void* uk_t, in
 
 // grid = (heads, tokens).  Eight neighbouring threads share a row of W.
 __global__ void __launch_bounds__(V_THREADS)
-latent_value_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int n_splits,
-                    const bf16* __restrict__ latent, const float* __restrict__ sinks, const bf16* __restrict__ uv, int n,
-                    int rank, int dv, const bf16* __restrict__ gate, int gate_stride, int per_head, int act, float scale,
-                    bf16* __restrict__ out, int out_stride) {
+latent_value_kernel(const float* part_o, const float* part_ml, int n_splits,
+                    const bf16* latent, const float* __restrict__ sinks, const bf16* __restrict__ uv, int n,
+                    int rank, int dv, const bf16* gate, int gate_stride, int per_head, int act, float scale,
+                    bf16* out, int out_stride) {
   mi_pdl_launch_dependents();
   extern __shared__ __align__(16) float lat[];       // [rank]
   __shared__ float weight[V_MAX_SPLITS];
