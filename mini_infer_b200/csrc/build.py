@@ -39,12 +39,12 @@ LIBRARIES: dict[str, tuple[list[str], list[str], list[str]]] = {
     "gemm_tma": (["gemm_tma.cu"], ["common.cuh", "bulk_copy.cuh"], []),
     "attention_tc": (["attention_tc.cu"], ["common.cuh"], []),
     "layernorm": (["layernorm.cu"], ["common.cuh"], []),
-    "rope_norm": (["rope_norm.cu"], ["common.cuh"], []),
+    "rope_norm": (["rope_norm.cu"], ["common.cuh", "heads_per_warp.cuh"], []),
     "recurrent": (["recurrent.cu"], ["common.cuh"], []),
     "gla_chunks": (["gla_chunks.cu"], ["common.cuh"], []),
     "moe": (["moe.cu"], ["common.cuh"], []),
     "stream": (["stream.cu"], ["common.cuh"], []),
-    "qk_prepare": (["qk_prepare.cu"], ["common.cuh"], []),
+    "qk_prepare": (["qk_prepare.cu"], ["common.cuh", "heads_per_warp.cuh"], []),
     "attention_rows": (["attention_rows.cu"], ["common.cuh"], []),
     "depth": (["depth.cu"], ["common.cuh"], []),
     "latent_decode": (["latent_decode.cu"], ["common.cuh"], []),

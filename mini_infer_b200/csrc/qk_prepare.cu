@@ -32,7 +32,7 @@
 //                           written back in place as well (a later layer may ask for them) and go to the
 //                           value pages.  Without pages nothing is stored: a mixer that keeps a state instead
 //                           of keys uses the kernel for the rotation alone.
-#include "common.cuh"
+#include "heads_per_warp.cuh"
 
 #include <initializer_list>
 
@@ -228,7 +228,7 @@ extern "C" int mi_qk_bias_norm_store(void* packed, int stride, int q_off, int k_
   if (writes && (!slots || !kcache || !vcache || page_size <= 0)) MI_REFUSE("qk_prepare: a cache write needs slots and pages");
   const int n_heads = nq + nkv + (values_are_keys ? 0 : nkv);
   const dim3 grid((unsigned)M, (unsigned)((n_heads + 3) / 4 < 64 ? (n_heads + 3) / 4 : 64));
-  const int per_warp = M <= 64 ? 1 : 4;      // a head per warp for few tokens; fewer, longer blocks for many
+  const int per_warp = heads_per_warp((long long)M * n_heads);
   const dim3 grid4((unsigned)M, (unsigned)((n_heads + 4 * per_warp - 1) / (4 * per_warp)));
   const int size = dtype == MI_DTYPE_F32 ? 4 : 2;
   bool pieces = d % 4 == 0 && dv % 4 == 0 && stride % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && (values_are_keys || v_off % 4 == 0) &&
@@ -704,7 +704,7 @@ extern "C" int mi_qk_norm_rope_store(void* packed, int stride, int q_off, int k_
   const dim3 grid((unsigned)M, (unsigned)((n_heads + 3) / 4 < 64 ? (n_heads + 3) / 4 : 64));
   // heads of 64, 128 or 256, rotated wholly, by half or not at all
   if ((d == 64 || d == 128 || d == 256) && (rot == 0 || rot == d || (2 * rot == d && d >= 128))) {
-    const int per_warp = M <= 64 ? 1 : 4;      // a head per warp for few tokens
+    const int per_warp = heads_per_warp((long long)M * n_heads);
     const dim3 lanes_grid((unsigned)M, (unsigned)((n_heads + 4 * per_warp - 1) / (4 * per_warp)));
 #define MI_LANES(T, PER)                                                                                                \
   MI_LAUNCH((qk_norm_rope_store_lanes_kernel<T, PER>), lanes_grid, 128, 0, stream, (T*)packed, stride, q_off, k_off, v_off, nq, \

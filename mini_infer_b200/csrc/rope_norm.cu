@@ -12,7 +12,7 @@
 //                        gate per element, per = a head's size: one gate per head.
 //
 // q, k, v and the gate are column ranges of one packed projection [tokens, stride].
-#include "common.cuh"
+#include "heads_per_warp.cuh"
 
 MI_DEFINE_ERROR_API()
 
@@ -157,8 +157,7 @@ extern "C" int mi_rope_norm_store(void* qkv, int stride, int q_off, int k_off, i
   const int size = dtype == MI_DTYPE_F32 ? 4 : 2, heads = nq + 2 * nkv;
   const bool vec = d % 2 == 0 && dv % 2 == 0 && stride % 2 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && v_off % 2 == 0 &&
                    mi_aligned(qkv, 2 * size) && (!writes || (mi_aligned(kcache, 16) && mi_aligned(vcache, 16)));
-  // a head per warp for few tokens; up to four for many, which share their angles
-  const int per_warp = M <= 64 ? 1 : 4;
+  const int per_warp = heads_per_warp((long long)M * heads);
   const dim3 grid((unsigned)M, (unsigned)((heads + 4 * per_warp - 1) / (4 * per_warp)));
 #define MI_GO(T, VEC)                                                                                                   \
   MI_LAUNCH((rope_norm_store_kernel<T, VEC>), grid, 128, 0, stream, (T*)qkv, stride, q_off, k_off, v_off, positions, inv_freq, \

@@ -265,3 +265,30 @@ def test_gains_that_the_kernel_before_writes(dtype):
             want = norm(gain[0].clone())
             assert torch.isfinite(want).all() and torch.equal(got, want)
         assert torch.equal(norm(gain[0], w_constant=True), want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M", [1137, 1139, 2730, 2731])
+def test_heads_of_many_tokens_have_the_bits_of_few(dtype, M):
+    """A warp takes one, two or four heads by the number of tokens times heads (9 a token here: 10240 and 24576 lie between the
+    sizes): what a token gives does not depend on it."""
+    o, nq, nkv, d, page = ops(), 5, 2, 64, 16
+    width, pages = (nq + 2 * nkv) * d, -(-M // page)
+    x, slots = rnd(M, width, dtype=dtype, seed=1), torch.arange(M, dtype=torch.int32, device=DEV)
+    inv = 1000.0 ** (-torch.arange(0, d, 2, dtype=torch.float32, device=DEV) / d)
+    gains, bias = (rnd(d, seed=2), rnd(d, seed=3)), (rnd(nq * d, seed=4), rnd(nkv * d, seed=5))
+    calls = [lambda p, s, k, v: o.rope_norm_store(p, 0, nq * d, (nq + nkv) * d, nq, nkv, d, d, positions=s * 3 + 1, inv_freq=inv,
+                                                  rot=d, unit_norm=True, eps=1e-6, slots=s, kcache=k, vcache=v),
+             lambda p, s, k, v: o.qk_norm_rope_store(p, 0, nq * d, (nq + nkv) * d, nq, nkv, d, d, q_gain=gains[0], k_gain=gains[1],
+                                                     eps=1e-6, rot=d, positions=s * 3 + 1, freq=inv.double(), slots=s, kcache=k,
+                                                     vcache=v),
+             lambda p, s, k, v: o.qk_bias_norm_store(p, 0, nq * d, (nq + nkv) * d, nq, nkv, d, d, q_bias=bias[0], k_bias=bias[1],
+                                                     q_gain=gains[0], k_gain=gains[1], eps=1e-6, values_are_keys=False, slots=s,
+                                                     kcache=k, vcache=v)]
+    for call in calls:
+        whole, cut = (x.clone() for _ in range(2))
+        caches = [cache_pair(pages * page, nkv, d, page, dtype) for _ in range(2)]
+        call(whole, slots, *caches[0])
+        for t in range(0, M, 100):
+            call(cut[t:t + 100], slots[t:t + 100], *caches[1])
+        assert torch.equal(whole, cut) and all(torch.equal(a, b) for a, b in zip(*caches))
