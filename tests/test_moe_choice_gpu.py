@@ -64,3 +64,22 @@ def test_ids_that_are_no_experts_leave_the_other_tokens_alone(M, E, dtype):
     with o.kept_sums():
         want, got = run(ids), run(bad)
     assert torch.isnan(got[broken]).all() and torch.equal(got[rest], want[rest])
+
+
+@pytest.mark.parametrize("E,top,groups", [(1, 1, 0), (31, 8, 0), (33, 3, 0), (64, 6, 8), (65, 3, 0), (96, 8, 8), (128, 8, 8), (255, 4, 0),
+                                          (256, 32, 16)])
+def test_choice_among_few_and_many_experts(E, top, groups):
+    """One, two and eight experts per lane: the choice and the weights that float64 gives."""
+    z = rnd(37, E, seed=E + 1)
+    keep = max(1, groups // 2)
+    ids, weights = select(z, top, "all", groups, keep)
+    c = z.double()
+    if groups:
+        best = c.view(37, groups, -1).max(dim=-1).values
+        kept = torch.zeros_like(best).scatter_(1, best.topk(keep, dim=1).indices, 1.0).repeat_interleave(E // groups, dim=1)
+        c = c.masked_fill(kept == 0, float("-inf"))
+    p, want = torch.softmax(z.double(), dim=1), c.topk(top, dim=1).indices
+    assert torch.equal(ids.long(), want)
+    share = p.gather(1, want)
+    share = 1.5 * share / share.sum(dim=1, keepdim=True)
+    assert (weights.double() - share).abs().max().item() <= 1e-5

@@ -268,6 +268,57 @@ def test_gains_that_the_kernel_before_writes(dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("M,heads,dv", [(1, 2, 64), (3, 3, 128), (70, 2, 256), (5, 4, 96), (2, 2, 288)])
+def test_gated_norm_of_heads_in_lanes_and_in_a_loop(dtype, per_head, M, heads, dv):
+    """Heads of 64, 128 and 256 stay in registers, others (the last two) are walked: against float64, with one gain for all heads
+    and one for each, without a gate and with either."""
+    o = ops()
+    x, g = rnd(M, heads * dv, seed=1), rnd(M, heads * dv, dtype=dtype, seed=2)
+    w = rnd(heads * dv if per_head else dv, seed=3)
+    h = x.double().view(M, heads, dv)
+    y = h * torch.rsqrt((h * h).mean(dim=-1, keepdim=True) + 1e-6) * (w.double().view(heads, dv) if per_head else w.double())
+    for act in (None, "sigmoid", "silu"):
+        out = torch.empty(M, heads * dv, dtype=dtype, device=DEV)
+        o.headnorm_gate(x, w, None if act is None else g, out, heads, dv, 1e-6, act, 0.7)
+        z = g.double().view(M, heads, dv)
+        want = 0.7 * y * (1.0 if act is None else torch.sigmoid(z) * (z if act == "silu" else 1.0))
+        assert (out.double().view(M, heads, dv) - want).abs().max().item() <= bound(dtype, want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,H", [(1, 8), (31, 12), (32, 8), (33, 7), (65, 512)])
+def test_pair_hash_embedding_of_many_requests(dtype, n, H):
+    """A token's request is looked for 32 requests at a time; portions of 0 to 3 tokens."""
+    from types import SimpleNamespace
+    V, buckets, mul_prev, mul_cur = 50, 37, 7919, 104729
+    lens = [(5 * i + 1) % 4 for i in range(n)]
+    lens[0] = lens[-1] = 2
+    starts = [sum(lens[:i]) for i in range(n)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    ids = [(11 * t + 3) % V for t in range(sum(lens))]
+    before = [(3 * i + 1) % V for i in range(n)]
+    first = [i % 3 == 0 for i in range(n)]              # sequences at their beginning
+    positions = [(0 if f else 9) + j for f, m in zip(first, lens) for j in range(m)]
+    table, pairs = rnd(V, H, dtype=dtype, seed=1), rnd(buckets + 1, H, dtype=dtype, seed=2)
+    slots = [(7 * i) % n if n % 7 else i for i in range(n)]
+    last = torch.zeros(n, 1, dtype=torch.int32, device=DEV)
+    for i, s in enumerate(slots):
+        last[s] = before[i]
+    ctx = SimpleNamespace(token_ids=i32(ids), positions=i32(positions), q_start=i32(starts), q_len=i32(lens), state_slot=i32(slots),
+                          n_requests=n, n_tokens=len(ids))
+    out = ops().embedding_pair_hash(table, pairs, ctx, last, buckets, mul_prev, mul_cur)
+    for i, (start, m) in enumerate(zip(starts, lens)):
+        prev = None if first[i] else before[i]
+        for t in range(start, start + m):
+            row = buckets if prev is None else (prev * mul_prev + ids[t] * mul_cur) % buckets
+            assert torch.equal(out[t], table[ids[t]].float() + pairs[row].float()), (i, t)
+            prev = ids[t]
+        if m:
+            assert last[slots[i], 0].item() == ids[start + m - 1]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("M", [1137, 1139, 2730, 2731])
 def test_heads_of_many_tokens_have_the_bits_of_few(dtype, M):
     """A warp takes one, two or four heads by the number of tokens times heads (9 a token here: 10240 and 24576 lie between the
