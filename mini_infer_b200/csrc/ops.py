@@ -1828,7 +1828,8 @@ def moe_route(x: torch.Tensor, router: torch.Tensor, top: int, *, all_scores: bo
     scores times ``scale``, with no division by their sum).  ``group_top2``: a group counts as the sum of its two best
     choice scores.  ``experts``: only the router's first ``experts`` rows are experts; the other rows ride
     along in the product and ``return_logits`` hands all logits back as a third result.  ``bias`` (fp32
-    ``[experts]``) is added to the logits before anything else."""
+    ``[experts]``) is added to the logits before anything else.  A token with fewer than ``top`` candidates (logits that are
+    NaN or minus infinity) gets valid ids for the others, with weights of NaN."""
     _cuda(x, router, correction, bias)
     _cols(x, "moe")
     if router.dim() != 2 or router.shape[1] != x.shape[1] or router.dtype != x.dtype or not router.is_contiguous():
@@ -1867,6 +1868,7 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gat
     ``w_gate_up [E, 2 ff, H]`` (an expert's gate rows, then its up rows), ``w_down [E, H, ff]``.
     ``shared_gate`` (fp32, one number per token, any row stride): its sigmoid multiplies ``shared[t]``.
     ``shared`` may also be a function that returns it, called when the experts' products are launched.
+    A token with an id that is no expert's comes out NaN; the others do not feel it.
     Entries are sorted by expert on the device; nothing is read back.  Three routes: a step that
     brings an expert only a few rows streams the weights (bfloat16); large bfloat16 steps gather
     each expert's rows and use the library's grouped product (as the dense layers use the library's

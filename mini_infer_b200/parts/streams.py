@@ -11,6 +11,8 @@ Replays of decode steps of 8 requests, us, one branch and two: Ruvurax 4096 wide
 branch on a stream of higher priority 821, 318 and 238: its kernels, launched ahead of their inputs, then hold the SMs
 while they wait.  Steps that are launched kernel by kernel stay one chain: they are bound by the host (two prompt steps of Ruvurax
 with two branches 4.9 ms where one takes 4.0), and so nothing is allocated on one stream and freed on another outside a capture.
+What it costs: a branch takes memory of its graph's pool for itself, and its result is not used again before the capture ends; a
+captured batch size holds 8 MB where one chain holds 2 (Ruvurax 4096 wide), 24 where it holds 22 (Lilulix 2048 wide).
 """
 
 from __future__ import annotations
